@@ -1322,6 +1322,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                    ptr<float>(lr), spin, cur_stream());
     check_launch("push_apply");
   });
+  m.def("local_push_update", [](const cu::TableHost& table, const torch::Tensor& ugrad, const torch::Tensor& off,
+                                const torch::Tensor& slot_cache, int max_n, const OptimPOD& optim,
+                                const torch::Tensor& lr) {
+    need_cuda(lr, "lr", torch::kFloat32);
+    need_cuda(ugrad, "ugrad", torch::kFloat32);
+    TORCH_CHECK(ugrad.dim() == 2 && ugrad.size(1) == table.dim && off.numel() >= 2, "ugrad must be [cap, dim]");
+    cu::local_push_update(table, ptr<float>(ugrad), ptr<int>(off), ptr<int>(slot_cache), max_n,
+                          static_cast<int>(slot_cache.numel()), optim, ptr<float>(lr), cur_stream());
+    check_launch("local_push_update");
+  });
 
   // ---------------- one exchange for several tables of one row width
   m.def("group_table_views", [](const std::vector<cu::TableHost>& tables) {

@@ -116,6 +116,12 @@ void push_dispatch(SymHost sym, ChanLayout lay, Ctrl* ctrl, float* ugrad, const 
 void push_apply(SymHost sym, ChanLayout lay, Ctrl* ctrl, TableHost table, const int* slot_cache, OptimPOD optim,
                 const float* lr, uint32_t spin_limit, cudaStream_t stream);
 
+// ---- the same on a job of one GPU (sparse_local.cu) ----
+// push_dispatch + push_apply without the inbox: updates the rows of the U = off[1] unique ids of the lookup from
+// ugrad and zeroes it.  slot_cache[u] is the row of unique id u (u < cap_s); max_n bounds U.
+void local_push_update(TableHost table, float* ugrad, const int* off, const int* slot_cache, int max_n, int cap_s,
+                       OptimPOD optim, const float* lr, cudaStream_t stream);
+
 // One of the channel's rendezvous points as a launch of its own: kind 0 = every source's request has
 // arrived (also snapshots the counts), 1 = every owner has answered the pull, 2 = every source's gradient
 // rows have arrived.  Nothing is launched when world == 1.

@@ -401,11 +401,19 @@ class SparseChannel:
         ``self.ugrad`` (the pull's ticket must still be current)."""
         if ticket.channel is not self or ticket.serial != self.serial:
             raise C.KrakenError("push_accumulated needs the ticket of this channel's latest pull")
+        self._apply_accumulated(lr, ticket.n)
+        self.serial += 1
+
+    def _apply_accumulated(self, lr: torch.Tensor, n: int) -> None:
+        """Sends the summed gradients of ``self.ugrad`` to the owners and runs the optimizer there."""
+        if self.world == 1:
+            C.local_push_update(self.table.host(), self.ugrad, self.off, self.slot_cache, n, self.table.optim, lr)
+            self.launches += 1
+            return
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
-        C.push_dispatch(h, lay, ctrl, self.ugrad, self.off, ticket.n, self.table.dim)
+        C.push_dispatch(h, lay, ctrl, self.ugrad, self.off, n, self.table.dim)
         C.push_apply(h, lay, ctrl, tbl, self.slot_cache, self.table.optim, lr, self.spin)
         self.launches += 2 + 2 * self._wait  # dispatch, (push wait, merge,) update
-        self.serial += 1
 
     # ------------------------------------------------------------------ pull
     def pull(self, ids: torch.Tensor, bag_offsets: Optional[torch.Tensor] = None,
@@ -446,15 +454,13 @@ class SparseChannel:
             if ids is None:
                 raise C.KrakenError("push without a current ticket needs the ids")
             n = self._lookup_phase(ids.reshape(-1), insert=False)
-        h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
         dim = self.table.dim
         grads = grads.reshape(-1, dim)
         if grads.dtype != torch.float32 or not grads.is_contiguous():
             grads = grads.to(torch.float32).contiguous()
         C.push_scatter(grads, self.inv, n, dim, bag_offsets, weights, mean, bag_mean, self.ugrad)
-        C.push_dispatch(h, lay, ctrl, self.ugrad, self.off, n, dim)
-        C.push_apply(h, lay, ctrl, tbl, self.slot_cache, self.table.optim, lr, self.spin)
-        self.launches += 3 + 2 * self._wait  # scatter, dispatch, (push wait, merge,) update
+        self.launches += 1
+        self._apply_accumulated(lr, n)
         # A push consumes the pull's bookkeeping: a second push needs a new lookup.
         self.serial += 1
 

@@ -1,0 +1,62 @@
+"""The one-GPU kernels of the sparse path (csrc/cuda/sparse_local.cu) against the CPU shard (B200 only)."""
+import pytest
+import torch
+
+import kraken_b200.pytorch as kk
+from kraken_b200._native import C
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+OPTIMS = [(kk.OptimType.kSGD, {}), (kk.OptimType.kSGD, {"momentum": "0.9"}),
+          (kk.OptimType.kAdagrad, {"initial_accumulator_value": "0.1"}), (kk.OptimType.kAdam, {}),
+          (kk.OptimType.kAdam, {"amsgrad": "true"}), (kk.OptimType.kRMSprop, {"momentum": "0.5", "centered": "true"})]
+
+
+def make(dim, optim, conf, capacity=1 << 12, **options):
+    kk.initialize("gpu", seed=11, table_capacity=capacity, **options)
+    kk.init_model("m", optim, conf)
+    kk.update_lr(0.05)
+    t = kk.register_sparse_table("e", dim, torch.float32, kk.InitializerType.kNormal, {"stddev": "0.5"})
+    shard = C.CpuShard(11)
+    shard.init_model("m", optim, conf)
+    shard.create_sparse_table(t, "e", dim, kk.InitializerType.kNormal, {"stddev": "0.5"})
+    return t, shard
+
+
+# Row widths on both sides of the vector width, of a power of two and of a block's threads; id counts around
+# a block's rows (256 / chunks) and with one id only.
+@pytest.mark.parametrize("optim,conf", OPTIMS)
+@pytest.mark.parametrize("dim,ids", [(1, 255), (1, 257), (3, 85), (10, 26), (16, 65), (20, 52), (64, 1), (100, 11),
+                                     (1028, 5), (1030, 3)])
+def test_push_updates_rows_as_the_cpu_shard(optim, conf, dim, ids):
+    t, shard = make(dim, optim, conf)
+    torch.manual_seed(dim + ids)
+    for step in range(3):
+        batch = torch.randint(0, ids, (2 * ids + 1,)) if step else torch.arange(ids)
+        rows = kk.pull_sparse_table(t, batch.to(DEV))
+        uniq, inv = C.cpu_dedup(batch)
+        # pull: a copy of the rows; after k updates the rows carry their rounding, see below
+        assert torch.allclose(rows.cpu(), shard.pull_sparse(t, uniq)[inv], atol=2e-4)
+        g = torch.randn(batch.numel(), dim)
+        kk.push_sparse_table(t, batch.to(DEV), g.to(DEV))
+        assert shard.push_sparse(t, uniq, C.cpu_segment_sum(g, inv, uniq.numel()), 0.05) == 0
+    kk.native.engine().check()
+    every = torch.arange(ids)
+    # three updates of at most lr = 0.05 each, their gradient sums added in another order: 1e-5 relative per sum,
+    # amplified where Adam and RMSprop divide two small numbers
+    assert torch.allclose(kk.pull_sparse_table(t, every.to(DEV)).cpu(), shard.pull_sparse(t, every), atol=2e-4)
+    ch = kk.native.engine().channels[t]
+    assert float(ch.ugrad.abs().max()) == 0.0  # zero again for the next step
+
+
+def test_push_drops_the_gradient_of_an_unknown_id():
+    t, _ = make(8, kk.OptimType.kSGD, {})
+    known = torch.arange(4, device=DEV)
+    before = kk.pull_sparse_table(t, known).clone()
+    kk.push_sparse_table(t, torch.tensor([2, 900, 3], device=DEV), torch.ones(3, 8, device=DEV))
+    with pytest.raises(kk.KrakenError):
+        kk.native.engine().check()
+    after = kk.pull_sparse_table(t, known)
+    assert torch.allclose(after, before - 0.05 * torch.tensor([0, 0, 1.0, 1.0], device=DEV)[:, None])
+    assert float(kk.native.engine().channels[t].ugrad.abs().max()) == 0.0

@@ -1322,6 +1322,52 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                    ptr<float>(lr), spin, cur_stream());
     check_launch("push_apply");
   });
+  m.def("local_lookup", [](const torch::Tensor& ids, const torch::Tensor& set, const torch::Tensor& first,
+                           const torch::Tensor& pos, uint32_t hbits, const torch::Tensor& cnt, const torch::Tensor& off,
+                           const torch::Tensor& uniq, const torch::Tensor& inv, int cap_u, const cu::TableHost& table,
+                           const torch::Tensor& slot_cache, bool insert, const torch::Tensor& ctrl) {
+    need_cuda(ids, "ids", torch::kInt64);
+    need_cuda(set, "set", torch::kInt32);
+    const int n = static_cast<int>(ids.numel());
+    TORCH_CHECK(hbits <= 31 && set.numel() == (1ll << hbits) && set.numel() > n,
+                "dedup scratch must be an int32 [1 << hbits] tensor with more than n slots");
+    TORCH_CHECK(first.numel() >= n && pos.numel() >= n && inv.numel() >= n && uniq.numel() >= cap_u,
+                "dedup outputs too small");
+    TORCH_CHECK(cnt.numel() >= 1 && off.numel() >= 2, "cnt/off too small");
+    c10::cuda::CUDAGuard guard(ids.device());
+    cu::local_lookup(ptr<int64_t>(ids), n, cu::LocalScratch{ptr<int>(set), ptr<int>(first), ptr<int>(pos), hbits},
+                     ptr<int>(cnt), ptr<int>(off), ptr<int64_t>(uniq), ptr<int>(inv), cap_u, table, ptr<int>(slot_cache),
+                     static_cast<int>(slot_cache.numel()), insert, ctrl_ptr(ctrl), cur_stream());
+    check_launch("local_lookup");
+  });
+  m.def("local_probe", [](const torch::Tensor& uniq, const torch::Tensor& off, int max_n, const cu::TableHost& table,
+                          const torch::Tensor& slot_cache, bool insert, const torch::Tensor& ctrl) {
+    need_cuda(uniq, "uniq", torch::kInt64);
+    cu::local_probe(ptr<int64_t>(uniq), ptr<int>(off), max_n, table, ptr<int>(slot_cache),
+                    static_cast<int>(slot_cache.numel()), insert, ctrl_ptr(ctrl), cur_stream());
+    check_launch("local_probe");
+  });
+  m.def("local_gather", [](const cu::TableHost& table, const torch::Tensor& off, const torch::Tensor& slot_cache,
+                           int max_n, const torch::Tensor& rows) {
+    need_cuda(rows, "rows", torch::kFloat32);
+    TORCH_CHECK(rows.dim() == 2 && rows.size(1) == table.dim, "rows must be [cap, dim]");
+    cu::local_gather(table, ptr<int>(off), ptr<int>(slot_cache), max_n, static_cast<int>(slot_cache.numel()),
+                     ptr<float>(rows), cur_stream());
+    check_launch("local_gather");
+  });
+  m.def("local_combine",
+        [](const cu::TableHost& table, const torch::Tensor& inv, const torch::Tensor& slot_cache, int n,
+           const c10::optional<torch::Tensor>& bag_offsets, const c10::optional<torch::Tensor>& weights, bool mean,
+           const c10::optional<torch::Tensor>& bag_mean, float patch_value, const torch::Tensor& out) {
+          const int k = bag_offsets.has_value() ? static_cast<int>(bag_offsets->numel()) - 1 : 0;
+          need_cuda(out, "out", torch::kFloat32);
+          TORCH_CHECK(out.numel() == static_cast<int64_t>(bag_offsets.has_value() ? k : n) * table.dim,
+                      "out has the wrong size");
+          cu::local_combine(table, ptr<int>(inv), ptr<int>(slot_cache), n, static_cast<int>(slot_cache.numel()),
+                            optr<int64_t>(bag_offsets), k, optr<float>(weights), mean, optr<uint8_t>(bag_mean),
+                            patch_value, ptr<float>(out), cur_stream());
+          check_launch("local_combine");
+        });
   m.def("local_push_update", [](const cu::TableHost& table, const torch::Tensor& ugrad, const torch::Tensor& off,
                                 const torch::Tensor& slot_cache, int max_n, const OptimPOD& optim,
                                 const torch::Tensor& lr) {

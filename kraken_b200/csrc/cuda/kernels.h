@@ -117,6 +117,27 @@ void push_apply(SymHost sym, ChanLayout lay, Ctrl* ctrl, TableHost table, const 
                 const float* lr, uint32_t spin_limit, cudaStream_t stream);
 
 // ---- the same on a job of one GPU (sparse_local.cu) ----
+// Scratch of its dedup: an open-addressing set of 1 << hbits occurrence indexes (more than n), -1 between calls.
+struct LocalScratch {
+  int* set;    // [1 << hbits]
+  int* first;  // [n]
+  int* pos;    // [n]
+  uint32_t hbits;
+};
+// dedup_bucketize_dispatch + pull_probe without the inbox.  cnt[0] must be zero on entry and is again when the call
+// has run; off[2] = {0, U}.
+void local_lookup(const int64_t* ids, int n, LocalScratch sc, int* cnt, int* off, int64_t* uniq, int* inv, int cap_u,
+                  TableHost table, int* slot_cache, int cap_s, bool insert, Ctrl* ctrl, cudaStream_t stream);
+// pull_dispatch + pull_probe without the inbox: rows of the off[1] ids in uniq (another channel's dedup).
+void local_probe(const int64_t* uniq, const int* off, int max_n, TableHost table, int* slot_cache, int cap_s, bool insert,
+                 Ctrl* ctrl, cudaStream_t stream);
+// The unique rows of a lookup as a compact buffer [U, dim].
+void local_gather(TableHost table, const int* off, const int* slot_cache, int max_n, int cap_s, float* rows_out,
+                  cudaStream_t stream);
+// pull_gather + pull_combine without the copy: out[n, dim], or pooled out[k, dim], read from the table.
+void local_combine(TableHost table, const int* inv, const int* slot_cache, int n, int cap_s, const int64_t* bag_offsets,
+                   int k, const float* weights, bool mean, const uint8_t* bag_mean, float patch_value, float* out,
+                   cudaStream_t stream);
 // push_dispatch + push_apply without the inbox: updates the rows of the U = off[1] unique ids of the lookup from
 // ugrad and zeroes it.  slot_cache[u] is the row of unique id u (u < cap_s); max_n bounds U.
 void local_push_update(TableHost table, float* ugrad, const int* off, const int* slot_cache, int max_n, int cap_s,

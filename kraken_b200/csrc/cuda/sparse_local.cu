@@ -104,7 +104,347 @@ void launch_local_update(int grid, cudaStream_t stream, const TableView& t, floa
   }
 }
 
+// ------------------------------------------------------------------ lookup
+// The id that marks a free slot is not available as a key; it is treated as its neighbour.
+__device__ __forceinline__ uint64_t canonical_id(uint64_t id) { return id == kEmptyKey ? kEmptyKey - 1 : id; }
+
+// Dedup without an exchange.  The scratch set holds 4-byte OCCURRENCE INDEXES instead of keys: entry h is the index of
+// the occurrence that claimed it (the winner of its id), and a probe compares ids[entry].  What is accessed at random is
+// then the set (4 bytes a slot) and the ids themselves, both of which stay in L2 at millions of ids, where the 16-byte
+// {key, position} entries of the multi-rank dedup cost a sector of HBM each on the way in, at the number's read-back and
+// at the clearing.  Measured for 3.4 M ids of which 2.3 M are distinct: insert + finalize + probe 260 us
+// before, 185 us now; 1.7 M ids, 0.55 M distinct: 102 and 58 us.
+
+// First kernel: every occurrence finds or claims its id's entry; the winner numbers the id.  first[i] = the winner's
+// index for the others, ~entry for the winner itself; pos[i] = the number, written by winners only.  One id per thread:
+// two or four were slower (3.4 M ids: 80, 85 and 107 us), the claims of a thread wait for one another.  The first look
+// at an entry may be a stale one from L1, where the entries of frequent ids stay: an entry only ever goes from free to
+// claimed within a launch, and a claim is made by compare-and-swap.
+__global__ void __launch_bounds__(kThreads)
+local_insert_kernel(const int64_t* __restrict__ ids, int n, int* set, uint32_t hbits, int* __restrict__ first,
+                    int* __restrict__ pos, int* cnt, int* status) {
+  pdl_enter();
+  constexpr int kWarps = kThreads / 32;
+  __shared__ int s_cnt[kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  const uint32_t mask = static_cast<uint32_t>((1ull << hbits) - 1);
+  bool won = false;
+  if (i < n) {
+    uint64_t id = static_cast<uint64_t>(ids[i]);
+    if (id == kEmptyKey) set_status(status, err::kBadArgument);  // reserved: reported, then treated as its neighbour
+    id = canonical_id(id);
+    uint32_t slot = static_cast<uint32_t>(SlotHash(id ^ kDedupSalt, hbits));
+    int e = __ldca(&set[slot]);
+    for (uint32_t probe = 0; probe <= mask; ++probe) {
+      if (e < 0) {
+        e = atomicCAS(&set[slot], -1, i);
+        if (e < 0) {
+          won = true;
+          break;
+        }
+      }
+      if (canonical_id(static_cast<uint64_t>(__ldg(ids + e))) == id) break;
+      slot = (slot + 1) & mask;
+      e = __ldca(&set[slot]);
+    }
+    first[i] = won ? static_cast<int>(~slot) : e;
+  }
+  const unsigned winners = __ballot_sync(0xffffffffu, won);
+  if (lane == 0) s_cnt[warp] = __popc(winners);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const int c = s_cnt[w];
+      s_cnt[w] = total;
+      total += c;
+    }
+    const int start = total > 0 ? atomicAdd(cnt, total) : 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) s_cnt[w] += start;
+  }
+  __syncthreads();
+  if (won) pos[i] = s_cnt[warp] + __popc(winners & ((1u << lane) - 1u));
+}
+
+// Rows that the warp's lanes have just created (bit set in `todo`, slot and id per lane), initialised by the whole
+// warp: `lpr` lanes per row, so that the Philox draws and the stores of a row are spread over lanes.
+template <int VEC>
+__device__ __forceinline__ void init_created(const TableView& t, unsigned todo, int slot, uint64_t id, int chunks, int lpr) {
+  const int lane = threadIdx.x & 31;
+  const int rows_per_pass = 32 / lpr;
+  while (todo) {
+    int src = -1;
+    for (int g = 0; g < rows_per_pass && todo; ++g) {
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      if (g == lane / lpr) src = l;
+    }
+    const int r_slot = __shfl_sync(0xffffffffu, slot, src < 0 ? 0 : src);
+    const uint64_t r_id = __shfl_sync(0xffffffffu, id, src < 0 ? 0 : src);
+    if (src < 0) continue;
+    float* row = t.val + static_cast<size_t>(r_slot) * t.dim;
+    for (int c = lane % lpr; c < chunks; c += lpr) {
+      float q[4];
+      if (VEC == 4) {
+        InitQuad(t.init, t.seed_key, r_id, c, t.dim, q);
+        *reinterpret_cast<float4*>(row + c * 4) = make_float4(q[0], q[1], q[2], q[3]);
+      } else {
+        InitQuad(t.init, t.seed_key, r_id, c >> 2, t.dim, q);
+        row[c] = q[c & 3];
+      }
+    }
+  }
+}
+
+// Second kernel, with the table probe: every occurrence learns its unique id's number; the winner also writes the
+// unique list, empties the set's entry, and finds (or, with `insert`, claims and initialises) the row.  The block that
+// finishes last zeroes `cnt` for the next call.  The ids do not pass through the inbox, and no block ends on a
+// system-scope fence.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+local_resolve_kernel(const int64_t* __restrict__ ids, int n, int* __restrict__ set, const int* __restrict__ first,
+                     const int* __restrict__ pos, int* cnt, int* off, int64_t* __restrict__ uniq, int* __restrict__ inv,
+                     int cap_u, TableView t, int* __restrict__ slot_cache, int cap_s, int insert, uint32_t* done, int* status,
+                     int chunks, int lpr) {
+  pdl_enter();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    // more unique ids than the channel's buffers hold: reported and clamped, so that no later kernel indexes
+    // past a buffer (the step's result is then invalid, not its memory)
+    const int U = *cnt;
+    if (U > cap_u || U > cap_s) set_status(status, err::kInboxOverflow);
+    off[0] = 0;
+    off[1] = min(U, cap_u);
+  }
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  bool created = false;
+  int slot = -1;
+  uint64_t id = 0;
+  if (i < n) {
+    const int f = first[i];
+    const int u = pos[f < 0 ? i : f];
+    inv[i] = u < cap_u ? u : 0;
+    if (f < 0) {
+      id = canonical_id(static_cast<uint64_t>(ids[i]));
+      set[~f] = -1;  // leave the set empty for the next call
+      if (u < cap_u) {
+        uniq[u] = static_cast<int64_t>(id);
+        if (u < cap_s) {
+          slot = table_find_or_insert(t, id, insert != 0, &created);
+          if (slot < 0 && !insert) set_status(status, err::kSparseIdNotExist);
+          slot_cache[u] = slot;
+        }
+      }
+    }
+  }
+  const unsigned todo = __ballot_sync(0xffffffffu, created);
+  if (todo) {
+    if ((threadIdx.x & 31) == __ffs(todo) - 1) atomicAdd(t.size, __popc(todo));
+    init_created<VEC>(t, todo, slot, id, chunks, lpr);
+  }
+  if (threadIdx.x == 0) {
+    // block 0 has read the count before it arrives here, so the last to arrive may clear it
+    if (blockIdx.x == 0) __threadfence();
+    if (atomicAdd(done, 1u) == gridDim.x - 1) {
+      *done = 0;
+      *cnt = 0;
+    }
+  }
+}
+
+// The lookup of unique ids that another channel has just deduplicated (the first-order table beside the embedding
+// table): only the probe is left.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+local_probe_kernel(const int64_t* __restrict__ uniq, const int* __restrict__ off, TableView t, int* __restrict__ slot_cache,
+                   int cap_s, int insert, int* status, int chunks, int lpr) {
+  pdl_enter();
+  const int U = off[1];
+  if (blockIdx.x == 0 && threadIdx.x == 0 && U > cap_s) set_status(status, err::kInboxOverflow);
+  const int limit = min(U, cap_s);
+  for (int base = blockIdx.x * blockDim.x; base < limit; base += gridDim.x * blockDim.x) {
+    const int u = base + threadIdx.x;
+    bool created = false;
+    int slot = -1;
+    uint64_t id = 0;
+    if (u < limit) {
+      id = static_cast<uint64_t>(uniq[u]);
+      slot = table_find_or_insert(t, id, insert != 0, &created);
+      if (slot < 0 && !insert) set_status(status, err::kSparseIdNotExist);
+      slot_cache[u] = slot;
+    }
+    const unsigned todo = __ballot_sync(0xffffffffu, created);
+    if (todo) {
+      if ((threadIdx.x & 31) == __ffs(todo) - 1) atomicAdd(t.size, __popc(todo));
+      init_created<VEC>(t, todo, slot, id, chunks, lpr);
+    }
+  }
+}
+
+// Row of unique entry u: its slot in the table, or -1 for one that was not found (its row reads as zeros).
+__device__ __forceinline__ int slot_at(const int* __restrict__ slot_cache, int u, int cap_s) {
+  return u < cap_s ? slot_cache[u] : -1;
+}
+
+// Unique rows into a compact buffer, for consumers that visit every occurrence of small rows (the DeepFM pack
+// kernels): `tpr` threads per row, four rows of a thread in flight.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+local_gather_kernel(TableView t, const int* __restrict__ off, const int* __restrict__ slot_cache, int cap_s, int chunks,
+                    int tpr, float* __restrict__ rows_out) {
+  pdl_enter();
+  using V = Vec<VEC>;
+  constexpr int kUnroll = 4;
+  const int U = off[1];
+  const int rows = kThreads / tpr;
+  const int r = threadIdx.x / tpr, c0 = threadIdx.x - r * tpr;
+  if (r >= rows) return;
+  const int stride = gridDim.x * rows;
+  for (int u0 = blockIdx.x * rows + r; u0 < U; u0 += stride * kUnroll) {
+    int slot[kUnroll];
+#pragma unroll
+    for (int q = 0; q < kUnroll; ++q) slot[q] = u0 + q * stride < U ? slot_at(slot_cache, u0 + q * stride, cap_s) : -1;
+    for (int c = c0; c < chunks; c += tpr) {
+      typename V::T v[kUnroll];
+#pragma unroll
+      for (int q = 0; q < kUnroll; ++q)
+        v[q] = slot[q] < 0 ? V::zero() : V::ld(t.val + static_cast<size_t>(slot[q]) * t.dim + c * VEC);
+#pragma unroll
+      for (int q = 0; q < kUnroll; ++q)
+        if (u0 + q * stride < U) V::st(rows_out + static_cast<size_t>(u0 + q * stride) * t.dim + c * VEC, v[q]);
+    }
+  }
+}
+
+// out[i] = row of occurrence i, read from the table where it is.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+local_expand_kernel(TableView t, const int* __restrict__ inv, const int* __restrict__ slot_cache, int cap_s, int n,
+                    int chunks, int tpr, float* __restrict__ out) {
+  pdl_enter();
+  using V = Vec<VEC>;
+  constexpr int kUnroll = 4;
+  const int rows = kThreads / tpr;
+  const int r = threadIdx.x / tpr, c0 = threadIdx.x - r * tpr;
+  if (r >= rows) return;
+  const int stride = gridDim.x * rows;
+  for (int i0 = blockIdx.x * rows + r; i0 < n; i0 += stride * kUnroll) {
+    int slot[kUnroll];
+#pragma unroll
+    for (int q = 0; q < kUnroll; ++q) slot[q] = i0 + q * stride < n ? inv[i0 + q * stride] : -1;
+#pragma unroll
+    for (int q = 0; q < kUnroll; ++q) slot[q] = slot[q] < 0 ? -1 : slot_at(slot_cache, slot[q], cap_s);
+    for (int c = c0; c < chunks; c += tpr) {
+      typename V::T v[kUnroll];
+#pragma unroll
+      for (int q = 0; q < kUnroll; ++q)
+        v[q] = slot[q] < 0 ? V::zero() : V::ld(t.val + static_cast<size_t>(slot[q]) * t.dim + c * VEC);
+#pragma unroll
+      for (int q = 0; q < kUnroll; ++q)
+        if (i0 + q * stride < n) V::st(out + static_cast<size_t>(i0 + q * stride) * t.dim + c * VEC, v[q]);
+    }
+  }
+}
+
+// out[b] = pooled rows of bag b, read from the table where they are; four rows of a bag in flight per thread.  The
+// sum runs in the order of the occurrences, as in pull_combine_kernel.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+local_pool_kernel(TableView t, const int* __restrict__ inv, const int* __restrict__ slot_cache, int cap_s, int chunks,
+                  int tpr, const int64_t* __restrict__ bag_offsets, int nbags, const float* __restrict__ weights, int mean,
+                  const uint8_t* __restrict__ bag_mean, float patch_value, float* __restrict__ out) {
+  pdl_enter();
+  using V = Vec<VEC>;
+  constexpr int kUnroll = 4;
+  const int rows = kThreads / tpr;
+  const int g = threadIdx.x / tpr, c0 = threadIdx.x - g * tpr;
+  if (g >= rows) return;
+  for (int b = blockIdx.x * rows + g; b < nbags; b += gridDim.x * rows) {
+    const int64_t lo = bag_offsets[b], hi = bag_offsets[b + 1];
+    const bool is_mean = bag_mean ? bag_mean[b] != 0 : mean != 0;
+    for (int c = c0; c < chunks; c += tpr) {
+      typename V::T acc = V::zero();
+      for (int64_t r = lo; r < hi; r += kUnroll) {
+        int slot[kUnroll];
+        typename V::T v[kUnroll];
+#pragma unroll
+        for (int q = 0; q < kUnroll; ++q) slot[q] = r + q < hi ? inv[r + q] : -1;
+#pragma unroll
+        for (int q = 0; q < kUnroll; ++q) slot[q] = slot[q] < 0 ? -1 : slot_at(slot_cache, slot[q], cap_s);
+#pragma unroll
+        for (int q = 0; q < kUnroll; ++q)
+          v[q] = slot[q] < 0 ? V::zero() : V::ld(t.val + static_cast<size_t>(slot[q]) * t.dim + c * VEC);
+#pragma unroll
+        for (int q = 0; q < kUnroll; ++q)
+          if (r + q < hi) V::fma(acc, weights ? weights[r + q] : 1.f, v[q]);
+      }
+      if (hi <= lo)
+        acc = V::fill(patch_value);
+      else if (is_mean)
+        acc = V::scale(acc, 1.f / static_cast<float>(hi - lo));
+      V::st(out + static_cast<size_t>(b) * t.dim + c * VEC, acc);
+    }
+  }
+}
+
 }  // namespace
+
+void local_lookup(const int64_t* ids, int n, LocalScratch sc, int* cnt, int* off, int64_t* uniq, int* inv, int cap_u,
+                  TableHost table, int* slot_cache, int cap_s, bool insert, Ctrl* ctrl, cudaStream_t stream) {
+  if (n <= 0) {
+    cudaMemsetAsync(off, 0, 2 * sizeof(int), stream);
+    return;
+  }
+  const RowGeom g = row_geom(table.dim);
+  const dim3 grid((n + kThreads - 1) / kThreads);
+  const bool early = grid.x < kFullGrid;
+  launch_pdl_if(early, local_insert_kernel, grid, dim3(kThreads), 0, stream, ids, n, sc.set, sc.hbits, sc.first, sc.pos, cnt,
+                &ctrl->status);
+  auto kernel = g.vec == 4 ? local_resolve_kernel<4> : local_resolve_kernel<1>;
+  launch_pdl_if(early, kernel, grid, dim3(kThreads), 0, stream, ids, n, sc.set, static_cast<const int*>(sc.first),
+                static_cast<const int*>(sc.pos), cnt, off, uniq, inv, cap_u, to_view(table), slot_cache, cap_s,
+                insert ? 1 : 0, &ctrl->done[0], &ctrl->status, g.chunks, g.lpr);
+}
+
+void local_probe(const int64_t* uniq, const int* off, int max_n, TableHost table, int* slot_cache, int cap_s, bool insert,
+                 Ctrl* ctrl, cudaStream_t stream) {
+  const RowGeom g = row_geom(table.dim);
+  const int grid = grid_for(max_n);
+  auto kernel = g.vec == 4 ? local_probe_kernel<4> : local_probe_kernel<1>;
+  launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, uniq, off, to_view(table), slot_cache,
+                cap_s, insert ? 1 : 0, &ctrl->status, g.chunks, g.lpr);
+}
+
+void local_gather(TableHost table, const int* off, const int* slot_cache, int max_n, int cap_s, float* rows_out,
+                  cudaStream_t stream) {
+  const RowGeom g = row_geom(table.dim);
+  const int tpr = g.chunks < kThreads ? g.chunks : kThreads;
+  const int grid = grid_for(max_n, kThreads / tpr);
+  auto kernel = g.vec == 4 ? local_gather_kernel<4> : local_gather_kernel<1>;
+  launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, to_view(table), off, slot_cache, cap_s,
+                g.chunks, tpr, rows_out);
+}
+
+void local_combine(TableHost table, const int* inv, const int* slot_cache, int n, int cap_s, const int64_t* bag_offsets,
+                   int k, const float* weights, bool mean, const uint8_t* bag_mean, float patch_value, float* out,
+                   cudaStream_t stream) {
+  const RowGeom g = row_geom(table.dim);
+  const int tpr = g.chunks < kThreads ? g.chunks : kThreads;
+  const int grid = grid_for(bag_offsets ? k : n, kThreads / tpr, 148 * 16);
+  if ((bag_offsets ? k : n) <= 0) return;
+  const bool early = grid < kFullGrid;
+  if (bag_offsets == nullptr) {
+    auto kernel = g.vec == 4 ? local_expand_kernel<4> : local_expand_kernel<1>;
+    launch_pdl_if(early, kernel, dim3(grid), dim3(kThreads), 0, stream, to_view(table), inv, slot_cache, cap_s, n, g.chunks,
+                  tpr, out);
+  } else {
+    auto kernel = g.vec == 4 ? local_pool_kernel<4> : local_pool_kernel<1>;
+    launch_pdl_if(early, kernel, dim3(grid), dim3(kThreads), 0, stream, to_view(table), inv, slot_cache, cap_s, g.chunks, tpr,
+                  bag_offsets, k, weights, mean ? 1 : 0, bag_mean, patch_value, out);
+  }
+}
 
 void local_push_update(TableHost table, float* ugrad, const int* off, const int* slot_cache, int max_n, int cap_s,
                        OptimPOD optim, const float* lr, cudaStream_t stream) {

@@ -320,10 +320,13 @@ class SparseChannel:
 
         self.ctrl = torch.zeros(C.CTRL_INTS, dtype=torch.int32, device=dev)  # csrc/cuda/kernels.h: Ctrl
         self.hbits = _next_pow2_bits(2 * self.cap)
-        # dedup scratch set: entries of (key, position | winner << 32); every key is free between calls
-        self.hkeys = torch.zeros((1 << self.hbits, 2), dtype=torch.int64, device=dev)
-        self.hkeys[:, 0] = _EMPTY
+        self._hkeys: Optional[torch.Tensor] = None
         self.slot_of = torch.zeros(self.cap, dtype=torch.int32, device=dev)
+        if world == 1:
+            # dedup scratch set of occurrence indexes: at most 0.8 full when every id of the largest call is distinct
+            self.lbits = _next_pow2_bits(self.cap + self.cap // 4 + 1)
+            self.lset = torch.full((1 << self.lbits,), -1, dtype=torch.int32, device=dev)
+            self.pos = torch.zeros(self.cap, dtype=torch.int32, device=dev)
         self.cnt = torch.zeros(world, dtype=torch.int32, device=dev)
         self._own_off = torch.zeros(world + 1, dtype=torch.int32, device=dev)
         self._own_uniq = torch.zeros(self.cap_u, dtype=torch.int64, device=dev)
@@ -338,6 +341,15 @@ class SparseChannel:
         self.owner_world = world            # rows live on ranks 0 .. owner_world - 1 (smaller after a live reshard)
 
     # ------------------------------------------------------------------ helpers
+    @property
+    def hkeys(self) -> torch.Tensor:
+        """Scratch set of the multi-rank dedup: entries of (key, position | winner << 32); every key is free
+        between calls."""
+        if self._hkeys is None:
+            self._hkeys = torch.zeros((1 << self.hbits, 2), dtype=torch.int64, device=self.table.device)
+            self._hkeys[:, 0] = _EMPTY
+        return self._hkeys
+
     def _lookup_phase(self, ids: torch.Tensor, insert: bool, share_from: Optional["SparseChannel"] = None) -> int:
         """Dedup + dispatch + owner-side probe.  ``share_from``: another channel that has just
         deduplicated the SAME ids with the same owner salt; its unique list and occurrence map
@@ -347,13 +359,28 @@ class SparseChannel:
             raise C.KrakenError(f"table {self.table.name!r}: {n} ids in one call exceed the channel capacity "
                                 f"{self.cap}; raise max_ids_per_call")
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
-        if share_from is not None and share_from.salt == self.salt and share_from.world == self.world:
+        share = share_from is not None and share_from.salt == self.salt and share_from.world == self.world
+        if share:
             self.off, self.uniq, self.inv = share_from.off, share_from.uniq, share_from.inv
+        else:
+            self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
+        if self.world == 1:
+            # nobody to exchange with: the dedup's second kernel also finds the rows
+            if share:
+                C.local_probe(self.uniq, self.off, n, tbl, self.slot_cache, insert, ctrl)
+                self.launches += 1
+            else:
+                C.local_lookup(ids, self.lset, self.slot_of, self.pos, self.lbits, self.cnt, self.off, self.uniq, self.inv,
+                               self.cap_u, tbl, self.slot_cache, insert, ctrl)
+                self.launches += 2
+            self.serial += 1
+            self.last_n = n
+            return n
+        if share:
             C.pull_dispatch(h, lay, ctrl, self.uniq, self.off, n)
             self.launches += 1
         else:
             # the dedup's second kernel also sends the unique ids to their owners' inboxes
-            self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
             C.dedup_bucketize(ids, self.world, self.salt, self.hkeys, self.slot_of, self.hbits,
                               self.cnt, self.off, self.uniq, self.inv, self.ctrl[4:5], self.cap_u, h, lay, ctrl,
                               self.owner_world)
@@ -390,8 +417,10 @@ class SparseChannel:
         n = self._lookup_phase(ids, insert=True, share_from=share_from)
         if in_place and self.world == 1:
             return self.table.val, self.inv, Ticket(self, self.serial, n, None, None, False, None, self.slot_cache)
-        C.pull_gather(self.arena.heap, self.lay, self.ctrl, self.table.host(), self.slot_cache)
-        if self.world > 1:
+        if self.world == 1:
+            C.local_gather(self.table.host(), self.off, self.slot_cache, n, self.rows_recv)
+        else:
+            C.pull_gather(self.arena.heap, self.lay, self.ctrl, self.table.host(), self.slot_cache)
             C.pull_wait(self.arena.heap, self.lay, self.ctrl, self.spin)
         self.launches += 1 + self._wait
         return self.rows_recv, self.inv, Ticket(self, self.serial, n, None, None, False, None)
@@ -429,13 +458,17 @@ class SparseChannel:
         n = self._lookup_phase(ids, insert=True)
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
         dim = self.table.dim
-        C.pull_gather(h, lay, ctrl, tbl, self.slot_cache)
         rows = (int(bag_offsets.numel()) - 1) if bag_offsets is not None else n
         if out is None:
             out = torch.empty((rows, dim), dtype=torch.float32, device=self.table.device)
-        C.pull_combine(h, lay, ctrl, self.inv, n, dim, bag_offsets, weights, mean, bag_mean, patch_value, out,
-                       self.spin)
-        self.launches += 2 + self._wait  # gather, (response wait,) combine
+        if self.world == 1:  # the rows are read where they are
+            C.local_combine(tbl, self.inv, self.slot_cache, n, bag_offsets, weights, mean, bag_mean, patch_value, out)
+            self.launches += 1
+        else:
+            C.pull_gather(h, lay, ctrl, tbl, self.slot_cache)
+            C.pull_combine(h, lay, ctrl, self.inv, n, dim, bag_offsets, weights, mean, bag_mean, patch_value, out,
+                           self.spin)
+            self.launches += 3  # gather, response wait, combine
         return out, Ticket(self, self.serial, n, bag_offsets, weights, mean, bag_mean)
 
     # ------------------------------------------------------------------ push

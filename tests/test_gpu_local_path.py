@@ -60,3 +60,53 @@ def test_push_drops_the_gradient_of_an_unknown_id():
     after = kk.pull_sparse_table(t, known)
     assert torch.allclose(after, before - 0.05 * torch.tensor([0, 0, 1.0, 1.0], device=DEV)[:, None])
     assert float(kk.native.engine().channels[t].ugrad.abs().max()) == 0.0
+
+
+# Id counts around the threads of a block (256), around the point where a thread takes four ids (two full waves of
+# blocks: 606208), and with heavy repetition; rows that exist, rows that are created, and both.
+@pytest.mark.parametrize("n,space", [(1, 1), (255, 300), (256, 256), (257, 40), (5003, 4000), (606207, 500_000),
+                                     (606208, 500_000), (700_001, 9)])
+def test_lookup_numbers_every_id_once_and_finds_its_row(n, space):
+    t, shard = make(4, kk.OptimType.kSGD, {}, capacity=1 << 21, max_ids_per_call=800_000)
+    torch.manual_seed(n)
+    for _ in range(2):
+        ids = torch.randint(0, space, (n,)) * 7919 - 3
+        rows = kk.pull_sparse_table(t, ids.to(DEV))
+        ch = kk.native.engine().channels[t]
+        uniq, inv = ch.uniq[:int(ch.off[1])].cpu(), ch.inv[:n].cpu().long()
+        assert torch.equal(uniq[inv], ids) and torch.equal(uniq.sort().values, torch.unique(ids))
+        want, at = C.cpu_dedup(ids)
+        assert torch.allclose(rows.cpu(), shard.pull_sparse(t, want)[at], atol=1e-5)  # Box-Muller in float32, rows of ~0.5
+        assert int(ch.cnt[0]) == 0 and bool((ch.lset == -1).all())
+    kk.native.engine().check()
+    assert kk.native.engine().sparse[t].num_rows() <= space
+
+
+@pytest.mark.parametrize("dim", [1, 3, 20, 64, 1028])
+@pytest.mark.parametrize("mean", [False, True])
+def test_bags_are_pooled_from_the_table(dim, mean):
+    t, shard = make(dim, kk.OptimType.kSGD, {})
+    torch.manual_seed(dim)
+    lens = torch.tensor([0, 1, 3, 4, 5, 0, 8, 9, 17] * 30)
+    off = torch.cat([torch.zeros(1, dtype=torch.int64), lens.cumsum(0)])
+    ids = torch.randint(0, 90, (int(off[-1]),))
+    w = torch.rand(ids.numel())
+    out, ticket = kk.native.engine().pull_sparse_pooled(t, ids.to(DEV), off.to(DEV), weights=w.to(DEV), mean=mean,
+                                                        patch_value=0.5)
+    uniq, inv = C.cpu_dedup(ids)
+    rows = shard.pull_sparse(t, uniq)[inv] * w[:, None]
+    want = torch.zeros(lens.numel(), dim).index_add_(0, torch.repeat_interleave(torch.arange(lens.numel()), lens), rows)
+    if mean:
+        want = want / lens.clamp(min=1)[:, None]
+    want[lens == 0] = 0.5
+    assert torch.allclose(out.cpu(), want, atol=1e-4)  # up to 17 rows of ~0.5 in float32
+    kk.native.engine().check()
+
+
+def test_ids_beyond_the_unique_limit_are_reported():
+    t, _ = make(4, kk.OptimType.kSGD, {}, max_ids_per_call=4096, max_unique_per_call=100)
+    kk.pull_sparse_table(t, torch.arange(101, device=DEV))
+    with pytest.raises(kk.KrakenError):
+        kk.native.engine().check()
+    assert torch.isfinite(kk.pull_sparse_table(t, torch.arange(100, device=DEV))).all()
+    kk.native.engine().check()

@@ -1323,7 +1323,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     check_launch("push_apply");
   });
   m.def("local_lookup", [](const torch::Tensor& ids, const torch::Tensor& set, const torch::Tensor& first,
-                           const torch::Tensor& pos, uint32_t hbits, const torch::Tensor& cnt, const torch::Tensor& off,
+                           const torch::Tensor& pos, const torch::Tensor& win, uint32_t hbits,
+                           const torch::Tensor& cnt, const torch::Tensor& off,
                            const torch::Tensor& uniq, const torch::Tensor& inv, int cap_u, const cu::TableHost& table,
                            const torch::Tensor& slot_cache, bool insert, const torch::Tensor& ctrl) {
     need_cuda(ids, "ids", torch::kInt64);
@@ -1331,12 +1332,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     const int n = static_cast<int>(ids.numel());
     TORCH_CHECK(hbits <= 31 && set.numel() == (1ll << hbits) && set.numel() > n,
                 "dedup scratch must be an int32 [1 << hbits] tensor with more than n slots");
-    TORCH_CHECK(first.numel() >= n && pos.numel() >= n && inv.numel() >= n && uniq.numel() >= cap_u,
+    TORCH_CHECK(first.numel() >= n && pos.numel() >= n && inv.numel() >= n && uniq.numel() >= cap_u &&
+                    win.numel() >= cap_u,
                 "dedup outputs too small");
     TORCH_CHECK(cnt.numel() >= 1 && off.numel() >= 2, "cnt/off too small");
     c10::cuda::CUDAGuard guard(ids.device());
-    cu::local_lookup(ptr<int64_t>(ids), n, cu::LocalScratch{ptr<int>(set), ptr<int>(first), ptr<int>(pos), hbits},
-                     ptr<int>(cnt), ptr<int>(off), ptr<int64_t>(uniq), ptr<int>(inv), cap_u, table, ptr<int>(slot_cache),
+    cu::local_lookup(ptr<int64_t>(ids), n, cu::LocalScratch{ptr<int>(set), ptr<int>(first), ptr<int>(pos), ptr<int>(win), hbits}, ptr<int>(cnt), ptr<int>(off), ptr<int64_t>(uniq), ptr<int>(inv), cap_u, table, ptr<int>(slot_cache),
                      static_cast<int>(slot_cache.numel()), insert, ctrl_ptr(ctrl), cur_stream());
     check_launch("local_lookup");
   });
@@ -1378,6 +1379,30 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                           static_cast<int>(slot_cache.numel()), optim, ptr<float>(lr), cur_stream());
     check_launch("local_push_update");
   });
+  m.def("local_push",
+        [](const cu::TableHost& table, const torch::Tensor& grads, const torch::Tensor& inv, const torch::Tensor& first,
+           const torch::Tensor& win, int n, const c10::optional<torch::Tensor>& bag_offsets,
+           const c10::optional<torch::Tensor>& weights, bool mean, const c10::optional<torch::Tensor>& bag_mean,
+           const torch::Tensor& lookup_ctrl, const torch::Tensor& multi, const c10::optional<torch::Tensor>& bag_of,
+           const torch::Tensor& ugrad, const torch::Tensor& off, const torch::Tensor& slot_cache, const OptimPOD& optim,
+           const torch::Tensor& lr) {
+          need_cuda(grads, "grads", torch::kFloat32);
+          need_cuda(ugrad, "ugrad", torch::kFloat32);
+          need_cuda(lr, "lr", torch::kFloat32);
+          const int k = bag_offsets.has_value() ? static_cast<int>(bag_offsets->numel()) - 1 : 0;
+          TORCH_CHECK(grads.numel() == static_cast<int64_t>(bag_offsets.has_value() ? k : n) * table.dim,
+                      "grads has the wrong size");
+          TORCH_CHECK(ugrad.dim() == 2 && ugrad.size(1) == table.dim && inv.numel() >= n && first.numel() >= n &&
+                          win.numel() >= ugrad.size(0) && multi.numel() >= ugrad.size(0) &&
+                          (!bag_offsets.has_value() || (bag_of.has_value() && bag_of->numel() >= ugrad.size(0))),
+                      "the lookup's buffers do not fit this channel");
+          cu::LocalPush p{ptr<float>(grads), ptr<int>(inv), ptr<int>(first), ptr<int>(win), optr<int64_t>(bag_offsets), k,
+                          optr<float>(weights), mean, optr<uint8_t>(bag_mean), ctrl_ptr(lookup_ctrl),
+                          reinterpret_cast<uint32_t*>(ptr<int>(multi)), optr<int>(bag_of)};
+          cu::local_push(table, p, ptr<float>(ugrad), ptr<int>(off), ptr<int>(slot_cache), n,
+                         static_cast<int>(slot_cache.numel()), optim, ptr<float>(lr), cur_stream());
+          check_launch("local_push");
+        });
 
   // ---------------- one exchange for several tables of one row width
   m.def("group_table_views", [](const std::vector<cu::TableHost>& tables) {

@@ -122,6 +122,7 @@ struct LocalScratch {
   int* set;    // [1 << hbits]
   int* first;  // [n]
   int* pos;    // [n]
+  int* win;    // [cap_u] unique id -> its first occurrence
   uint32_t hbits;
 };
 // dedup_bucketize_dispatch + pull_probe without the inbox.  cnt[0] must be zero on entry and is again when the call
@@ -142,6 +143,25 @@ void local_combine(TableHost table, const int* inv, const int* slot_cache, int n
 // ugrad and zeroes it.  slot_cache[u] is the row of unique id u (u < cap_s); max_n bounds U.
 void local_push_update(TableHost table, float* ugrad, const int* off, const int* slot_cache, int max_n, int cap_s,
                        OptimPOD optim, const float* lr, cudaStream_t stream);
+
+// push_scatter + local_push_update of the gradients of a lookup; the gradient of an id's first occurrence is not summed
+// into ugrad but read from `grads` by the update.
+struct LocalPush {
+  const float* grads;          // [n, dim], or [nbags, dim] with bag_offsets
+  const int* inv;              // inv, first and win are the lookup's
+  const int* first;
+  const int* win;
+  const int64_t* bag_offsets;
+  int nbags;
+  const float* weights;
+  bool mean;
+  const uint8_t* bag_mean;
+  const Ctrl* lookup;          // control block of the channel that did the dedup
+  uint32_t* multi;             // [cap_u] of this channel: number of the last lookup in which the id occurred more than once
+  int* bag_of;                 // [cap_u] scratch (bags only)
+};
+void local_push(TableHost table, const LocalPush& p, float* ugrad, const int* off, const int* slot_cache, int n, int cap_s,
+                OptimPOD optim, const float* lr, cudaStream_t stream);
 
 // One of the channel's rendezvous points as a launch of its own: kind 0 = every source's request has
 // arrived (also snapshots the counts), 1 = every owner has answered the pull, 2 = every source's gradient

@@ -18,28 +18,59 @@ namespace {
 // update grid and 226 us with one in plain stream order, one of 65536 samples 980 and 963 us.
 constexpr int kFullGrid = 148 * 4;
 
+// Rows of less than a sector (8 floats) are summed in any case: telling the update where a gradient is takes as much
+// traffic as the gradient.
+constexpr int kDirectDim = 8;
+
+// Where the update finds the gradient of every id's first occurrence.
+struct DirectSource {
+  const float* grads;          // [n, dim], or [bags, dim]
+  const int64_t* bag_offsets;  // null: one gradient row per occurrence
+  const float* weights;        // per occurrence of a bag, or null
+  const uint8_t* bag_mean;
+  int mean;
+  const int* win;              // unique id -> its first occurrence
+  const int* bag_of;           // unique id -> the bag of its first occurrence (null without bags)
+  const uint32_t* multi;       // == *epoch: the id occurs more than once
+  const uint32_t* epoch;       // number of the lookup
+  __device__ __forceinline__ float bag_scale(int b) const {
+    const int64_t len = bag_offsets[b + 1] - bag_offsets[b];
+    const bool is_mean = bag_mean ? bag_mean[b] != 0 : mean != 0;
+    return is_mean && len > 0 ? 1.f / static_cast<float>(len) : 1.f;
+  }
+};
+
 // Optimizer update straight from the segment-sum buffer: entry u of `ugrad` is the gradient of the row
 // in slot_cache[u], and is zeroed here for the next step's segment-sum.
 //
-// Bound by HBM: per row it must read the gradient, read and write value and state rows and write the
-// zeros.  The two-kernel form (push_dispatch into the inbox, push_update out of it) wrote and read
-// every gradient row once more.  Measured for 2.3 M rows of 64 floats with Adagrad: 853 us before (310 + 543), 590 us
-// now, of 543 us at the copy rate; 0.55 M rows of 20 floats with Adam: 245 us before, 214 us now.  A row is handled by `chunks` neighbouring threads of a block, one
-// 16-byte chunk each (a row width like 20 floats leaves no lane idle, as a power-of-two group per row
-// would); the threads of a row may sit in two warps, so its step counter is read by all of them before
-// the block barrier and written behind it.
-template <int VEC, int OPT>
-__global__ void __launch_bounds__(kThreads, 4)
+// Bound by HBM: per row it must read the gradient, read and write value and state rows and write the zeros.  The
+// two-kernel form (push_dispatch into the inbox, push_update out of it) wrote and read every gradient row once more.
+// Measured for 0.55 M rows of 20 floats with Adam: 245 us before, 194 us now.  A row is handled by `chunks` neighbouring
+// threads of a block, one 16-byte chunk each (a row width like 20 floats leaves no lane idle, as a power-of-two group
+// per row would); the threads of a row may sit in two warps, so its step counter is read by all of them before the
+// block barrier and written behind it.  What is known of the next row is fetched one pass ahead.  Nine blocks of 128
+// threads per SM hold 56 registers a thread without spills; eight of them were 3 to 6 % slower, four or five blocks of
+// 256 threads up to 25 %.
+//
+// FROM: with kFromRows and kFromBags the gradient of every id's first occurrence is read from the caller's gradients
+// (`so`); `ugrad` holds the sum of the others, which is not read where there are none.  2.3 M rows of 64 floats, Adagrad: 853 us with two
+// kernels, 590 us with one that reads and clears every sum, 500 us so, of 460 us at the copy rate.
+constexpr int kUpdateThreads = 128;
+enum GradSource { kFromSum = 0, kFromRows = 1, kFromBags = 2 };
+
+template <int VEC, int OPT, int FROM>
+__global__ void __launch_bounds__(kUpdateThreads, 9)
 local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restrict__ off,
-                    const int* __restrict__ slot_cache, OptimPOD optim_in, const float* __restrict__ lr_ptr, int cap_s,
-                    int chunks, int tpr) {
+                    const int* __restrict__ slot_cache, DirectSource so, OptimPOD optim_in,
+                    const float* __restrict__ lr_ptr, int cap_s, int chunks, int tpr) {
   pdl_enter();
   using V = Vec<VEC>;
+  const uint32_t now = FROM != kFromSum ? *so.epoch : 0;
   OptimPOD optim = optim_in;
   optim.type = OPT;
   const float lr = *lr_ptr;
   const int U = off[1];
-  const int rows = kThreads / tpr;             // rows of one block and pass
+  const int rows = kUpdateThreads / tpr;             // rows of one block and pass
   const int r = threadIdx.x / tpr;
   const int c0 = threadIdx.x - r * tpr;
   const int stride = gridDim.x * rows;
@@ -47,19 +78,35 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
   const bool counts = t.steps != nullptr;
   const bool active = r < rows;
   int u = blockIdx.x * rows + r;
-  int slot = active && u < limit ? slot_cache[u] : -1;
+  // what is known of a row before its data: its slot, the row of `grads`, whether there is a sum of others
+  auto slot_of = [&](int v) { return active && v < limit ? slot_cache[v] : -1; };
+  auto src_of = [&](int v) { 
+    if (FROM == kFromSum || !active || v >= U) return 0;
+    return FROM == kFromBags ? so.bag_of[v] : so.win[v];
+  };
+  auto many_of = [&](int v) { return active && v < U && (FROM == kFromSum || so.multi[v] == now); };
+  int slot = slot_of(u), from = src_of(u);
+  bool many = many_of(u);
   for (int base = blockIdx.x * rows; base < U; base += stride, u += stride) {
-    const int next = active && u + stride < limit ? slot_cache[u + stride] : -1;
+    const int next = slot_of(u + stride), next_from = src_of(u + stride);
+    const bool next_many = many_of(u + stride);
     const bool mine = active && u < U;
     float* const gu = ugrad + static_cast<size_t>(u) * t.dim;
+    const float* const gd = so.grads + static_cast<size_t>(from) * t.dim;
+    float scale = 1.f, weight = 1.f;
+    if (FROM == kFromBags && mine) {
+      scale = so.bag_scale(from);
+      if (so.weights) weight = so.weights[so.win[u]];
+    }
     const size_t row = static_cast<size_t>(slot < 0 ? 0 : slot) * t.dim;
     // an id that was not found (reported by the lookup) has no row: its gradient is dropped
     const bool found = mine && slot >= 0;
     int step_i = 1;
     if (counts && found) step_i = t.steps[slot] + 1;
-    float g[VEC], w[VEC], a0[VEC], a1[VEC], a2[VEC];
+    float g[VEC], d[VEC], w[VEC], a0[VEC], a1[VEC], a2[VEC];
     auto load = [&](int c) {
-      *reinterpret_cast<typename V::T*>(g) = V::ldcg(gu + c * VEC);
+      *reinterpret_cast<typename V::T*>(g) = many ? V::ldcg(gu + c * VEC) : V::zero();
+      if (FROM != kFromSum) *reinterpret_cast<typename V::T*>(d) = V::ldcg(gd + c * VEC);
       *reinterpret_cast<typename V::T*>(w) = V::ld(t.val + row + c * VEC);
       if (t.s[0]) *reinterpret_cast<typename V::T*>(a0) = V::ld(t.s[0] + row + c * VEC);
       if (t.s[1]) *reinterpret_cast<typename V::T*>(a1) = V::ld(t.s[1] + row + c * VEC);
@@ -75,6 +122,10 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
       const AdamBias ab = optim.type == 1 ? AdamBiasAt(optim, step) : AdamBias{1.f, 1.f};
       for (int c = c0; c < chunks; c += tpr) {
         if (c != c0) load(c);
+        if (FROM != kFromSum) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) g[e] += FROM == kFromBags ? d[e] * scale * weight : d[e];
+        }
 #pragma unroll
         for (int e = 0; e < VEC; ++e) UpdateElem(optim, lr, g[e], step, ab, w[e], a0[e], a1[e], a2[e]);
         V::st(t.val + row + c * VEC, *reinterpret_cast<typename V::T*>(w));
@@ -83,24 +134,103 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
         if (t.s[2]) V::st(t.s[2] + row + c * VEC, *reinterpret_cast<typename V::T*>(a2));
       }
     }
-    if (mine)
+    if (many)
       for (int c = c0; c < chunks; c += tpr) V::st(gu + c * VEC, V::zero());
-    slot = next;
+    slot = next, from = next_from, many = next_many;
+  }
+}
+
+template <int VEC, int FROM>
+void launch_local_update(int grid, cudaStream_t stream, const TableView& t, float* ugrad, const int* off,
+                         const int* slot_cache, const DirectSource& so, const OptimPOD& optim, const float* lr, int cap_s,
+                         int chunks, int tpr) {
+  auto go = [&](auto kernel) {
+    launch_pdl_if(grid < 2 * kFullGrid, kernel, dim3(grid), dim3(kUpdateThreads), 0, stream, t, ugrad, off, slot_cache, so, optim, lr,
+                  cap_s, chunks, tpr);
+  };
+  switch (optim.type) {
+    case 0: go(local_update_kernel<VEC, 0, FROM>); break;
+    case 1: go(local_update_kernel<VEC, 1, FROM>); break;
+    case 2: go(local_update_kernel<VEC, 2, FROM>); break;
+    default: go(local_update_kernel<VEC, 3, FROM>); break;
+  }
+}
+
+// Segment-sum of the gradients of all but every id's first occurrence; `first` < 0 names that one, and its gradient is
+// left to the update, which for a bag is told the bag.  Bound by the 16-byte reductions in L2 and by the HBM traffic of
+// reductions into rows that are not there: an id that occurs once has its row neither read and written here nor read
+// and cleared in the update.  3.4 M rows of 64 floats: 490 us with every row summed, 245 us now.  The ids with a sum are
+// marked here, by plain stores: marking them in the dedup, with a look at the mark first, took 84 us for 240 k ids instead
+// of 7 - lines that are read and written from both dies move to and fro.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+local_scatter_kernel(const int* __restrict__ inv, const int* __restrict__ first, DirectSource so, uint32_t* multi, int n,
+                     int dim, int chunks, int tpr, float* ugrad) {
+  pdl_enter();
+  using V = Vec<VEC>;
+  constexpr int kUnroll = 4;
+  const uint32_t now = *so.epoch;
+  const int rows = kThreads / tpr;
+  const int r = threadIdx.x / tpr, c0 = threadIdx.x - r * tpr;
+  if (r >= rows) return;
+  const int stride = gridDim.x * rows;
+  for (int i0 = blockIdx.x * rows + r; i0 < n; i0 += stride * kUnroll) {
+    int u[kUnroll];
+#pragma unroll
+    for (int q = 0; q < kUnroll; ++q) {
+      const int i = i0 + q * stride;
+      u[q] = i < n && first[i] >= 0 ? inv[i] : -1;
+    }
+    for (int c = c0; c < chunks; c += tpr) {
+      typename V::T v[kUnroll];
+#pragma unroll
+      for (int q = 0; q < kUnroll; ++q)
+        if (u[q] >= 0) v[q] = V::ld(so.grads + static_cast<size_t>(i0 + q * stride) * dim + c * VEC);
+#pragma unroll
+      for (int q = 0; q < kUnroll; ++q)
+        if (u[q] >= 0) {
+          V::red(ugrad + static_cast<size_t>(u[q]) * dim + c * VEC, v[q]);
+          if (c == 0) multi[u[q]] = now;
+        }
+    }
   }
 }
 
 template <int VEC>
-void launch_local_update(int grid, cudaStream_t stream, const TableView& t, float* ugrad, const int* off,
-                         const int* slot_cache, const OptimPOD& optim, const float* lr, int cap_s, int chunks, int tpr) {
-  auto go = [&](auto kernel) {
-    launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, t, ugrad, off, slot_cache, optim, lr,
-                  cap_s, chunks, tpr);
-  };
-  switch (optim.type) {
-    case 0: go(local_update_kernel<VEC, 0>); break;
-    case 1: go(local_update_kernel<VEC, 1>); break;
-    case 2: go(local_update_kernel<VEC, 2>); break;
-    default: go(local_update_kernel<VEC, 3>); break;
+__global__ void __launch_bounds__(kThreads)
+local_bag_scatter_kernel(const int* __restrict__ inv, const int* __restrict__ first, DirectSource so, uint32_t* multi,
+                         int* __restrict__ bag_of, int nbags, int dim, int chunks, int tpr, float* ugrad) {
+  pdl_enter();
+  using V = Vec<VEC>;
+  constexpr int kUnroll = 4;
+  const uint32_t now = *so.epoch;
+  const int rows = kThreads / tpr;
+  const int g = threadIdx.x / tpr, c0 = threadIdx.x - g * tpr;
+  if (g >= rows) return;
+  for (int b = blockIdx.x * rows + g; b < nbags; b += gridDim.x * rows) {
+    const int64_t lo = so.bag_offsets[b], hi = so.bag_offsets[b + 1];
+    const float scale = so.bag_scale(b);
+    for (int c = c0; c < chunks; c += tpr) {
+      const typename V::T v = V::scale(V::ld(so.grads + static_cast<size_t>(b) * dim + c * VEC), scale);
+      for (int64_t i0 = lo; i0 < hi; i0 += kUnroll) {
+        int u[kUnroll], f[kUnroll];
+#pragma unroll
+        for (int q = 0; q < kUnroll; ++q) {
+          u[q] = i0 + q < hi ? inv[i0 + q] : -1;
+          f[q] = i0 + q < hi ? first[i0 + q] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < kUnroll; ++q) {
+          if (u[q] < 0) continue;
+          if (f[q] >= 0) {
+            V::red(ugrad + static_cast<size_t>(u[q]) * dim + c * VEC, so.weights ? V::scale(v, so.weights[i0 + q]) : v);
+            if (c == 0) multi[u[q]] = now;
+          } else if (c == 0) {
+            bag_of[u[q]] = b;
+          }
+        }
+      }
+    }
   }
 }
 
@@ -201,14 +331,14 @@ __device__ __forceinline__ void init_created(const TableView& t, unsigned todo, 
 
 // Second kernel, with the table probe: every occurrence learns its unique id's number; the winner also writes the
 // unique list, empties the set's entry, and finds (or, with `insert`, claims and initialises) the row.  The block that
-// finishes last zeroes `cnt` for the next call.  The ids do not pass through the inbox, and no block ends on a
+// finishes last zeroes `cnt` for the next call and counts the lookup.  The ids do not pass through the inbox, and no block ends on a
 // system-scope fence.
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 local_resolve_kernel(const int64_t* __restrict__ ids, int n, int* __restrict__ set, const int* __restrict__ first,
                      const int* __restrict__ pos, int* cnt, int* off, int64_t* __restrict__ uniq, int* __restrict__ inv,
-                     int cap_u, TableView t, int* __restrict__ slot_cache, int cap_s, int insert, uint32_t* done, int* status,
-                     int chunks, int lpr) {
+                     int* __restrict__ win, int cap_u, TableView t, int* __restrict__ slot_cache, int cap_s, int insert,
+                     uint32_t* epoch, uint32_t* done, int* status, int chunks, int lpr) {
   pdl_enter();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     // more unique ids than the channel's buffers hold: reported and clamped, so that no later kernel indexes
@@ -231,6 +361,7 @@ local_resolve_kernel(const int64_t* __restrict__ ids, int n, int* __restrict__ s
       set[~f] = -1;  // leave the set empty for the next call
       if (u < cap_u) {
         uniq[u] = static_cast<int64_t>(id);
+        win[u] = i;
         if (u < cap_s) {
           slot = table_find_or_insert(t, id, insert != 0, &created);
           if (slot < 0 && !insert) set_status(status, err::kSparseIdNotExist);
@@ -250,6 +381,7 @@ local_resolve_kernel(const int64_t* __restrict__ ids, int n, int* __restrict__ s
     if (atomicAdd(done, 1u) == gridDim.x - 1) {
       *done = 0;
       *cnt = 0;
+      *epoch += 1;
     }
   }
 }
@@ -404,8 +536,8 @@ void local_lookup(const int64_t* ids, int n, LocalScratch sc, int* cnt, int* off
                 &ctrl->status);
   auto kernel = g.vec == 4 ? local_resolve_kernel<4> : local_resolve_kernel<1>;
   launch_pdl_if(early, kernel, grid, dim3(kThreads), 0, stream, ids, n, sc.set, static_cast<const int*>(sc.first),
-                static_cast<const int*>(sc.pos), cnt, off, uniq, inv, cap_u, to_view(table), slot_cache, cap_s,
-                insert ? 1 : 0, &ctrl->done[0], &ctrl->status, g.chunks, g.lpr);
+                static_cast<const int*>(sc.pos), cnt, off, uniq, inv, sc.win, cap_u, to_view(table), slot_cache, cap_s,
+                insert ? 1 : 0, &ctrl->pull_epoch, &ctrl->done[0], &ctrl->status, g.chunks, g.lpr);
 }
 
 void local_probe(const int64_t* uniq, const int* off, int max_n, TableHost table, int* slot_cache, int cap_s, bool insert,
@@ -446,16 +578,57 @@ void local_combine(TableHost table, const int* inv, const int* slot_cache, int n
   }
 }
 
+namespace {
+template <int FROM>
+void update_all(TableHost table, float* ugrad, const int* off, const int* slot_cache, const DirectSource& so, int max_n,
+                int cap_s, OptimPOD optim, const float* lr, cudaStream_t stream) {
+  const RowGeom g = row_geom(table.dim);
+  const int tpr = g.chunks < kUpdateThreads ? g.chunks : kUpdateThreads;
+  const int grid = grid_for(max_n, kUpdateThreads / tpr, 148 * 80);
+  const TableView t = to_view(table);
+  if (g.vec == 4)
+    launch_local_update<4, FROM>(grid, stream, t, ugrad, off, slot_cache, so, optim, lr, cap_s, g.chunks, tpr);
+  else
+    launch_local_update<1, FROM>(grid, stream, t, ugrad, off, slot_cache, so, optim, lr, cap_s, g.chunks, tpr);
+}
+}  // namespace
+
 void local_push_update(TableHost table, float* ugrad, const int* off, const int* slot_cache, int max_n, int cap_s,
                        OptimPOD optim, const float* lr, cudaStream_t stream) {
+  update_all<kFromSum>(table, ugrad, off, slot_cache, DirectSource{}, max_n, cap_s, optim, lr, stream);
+}
+
+void local_push(TableHost table, const LocalPush& p, float* ugrad, const int* off, const int* slot_cache, int n, int cap_s,
+                OptimPOD optim, const float* lr, cudaStream_t stream) {
+  if (n <= 0) return;
+  const bool bags = p.bag_offsets != nullptr;
+  if (table.dim < kDirectDim) {
+    push_scatter(p.grads, p.inv, n, table.dim, p.bag_offsets, p.nbags, p.weights, p.mean, p.bag_mean, ugrad, stream);
+    update_all<kFromSum>(table, ugrad, off, slot_cache, DirectSource{}, n, cap_s, optim, lr, stream);
+    return;
+  }
+  DirectSource so{};
+  so.grads = p.grads, so.bag_offsets = p.bag_offsets, so.weights = p.weights, so.bag_mean = p.bag_mean;
+  so.mean = p.mean ? 1 : 0;
+  so.win = p.win, so.multi = p.multi, so.epoch = &p.lookup->pull_epoch;
+  so.bag_of = p.bag_of;
   const RowGeom g = row_geom(table.dim);
   const int tpr = g.chunks < kThreads ? g.chunks : kThreads;
-  const int rows = kThreads / tpr;
-  const int grid = grid_for(max_n, rows);
-  if (g.vec == 4)
-    launch_local_update<4>(grid, stream, to_view(table), ugrad, off, slot_cache, optim, lr, cap_s, g.chunks, tpr);
+  const int grid = grid_for(bags ? p.nbags : n, kThreads / tpr, 148 * 16);
+  if (bags) {
+    auto kernel = g.vec == 4 ? local_bag_scatter_kernel<4> : local_bag_scatter_kernel<1>;
+    if (p.nbags > 0)
+      launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, p.inv, p.first, so, p.multi, p.bag_of,
+                    p.nbags, table.dim, g.chunks, tpr, ugrad);
+  } else {
+    auto kernel = g.vec == 4 ? local_scatter_kernel<4> : local_scatter_kernel<1>;
+    launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, p.inv, p.first, so, p.multi, n, table.dim,
+                  g.chunks, tpr, ugrad);
+  }
+  if (bags)
+    update_all<kFromBags>(table, ugrad, off, slot_cache, so, n, cap_s, optim, lr, stream);
   else
-    launch_local_update<1>(grid, stream, to_view(table), ugrad, off, slot_cache, optim, lr, cap_s, g.chunks, tpr);
+    update_all<kFromRows>(table, ugrad, off, slot_cache, so, n, cap_s, optim, lr, stream);
 }
 
 }  // namespace cu

@@ -327,6 +327,10 @@ class SparseChannel:
             self.lbits = _next_pow2_bits(self.cap + self.cap // 4 + 1)
             self.lset = torch.full((1 << self.lbits,), -1, dtype=torch.int32, device=dev)
             self.pos = torch.zeros(self.cap, dtype=torch.int32, device=dev)
+            self.win = torch.zeros(self.cap_u, dtype=torch.int32, device=dev)
+            self.multi = torch.zeros(self.cap_u, dtype=torch.int32, device=dev)
+            self._bag_of: Optional[torch.Tensor] = None
+        self.dedup_by = self   # the channel whose dedup result off / uniq / inv are (another one after a shared pull)
         self.cnt = torch.zeros(world, dtype=torch.int32, device=dev)
         self._own_off = torch.zeros(world + 1, dtype=torch.int32, device=dev)
         self._own_uniq = torch.zeros(self.cap_u, dtype=torch.int64, device=dev)
@@ -362,7 +366,9 @@ class SparseChannel:
         share = share_from is not None and share_from.salt == self.salt and share_from.world == self.world
         if share:
             self.off, self.uniq, self.inv = share_from.off, share_from.uniq, share_from.inv
+            self.dedup_by = share_from.dedup_by
         else:
+            self.dedup_by = self
             self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
         if self.world == 1:
             # nobody to exchange with: the dedup's second kernel also finds the rows
@@ -370,7 +376,7 @@ class SparseChannel:
                 C.local_probe(self.uniq, self.off, n, tbl, self.slot_cache, insert, ctrl)
                 self.launches += 1
             else:
-                C.local_lookup(ids, self.lset, self.slot_of, self.pos, self.lbits, self.cnt, self.off, self.uniq, self.inv,
+                C.local_lookup(ids, self.lset, self.slot_of, self.pos, self.win, self.lbits, self.cnt, self.off, self.uniq, self.inv,
                                self.cap_u, tbl, self.slot_cache, insert, ctrl)
                 self.launches += 2
             self.serial += 1
@@ -491,9 +497,17 @@ class SparseChannel:
         grads = grads.reshape(-1, dim)
         if grads.dtype != torch.float32 or not grads.is_contiguous():
             grads = grads.to(torch.float32).contiguous()
-        C.push_scatter(grads, self.inv, n, dim, bag_offsets, weights, mean, bag_mean, self.ugrad)
-        self.launches += 1
-        self._apply_accumulated(lr, n)
+        if self.world == 1:
+            by = self.dedup_by
+            if self._bag_of is None and bag_offsets is not None:
+                self._bag_of = torch.zeros(self.cap_u, dtype=torch.int32, device=self.table.device)
+            C.local_push(self.table.host(), grads, self.inv, by.slot_of, by.win, n, bag_offsets, weights, mean, bag_mean,
+                         by.ctrl, self.multi, self._bag_of, self.ugrad, self.off, self.slot_cache, self.table.optim, lr)
+            self.launches += 2  # scatter, update
+        else:
+            C.push_scatter(grads, self.inv, n, dim, bag_offsets, weights, mean, bag_mean, self.ugrad)
+            self.launches += 1
+            self._apply_accumulated(lr, n)
         # A push consumes the pull's bookkeeping: a second push needs a new lookup.
         self.serial += 1
 

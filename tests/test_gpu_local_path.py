@@ -110,3 +110,41 @@ def test_ids_beyond_the_unique_limit_are_reported():
         kk.native.engine().check()
     assert torch.isfinite(kk.pull_sparse_table(t, torch.arange(100, device=DEV))).all()
     kk.native.engine().check()
+
+
+# The first occurrence of an id is updated from the caller's gradients, the others from their sum; widths on both sides
+# of the line below which every gradient is summed (8), with bags (weights, mean, empty ones) and without, and further
+# pushes of the same shape in which other ids are the ones that repeat.
+@pytest.mark.parametrize("dim", [7, 8, 10, 20, 64, 1028])
+@pytest.mark.parametrize("bags", [None, "sum", "mean"])
+def test_push_of_ids_that_occur_once_and_of_ids_that_repeat(dim, bags):
+    t, shard = make(dim, kk.OptimType.kAdagrad, {"initial_accumulator_value": "0.1"}, max_ids_per_call=4096)
+    torch.manual_seed(dim)
+    eng = kk.native.engine()
+    for step in range(3):
+        once = torch.randperm(600)[:300] + 1000 * (step % 2)
+        ids = torch.cat([once, torch.randint(0, 600, (200,)) + 1000, torch.full((40,), 7)])
+        ids = ids[torch.randperm(ids.numel())]
+        n = ids.numel()
+        uniq, inv = C.cpu_dedup(ids)
+        if bags is None:
+            kk.pull_sparse_table(t, ids.to(DEV))
+            g = torch.randn(n, dim)
+            kk.push_sparse_table(t, ids.to(DEV), g.to(DEV))
+        else:
+            lens = torch.tensor([0, 1, 5, 4, 8, 0, 9] * 20)
+            off = torch.cat([torch.zeros(1, dtype=torch.int64), lens.cumsum(0)])
+            assert int(off[-1]) == n
+            w = torch.rand(n)
+            _, ticket = eng.pull_sparse_pooled(t, ids.to(DEV), off.to(DEV), weights=w.to(DEV), mean=bags == "mean")
+            gb = torch.randn(lens.numel(), dim)
+            eng.push_sparse_pooled(t, ticket, gb.to(DEV), ids.to(DEV))
+            g = (gb / lens.clamp(min=1)[:, None] if bags == "mean" else gb).repeat_interleave(lens, 0) * w[:, None]
+        shard.pull_sparse(t, uniq)
+        assert shard.push_sparse(t, uniq, C.cpu_segment_sum(g, inv, uniq.numel()), 0.05) == 0
+    eng.check()
+    every = torch.arange(1600)
+    every = every[(every < 600) | (every >= 1000)]
+    # three Adagrad updates of at most 0.05 / sqrt(0.1) * |g|, their sums of up to 41 terms in another order
+    assert torch.allclose(kk.pull_sparse_table(t, every.to(DEV)).cpu(), shard.pull_sparse(t, every), atol=2e-4)
+    assert float(eng.channels[t].ugrad.abs().max()) == 0.0

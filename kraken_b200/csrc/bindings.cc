@@ -284,6 +284,48 @@ struct SymHeap {
   }
 };
 
+// A small device buffer's contents on their way to pinned host memory: start() enqueues the copy on the current
+// stream, ready() asks without waiting whether it has landed.
+struct AsyncRead {
+  torch::Tensor src;
+  int* host = nullptr;
+  cudaEvent_t event = nullptr;
+
+  explicit AsyncRead(const torch::Tensor& t) : src(t) {
+    need_cuda(t, "source", torch::kInt32);
+    CUDA_OK(cudaMallocHost(&host, t.numel() * sizeof(int)));
+    CUDA_OK(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+  }
+  AsyncRead(const AsyncRead&) = delete;
+  AsyncRead& operator=(const AsyncRead&) = delete;
+  ~AsyncRead() {
+    if (event) {
+      cudaEventSynchronize(event);  // a copy in flight still writes to `host`
+      cudaEventDestroy(event);
+    }
+    if (host) cudaFreeHost(host);
+  }
+  void Start(int n) {
+    TORCH_CHECK(n >= 0 && n <= src.numel(), "more values than the buffer holds");
+    CUDA_OK(cudaMemcpyAsync(host, src.data_ptr(), n * sizeof(int), cudaMemcpyDeviceToHost, cur_stream()));
+    CUDA_OK(cudaEventRecord(event, cur_stream()));
+  }
+  bool Ready() const {
+    const cudaError_t e = cudaEventQuery(event);
+    if (e == cudaErrorNotReady) return false;
+    CUDA_OK(e);
+    return true;
+  }
+  void Wait() const {
+    py::gil_scoped_release release;
+    CUDA_OK(cudaEventSynchronize(event));
+  }
+  std::vector<int> Values(int n) const {
+    TORCH_CHECK(n >= 0 && n <= src.numel(), "more values than the buffer holds");
+    return std::vector<int>(host, host + n);
+  }
+};
+
 cu::TableHost make_table(const torch::Tensor& keys, const torch::Tensor& val, const c10::optional<torch::Tensor>& s0,
                          const c10::optional<torch::Tensor>& s1, const c10::optional<torch::Tensor>& s2,
                          const c10::optional<torch::Tensor>& steps, const c10::optional<torch::Tensor>& lead,
@@ -1200,6 +1242,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       py::arg("offsets"), py::arg("grads"), py::arg("weights") = py::none());
 
   // ---------------- symmetric heap + device structs
+  py::class_<AsyncRead>(m, "AsyncRead")
+      .def(py::init<const torch::Tensor&>())
+      .def("start", &AsyncRead::Start)
+      .def("ready", &AsyncRead::Ready)
+      .def("wait", &AsyncRead::Wait)
+      .def("values", &AsyncRead::Values);
   py::class_<SymHeap>(m, "SymHeap")
       .def(py::init<size_t, int, int, bool>(), py::arg("bytes"), py::arg("rank"), py::arg("world"),
            py::arg("alias_peers") = false)

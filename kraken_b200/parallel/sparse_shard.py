@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import math
 import os
+import weakref
 from typing import Dict, Optional
 
 import torch
@@ -33,11 +34,63 @@ def _next_pow2_bits(n: int) -> int:
     return max(4, int(math.ceil(math.log2(max(2, n)))))
 
 
+class RowCounters:
+    """Row counters of a rank's tables, side by side in device memory, so that the host learns how full ALL of them are
+    with one asynchronous copy.  ``added`` of a table counts, on the host, the rows that the calls so far may have
+    created; a sample remembers it, so that ``bound(table)`` - the sampled rows plus what was added since - never lies
+    below the number of rows that the enqueued calls can lead to."""
+
+    BANK = 256
+
+    def __init__(self, device: torch.device) -> None:
+        self.device = device
+        self.banks = []            # (int32 [BANK] device tensor, its copy to the host); tables hold one-element views
+        self.tables = []
+        self._marks = None         # ``added`` of every table when the sample in flight was taken
+
+    def attach(self, table) -> torch.Tensor:
+        k = len(self.tables)
+        if k % self.BANK == 0:
+            bank = torch.zeros(self.BANK, dtype=torch.int32, device=self.device)
+            self.banks.append((bank, C.AsyncRead(bank)))
+        self.tables.append(weakref.ref(table))  # a table keeps its counters, not the other way round
+        return self.banks[-1][0][k % self.BANK:k % self.BANK + 1]
+
+    def start(self) -> None:
+        """Enqueues a sample on the current stream unless one is in flight.  The calls counted in ``added`` must have
+        been enqueued before it."""
+        if self._marks is not None or not self.tables:
+            return
+        n = len(self.tables)
+        for k, (_, read) in enumerate(self.banks):
+            read.start(min(self.BANK, n - k * self.BANK))
+        self._marks = [getattr(t(), "added", 0) for t in self.tables]
+
+    def poll(self, wait: bool = False) -> bool:
+        """Takes over the sample in flight if it has landed (``wait``: waits for it); True if it did."""
+        if self._marks is None:
+            return False
+        last = self.banks[(len(self._marks) - 1) // self.BANK][1]   # the copies land in order
+        if wait:
+            last.wait()
+        elif not last.ready():
+            return False
+        for k in range(0, len(self._marks), self.BANK):
+            rows = self.banks[k // self.BANK][1].values(min(self.BANK, len(self._marks) - k))
+            for ref, r, mark in zip(self.tables[k:], rows, self._marks[k:]):
+                t = ref()
+                if t is not None:
+                    t.sampled_rows, t.sampled_added = r, mark
+        self._marks = None
+        return True
+
+
 class GpuSparseTable:
     """One rank's shard of a sparse table."""
 
     def __init__(self, table_id: int, name: str, dim: int, init_type, init_conf: Dict[str, str], optim_type,
-                 optim_conf: Dict[str, str], seed: int, capacity: int, world: int, device: torch.device) -> None:
+                 optim_conf: Dict[str, str], seed: int, capacity: int, world: int, device: torch.device,
+                 counters: Optional[RowCounters] = None) -> None:
         self.table_id = table_id
         self.name = name
         self.dim = int(dim)
@@ -52,10 +105,12 @@ class GpuSparseTable:
         self.world = world
         self.device = device
         self.bits = _next_pow2_bits(capacity)
-        self.size = torch.zeros(1, dtype=torch.int32, device=device)
+        self.added = 0            # rows that the calls so far may have created (host-side count)
+        self.sampled_rows = 0     # the last sample of ``size`` ...
+        self.sampled_added = 0    # ... and ``added`` when it was taken
+        self.counters = counters if counters is not None else RowCounters(device)
+        self.size = self.counters.attach(self)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
-        self._size_host = torch.zeros(1, dtype=torch.int32).pin_memory() if device.type == "cuda" else None
-        self._size_event: Optional[torch.cuda.Event] = None
         self._alloc(self.bits)
 
     # ------------------------------------------------------------------ storage
@@ -194,9 +249,8 @@ class GpuSparseTable:
         n = int(ids.numel())
         if n == 0:
             return
-        total = self.num_rows() + n
-        self.reserve(total)
-        self.rows_hi = max(getattr(self, "rows_hi", 0), total)  # host-side upper bound used by the engine's growth check
+        self.reserve(self.num_rows() + n)
+        self.added += n
         dev = self.device
         ids = ids.to(dev, torch.int64).contiguous()
         vals = vals.to(dev, torch.float32).contiguous()
@@ -224,23 +278,23 @@ class GpuSparseTable:
                        old["states_i"][0].to(torch.int32) if self.steps is not None else None)
         return True
 
+    def rows_bound(self) -> int:
+        """Upper bound of the rows after every call enqueued so far, without a look at the device."""
+        return self.sampled_rows + self.added - self.sampled_added
+
+    def grow_for_pace(self, max_load: float = 0.6) -> bool:
+        """Grows the table if its last sampled row count, at the pace seen since the one before, nears the limit."""
+        rows = self.sampled_rows
+        # the sample is a step or two old: leave room for what arrives at the pace seen since the last one
+        pace = max(0, rows - getattr(self, "_rows_seen", rows))
+        self._rows_seen = rows
+        return rows + 2 * pace > max_load * self.capacity and self.reserve(int((rows + 2 * pace) * 2))
+
     def poll_growth(self, max_load: float = 0.6) -> bool:
-        """Non-blocking load-factor check: looks at the size counter copied out
-        during the previous call and starts the next copy.  Call between steps."""
-        grew = False
-        if self._size_host is not None:
-            if self._size_event is not None and self._size_event.query():
-                rows = int(self._size_host[0])
-                # the sample is a step or two old: leave room for what arrives at the pace seen since the last one
-                pace = max(0, rows - getattr(self, "_rows_seen", rows))
-                self._rows_seen = rows
-                if rows + 2 * pace > max_load * self.capacity:
-                    grew = self.reserve(int((rows + 2 * pace) * 2))
-                self._size_event = None
-            if self._size_event is None:
-                self._size_host.copy_(self.size, non_blocking=True)
-                self._size_event = torch.cuda.Event()
-                self._size_event.record()
+        """Non-blocking load-factor check of a table by itself: looks at the row counter copied out during the
+        previous call and starts the next copy.  Call between steps."""
+        grew = self.counters.poll() and self.grow_for_pace(max_load)
+        self.counters.start()
         return grew
 
     def evict(self, min_steps: int) -> int:

@@ -17,7 +17,7 @@ import torch.distributed as dist
 from .._native import C
 from ..parallel.dense_bucket import BucketSet
 from ..parallel.nccl_baseline import NcclSparseChannel
-from ..parallel.sparse_shard import GpuSparseTable, GroupChannel, SparseChannel, Ticket
+from ..parallel.sparse_shard import GpuSparseTable, GroupChannel, RowCounters, SparseChannel, Ticket
 from ..utils import profiler as _profiler
 from .engine import Engine, EngineConfig, TableInfo
 
@@ -33,6 +33,8 @@ class GpuEngine(Engine):
         self.lr_dev = torch.zeros(1, dtype=torch.float32, device=self.device)
         self._lr_host = torch.zeros(1, dtype=torch.float32).pin_memory()
         self.sparse: Dict[int, GpuSparseTable] = {}
+        self.counters = RowCounters(self.device)
+        self._sample_next = False
         self.channels: Dict[int, SparseChannel] = {}
         self.tickets: Dict[int, Tuple[Ticket, int, int, int]] = {}
         self.group_channels: Dict[Tuple[int, ...], GroupChannel] = {}
@@ -71,7 +73,7 @@ class GpuEngine(Engine):
     def _on_register_sparse(self, info: TableInfo) -> None:
         self.sparse[info.id] = GpuSparseTable(info.id, info.name, info.dimension, info.init_type, info.init_conf,
                                               self.optim_type, self.optim_conf, self.cfg.seed,
-                                              self.cfg.table_capacity, self.world, self.device)
+                                              self.cfg.table_capacity, self.world, self.device, self.counters)
 
     def _salt(self, table_id: int) -> int:
         return C.table_salt(table_id) if self.cfg.owner_salt_per_table else 0
@@ -306,6 +308,7 @@ class GpuEngine(Engine):
         self._ensure_room(table_id, idx.numel())
         with self._region("pull"):
             rows, ticket = ch.pull(idx)
+        self._looked_up()
         self._remember(table_id, ticket, indices)
         return rows.view(*indices.shape, info.dimension)
 
@@ -332,6 +335,7 @@ class GpuEngine(Engine):
                 part = flat[k * ch.cap:(k + 1) * ch.cap]
                 self._ensure_room(table_id, part.numel())
                 ch.pull(part, out=out[k * ch.cap:k * ch.cap + part.numel()])
+                self._looked_up()
         return out
 
     def _push_in_rounds(self, ch: SparseChannel, idx: torch.Tensor, g: torch.Tensor, rounds: int) -> None:
@@ -388,10 +392,10 @@ class GpuEngine(Engine):
             flat = [self._prep_ids(indices[p]).reshape(-1) for p in pos]
             counts = [int(f.numel()) for f in flat]
             ch = self._group_channel(tids, sum(counts))
-            for t, c in zip(tids, counts):
-                self._ensure_room(t, c)
+            self._ensure_rooms(tids, counts)
             with self._region("pull"):
                 rows, ticket = ch.pull(torch.cat(flat), counts)
+            self._looked_up()
             self.group_tickets[tids] = (ticket, [indices[p] for p in pos], [self._sig(indices[p]) for p in pos])
             for p, part in zip(pos, rows.split(counts)):
                 out[p] = part.view(*indices[p].shape, dim)
@@ -469,11 +473,11 @@ class GpuEngine(Engine):
             bag_mean = torch.cat([torch.full((bags[k],), 1 if means[p] else 0, dtype=torch.uint8, device=self.device)
                                   for k, p in enumerate(pos)])
             ch = self._group_channel(tids, sum(counts))
-            for t, c in zip(tids, counts):
-                self._ensure_room(t, c)
+            self._ensure_rooms(tids, counts)
             with self._region("pull"):
                 rows, ticket = ch.pull(torch.cat(vals), counts, bag_offsets=torch.cat(offs).contiguous(),
                                        weights=weights, bag_mean=bag_mean, patch_value=patch)
+            self._looked_up()
             for p, part in zip(pos, rows.split(bags)):
                 outs[p] = part
             handles.append(("group", tids, ticket, (vals, counts, bags), list(pos)))
@@ -519,7 +523,9 @@ class GpuEngine(Engine):
         bm = bag_mean.detach().to(self.device, torch.uint8).contiguous() if bag_mean is not None else None
         ch = self._channel(table_id, idx.numel())
         self._ensure_room(table_id, idx.numel())
-        return ch.pull(idx, bag_offsets=off, weights=w, mean=mean, bag_mean=bm, patch_value=patch_value)
+        out = ch.pull(idx, bag_offsets=off, weights=w, mean=mean, bag_mean=bm, patch_value=patch_value)
+        self._looked_up()
+        return out
 
     def push_sparse_pooled(self, table_id: int, ticket: Ticket, grads: torch.Tensor,
                            values: Optional[torch.Tensor] = None) -> None:
@@ -540,7 +546,9 @@ class GpuEngine(Engine):
         share = self.channels.get(share_with) if share_with is not None else None
         self._ensure_room(table_id, idx.numel())
         with self._region("pull"):
-            return ch.pull_unique(idx, share_from=share, in_place=in_place)
+            out = ch.pull_unique(idx, share_from=share, in_place=in_place)
+        self._looked_up()
+        return out
 
     def grad_accumulator(self, table_id: int) -> torch.Tensor:
         """Per-unique-id gradient buffer [cap, dim] of the table's channel (zero between steps)."""
@@ -627,7 +635,6 @@ class GpuEngine(Engine):
                     slab.fill_(t.optim_info["initial_accumulator_value"] if (t.optim_info["type"] == 0 and k == 0) else 0.0)
             if t.steps is not None:
                 t.steps.zero_()
-            t.rows_hi = 0
             t.import_rows(keep["ids"], keep["vals"], keep["states"], keep["states_i"])
             t.import_rows(in_ids, in_vals, in_states, in_steps)
         self.owner_world = owner_world
@@ -658,8 +665,11 @@ class GpuEngine(Engine):
         if self.profiler is not None:
             self.profiler.end_step()
         grew = False
-        for t in self.sparse.values():
-            grew = t.poll_growth() or grew
+        if self.sparse:
+            if self.counters.poll():
+                for t in self.sparse.values():
+                    grew = t.grow_for_pace() or grew
+            self.counters.start()
         self._poll_status()
         return grew
 
@@ -699,35 +709,54 @@ class GpuEngine(Engine):
         host = getattr(self, "_status_host", None)
         if host is None or host.numel() < len(words):
             host = self._status_host = torch.zeros(max(16, 2 * len(words)), dtype=torch.int32).pin_memory()
-        for k, (_, w) in enumerate(words):
-            host[k:k + 1].copy_(w, non_blocking=True)
+        host[:len(words)].copy_(torch.cat([w.reshape(1) for _, w in words]), non_blocking=True)
         ev = torch.cuda.Event()
         ev.record()
         self._status_pending = (ev, host[:len(words)], words)
 
     def _ensure_room(self, table_id: int, n_ids: int) -> None:
-        """Makes sure the shard can take the rows this lookup may create BEFORE the kernels run (growth
-        by ``end_step`` reacts one step late: a first batch larger than the free slots would otherwise
-        hit the probe limit and come back as kTableFull).  A host-side upper bound of the row count is
-        kept per table; only when it nears the load limit is the exact counter read (one synchronisation)."""
+        """``_ensure_rooms`` for one table."""
+        self._ensure_rooms((table_id,), (n_ids,))
+
+    def _ensure_rooms(self, table_ids: Sequence[int], counts: Sequence[int]) -> None:
+        """Makes sure the shards can take the rows that a lookup of ``counts`` ids may create BEFORE its kernels run
+        (growth by ``end_step`` reacts one step late: a first batch larger than the free slots would otherwise
+        hit the probe limit and come back as kTableFull).  Decided on a host-side upper bound of the row counts.  When a
+        table is within two calls of its limit, the counters of all tables are sampled in one asynchronous copy behind
+        the lookup (``_looked_up``), so that a call waits for the device only if the bound passes the limit all the same."""
         if torch.cuda.is_current_stream_capturing():
             return
-        t = self.sparse[table_id]
-        ch = self.channels.get(table_id)
-        inflow = n_ids * self.world  # worst case: every rank's ids of this call belong to this shard
-        if ch is not None:
-            # no more than the exchange buffers admit (world x cap_s), and with a uniform owner hash about
-            # 1 / world of every rank's unique ids - twice that is reserved; a shard that still runs full
-            # reports kTableFull and is grown by end_step()
-            n_ids = min(n_ids, ch.cap_u)
-            inflow = min(self.world * ch.cap_s, 2 * n_ids) if self.world > 1 else n_ids
-        hi = getattr(t, "rows_hi", 0) + inflow
-        if hi > 0.6 * t.capacity:
-            exact = t.num_rows()
-            hi = exact + inflow
-            if hi > 0.6 * t.capacity:
-                t.reserve(hi)
-        t.rows_hi = hi
+        want = []
+        for table_id, n_ids in zip(table_ids, counts):
+            t = self.sparse[table_id]
+            ch = self.channels.get(table_id)
+            inflow = n_ids * self.world  # worst case: every rank's ids of this call belong to this shard
+            if ch is not None:
+                # no more than the exchange buffers admit (world x cap_s), and with a uniform owner hash about
+                # 1 / world of every rank's unique ids - twice that is reserved; a shard that still runs full
+                # reports kTableFull and is grown by end_step()
+                n_ids = min(n_ids, ch.cap_u)
+                inflow = min(self.world * ch.cap_s, 2 * n_ids) if self.world > 1 else n_ids
+            want.append((t, inflow))
+        self._sample_next = any(t.rows_bound() + 2 * inflow > 0.6 * t.capacity for t, inflow in want)
+        if self._sample_next:
+            self.counters.poll()
+            for _ in range(2):  # the sample that is waited for first may be an older one
+                if any(t.rows_bound() + inflow > 0.6 * t.capacity for t, inflow in want):
+                    self.counters.start()
+                    self.counters.poll(wait=True)
+            for t, inflow in want:
+                hi = t.rows_bound() + inflow
+                if hi > 0.6 * t.capacity:
+                    t.reserve(hi)
+        for t, inflow in want:
+            t.added += inflow
+
+    def _looked_up(self) -> None:
+        """Behind a lookup that ``_ensure_rooms`` found close to a table's limit: starts the sample the next call uses."""
+        if self._sample_next:
+            self._sample_next = False
+            self.counters.start()
 
     def check(self) -> None:
         """Raises if any kernel recorded an error (synchronises)."""

@@ -1,0 +1,59 @@
+"""Growth decisions on sampled row counters (B200 only)."""
+import pytest
+import torch
+
+import kraken_b200.pytorch as kk
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# Tables that fill up call by call, alone and in a combined call, with and without housekeeping between the calls: the
+# bound never falls below the rows there are, no lookup finds a full table, and no row is lost by growing.
+@pytest.mark.parametrize("combined", [False, True])
+@pytest.mark.parametrize("end_step", [False, True])
+def test_tables_grow_before_they_are_full(combined, end_step):
+    kk.initialize("gpu", table_capacity=1 << 10)
+    eng = kk.native.engine()
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    kk.update_lr(1.0)
+    tids = [kk.register_sparse_table(f"t{k}", 4, torch.float32, kk.InitializerType.kConstant, {"value": "1"})
+            for k in range(3)]
+    n = 500
+    for step in range(12):
+        ids = [torch.arange(n, device=DEV) + step * n // (k + 1) for k in range(3)]
+        g = [torch.ones(n, 4, device=DEV) for _ in tids]
+        if combined:
+            kk.combine_pull_sparse_table(tids, ids)
+            kk.combine_push_sparse_table(tids, ids, g)
+        else:
+            for t, i, x in zip(tids, ids, g):
+                kk.pull_sparse_table(t, i)
+                kk.push_sparse_table(t, i, x)
+        if end_step:
+            eng.end_step()
+        for k, t in enumerate(tids):
+            table = eng.sparse[t]
+            rows = table.num_rows()
+            assert rows == n + step * n // (k + 1) and table.rows_bound() >= rows and rows < 0.9 * table.capacity
+    eng.check()
+    for k, t in enumerate(tids):
+        last = 11 * n // (k + 1)
+        ids = torch.arange(n + last, device=DEV)
+        times = torch.zeros(n + last, device=DEV)
+        for step in range(12):
+            times[step * n // (k + 1):step * n // (k + 1) + n] += 1
+        rows, found = eng.sparse[t].lookup(ids)
+        assert bool(found.bool().all()) and torch.equal(rows, (1 - times)[:, None].expand(-1, 4))
+
+
+def test_imported_rows_count_while_a_sample_is_in_flight():
+    kk.initialize("gpu", table_capacity=1 << 12)
+    eng = kk.native.engine()
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    t = kk.register_sparse_table("t", 4, torch.float32, kk.InitializerType.kConstant, {"value": "1"})
+    eng.counters.start()                      # taken before the rows arrive
+    eng.sparse[t].import_rows(torch.arange(2000, device=DEV), torch.zeros(2000, 4, device=DEV))
+    assert eng.counters.poll(wait=True) and eng.sparse[t].rows_bound() >= 2000
+    eng.counters.start()
+    assert eng.counters.poll(wait=True) and eng.sparse[t].rows_bound() == 2000

@@ -66,6 +66,25 @@ void bind_dense(py::module_& m) {
                          use_coo ? 1 : 0, spin, cur_stream());
           check_launch("dense_step");
         });
+  m.def("dense_step_dct",
+        [](const std::vector<uintptr_t>& bases, int rank, const cu::DenseLayout& lay, const torch::Tensor& ctrl,
+           int64_t n_pad, const c10::optional<torch::Tensor>& s0, const c10::optional<torch::Tensor>& s1,
+           const c10::optional<torch::Tensor>& s2, const torch::Tensor& residual, const torch::Tensor& tau, bool add,
+           const torch::Tensor& chunk_table, const torch::Tensor& table_steps, const torch::Tensor& table_active,
+           const OptimPOD& optim, const torch::Tensor& lr, float grad_scale) {
+          TORCH_CHECK(bases.size() == 1 && n_pad % cu::kDenseChunk == 0, "dense_step_dct: one GPU, n_pad a multiple of 256");
+          TORCH_CHECK(chunk_table.numel() == n_pad / cu::kDenseChunk && residual.numel() == n_pad &&
+                          tau.numel() == table_steps.numel(),
+                      "chunk_table, residual or tau has the wrong size");
+          TORCH_CHECK(ctrl.is_cuda() && ctrl.scalar_type() == torch::kInt32 && ctrl.numel() >= cu::kDenseCtrlInts,
+                      "ctrl must be an int32 CUDA tensor of at least ", cu::kDenseCtrlInts, " elements");
+          cu::dense_step_dct(sym_from(bases, rank), lay, reinterpret_cast<cu::DenseCtrl*>(ctrl.data_ptr()), n_pad,
+                             optr<float>(s0), optr<float>(s1), optr<float>(s2), residual.data_ptr<float>(),
+                             tau.data_ptr<float>(), add, chunk_table.data_ptr<int>(), table_steps.data_ptr<int>(),
+                             table_active.data_ptr<uint8_t>(), static_cast<int>(table_steps.numel()), optim,
+                             lr.data_ptr<float>(), grad_scale, cur_stream());
+          check_launch("dense_step_dct");
+        });
   m.def("dct_accumulate", [](const torch::Tensor& grad, const torch::Tensor& residual) {
     TORCH_CHECK(grad.numel() == residual.numel(), "grad and residual differ in size");
     cu::dct_accumulate(grad.data_ptr<float>(), residual.data_ptr<float>(), grad.numel(), cur_stream());

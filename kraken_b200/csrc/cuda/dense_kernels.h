@@ -42,7 +42,7 @@ constexpr int kDenseCtrlInts = static_cast<int>(sizeof(DenseCtrl) / sizeof(int))
 //   stores the new values into every rank's parameter copy.
 // chunk_table[n_pad / 256] maps a chunk to its table; table_active[t] == 0
 // leaves table t untouched; table_steps[t] is bumped for active tables.
-// use_coo != 0: gradients arrive as the (idx, val) lists written by dct_compact.
+// use_coo != 0 (between GPUs): gradients arrive as the (idx, val) lists written by dct_compact.
 // The local gradient buffer is zero again when the call's last kernel ends.
 // Between GPUs the call is a short sequence in stream order - a one-warp rendezvous ("my gradient is
 // complete" to every peer, wait for theirs), the update grid, a one-warp wait for every owner's
@@ -53,6 +53,12 @@ void dense_step(SymHost sym, DenseLayout lay, DenseCtrl* ctrl, long long n_pad, 
                 cudaStream_t stream);
 
 // ---- DCT ----
+// The step of one GPU with DCT, one pass: f = gradient + residual (`add` false: the gradient buffer holds f already);
+// entries with |f| >= tau[table] are applied, the others become the residual.
+void dense_step_dct(SymHost sym, DenseLayout lay, DenseCtrl* ctrl, long long n_pad, float* s0, float* s1, float* s2,
+                    float* residual, const float* tau, bool add, const int* chunk_table, int* table_steps,
+                    const uint8_t* table_active, int n_tables, OptimPOD optim, const float* lr, float grad_scale,
+                    cudaStream_t stream);
 // f = g + e written over g (in place); returns nothing.  Part of every DCT step.
 void dct_accumulate(float* grad, const float* residual, long long n, cudaStream_t stream);
 // k-th largest |x| over x[0..n) by 4-pass radix select on the float bits.

@@ -66,8 +66,9 @@ class DenseBucket:
         lay.add("flag_done", (world,), torch.int32)
         lay.add("coo_cnt", (world,), torch.int32)
         if self.dct:
-            lay.add("coo_idx", (self.n_pad,), torch.int32)
-            lay.add("coo_val", (self.n_pad,), torch.float32)
+            listed = self.n_pad if world > 1 else 1  # one GPU applies what it keeps where it is
+            lay.add("coo_idx", (listed,), torch.int32)
+            lay.add("coo_val", (listed,), torch.float32)
         self.arena = SymmetricArena(lay, rank, world, group)
         self.lay = C.DenseLayout()
         for name in lay.entries:
@@ -90,7 +91,7 @@ class DenseBucket:
                 self.state.append(torch.full((self.slice,), fill, dtype=torch.float32, device=device))
             else:
                 self.state.append(None)
-        self.acc = torch.zeros(self.slice, dtype=torch.float32, device=device) if self.dct else None
+        self.acc = torch.zeros(self.slice, dtype=torch.float32, device=device) if self.dct and world > 1 else None
         if self.dct:
             self.residual = torch.zeros(self.n_pad, dtype=torch.float32, device=device)
             self.tau = torch.zeros(n_tables, dtype=torch.float32, device=device)
@@ -119,8 +120,12 @@ class DenseBucket:
         """Collective.  Consumes the gradient buffer (zero afterwards) and leaves
         the updated parameters in every rank's ``param`` buffer."""
         if self.dct:
-            C.dct_accumulate(self.grad, self.residual)
-            if self.dct_step % self.life_span == 0:
+            refresh = self.dct_step % self.life_span == 0
+            self.dct_step += 1
+            if refresh or self.world > 1:
+                C.dct_accumulate(self.grad, self.residual)
+                self.launches += 1
+            if refresh:
                 for idx, tid in enumerate(self.table_ids):
                     off, numel = self.offsets[tid]
                     if numel < DCT_MIN_SIZE:
@@ -130,13 +135,18 @@ class DenseBucket:
                         raise C.KrakenError("DCT keeps no element: eta too close to 1")
                     C.dct_select_tau(self.grad[off:off + numel], k, self.hist, self.prefix, self.tau[idx:idx + 1])
                     self.launches += 9
+            if self.world == 1:
+                C.dense_step_dct(self.bases, self.rank, self.lay, self.ctrl, self.n_pad, self.state[0], self.state[1],
+                                 self.state[2], self.residual, self.tau, not refresh, self.chunk_table, self.table_steps,
+                                 self.table_active, self.optim, lr, float(grad_scale))
+                self.launches += 1
+                return
             C.dct_compact(self.bases, self.rank, self.lay, self.n_pad, self.residual, self.tau, self.chunk_table)
-            self.dct_step += 1
-            self.launches += 2
+            self.launches += 1
         C.dense_step(self.bases, self.rank, self.lay, self.ctrl, self.n_pad, self.state[0], self.state[1],
                      self.state[2], self.acc, self.chunk_table, self.table_steps, self.table_active, self.optim, lr,
                      float(grad_scale), self.dct, self.spin)
-        # between GPUs: rendezvous, (COO gather,) update, wait for the owners, zero; one GPU: (COO gather,) update
+        # between GPUs: rendezvous, (COO gather,) update, wait for the owners, zero; one GPU: update
         self.launches += (4 if self.world > 1 else 1) + (1 if self.dct else 0)
 
     def check(self) -> None:

@@ -148,3 +148,33 @@ def test_push_of_ids_that_occur_once_and_of_ids_that_repeat(dim, bags):
     # three Adagrad updates of at most 0.05 / sqrt(0.1) * |g|, their sums of up to 41 terms in another order
     assert torch.allclose(kk.pull_sparse_table(t, every.to(DEV)).cpu(), shard.pull_sparse(t, every), atol=2e-4)
     assert float(eng.channels[t].ugrad.abs().max()) == 0.0
+
+
+# The step of dense tables on one GPU with DCT, residual and threshold carried over steps and refreshed every second:
+# tables around the size below which one travels whole (256) and around a block's elements (4096).
+@pytest.mark.parametrize("optim,conf", OPTIMS)
+def test_dct_step_matches_the_cpu_compressor(optim, conf):
+    kk.initialize("gpu", emitter_type=kk.EmitterType.kDCT, life_span=2, eta=0.75)
+    kk.init_model("m", optim, conf)
+    kk.update_lr(0.05)
+    torch.manual_seed(3)
+    sizes = [1, 255, 256, 257, 4095, 4097, 9000]
+    ids = [kk.register_dense_table(f"w{n}", torch.randn(n)) for n in sizes]
+    shard = C.CpuShard(0)
+    shard.init_model("m", optim, conf)
+    states = {i: C.DctState() for i in ids}
+    for i, n, v in zip(ids, sizes, kk.combine_pull_dense_table(ids)):
+        shard.create_dense_table(i, f"w{n}", v.cpu().clone())
+    for step in range(5):
+        for i, n in zip(ids, sizes):
+            g = torch.randn(n)
+            kk.push_dense_table(i, g.to(DEV))
+            packed = C.cpu_dct_compress(g, 2, 0.75, states[i])
+            if packed is not None:
+                shard.push_dense_coo(i, packed[0], packed[1], 0.05)
+            else:
+                shard.push_dense(i, g, 0.05)
+        for i, v in zip(ids, kk.combine_pull_dense_table(ids)):
+            # the same float32 formulas element by element, compiled by two compilers
+            assert torch.allclose(v.cpu(), shard.pull_dense(i).view(-1), atol=1e-5), (step, i)
+    kk.native.engine().check()

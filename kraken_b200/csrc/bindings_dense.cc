@@ -234,4 +234,52 @@ void bind_dense(py::module_& m) {
     check_launch("cast_w_wt");
     return std::make_pair(w16, wt16);
   });
+  // All matrices in as few launches as possible, their bf16 copies (and transposes) in ONE buffer, which is returned
+  // with the views so that a caller on another stream has one tensor to record.
+  m.def("cast_weights", [](const std::vector<torch::Tensor>& ws, bool transpose) {
+    int64_t total = 0;
+    auto room = [](int64_t n) { return (n + 63) / 64 * 64; };
+    for (const auto& w : ws) {
+      TORCH_CHECK(w.is_cuda() && w.scalar_type() == torch::kFloat32 && w.dim() == 2 && w.is_contiguous(),
+                  "weights must be contiguous 2-D CUDA f32 tensors");
+      total += room(w.numel()) * (transpose ? 2 : 1);
+    }
+    std::vector<torch::Tensor> w16s, wt16s;
+    if (ws.empty()) return std::make_tuple(w16s, wt16s, torch::Tensor());
+    torch::Tensor buf = torch::empty({total}, ws[0].options().dtype(torch::kBFloat16));
+    __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(buf.data_ptr());
+    cu::CastBatch batch{};
+    int64_t at = 0;
+    for (const auto& w : ws) {
+      const int N = w.size(0), K = w.size(1);
+      w16s.push_back(buf.narrow(0, at, w.numel()).view({N, K}));
+      __nv_bfloat16* const w16 = base + at;
+      at += room(w.numel());
+      __nv_bfloat16* wt16 = nullptr;
+      if (transpose) {
+        wt16s.push_back(buf.narrow(0, at, w.numel()).view({K, N}));
+        wt16 = base + at;
+        at += room(w.numel());
+      }
+      const float* src = w.data_ptr<float>();
+      if (N % 8 != 0 || K % 8 != 0 || reinterpret_cast<uintptr_t>(src) % 16 != 0) {
+        torch::Tensor spare;
+        if (wt16 == nullptr) {
+          spare = torch::empty({w.numel()}, buf.options());
+          wt16 = reinterpret_cast<__nv_bfloat16*>(spare.data_ptr());
+        }
+        cu::cast_w_wt(src, N, K, w16, wt16, cur_stream());
+        continue;
+      }
+      const int l = batch.layers++;
+      batch.w[l] = src, batch.w16[l] = w16, batch.wt16[l] = wt16, batch.N[l] = N, batch.K[l] = K;
+      if (batch.layers == cu::CastBatch::kMax) {
+        cu::cast_weights(batch, cur_stream());
+        batch.layers = 0;
+      }
+    }
+    if (batch.layers > 0) cu::cast_weights(batch, cur_stream());
+    check_launch("cast_weights");
+    return std::make_tuple(w16s, wt16s, buf);
+  });
 }

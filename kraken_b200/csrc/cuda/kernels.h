@@ -250,6 +250,18 @@ void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2
 // bf16 copy [N, K] and bf16 transpose [K, N] of an fp32 weight matrix [N, K], one pass.
 void cast_w_wt(const float* w, int N, int K, __nv_bfloat16* w16, __nv_bfloat16* wt16, cudaStream_t stream);
 
+// The same for several matrices in one launch.  Every K and N a multiple of 8, every pointer on 16 bytes; a null wt16[l]
+// leaves that transpose out.  first[] is filled by the call.
+struct CastBatch {
+  static constexpr int kMax = 8;
+  int layers;
+  const float* w[kMax];
+  __nv_bfloat16* w16[kMax];
+  __nv_bfloat16* wt16[kMax];
+  int N[kMax], K[kMax], first[kMax];
+};
+void cast_weights(CastBatch b, cudaStream_t stream);
+
 // Linear layer with one output over bf16 rows x[M, K] (pitch ldx):
 // y[m] = x[m, :] . w + bias[0] + addend[m]   (bias and addend optional).
 void rowdot_forward(const __nv_bfloat16* x, int ldx, const float* w, const float* bias, const float* addend, int M,

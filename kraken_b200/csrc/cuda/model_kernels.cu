@@ -280,7 +280,65 @@ cast_w_wt_kernel(const float* __restrict__ w, int N, int K, __nv_bfloat16* __res
   }
 }
 
+// The same for all layers of an MLP in one launch, 64 x 64 tiles: 16-byte loads, 8-byte stores of the copy, 16-byte stores
+// of the transpose (which is left out where no backward pass will want it).  Bound by HBM: 4 bytes read, 2 or 4 written
+// per weight.  The 32 x 32 kernel above, with its 2-byte stores, takes 110 us for 784-4096-4096-4096, 48 us this
+// one, of 45 us at the copy rate.
+__global__ void __launch_bounds__(256)
+cast_weights_kernel(CastBatch b) {
+  pdl_enter();
+  constexpr int kPitch = 66;  // columns of the tile are read 8 rows apart: 33 words of pitch spread them over the banks
+  __shared__ __nv_bfloat16 tile[64 * kPitch];
+  int l = 0;
+  while (l + 1 < b.layers && static_cast<int>(blockIdx.x) >= b.first[l + 1]) ++l;
+  const int N = b.N[l], K = b.K[l];
+  const int at = blockIdx.x - b.first[l];
+  const int tiles_k = (K + 63) / 64;
+  const int n0 = at / tiles_k * 64, k0 = at % tiles_k * 64;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float4 v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int n = n0 + ty + 16 * j, k = k0 + tx * 4;
+    v[j] = n < N && k < K ? __ldcs(reinterpret_cast<const float4*>(b.w[l] + static_cast<size_t>(n) * K + k))
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int n = n0 + ty + 16 * j, k = k0 + tx * 4;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[j].x, v[j].y), hi = __floats2bfloat162_rn(v[j].z, v[j].w);
+    uint2 packed;
+    packed.x = *reinterpret_cast<const uint32_t*>(&lo);
+    packed.y = *reinterpret_cast<const uint32_t*>(&hi);
+    if (n < N && k < K) *reinterpret_cast<uint2*>(b.w16[l] + static_cast<size_t>(n) * K + k) = packed;
+    uint32_t* t = reinterpret_cast<uint32_t*>(tile + (ty + 16 * j) * kPitch + tx * 4);
+    t[0] = packed.x;
+    t[1] = packed.y;
+  }
+  if (b.wt16[l] == nullptr) return;  // the same for the whole block
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int kk = (threadIdx.x >> 3) + 32 * j, nn = (threadIdx.x & 7) * 8;
+    const int k = k0 + kk, n = n0 + nn;
+    if (k >= K || n >= N) continue;
+    __align__(16) __nv_bfloat16 col[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) col[i] = tile[(nn + i) * kPitch + kk];
+    *reinterpret_cast<uint4*>(b.wt16[l] + static_cast<size_t>(k) * N + n) = *reinterpret_cast<const uint4*>(col);
+  }
+}
+
 }  // namespace
+
+void cast_weights(CastBatch b, cudaStream_t stream) {
+  int tiles = 0;
+  for (int l = 0; l < b.layers; ++l) {
+    b.first[l] = tiles;
+    tiles += ((b.N[l] + 63) / 64) * ((b.K[l] + 63) / 64);
+  }
+  if (tiles > 0) launch_pdl(cast_weights_kernel, dim3(tiles), dim3(256), 0, stream, b);
+}
 
 void jagged_forward(const float* values, const float* weights, const int64_t* offsets, int k, int dim, bool mean,
                     float patch_value, float* out, cudaStream_t stream) {

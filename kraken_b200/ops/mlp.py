@@ -72,10 +72,16 @@ def _side_stream(device: torch.device) -> torch.cuda.Stream:
 
 
 class PreparedWeights:
-    """bf16 copies of the hidden layers' weights (both layouts), cast on the side stream."""
+    """bf16 copies of the hidden layers' weights, cast on the side stream: as they are and, for a forward pass that a
+    backward pass will follow, transposed (``wt16s`` is empty otherwise)."""
 
     def __init__(self, w16s, wt16s, event):
         self.w16s, self.wt16s, self.event = w16s, wt16s, event
+
+
+def _cast(weights: Sequence[torch.Tensor], transpose: bool):
+    counters.add()
+    return C.cast_weights([w.detach().contiguous() for w in weights], transpose)
 
 
 def prepare_weights(weights: Sequence[torch.Tensor]) -> PreparedWeights:
@@ -87,15 +93,10 @@ def prepare_weights(weights: Sequence[torch.Tensor]) -> PreparedWeights:
     main = torch.cuda.current_stream(dev)
     side = _side_stream(dev)
     side.wait_stream(main)
-    w16s, wt16s = [], []
     with torch.cuda.stream(side):
-        for w in weights[:-1]:
-            counters.add()
-            w16, wt16 = C.cast_w_wt(w.detach().contiguous())
-            w16.record_stream(main)
-            wt16.record_stream(main)
-            w16s.append(w16)
-            wt16s.append(wt16)
+        w16s, wt16s, buf = _cast(weights[:-1], torch.is_grad_enabled())
+        if buf is not None:
+            buf.record_stream(main)
         event = torch.cuda.Event()
         event.record(side)
     return PreparedWeights(w16s, wt16s, event)
@@ -134,24 +135,21 @@ def _grad_target(p: torch.Tensor) -> torch.Tensor:
 
 class _FusedMLP(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, addend, n_layers, input_grad_cols, prepared, *params):
+    def forward(ctx, x, addend, n_layers, input_grad_cols, prepared, with_grad, *params):
         ws, bs = params[:n_layers], params[n_layers:]
         dev = x.device
-        if prepared is not None:
+        if prepared is not None and (prepared.wt16s or not with_grad):
             torch.cuda.current_stream(dev).wait_event(prepared.event)
+            w16s, wts = prepared.w16s, prepared.wt16s
+        else:
+            w16s, wts, _ = _cast(ws[:-1], with_grad)
         st = gemm_status(dev)
         h = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
         acts = [h]
         M = h.shape[0]
-        wts = []
         masks = [None]  # masks[i] belongs to acts[i]; the MLP input has none
         for i in range(n_layers - 1):
-            if prepared is not None:
-                w16, wt16 = prepared.w16s[i], prepared.wt16s[i]
-            else:
-                counters.add()
-                w16, wt16 = C.cast_w_wt(ws[i].detach().contiguous())  # both layouts in one pass; wt16 is for backward
-            wts.append(wt16)
+            w16 = w16s[i]
             y = torch.empty((M, w16.shape[0]), dtype=torch.bfloat16, device=dev)
             # one bit per output (> 0): the next layer's input gradient masks with it instead of re-reading y
             mask = torch.empty(((w16.shape[0] + 15) // 16, (M + 63) // 64 * 64), dtype=torch.int16, device=dev)
@@ -264,7 +262,7 @@ class _FusedMLP(torch.autograd.Function):
         if ctx.x_needs_grad and dh is not None:
             dx = dh if ctx.x_dtype == torch.bfloat16 else dh.to(ctx.x_dtype)
         # parameter gradients were accumulated in place
-        return (dx, gout.reshape(-1) if ctx.needs_input_grad[1] else None, None, None, None) + (None,) * (2 * L)
+        return (dx, gout.reshape(-1) if ctx.needs_input_grad[1] else None, None, None, None, None) + (None,) * (2 * L)
 
 
 def fused_mlp(x: torch.Tensor, weights: List[torch.Tensor], biases: List[torch.Tensor],
@@ -279,4 +277,5 @@ def fused_mlp(x: torch.Tensor, weights: List[torch.Tensor], biases: List[torch.T
     with engine_region("mlp_fwd"):
         if addend is not None and weights[-1].shape[0] != 1:
             raise ValueError("addend needs a single-output head")
-        return _FusedMLP.apply(x, addend, len(weights), int(input_grad_cols), prepared, *weights, *biases)
+        return _FusedMLP.apply(x, addend, len(weights), int(input_grad_cols), prepared, torch.is_grad_enabled(), *weights,
+                               *biases)

@@ -1,0 +1,45 @@
+"""Weight casts and fused gradients of the MLP path (csrc/cuda/model_kernels.cu, mlp_gemm.cu) (B200 only)."""
+import pytest
+import torch
+
+from kraken_b200._native import C
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# Matrix edges around the 64 x 64 tiles, more layers than one launch takes (8), widths and addresses that only the
+# general kernel can read; the copies are roundings of the same floats, so they are equal bit for bit.
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("shapes", [[(8, 8)], [(64, 64), (72, 56), (400, 432)], [(128, 8), (8, 200)] * 5, [(10, 24), (16, 12)],
+                                    [(4096, 784)]])
+def test_cast_weights(shapes, transpose):
+    torch.manual_seed(0)
+    ws = [torch.randn(s, device=DEV) for s in shapes]
+    if len(shapes) == 1:  # an address that is not on 16 bytes
+        n, k = shapes[0]
+        ws.append(torch.randn(n * k + 1, device=DEV)[1:].view(n, k))
+    w16s, wt16s, buf = C.cast_weights(ws, transpose)
+    assert len(w16s) == len(ws) and len(wt16s) == (len(ws) if transpose else 0) and buf is not None
+    for k, w in enumerate(ws):
+        assert torch.equal(w16s[k], w.to(torch.bfloat16))
+        if transpose:
+            assert torch.equal(wt16s[k], w.t().to(torch.bfloat16))
+
+
+def test_scoring_between_training_steps_leaves_the_gradients_right():
+    from kraken_b200.models import MLP
+    torch.manual_seed(1)
+    model = MLP(64, [128, 64, 1]).to(DEV)
+    x = torch.randn(300, 64, device=DEV)
+    model(x).sum().backward()
+    want = [p.grad.clone() for p in model.parameters()]
+    for p in model.parameters():
+        p.grad = None
+    with torch.no_grad():
+        prepared = model.prepare()   # no transposes
+        model(x, prepared=prepared)
+    model(x, prepared=prepared).sum().backward()
+    for p, w in zip(model.parameters(), want):
+        # split sums added in another order
+        assert torch.allclose(p.grad, w, rtol=1e-4, atol=1e-4 * float(w.abs().max()))

@@ -1441,7 +1441,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           TORCH_CHECK(grads.numel() == static_cast<int64_t>(bag_offsets.has_value() ? k : n) * table.dim,
                       "grads has the wrong size");
           TORCH_CHECK(ugrad.dim() == 2 && ugrad.size(1) == table.dim && inv.numel() >= n && first.numel() >= n &&
-                          win.numel() >= ugrad.size(0) && multi.numel() >= ugrad.size(0) &&
+                          multi.numel() >= ugrad.size(0) &&
                           (!bag_offsets.has_value() || (bag_of.has_value() && bag_of->numel() >= ugrad.size(0))),
                       "the lookup's buffers do not fit this channel");
           cu::LocalPush p{ptr<float>(grads), ptr<int>(inv), ptr<int>(first), ptr<int>(win), optr<int64_t>(bag_offsets), k,

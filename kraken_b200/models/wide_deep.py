@@ -80,13 +80,14 @@ class MultiHotWideAndDeep(torch.nn.Module):
 
         k = bags.num_bags()
         B = k // self.num_fields
-        wide = self.wide(bags).view(B, self.num_fields).sum(1)
-        tid = self.deep.sparse_table.table_id()
         eng = native.engine()
         if hasattr(eng, "pull_sparse_pooled"):
-            bag_mean = self.field_is_mean.repeat(B)
-            pooled = _PooledLookup.apply(self.deep.sparse_table, bags.values(), bags.offsets(), bag_mean)
+            # both tables look the same ids up: one dedup serves both
+            wide, pooled = _PooledLookups.apply(self.wide.embedding.sparse_table, self.deep.sparse_table, bags.values(),
+                                                bags.offsets(), bags.weights(), self.field_is_mean.repeat(B))
+            wide = wide.view(B, self.num_fields).sum(1)
         else:
+            wide = self.wide(bags).view(B, self.num_fields).sum(1)
             emb = self.deep(bags.values())
             off = bags.offsets()
             s = native.jagged_sum_forward(emb, off, 0.0)  # plain CPU path: sum, then scale the mean fields
@@ -101,22 +102,26 @@ class MultiHotWideAndDeep(torch.nn.Module):
         return wide + self.mlp(torch.cat(parts, dim=1)).squeeze(-1) + self.bias
 
 
-class _PooledLookup(torch.autograd.Function):
-    """Fused bag lookup with a per-bag sum / mean switch (GPU engine)."""
+class _PooledLookups(torch.autograd.Function):
+    """Fused bag lookups of the wide table (sum) and of the deep table (sum / mean per bag) for the same ids (GPU
+    engine).  The second lookup reuses the first one's dedup."""
 
     @staticmethod
-    def forward(ctx, sparse_table, values, offsets, bag_mean):
+    def forward(ctx, wide_table, deep_table, values, offsets, wide_weights, bag_mean):
         from ..pytorch import native
         eng = native.engine()
-        out, ticket = eng.pull_sparse_pooled(sparse_table.table_id(), values, offsets, bag_mean=bag_mean)
-        ctx.state = (eng, sparse_table.table_id(), ticket, values)
-        return out
+        wide_id, deep_id = wide_table.table_id(), deep_table.table_id()
+        deep, deep_ticket = eng.pull_sparse_pooled(deep_id, values, offsets, bag_mean=bag_mean)
+        wide, wide_ticket = eng.pull_sparse_pooled(wide_id, values, offsets, weights=wide_weights, share_with=deep_id)
+        ctx.state = (eng, values, (wide_id, wide_ticket), (deep_id, deep_ticket))
+        return wide, deep
 
     @staticmethod
-    def backward(ctx, grad):
-        eng, tid, ticket, values = ctx.state
-        eng.push_sparse_pooled(tid, ticket, grad.contiguous(), values)
-        return None, None, None, None
+    def backward(ctx, *grads):
+        eng, values, *pulls = ctx.state
+        for (tid, ticket), g in zip(pulls, grads):
+            eng.push_sparse_pooled(tid, ticket, g.contiguous(), values)
+        return None, None, None, None, None, None
 
 
 class _CpuPool(torch.autograd.Function):

@@ -320,9 +320,11 @@ class Ticket:
     """Identifies one pull so that the matching push can reuse its dedup result
     and the slots the owners resolved."""
 
-    __slots__ = ("channel", "serial", "n", "bag_offsets", "weights", "mean", "bag_mean", "slots")
+    __slots__ = ("channel", "serial", "n", "bag_offsets", "weights", "mean", "bag_mean", "slots", "lookups")
 
     def __init__(self, channel, serial, n, bag_offsets, weights, mean, bag_mean, slots=None):
+        # which dedup the unique list and occurrence map are from: after a shared pull another channel's
+        self.lookups = getattr(channel.dedup_by, "lookups", 0) if hasattr(channel, "dedup_by") else 0
         self.slots = slots  # in-place pulls: table slot of every unique entry (rows are the table's value slab)
         self.channel = channel
         self.serial = serial
@@ -331,6 +333,12 @@ class Ticket:
         self.weights = weights
         self.mean = mean
         self.bag_mean = bag_mean
+
+
+    def current(self, channel) -> bool:
+        """Whether ``channel``'s buffers still hold what this pull left in them."""
+        return (self.channel is channel and self.serial == channel.serial
+                and self.lookups == getattr(getattr(channel, "dedup_by", None), "lookups", 0))
 
 
 class SparseChannel:
@@ -385,6 +393,7 @@ class SparseChannel:
             self.multi = torch.zeros(self.cap_u, dtype=torch.int32, device=dev)
             self._bag_of: Optional[torch.Tensor] = None
         self.dedup_by = self   # the channel whose dedup result off / uniq / inv are (another one after a shared pull)
+        self.lookups = 0       # dedups run into this channel's own buffers
         self.cnt = torch.zeros(world, dtype=torch.int32, device=dev)
         self._own_off = torch.zeros(world + 1, dtype=torch.int32, device=dev)
         self._own_uniq = torch.zeros(self.cap_u, dtype=torch.int64, device=dev)
@@ -417,12 +426,15 @@ class SparseChannel:
             raise C.KrakenError(f"table {self.table.name!r}: {n} ids in one call exceed the channel capacity "
                                 f"{self.cap}; raise max_ids_per_call")
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
-        share = share_from is not None and share_from.salt == self.salt and share_from.world == self.world
+        # the other channel's unique ids must fit this one's buffers
+        share = (share_from is not None and share_from.salt == self.salt and share_from.world == self.world
+                 and share_from.dedup_by.cap_u <= min(self.cap_u, self.cap_s))
         if share:
             self.off, self.uniq, self.inv = share_from.off, share_from.uniq, share_from.inv
             self.dedup_by = share_from.dedup_by
         else:
             self.dedup_by = self
+            self.lookups += 1
             self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
         if self.world == 1:
             # nobody to exchange with: the dedup's second kernel also finds the rows
@@ -430,8 +442,8 @@ class SparseChannel:
                 C.local_probe(self.uniq, self.off, n, tbl, self.slot_cache, insert, ctrl)
                 self.launches += 1
             else:
-                C.local_lookup(ids, self.lset, self.slot_of, self.pos, self.win, self.lbits, self.cnt, self.off, self.uniq, self.inv,
-                               self.cap_u, tbl, self.slot_cache, insert, ctrl)
+                C.local_lookup(ids, self.lset, self.slot_of, self.pos, self.win, self.lbits, self.cnt, self.off,
+                               self.uniq, self.inv, self.cap_u, tbl, self.slot_cache, insert, ctrl)
                 self.launches += 2
             self.serial += 1
             self.last_n = n
@@ -488,7 +500,7 @@ class SparseChannel:
     def push_accumulated(self, lr: torch.Tensor, ticket: Ticket) -> None:
         """Push for gradients that a fused kernel has already summed per unique id into
         ``self.ugrad`` (the pull's ticket must still be current)."""
-        if ticket.channel is not self or ticket.serial != self.serial:
+        if not ticket.current(self):
             raise C.KrakenError("push_accumulated needs the ticket of this channel's latest pull")
         self._apply_accumulated(lr, ticket.n)
         self.serial += 1
@@ -507,15 +519,17 @@ class SparseChannel:
     # ------------------------------------------------------------------ pull
     def pull(self, ids: torch.Tensor, bag_offsets: Optional[torch.Tensor] = None,
              weights: Optional[torch.Tensor] = None, mean: bool = False, bag_mean: Optional[torch.Tensor] = None,
-             patch_value: float = 0.0, out: Optional[torch.Tensor] = None):
+             patch_value: float = 0.0, out: Optional[torch.Tensor] = None,
+             share_from: Optional["SparseChannel"] = None):
         """Looks up (inserting unseen ids) and returns (rows, ticket).
 
         Without ``bag_offsets`` rows is [n, dim], one per id.  With ``bag_offsets``
         ([k + 1], int64) rows is [k, dim]: each bag's rows pooled by sum, or mean
         where ``mean`` / ``bag_mean[b]`` says so; empty bags give ``patch_value``.
+        ``share_from``: a channel that has just looked up the same ids (see ``_lookup_phase``).
         """
         ids = ids.reshape(-1)
-        n = self._lookup_phase(ids, insert=True)
+        n = self._lookup_phase(ids, insert=True, share_from=share_from)
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
         dim = self.table.dim
         rows = (int(bag_offsets.numel()) - 1) if bag_offsets is not None else n
@@ -540,7 +554,7 @@ class SparseChannel:
         the optimizer there.  With the ticket of the latest pull of this channel
         the dedup result and the owners' slots are reused; otherwise ``ids`` are
         looked up again (an id the table does not hold is kSparseIdNotExist)."""
-        if ticket is not None and ticket.channel is self and ticket.serial == self.serial:
+        if ticket is not None and ticket.current(self):
             n = ticket.n
             bag_offsets, weights, mean, bag_mean = ticket.bag_offsets, ticket.weights, ticket.mean, ticket.bag_mean
         else:

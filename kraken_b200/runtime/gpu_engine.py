@@ -514,8 +514,10 @@ class GpuEngine(Engine):
 
     def pull_sparse_pooled(self, table_id: int, values: torch.Tensor, offsets: torch.Tensor,
                            weights: Optional[torch.Tensor] = None, mean: bool = False,
-                           bag_mean: Optional[torch.Tensor] = None, patch_value: float = 0.0):
-        """EmbeddingBag in one fused pull: returns (pooled [k, dim], ticket)."""
+                           bag_mean: Optional[torch.Tensor] = None, patch_value: float = 0.0,
+                           share_with: Optional[int] = None):
+        """EmbeddingBag in one fused pull: returns (pooled [k, dim], ticket).  ``share_with`` names a table whose
+        channel has just pulled the same ids: its dedup result is reused."""
         self._table(table_id, "sparse")
         idx = self._prep_ids(values)
         off = offsets.detach().to(self.device, torch.int64).contiguous()
@@ -523,7 +525,8 @@ class GpuEngine(Engine):
         bm = bag_mean.detach().to(self.device, torch.uint8).contiguous() if bag_mean is not None else None
         ch = self._channel(table_id, idx.numel())
         self._ensure_room(table_id, idx.numel())
-        out = ch.pull(idx, bag_offsets=off, weights=w, mean=mean, bag_mean=bm, patch_value=patch_value)
+        share = self.channels.get(share_with) if share_with is not None else None
+        out = ch.pull(idx, bag_offsets=off, weights=w, mean=mean, bag_mean=bm, patch_value=patch_value, share_from=share)
         self._looked_up()
         return out
 

@@ -178,3 +178,35 @@ def test_dct_step_matches_the_cpu_compressor(optim, conf):
             # the same float32 formulas element by element, compiled by two compilers
             assert torch.allclose(v.cpu(), shard.pull_dense(i).view(-1), atol=1e-5), (step, i)
     kk.native.engine().check()
+
+
+# Two tables that share one dedup, with another lookup of the first between pull and push of the second: the second's
+# ticket is out of date then and its ids are resolved again.
+# A third case has the second table's buffers smaller than the first's: it runs its own dedup.
+@pytest.mark.parametrize("between", [False, True, "smaller"])
+def test_tables_that_share_a_dedup(between):
+    kk.initialize("gpu", table_capacity=1 << 12, **({} if between == "smaller" else {"max_ids_per_call": 4096}))
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    kk.update_lr(1.0)
+    a, b = (kk.register_sparse_table(n, d, torch.float32, kk.InitializerType.kConstant, {"value": "3"})
+            for n, d in (("a", 16), ("b", 1)))
+    eng = kk.native.engine()
+    if between == "smaller":
+        kk.pull_sparse_table(a, torch.arange(2000, device=DEV))
+        kk.pull_sparse_table(b, torch.arange(600, device=DEV))
+        assert eng.channels[a].cap_u > eng.channels[b].cap_u
+    ids = torch.randint(0, 50, (200,), device=DEV)
+    off = torch.arange(0, 201, 4, device=DEV)
+    pa, ta = eng.pull_sparse_pooled(a, ids, off)
+    pb, tb = eng.pull_sparse_pooled(b, ids, off, share_with=a)
+    assert torch.equal(pa, torch.full((50, 16), 12.0, device=DEV)) and torch.equal(pb, torch.full((50, 1), 12.0, device=DEV))
+    if between is True:
+        kk.pull_sparse_table(a, torch.arange(100, 400, device=DEV))
+    eng.push_sparse_pooled(b, tb, torch.ones(50, 1, device=DEV), ids)
+    eng.push_sparse_pooled(a, ta, torch.ones(50, 16, device=DEV), ids)
+    eng.check()
+    every = torch.arange(50, device=DEV)
+    count = torch.bincount(ids, minlength=50).float()[:, None]
+    for t, d in ((a, 16), (b, 1)):
+        rows, found = eng.sparse[t].lookup(every)
+        assert torch.equal(rows[found.bool()], (3 - count).expand(-1, d)[found.bool()])

@@ -172,17 +172,20 @@ void bind_dense(py::module_& m) {
     TORCH_CHECK(rc == 0, "linear_dgrad: cannot encode the TMA descriptors (pitches must be multiples of 8)");
   }, py::arg("dy"), py::arg("wt"), py::arg("h"), py::arg("dx"), py::arg("status"), py::arg("mask") = py::none());
   m.def("linear_wgrad", [bf, need_bf16](const torch::Tensor& dy, const torch::Tensor& x, const torch::Tensor& dw,
-                                        const torch::Tensor& status) {
+                                        const torch::Tensor& status, const c10::optional<torch::Tensor>& db) {
     need_bf16(dy, "dy");
     need_bf16(x, "x");
+    TORCH_CHECK(!db.has_value() || (db->is_cuda() && db->scalar_type() == torch::kFloat32 && db->is_contiguous() &&
+                                    db->numel() >= dy.size(1)),
+                "db too small");
     TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == torch::kFloat32 && dw.dim() == 2 && dw.stride(1) == 1,
                 "dw must be a 2-D CUDA f32 tensor");
     const int M = dy.size(0), N = dy.size(1), K = x.size(1);
     TORCH_CHECK(x.size(0) == M && dw.size(0) == N && dw.size(1) == K, "linear_wgrad: shape mismatch");
-    const int rc = cu::linear_wgrad(bf(dy), dy.stride(0), bf(x), x.stride(0), dw.data_ptr<float>(), dw.stride(0), M,
-                                    N, K, status.data_ptr<int>(), cur_stream());
+    const int rc = cu::linear_wgrad(bf(dy), dy.stride(0), bf(x), x.stride(0), dw.data_ptr<float>(), dw.stride(0),
+                                    db.has_value() ? db->data_ptr<float>() : nullptr, M, N, K, status.data_ptr<int>(), cur_stream());
     TORCH_CHECK(rc == 0, "linear_wgrad: cannot encode the TMA descriptors (pitches must be multiples of 8)");
-  });
+  }, py::arg("dy"), py::arg("x"), py::arg("dw"), py::arg("status"), py::arg("db") = py::none());
   m.def("gemm_set_tuning", &cu::gemm_set_tuning, py::arg("variant") = 0, py::arg("n_tiles") = 0);
   m.def("colsum_bf16", [bf, need_bf16](const torch::Tensor& dy, const torch::Tensor& db) {
     need_bf16(dy, "dy");

@@ -57,6 +57,7 @@ struct GemmArgs {
   int ldo;
   float* out32;           // [M, ldo32] f32 (EPI_RED_F32)
   int ldo32;
+  float* col_sums;        // [M] += column sums of A, or null (EPI_RED_F32 with an MN-major A: the bias gradient)
   int* status;
 };
 
@@ -246,6 +247,24 @@ __device__ __forceinline__ void epi_cols(int bn, int ew, int* c_begin, int* c_en
   }
 }
 
+// Adds one stage of an MN-major A tile (two boxes of 64 rows x 64 columns, 128-byte swizzle) to the column sums that the
+// 256 epilogue threads keep: a thread owns 8 columns of a box and 4 of its rows, 16-byte reads.
+__device__ __forceinline__ void add_stage_columns(const uint8_t* a, int t, float (&acc)[8]) {
+  const uint8_t* box = a + (t >> 7) * 8192;
+  const int chunk = t & 7, r0 = (t >> 3) & 15;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int r = r0 + 16 * j;
+    const uint4 v = *reinterpret_cast<const uint4*>(box + r * 128 + ((chunk ^ (r & 7)) << 4));
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      acc[2 * q] += __uint_as_float(w[q] << 16);
+      acc[2 * q + 1] += __uint_as_float(w[q] & 0xFFFF0000u);
+    }
+  }
+}
+
 // Bias of the tile's columns into shared memory (zeros where there is none).
 __device__ __forceinline__ void stage_bias(const GemmArgs& g, float* s_bias, int n0, int tid, int nthreads) {
   for (int j = tid; j < 256; j += nthreads) s_bias[j] = (g.bias && j < g.BN && n0 + j < g.N) ? g.bias[n0 + j] : 0.f;
@@ -278,10 +297,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint32_t tmem_cols = 32;
   while (tmem_cols < static_cast<uint32_t>(g.BN)) tmem_cols <<= 1;
 
+  // The epilogue warps are idle until the accumulator is complete: in one column of tiles they sum the columns of A as
+  // it passes through shared memory, which is the bias gradient of the layer.  A kernel of its own read all of dY again:
+  // three layers of 65536 x 400 took 125 us of the stream that the weight gradients share with the backward chain.
+  const bool sums = A_MN && EPI == EPI_RED_F32 && g.col_sums != nullptr && blockIdx.y == 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < g.stages; ++s) {
       tc::mbar_init(&full_bar[s], 1);
-      tc::mbar_init(&empty_bar[s], 1);
+      tc::mbar_init(&empty_bar[s], sums ? 1 + kEpiWarps : 1);  // the MMAs that read the stage, and the summing warps
     }
     tc::mbar_init(&acc_bar, 1);
     abort_flag = 0;
@@ -291,6 +314,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   }
   if (warp == 1) tc::tmem_alloc(&tmem_slot, tmem_cols);
   if (EPI == EPI_BIAS_ACT) stage_bias(g, s_bias, n0, threadIdx.x, blockDim.x);
+  if (EPI == EPI_RED_F32 && threadIdx.x < kBM) s_bias[threadIdx.x] = 0.f;  // the column sums meet here
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -358,6 +382,32 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     epi_cols(g.BN, warp - 2, &c_begin, &c_end);
     RowMask rm{~0ull, ~0ull};
     if (EPI == EPI_RELU_MASK) rm = load_row_mask(g, row, (n0 + c_begin) >> 4, (c_end - c_begin + 15) >> 4);
+    if (A_MN && EPI == EPI_RED_F32 && sums) {
+      const int t = threadIdx.x - 64;
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      bool fine = true;
+      for (int i = 0; i < num_kb && fine; ++i) {
+        const int s = i % g.stages;
+        fine = tc::mbar_wait(&full_bar[s], static_cast<uint32_t>(i / g.stages) & 1, kWaitLimit);
+        fine = __all_sync(0xffffffffu, fine);
+        if (!fine) break;
+        add_stage_columns(smem + static_cast<size_t>(s) * stage_bytes, t, acc);
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&empty_bar[s]);
+      }
+      if (!fine && lane == 0) atomicCAS(g.status, 0, err::kTimeout);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {  // lanes 8 apart hold other rows of the same columns
+        acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 8);
+        acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 16);
+      }
+      if (lane < 8) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) atomicAdd(&s_bias[(t >> 7) * 64 + lane * 8 + q], acc[q]);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");  // the epilogue warps only
+      if (fine && t < kBM && m0 + t < g.M) atomicAdd(g.col_sums + m0 + t, s_bias[t]);
+    }
     const bool ok = tc::mbar_wait(&acc_bar, 0, kWaitLimit);
     tc::fence_after_sync();
     if (!ok && lane == 0) atomicCAS(g.status, 0, err::kTimeout);
@@ -943,7 +993,7 @@ int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int
   return launch<false, false, EPI_RELU_MASK>(ta, tb, g, 1, stream);
 }
 
-int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int ldx, float* dW, int lddw, int M,
+int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int ldx, float* dW, int lddw, float* db, int M,
                  int N, int K, int* status, cudaStream_t stream) {
   // out dW is [N, K]; the contraction runs over the M batch rows, split across blockIdx.z
   GemmArgs g{};
@@ -958,6 +1008,7 @@ int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int 
   g.kb_per_split = (total_kb + splits - 1) / splits;
   splits = (total_kb + g.kb_per_split - 1) / g.kb_per_split;  // no empty split
   g.out32 = dW, g.ldo32 = lddw;
+  g.col_sums = db;
   g.status = status;
   CUtensorMap ta, tb;
   if ((lddw % 4) != 0 || (reinterpret_cast<uintptr_t>(dW) & 15) != 0 || !make_tmap(&ta, dY, M, N, lddy, 64, 64) ||

@@ -5,7 +5,8 @@
 //
 //   linear_forward   Y[M,N]  = act(X[M,K] * W[N,K]^T + bias)         bf16 out
 //   linear_dgrad     dX[M,K] = (dY[M,N] * Wt[K,N]^T) .* (H > 0)       bf16 out, Wt = W^T stored [K,N]
-//   linear_wgrad     dW[N,K] += dY[M,N]^T * X[M,K]                    fp32 red-add, split over M
+//   linear_wgrad     dW[N,K] += dY[M,N]^T * X[M,K]                    fp32 red-add, split over M;
+//                    db[N] += column sums of dY in the same pass (db may be null)
 //
 // All matrices are row-major with leading dimensions (in elements) that are
 // multiples of 8, so every TMA row pitch is a multiple of 16 bytes.
@@ -38,8 +39,8 @@ int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int
                  int ldh, const uint16_t* mask, int ldm, __nv_bfloat16* dX, int lddx, int M, int N, int K, int* status,
                  cudaStream_t stream);
 
-int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int ldx, float* dW, int lddw, int M,
-                 int N, int K, int* status, cudaStream_t stream);
+int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int ldx, float* dW, int lddw, float* db,
+                 int M, int N, int K, int* status, cudaStream_t stream);
 
 // Knobs for measurements.  variant: 0 = chosen from the shape, 1 = weight-resident CTA pair
 // (cta_group::2), 2 = weight-resident single CTA, 3 = one output tile per CTA.  n_tiles: column

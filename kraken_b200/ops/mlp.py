@@ -5,8 +5,8 @@ with fp32 parameters and fp32 accumulation; the last layer has no activation
 and, when it has a single output, runs as a row-dot kernel that keeps the
 logit in fp32.  The backward pass is hand-scheduled: per layer one split-K
 weight-gradient GEMM that red-adds straight into the parameter's gradient
-buffer, one column-sum for the bias and one input-gradient GEMM with the ReLU
-mask of the previous layer fused into its epilogue.
+buffer and sums the bias gradient on the way, and one input-gradient GEMM with
+the ReLU mask of the previous layer fused into its epilogue.
 """
 from __future__ import annotations
 
@@ -216,9 +216,7 @@ class _FusedMLP(torch.autograd.Function):
         else:
             dy16 = gout.to(torch.bfloat16).contiguous()
             counters.add()
-            C.linear_wgrad(dy16, h_last, _grad_target(wl), st)
-            counters.add()
-            C.colsum_bf16(dy16, _grad_target(bs[-1]))
+            C.linear_wgrad(dy16, h_last, _grad_target(wl), st, _grad_target(bs[-1]))
             dh = None
             if need_dx_last:
                 dh = torch.empty_like(h_last)
@@ -235,9 +233,8 @@ class _FusedMLP(torch.autograd.Function):
             # dh is d(loss)/d(acts[i + 1]) with layer i's ReLU mask already applied
             side.wait_stream(main)
             with torch.cuda.stream(side):
-                counters.add(2)
-                C.linear_wgrad(dh, acts[i], _grad_target(ws[i]), st)
-                C.colsum_bf16(dh, _grad_target(bs[i]))
+                counters.add()
+                C.linear_wgrad(dh, acts[i], _grad_target(ws[i]), st, _grad_target(bs[i]))
                 dh.record_stream(side)
             _notify((ws[i], bs[i]), side)
             if i > 0 or ctx.x_needs_grad:

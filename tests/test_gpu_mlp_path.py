@@ -43,3 +43,23 @@ def test_scoring_between_training_steps_leaves_the_gradients_right():
     for p, w in zip(model.parameters(), want):
         # split sums added in another order
         assert torch.allclose(p.grad, w, rtol=1e-4, atol=1e-4 * float(w.abs().max()))
+
+
+# Batches around the 64 rows of a stage and the stages of the ring, widths around the 128 columns of a tile and with
+# several column tiles of dW; the bias gradient is added to what is there and is float32 sums of bf16 values.
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (63, 128, 64), (64, 136, 256), (65, 400, 432), (257, 120, 520), (1000, 256, 64),
+                                   (40001, 400, 432)])
+def test_wgrad_sums_the_bias_gradient(m, n, k):
+    torch.manual_seed(m)
+    dy = torch.randn(m, n, device=DEV).to(torch.bfloat16)
+    x = torch.randn(m, k, device=DEV).to(torch.bfloat16)
+    dw, db = torch.zeros(n, k, device=DEV), torch.full((n,), 3.0, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    C.linear_wgrad(dy, x, dw, status, db)
+    want = dy.double().sum(0) + 3.0
+    # float32 sums of m values of magnitude 1: at most m roundings of 2^-24 of the running sum's size, ~sqrt(m)
+    assert float((db.double() - want).abs().max()) <= 1e-6 * (10 + m ** 0.5) * max(1.0, m ** 0.5 / 8)
+    ref = torch.zeros_like(dw)
+    C.linear_wgrad(dy, x, ref, status)
+    assert torch.allclose(dw, ref, rtol=1e-4, atol=1e-4 * float(ref.abs().max()))
+    assert int(status) == 0

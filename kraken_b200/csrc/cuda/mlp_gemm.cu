@@ -8,7 +8,7 @@
 //   warps 2-9          epilogue: two warps per TMEM lane quarter, each taking half of the tile's
 //                      columns; tcgen05.ld the accumulator (one row per thread) and fuse bias + ReLU
 //                      (+ a one-bit ReLU mask) in the forward pass, the ReLU mask in the input
-//                      gradient, or a split-K vector red.add into the fp32 gradient buffer.
+//                      gradient, or a split-K TMA reduce-add into the fp32 gradient buffer.
 // gemm_kernel computes one 128 x BN tile per CTA; gemm_bres_kernel and gemm_pair_kernel are
 // persistent, keep their slice of the weights in shared memory and stream activation tiles past it
 // with two TMEM accumulators (the pair variant runs tcgen05.mma.cta_group::2 on two CTAs).
@@ -39,6 +39,9 @@ constexpr int kMaxStages = 8;
 
 enum { EPI_BIAS_ACT = 0, EPI_RELU_MASK = 1, EPI_RED_F32 = 2 };
 
+// Passed as a __grid_constant__: the slow path below takes its address, and a by-value parameter was copied to each
+// thread's local memory for that, where every access of the epilogues then went (65536 x 400 x 432: 46 us a forward layer
+// so, 37 us from constant memory).
 struct GemmArgs {
   int M, N, K;            // output is M x N, contraction length K
   int BN;                 // tile width (multiple of 16; of 64 when B is MN-major)
@@ -55,8 +58,6 @@ struct GemmArgs {
   int out_v8;             // bf16 output rows and tile columns are 32-byte aligned: one 256-bit store per chunk
   __nv_bfloat16* out;     // [M, ldo] bf16  (EPI_BIAS_ACT, EPI_RELU_MASK)
   int ldo;
-  float* out32;           // [M, ldo32] f32 (EPI_RED_F32)
-  int ldo32;
   float* col_sums;        // [M] += column sums of A, or null (EPI_RED_F32 with an MN-major A: the bias gradient)
   int* status;
 };
@@ -92,10 +93,7 @@ __device__ __noinline__ void epilogue_tail(const GemmArgs& g, const float* s_bia
     if (EPI == EPI_RELU_MASK && g.mask == nullptr && g.H != nullptr &&
         !(__bfloat162float(g.H[static_cast<size_t>(row) * g.ldh + col + j]) > 0.f))
       v = 0.f;
-    if (EPI == EPI_RED_F32)
-      atomicAdd(g.out32 + static_cast<size_t>(row) * g.ldo32 + col + j, v);
-    else
-      g.out[static_cast<size_t>(row) * g.ldo + col + j] = __float2bfloat16(v);
+    g.out[static_cast<size_t>(row) * g.ldo + col + j] = __float2bfloat16(v);
   }
   if (EPI == EPI_BIAS_ACT && g.mask_out != nullptr)
     g.mask_out[static_cast<size_t>(col >> 4) * g.ldm + row] = static_cast<uint16_t>(bits_out);
@@ -124,29 +122,20 @@ __device__ __forceinline__ void epilogue_full(const GemmArgs& g, const float* s_
     for (int j = 0; j < 16; ++j)
       if (!((keep_bits >> j) & 1u)) v[j] = 0.f;
   }
-  if (EPI == EPI_RED_F32) {
-    float* o = g.out32 + static_cast<size_t>(row) * g.ldo32 + col;
-#pragma unroll
-    for (int j = 0; j < 16; j += 4)
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o + j), "f"(v[j]), "f"(v[j + 1]),
-                   "f"(v[j + 2]), "f"(v[j + 3])
-                   : "memory");
+  __nv_bfloat16* o = g.out + static_cast<size_t>(row) * g.ldo + col;
+  uint4 w0, w1;
+  w0.x = pack_bf16(v[0], v[1]);   w0.y = pack_bf16(v[2], v[3]);
+  w0.z = pack_bf16(v[4], v[5]);   w0.w = pack_bf16(v[6], v[7]);
+  w1.x = pack_bf16(v[8], v[9]);   w1.y = pack_bf16(v[10], v[11]);
+  w1.z = pack_bf16(v[12], v[13]); w1.w = pack_bf16(v[14], v[15]);
+  if (g.out_v8) {
+    // one 32-byte sector per request: the L2 write-request rate, not bytes, bounds this epilogue
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o), "r"(w0.x), "r"(w0.y), "r"(w0.z),
+                 "r"(w0.w), "r"(w1.x), "r"(w1.y), "r"(w1.z), "r"(w1.w)
+                 : "memory");
   } else {
-    __nv_bfloat16* o = g.out + static_cast<size_t>(row) * g.ldo + col;
-    uint4 w0, w1;
-    w0.x = pack_bf16(v[0], v[1]);   w0.y = pack_bf16(v[2], v[3]);
-    w0.z = pack_bf16(v[4], v[5]);   w0.w = pack_bf16(v[6], v[7]);
-    w1.x = pack_bf16(v[8], v[9]);   w1.y = pack_bf16(v[10], v[11]);
-    w1.z = pack_bf16(v[12], v[13]); w1.w = pack_bf16(v[14], v[15]);
-    if (g.out_v8) {
-      // one 32-byte sector per request: the L2 write-request rate, not bytes, bounds this epilogue
-      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o), "r"(w0.x), "r"(w0.y), "r"(w0.z),
-                   "r"(w0.w), "r"(w1.x), "r"(w1.y), "r"(w1.z), "r"(w1.w)
-                   : "memory");
-    } else {
-      *reinterpret_cast<uint4*>(o) = w0;
-      *reinterpret_cast<uint4*>(o + 8) = w1;
-    }
+    *reinterpret_cast<uint4*>(o) = w0;
+    *reinterpret_cast<uint4*>(o + 8) = w1;
   }
 }
 
@@ -233,6 +222,38 @@ __device__ __forceinline__ void epilogue_rows(const GemmArgs& g, const float* s_
   }
 }
 
+// The same for EPI_RED_F32: 32 x 32 boxes of the accumulator go through two 4 KB buffers of the warp in shared memory
+// (128-byte swizzle: a lane holds a row, and 8 lanes' 16-byte chunks fall into 8 different columns of banks) and are
+// added to dW by the TMA unit, in whole lines.  As 16-byte red.global.add from every lane's own row each warp instruction
+// touched 32 lines, half a sector each, and that, not the MMAs, set the time: the three layers 784-4096-4096-4096 at
+// batch 1024 took 173 us, 142 us so.
+__device__ __forceinline__ void epilogue_reduce(const GemmArgs& g, const CUtensorMap* tmD, uint8_t* buf, uint32_t t_row,
+                                                int row0, int n0, int c_begin, int c_end) {
+  const int lane = threadIdx.x & 31;
+  if (row0 >= g.M) return;  // the same for the whole warp
+  int turn = 0;
+  for (int c = c_begin; c < c_end && n0 + c < g.N; c += 32, ++turn) {
+    uint8_t* const b = buf + (turn & 1) * 4096;
+    uint32_t r0[16], r1[16];
+    tc::tmem_ld16(t_row + c, r0);
+    tc::tmem_ld16(t_row + c + 16, r1);
+    if (turn >= 2 && lane == 0) tc::bulk_wait_read<1>();
+    __syncwarp();
+    tc::tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      *reinterpret_cast<uint4*>(b + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+          make_uint4(r0[4 * j], r0[4 * j + 1], r0[4 * j + 2], r0[4 * j + 3]);
+      *reinterpret_cast<uint4*>(b + lane * 128 + (((j + 4) ^ (lane & 7)) << 4)) =
+          make_uint4(r1[4 * j], r1[4 * j + 1], r1[4 * j + 2], r1[4 * j + 3]);
+    }
+    tc::fence_async_shared();
+    __syncwarp();
+    if (lane == 0) tc::tma_reduce_add_2d(tmD, b, n0 + c, row0);
+  }
+  if (lane == 0) tc::bulk_wait_all();
+}
+
 // Column range of epilogue warp `ew` (0 .. kEpiWarps - 1): the tile's 16-column chunks are split
 // between the two warps that share a TMEM lane quarter.
 __device__ __forceinline__ void epi_cols(int bn, int ew, int* c_begin, int* c_end) {
@@ -272,7 +293,8 @@ __device__ __forceinline__ void stage_bias(const GemmArgs& g, float* s_bias, int
 
 template <bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(kThreads)
-gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
+gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+            const __grid_constant__ CUtensorMap tmD, const __grid_constant__ GemmArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t a_bytes = kBM * 128;
@@ -411,7 +433,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const bool ok = tc::mbar_wait(&acc_bar, 0, kWaitLimit);
     tc::fence_after_sync();
     if (!ok && lane == 0) atomicCAS(g.status, 0, err::kTimeout);
-    if (ok && abort_flag == 0 && num_kb > 0)
+    if (EPI == EPI_RED_F32) {
+      // every stage has been read by then: by the MMAs (acc_bar) and by the summing warps (their barrier)
+      if (ok && abort_flag == 0 && num_kb > 0)
+        epilogue_reduce(g, &tmD, smem + (warp - 2) * 8192, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16),
+                        m0 + quarter * 32, n0, c_begin, c_end);
+    } else if (ok && abort_flag == 0 && num_kb > 0)
       epilogue_rows<EPI>(g, s_bias, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16), row, n0, c_begin, c_end, rm);
   }
 
@@ -435,7 +462,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 // epilogue of tile j overlaps the MMAs of tile j + 1.
 template <int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_bres_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
+gemm_bres_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ GemmArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int total_kb = (g.K + kBK - 1) / kBK;
@@ -593,7 +621,8 @@ gemm_bres_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 //   release an accumulator buffer by arriving on the even CTA's barrier.
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ GemmArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int total_kb = (g.K + kBK - 1) / kBK;
@@ -806,6 +835,19 @@ bool make_tmap(CUtensorMap* m, const __nv_bfloat16* base, int rows, int cols, in
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// 2-D fp32 row-major tensor [rows, cols] with pitch ld (elements), for 32 x 32 boxes in the 128-byte swizzle.
+bool make_tmap_f32(CUtensorMap* m, float* base, int rows, int cols, int ld) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (ld % 4) != 0) return false;
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 4};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int pick_bn(int n, int granule) {
   // fewest tiles first, then the narrowest tile that still covers n with that many tiles
   const int tiles = (n + 255) / 256;
@@ -822,7 +864,7 @@ int one_wave_stages(int m, int n, int bn) {
 }
 
 template <bool A_MN, bool B_MN, int EPI>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs g, int splits, cudaStream_t stream) {
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, GemmArgs g, int splits, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(g.stages) * (kBM + g.BN) * 128 + 1024;
   static bool attr_set = false;
   if (!attr_set) {
@@ -830,7 +872,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs g, int splits,
     attr_set = true;
   }
   dim3 grid((g.M + kBM - 1) / kBM, (g.N + g.BN - 1) / g.BN, splits);
-  launch_pdl(gemm_kernel<A_MN, B_MN, EPI>, grid, dim3(kThreads), smem, stream, ta, tb, g);
+  launch_pdl(gemm_kernel<A_MN, B_MN, EPI>, grid, dim3(kThreads), smem, stream, ta, tb, td, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -963,7 +1005,7 @@ int linear_forward(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, int 
   if (pair) return launch_pair<EPI_BIAS_ACT>(ta, tb, g, stream);
   if (resident) return launch_resident<EPI_BIAS_ACT>(ta, tb, g, stream);
   g.stages = one_wave_stages(M, N, g.BN);
-  return launch<false, false, EPI_BIAS_ACT>(ta, tb, g, 1, stream);
+  return launch<false, false, EPI_BIAS_ACT>(ta, tb, ta, g, 1, stream);  // no third map is read
 }
 
 int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int ldwt, const __nv_bfloat16* H,
@@ -990,7 +1032,7 @@ int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int
   if (pair) return launch_pair<EPI_RELU_MASK>(ta, tb, g, stream);
   if (resident) return launch_resident<EPI_RELU_MASK>(ta, tb, g, stream);
   g.stages = one_wave_stages(M, K, g.BN);
-  return launch<false, false, EPI_RELU_MASK>(ta, tb, g, 1, stream);
+  return launch<false, false, EPI_RELU_MASK>(ta, tb, ta, g, 1, stream);
 }
 
 int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int ldx, float* dW, int lddw, float* db, int M,
@@ -1007,14 +1049,13 @@ int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int 
   if (splits > total_kb) splits = total_kb;
   g.kb_per_split = (total_kb + splits - 1) / splits;
   splits = (total_kb + g.kb_per_split - 1) / g.kb_per_split;  // no empty split
-  g.out32 = dW, g.ldo32 = lddw;
   g.col_sums = db;
   g.status = status;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, td;
   if ((lddw % 4) != 0 || (reinterpret_cast<uintptr_t>(dW) & 15) != 0 || !make_tmap(&ta, dY, M, N, lddy, 64, 64) ||
-      !make_tmap(&tb, X, M, K, ldx, 64, 64))
+      !make_tmap(&tb, X, M, K, ldx, 64, 64) || !make_tmap_f32(&td, dW, N, K, lddw))
     return -1;
-  return launch<true, true, EPI_RED_F32>(ta, tb, g, splits, stream);
+  return launch<true, true, EPI_RED_F32>(ta, tb, td, g, splits, stream);
 }
 
 void gemm_set_tuning(int variant, int n_tiles) {

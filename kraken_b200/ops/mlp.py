@@ -231,13 +231,11 @@ class _FusedMLP(torch.autograd.Function):
         side = _side_stream(dev)
         for i in range(L - 2, -1, -1):
             # dh is d(loss)/d(acts[i + 1]) with layer i's ReLU mask already applied
-            side.wait_stream(main)
-            with torch.cuda.stream(side):
-                counters.add()
-                C.linear_wgrad(dh, acts[i], _grad_target(ws[i]), st, _grad_target(bs[i]))
-                dh.record_stream(side)
-            _notify((ws[i], bs[i]), side)
+            ready = torch.cuda.Event()
+            ready.record(main)
+            dprev = None
             if i > 0 or ctx.x_needs_grad:
+                # the chain first: it is what the rest of the backward pass waits for
                 dprev = torch.empty_like(acts[i])
                 wt16 = ctx.wts[i]
                 counters.add()
@@ -248,9 +246,13 @@ class _FusedMLP(torch.autograd.Function):
                     C.linear_dgrad(dh, wt16[:cols], None, dprev[:, :cols], st)
                 else:
                     C.linear_dgrad(dh, wt16, None, dprev, st, ctx.masks[i])
-                dh = dprev
-            else:
-                dh = None
+            side.wait_event(ready)
+            with torch.cuda.stream(side):
+                counters.add()
+                C.linear_wgrad(dh, acts[i], _grad_target(ws[i]), st, _grad_target(bs[i]))
+                dh.record_stream(side)
+            _notify((ws[i], bs[i]), side)
+            dh = dprev
         if _deferred_join:
             _pending_join.add((dev.type, dev.index))
         else:

@@ -414,8 +414,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         fine = __all_sync(0xffffffffu, fine);
         if (!fine) break;
         add_stage_columns(smem + static_cast<size_t>(s) * stage_bytes, t, acc);
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&empty_bar[s]);
+        // The stage may be refilled once the warp has arrived, so what was read must be in registers by then: which lane
+        // arrives depends on a vote over values that all of the lanes' reads went into.  (An arrival behind a mere
+        // __syncwarp overtook reads that other kernels' memory traffic on the SM had held up.)
+        const unsigned landed = __ballot_sync(0xffffffffu, __float_as_uint(acc[0]) != 0x7FFFDEADu);
+        if (lane == (landed ? __ffs(landed) - 1 : 0)) tc::mbar_arrive(&empty_bar[s]);
       }
       if (!fine && lane == 0) atomicCAS(g.status, 0, err::kTimeout);
 #pragma unroll

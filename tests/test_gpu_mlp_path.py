@@ -63,3 +63,28 @@ def test_wgrad_sums_the_bias_gradient(m, n, k):
     C.linear_wgrad(dy, x, ref, status)
     assert torch.allclose(dw, ref, rtol=1e-4, atol=1e-4 * float(ref.abs().max()))
     assert int(status) == 0
+
+
+# The bias gradient beside a kernel that floods the SMs' memory units with reductions, as the sparse backward does: reads
+# of a stage that are held up must still be done before the stage is refilled.
+def test_bias_gradient_is_right_beside_heavy_memory_traffic():
+    torch.manual_seed(5)
+    m, n, k = 65536, 400, 432
+    dy = torch.randn(m, n, device=DEV).to(torch.bfloat16)
+    x = torch.randn(m, k, device=DEV).to(torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    want = dy.double().sum(0)
+    rows = torch.randint(0, 400_000, (1_700_000,), device=DEV)
+    grads, table = torch.randn(1_700_000, 16, device=DEV), torch.zeros(400_000, 16, device=DEV)
+    dbs = [torch.zeros(n, device=DEV) for _ in range(20)]
+    dw = torch.zeros(n, k, device=DEV)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for db in dbs:
+        with torch.cuda.stream(side):
+            C.linear_wgrad(dy, x, dw, status, db)
+        table.index_add_(0, rows, grads)
+    torch.cuda.synchronize()
+    for db in dbs:
+        # 65536 float32 additions of values of magnitude 1 in blocks: sums of ~256, roundings of 2^-24 of them
+        assert float((db.double() - want).abs().max()) < 2e-3

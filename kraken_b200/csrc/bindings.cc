@@ -288,12 +288,14 @@ struct SymHeap {
 // stream, ready() asks without waiting whether it has landed.
 struct AsyncRead {
   torch::Tensor src;
+  torch::Tensor pinned;  // from torch's cache of pinned memory: an engine's set-up and end do not pay for the pinning
   int* host = nullptr;
   cudaEvent_t event = nullptr;
 
   explicit AsyncRead(const torch::Tensor& t) : src(t) {
     need_cuda(t, "source", torch::kInt32);
-    CUDA_OK(cudaMallocHost(&host, t.numel() * sizeof(int)));
+    pinned = torch::empty({t.numel()}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
+    host = pinned.data_ptr<int>();
     CUDA_OK(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
   }
   AsyncRead(const AsyncRead&) = delete;
@@ -303,7 +305,6 @@ struct AsyncRead {
       cudaEventSynchronize(event);  // a copy in flight still writes to `host`
       cudaEventDestroy(event);
     }
-    if (host) cudaFreeHost(host);
   }
   void Start(int n) {
     TORCH_CHECK(n >= 0 && n <= src.numel(), "more values than the buffer holds");

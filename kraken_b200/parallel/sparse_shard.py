@@ -365,11 +365,13 @@ class SparseChannel:
         dim = table.dim
         dev = table.device
 
+        # one GPU has no peers that write to it: its lookups and pushes use none of the large buffers
+        inbox, recv = (self.cap_s, self.cap_u) if world > 1 else (1, 1)
         lay = Layout()
-        lay.add("inbox_ids", (world, self.cap_s), torch.int64)
+        lay.add("inbox_ids", (world, inbox), torch.int64)
         lay.add("inbox_meta", (world, 2), torch.int32)
-        lay.add("rows_recv", (self.cap_u, dim), torch.float32)
-        lay.add("inbox_grad", (world, self.cap_s, dim), torch.float32)
+        lay.add("rows_recv", (recv, dim), torch.float32)
+        lay.add("inbox_grad", (world, inbox, dim), torch.float32)
         lay.add("flag_req", (world,), torch.int32)
         lay.add("flag_rsp", (world,), torch.int32)
         lay.add("flag_push", (world,), torch.int32)
@@ -392,14 +394,14 @@ class SparseChannel:
             self.win = torch.zeros(self.cap_u, dtype=torch.int32, device=dev)
             self.multi = torch.zeros(self.cap_u, dtype=torch.int32, device=dev)
             self._bag_of: Optional[torch.Tensor] = None
-        self.dedup_by = self   # the channel whose dedup result off / uniq / inv are (another one after a shared pull)
+        self._dedup_by = None  # weak reference to the channel whose dedup off / uniq / inv are, None: this one's own
         self.lookups = 0       # dedups run into this channel's own buffers
         self.cnt = torch.zeros(world, dtype=torch.int32, device=dev)
         self._own_off = torch.zeros(world + 1, dtype=torch.int32, device=dev)
         self._own_uniq = torch.zeros(self.cap_u, dtype=torch.int64, device=dev)
         self._own_inv = torch.zeros(self.cap, dtype=torch.int32, device=dev)
         self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
-        self.rows_recv = self.arena.window("rows_recv")
+        self._rows_recv = self.arena.window("rows_recv") if world > 1 else None
         self.slot_cache = torch.full((world * self.cap_s,), -1, dtype=torch.int32, device=dev)
         self.ugrad = torch.zeros((self.cap_u, dim), dtype=torch.float32, device=dev)
         self.serial = 0
@@ -408,6 +410,18 @@ class SparseChannel:
         self.owner_world = world            # rows live on ranks 0 .. owner_world - 1 (smaller after a live reshard)
 
     # ------------------------------------------------------------------ helpers
+    @property
+    def dedup_by(self) -> "SparseChannel":
+        """The channel whose dedup result ``off`` / ``uniq`` / ``inv`` are: another one after a shared pull."""
+        return self if self._dedup_by is None else self._dedup_by()
+
+    @property
+    def rows_recv(self) -> torch.Tensor:
+        """The rows of the latest ``pull_unique``: the buffer peers write, or, on one GPU, a local one made on first use."""
+        if self._rows_recv is None:
+            self._rows_recv = torch.zeros((self.cap_u, self.table.dim), dtype=torch.float32, device=self.table.device)
+        return self._rows_recv
+
     @property
     def hkeys(self) -> torch.Tensor:
         """Scratch set of the multi-rank dedup: entries of (key, position | winner << 32); every key is free
@@ -431,9 +445,9 @@ class SparseChannel:
                  and share_from.dedup_by.cap_u <= min(self.cap_u, self.cap_s))
         if share:
             self.off, self.uniq, self.inv = share_from.off, share_from.uniq, share_from.inv
-            self.dedup_by = share_from.dedup_by
+            self._dedup_by = weakref.ref(share_from.dedup_by)
         else:
-            self.dedup_by = self
+            self._dedup_by = None
             self.lookups += 1
             self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
         if self.world == 1:

@@ -57,3 +57,27 @@ def test_imported_rows_count_while_a_sample_is_in_flight():
     assert eng.counters.poll(wait=True) and eng.sparse[t].rows_bound() >= 2000
     eng.counters.start()
     assert eng.counters.poll(wait=True) and eng.sparse[t].rows_bound() == 2000
+
+
+def test_an_engine_that_is_let_go_is_freed_at_once():
+    """Tables and exchange buffers are gigabytes: nothing may keep them until the garbage collector looks for cycles."""
+    import gc
+    import weakref
+    kk.initialize("gpu", table_capacity=1 << 12)
+    eng = kk.native.engine()
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    a, b = (kk.register_sparse_table(n, 8, torch.float32, kk.InitializerType.kConstant, {"value": "1"}) for n in "ab")
+    ids, off = torch.arange(64, device=DEV), torch.arange(0, 65, 2, device=DEV)
+    eng.pull_sparse_pooled(a, ids, off)
+    eng.pull_sparse_pooled(b, ids, off, share_with=a)
+    kk.combine_pull_sparse_table([a, b], [ids, ids])
+    eng.end_step()
+    gone = [weakref.ref(x) for x in (eng.channels[a], eng.channels[b], eng.sparse[a])]
+    gc.collect()
+    gc.disable()
+    try:
+        kk.stop()
+        del eng
+        assert [r() is None for r in gone] == [True] * 3
+    finally:
+        gc.enable()

@@ -26,11 +26,15 @@ constexpr int kDirectDim = 8;
 struct DirectSource {
   const float* grads;          // [n, dim], or [bags, dim]
   const int64_t* bag_offsets;  // null: one gradient row per occurrence
+  int nbags;
   const float* weights;        // per occurrence of a bag, or null
   const uint8_t* bag_mean;
   int mean;
   const int* win;              // unique id -> its first occurrence
-  const int* bag_of;           // unique id -> the bag of its first occurrence (null without bags)
+  // Unique id -> the bag of its first occurrence (null without bags).  Occurrences may lie outside every bag (offsets
+  // that start behind the first id or end before the last); the entry of such an id is what an earlier push left there,
+  // of ANY number of bags, and holds only if that bag is one of this push and contains the occurrence.
+  const int* bag_of;
   const uint32_t* multi;       // == *epoch: the id occurs more than once
   const uint32_t* epoch;       // number of the lookup
   __device__ __forceinline__ float bag_scale(int b) const {
@@ -54,7 +58,8 @@ struct DirectSource {
 //
 // FROM: with kFromRows and kFromBags the gradient of every id's first occurrence is read from the caller's gradients
 // (`so`); `ugrad` holds the sum of the others, which is not read where there are none.  2.3 M rows of 64 floats, Adagrad: 853 us with two
-// kernels, 590 us with one that reads and clears every sum, 500 us so, of 460 us at the copy rate.
+// kernels, 590 us with one that reads and clears every sum, 500 us so, of 460 us at the copy rate.  A first occurrence
+// outside every bag has no gradient: the row is updated with the sum of the others, or with zeros.
 constexpr int kUpdateThreads = 128;
 enum GradSource { kFromSum = 0, kFromRows = 1, kFromBags = 2 };
 
@@ -94,9 +99,13 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
     float* const gu = ugrad + static_cast<size_t>(u) * t.dim;
     const float* const gd = so.grads + static_cast<size_t>(from) * t.dim;
     float scale = 1.f, weight = 1.f;
-    if (FROM == kFromBags && mine) {
+    const bool in_grads = FROM == kFromRows || (FROM == kFromBags && from < so.nbags);
+    bool direct = in_grads;
+    if (FROM == kFromBags && mine && in_grads) {
+      const int i = so.win[u];
+      direct = so.bag_offsets[from] <= i && i < so.bag_offsets[from + 1];
       scale = so.bag_scale(from);
-      if (so.weights) weight = so.weights[so.win[u]];
+      if (so.weights) weight = so.weights[i];
     }
     const size_t row = static_cast<size_t>(slot < 0 ? 0 : slot) * t.dim;
     // an id that was not found (reported by the lookup) has no row: its gradient is dropped
@@ -106,7 +115,7 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
     float g[VEC], d[VEC], w[VEC], a0[VEC], a1[VEC], a2[VEC];
     auto load = [&](int c) {
       *reinterpret_cast<typename V::T*>(g) = many ? V::ldcg(gu + c * VEC) : V::zero();
-      if (FROM != kFromSum) *reinterpret_cast<typename V::T*>(d) = V::ldcg(gd + c * VEC);
+      if (FROM != kFromSum) *reinterpret_cast<typename V::T*>(d) = in_grads ? V::ldcg(gd + c * VEC) : V::zero();
       *reinterpret_cast<typename V::T*>(w) = V::ld(t.val + row + c * VEC);
       if (t.s[0]) *reinterpret_cast<typename V::T*>(a0) = V::ld(t.s[0] + row + c * VEC);
       if (t.s[1]) *reinterpret_cast<typename V::T*>(a1) = V::ld(t.s[1] + row + c * VEC);
@@ -122,7 +131,7 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
       const AdamBias ab = optim.type == 1 ? AdamBiasAt(optim, step) : AdamBias{1.f, 1.f};
       for (int c = c0; c < chunks; c += tpr) {
         if (c != c0) load(c);
-        if (FROM != kFromSum) {
+        if (FROM != kFromSum && direct) {
 #pragma unroll
           for (int e = 0; e < VEC; ++e) g[e] += FROM == kFromBags ? d[e] * scale * weight : d[e];
         }
@@ -608,7 +617,7 @@ void local_push(TableHost table, const LocalPush& p, float* ugrad, const int* of
     return;
   }
   DirectSource so{};
-  so.grads = p.grads, so.bag_offsets = p.bag_offsets, so.weights = p.weights, so.bag_mean = p.bag_mean;
+  so.grads = p.grads, so.bag_offsets = p.bag_offsets, so.nbags = p.nbags, so.weights = p.weights, so.bag_mean = p.bag_mean;
   so.mean = p.mean ? 1 : 0;
   so.win = p.win, so.multi = p.multi, so.epoch = &p.lookup->pull_epoch;
   so.bag_of = p.bag_of;

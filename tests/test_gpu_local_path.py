@@ -150,6 +150,40 @@ def test_push_of_ids_that_occur_once_and_of_ids_that_repeat(dim, bags):
     assert float(eng.channels[t].ugrad.abs().max()) == 0.0
 
 
+# Offsets that leave ids out in front of the first bag, behind the last, or altogether, after pushes of more bags: such an
+# occurrence has no gradient, whichever occurrence of its id the lookup found first.  Momentum moves every row that was
+# looked up, with a gradient of zero too.
+@pytest.mark.parametrize("dim", [7, 10, 64])
+@pytest.mark.parametrize("mode", ["sum", "mean", "weights"])
+def test_ids_outside_every_bag_have_no_gradient(dim, mode):
+    t, shard = make(dim, kk.OptimType.kSGD, {"momentum": "0.9"}, max_ids_per_call=4096)
+    torch.manual_seed(dim)
+    eng = kk.native.engine()
+    for head, lens, tail in [(0, [3, 2, 4] * 40, 0), (7, [2, 0, 3] * 5, 0), (0, [1, 4], 200), (300, [5], 300), (40, [], 0),
+                             (5, [0, 0], 5), (0, [3, 1] * 30, 60)]:
+        inside = sum(lens)
+        lens = torch.tensor(lens, dtype=torch.int64)
+        off = torch.cat([torch.zeros(1, dtype=torch.int64), lens.cumsum(0)]) + head
+        ids = torch.randint(0, 300, (head + inside + tail,))
+        w = torch.rand(ids.numel()) if mode == "weights" else None
+        _, ticket = eng.pull_sparse_pooled(t, ids.to(DEV), off.to(DEV), weights=w.to(DEV) if w is not None else None,
+                                           mean=mode == "mean")
+        gb = torch.randn(lens.numel(), dim)
+        eng.push_sparse_pooled(t, ticket, gb.to(DEV), ids.to(DEV))
+        g = torch.zeros(ids.numel(), dim)
+        per_bag = gb / lens.clamp(min=1)[:, None] if mode == "mean" else gb
+        g[head:head + inside] = per_bag.repeat_interleave(lens, 0)
+        if w is not None:
+            g *= w[:, None]
+        uniq, inv = C.cpu_dedup(ids)
+        shard.pull_sparse(t, uniq)
+        assert shard.push_sparse(t, uniq, C.cpu_segment_sum(g, inv, uniq.numel()), 0.05) == 0
+    eng.check()
+    every = torch.arange(300)
+    # seven updates of 0.05 times sums of ~10 values of ~1, added in another order
+    assert torch.allclose(kk.pull_sparse_table(t, every.to(DEV)).cpu(), shard.pull_sparse(t, every), atol=2e-4)
+
+
 # The step of dense tables on one GPU with DCT, residual and threshold carried over steps and refreshed every second:
 # tables around the size below which one travels whole (256) and around a block's elements (4096).
 @pytest.mark.parametrize("optim,conf", OPTIMS)

@@ -119,8 +119,9 @@ class _PooledLookups(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grads):
         eng, values, *pulls = ctx.state
-        for (tid, ticket), g in zip(pulls, grads):
-            eng.push_sparse_pooled(tid, ticket, g.contiguous(), values)
+        for trains, (tid, ticket), g in zip(ctx.needs_input_grad, pulls, grads):
+            if trains:  # a table whose parameter does not require a gradient is frozen
+                eng.push_sparse_pooled(tid, ticket, g.contiguous(), values)
         return None, None, None, None, None, None
 
 

@@ -16,6 +16,7 @@ from __future__ import annotations
 from typing import List, Sequence
 
 import torch
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import pytorch as kk
 from .mlp import MLP
@@ -80,14 +81,14 @@ class MultiHotWideAndDeep(torch.nn.Module):
 
         k = bags.num_bags()
         B = k // self.num_fields
+        wide = self.wide(bags).view(B, self.num_fields).sum(1)
         eng = native.engine()
         if hasattr(eng, "pull_sparse_pooled"):
-            # both tables look the same ids up: one dedup serves both
-            wide, pooled = _PooledLookups.apply(self.wide.embedding.sparse_table, self.deep.sparse_table, bags.values(),
-                                                bags.offsets(), bags.weights(), self.field_is_mean.repeat(B))
-            wide = wide.view(B, self.num_fields).sum(1)
+            # both tables look the same ids up: where the wide one's lookup is known to be that, its dedup serves both
+            share = self.wide.embedding.sparse_table.table_id() if self._wide_is_one_lookup(bags) else None
+            pooled = _PooledLookup.apply(self.deep.sparse_table, bags.values(), bags.offsets(), self.field_is_mean.repeat(B),
+                                         share)
         else:
-            wide = self.wide(bags).view(B, self.num_fields).sum(1)
             emb = self.deep(bags.values())
             off = bags.offsets()
             s = native.jagged_sum_forward(emb, off, 0.0)  # plain CPU path: sum, then scale the mean fields
@@ -101,28 +102,33 @@ class MultiHotWideAndDeep(torch.nn.Module):
             parts.append(torch.zeros(B, pad, dtype=pooled.dtype, device=pooled.device))
         return wide + self.mlp(torch.cat(parts, dim=1)).squeeze(-1) + self.bias
 
+    def _wide_is_one_lookup(self, bags: kk.JaggedTensor) -> bool:
+        """Whether calling ``self.wide`` on ``bags`` has been one fused lookup of exactly their ids, with nothing behind
+        it: the module as it was made, without hooks that might change the ids or look others up, on the fused path."""
+        w = self.wide
+        return (type(w) is kk.JaggedEmbedding and type(w.embedding) is kk.Embedding and "forward" not in vars(w)
+                and not w._forward_pre_hooks and not w._forward_hooks and not _has_any_global_hook()
+                and w.fused(bags))
 
-class _PooledLookups(torch.autograd.Function):
-    """Fused bag lookups of the wide table (sum) and of the deep table (sum / mean per bag) for the same ids (GPU
-    engine).  The second lookup reuses the first one's dedup."""
+
+class _PooledLookup(torch.autograd.Function):
+    """Fused bag lookup with a per-bag sum / mean switch (GPU engine).  ``share_with``: id of a table that has just looked
+    the same ids up, whose dedup is used again."""
 
     @staticmethod
-    def forward(ctx, wide_table, deep_table, values, offsets, wide_weights, bag_mean):
+    def forward(ctx, sparse_table, values, offsets, bag_mean, share_with):
         from ..pytorch import native
         eng = native.engine()
-        wide_id, deep_id = wide_table.table_id(), deep_table.table_id()
-        deep, deep_ticket = eng.pull_sparse_pooled(deep_id, values, offsets, bag_mean=bag_mean)
-        wide, wide_ticket = eng.pull_sparse_pooled(wide_id, values, offsets, weights=wide_weights, share_with=deep_id)
-        ctx.state = (eng, values, (wide_id, wide_ticket), (deep_id, deep_ticket))
-        return wide, deep
+        tid = sparse_table.table_id()
+        out, ticket = eng.pull_sparse_pooled(tid, values, offsets, bag_mean=bag_mean, share_with=share_with)
+        ctx.state = (eng, tid, ticket, values)
+        return out
 
     @staticmethod
-    def backward(ctx, *grads):
-        eng, values, *pulls = ctx.state
-        for trains, (tid, ticket), g in zip(ctx.needs_input_grad, pulls, grads):
-            if trains:  # a table whose parameter does not require a gradient is frozen
-                eng.push_sparse_pooled(tid, ticket, g.contiguous(), values)
-        return None, None, None, None, None, None
+    def backward(ctx, grad):
+        eng, tid, ticket, values = ctx.state
+        eng.push_sparse_pooled(tid, ticket, grad.contiguous(), values)
+        return None, None, None, None, None
 
 
 class _CpuPool(torch.autograd.Function):

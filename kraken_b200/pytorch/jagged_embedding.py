@@ -38,8 +38,13 @@ class JaggedEmbedding(torch.nn.Module):
         self._mode = mode
         self._patch_value = float(patch_value)
 
+    @staticmethod
+    def fused(input: JaggedTensor) -> bool:
+        """Whether ``forward`` looks ``input`` up and pools it in one fused pull."""
+        return _fused_available() and input.values().dim() == 1
+
     def forward(self, input: JaggedTensor):
-        if _fused_available() and input.values().dim() == 1:
+        if self.fused(input):
             return FusedJaggedLookupFunction.apply(self.embedding.sparse_table, input.values(), input.offsets(),
                                                    input.weights(), self._mode == "mean", self._patch_value)
         emb = self.embedding(input.values())

@@ -49,3 +49,28 @@ def test_a_frozen_table_is_not_trained(frozen):
     for name, t in tables.items():
         assert torch.equal(rows(t), before[name]) == (frozen in (name, "both")), name
     kk.native.engine().check()
+
+
+# The same steps with the shared lookup and, because of a hook that does nothing, with one lookup per table.
+def test_shared_and_separate_lookups_train_alike():
+    results = []
+    for hook in (False, True):
+        model, opt = make()
+        if hook:
+            model.wide.register_forward_hook(lambda m, i, o: None)
+        outs = []
+        for seed in range(3):
+            opt.zero_grad()
+            out = model(*batch(seed))
+            out.sum().backward()
+            opt.step()
+            outs.append(out.detach().clone())
+        eng = kk.native.engine()
+        eng.check()
+        wide, deep = (eng.channels[t.table_id()] for t in (model.wide.embedding.sparse_table, model.deep.sparse_table))
+        assert wide.lookups == 3 and deep.lookups == (3 if hook else 0)
+        results.append((torch.stack(outs), rows(model.wide.embedding.sparse_table), rows(model.deep.sparse_table)))
+        kk.stop()
+    for a, b in zip(*results):
+        # sums of a few dozen float32 values in another order, through a bf16 layer: one rounding of 2^-8 may differ
+        assert torch.allclose(a, b, rtol=2e-2, atol=2e-2 * float(b.abs().max()))

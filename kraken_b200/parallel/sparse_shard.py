@@ -316,15 +316,28 @@ class GpuSparseTable:
         return C.table_lookup(self._host, ids.to(self.device, torch.int64).contiguous())
 
 
+class Dedup:
+    """Buffers that the dedup of a channel leaves behind.  Channels that look the same ids up share the object, and keep it
+    when the channel that ran the dedup goes; it does not refer to any of them."""
+
+    __slots__ = ("cap_u", "off", "uniq", "inv", "first", "win", "ctrl", "runs")
+
+    def __init__(self, cap_u, off, uniq, inv, first, win, ctrl):
+        self.cap_u = cap_u
+        self.off, self.uniq, self.inv = off, uniq, inv
+        self.first, self.win, self.ctrl = first, win, ctrl  # what a push on one GPU wants to know of it
+        self.runs = 0  # how often the buffers have been written
+
+
 class Ticket:
     """Identifies one pull so that the matching push can reuse its dedup result
     and the slots the owners resolved."""
 
-    __slots__ = ("channel", "serial", "n", "bag_offsets", "weights", "mean", "bag_mean", "slots", "lookups")
+    __slots__ = ("channel", "serial", "n", "bag_offsets", "weights", "mean", "bag_mean", "slots", "dedup", "runs")
 
     def __init__(self, channel, serial, n, bag_offsets, weights, mean, bag_mean, slots=None):
-        # which dedup the unique list and occurrence map are from: after a shared pull another channel's
-        self.lookups = getattr(channel.dedup_by, "lookups", 0) if hasattr(channel, "dedup_by") else 0
+        self.dedup = getattr(channel, "dedup", None)  # after a shared pull it can be run again by another channel
+        self.runs = self.dedup.runs if self.dedup is not None else 0
         self.slots = slots  # in-place pulls: table slot of every unique entry (rows are the table's value slab)
         self.channel = channel
         self.serial = serial
@@ -334,11 +347,10 @@ class Ticket:
         self.mean = mean
         self.bag_mean = bag_mean
 
-
     def current(self, channel) -> bool:
         """Whether ``channel``'s buffers still hold what this pull left in them."""
         return (self.channel is channel and self.serial == channel.serial
-                and self.lookups == getattr(getattr(channel, "dedup_by", None), "lookups", 0))
+                and (self.dedup is None or self.runs == self.dedup.runs))
 
 
 class SparseChannel:
@@ -394,13 +406,12 @@ class SparseChannel:
             self.win = torch.zeros(self.cap_u, dtype=torch.int32, device=dev)
             self.multi = torch.zeros(self.cap_u, dtype=torch.int32, device=dev)
             self._bag_of: Optional[torch.Tensor] = None
-        self._dedup_by = None  # weak reference to the channel whose dedup off / uniq / inv are, None: this one's own
-        self.lookups = 0       # dedups run into this channel's own buffers
         self.cnt = torch.zeros(world, dtype=torch.int32, device=dev)
-        self._own_off = torch.zeros(world + 1, dtype=torch.int32, device=dev)
-        self._own_uniq = torch.zeros(self.cap_u, dtype=torch.int64, device=dev)
-        self._own_inv = torch.zeros(self.cap, dtype=torch.int32, device=dev)
-        self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
+        self._own = Dedup(self.cap_u, torch.zeros(world + 1, dtype=torch.int32, device=dev),
+                          torch.zeros(self.cap_u, dtype=torch.int64, device=dev),
+                          torch.zeros(self.cap, dtype=torch.int32, device=dev), self.slot_of,
+                          self.win if world == 1 else None, self.ctrl)
+        self.dedup = self._own  # after a shared pull another channel's
         self._rows_recv = self.arena.window("rows_recv") if world > 1 else None
         self.slot_cache = torch.full((world * self.cap_s,), -1, dtype=torch.int32, device=dev)
         self.ugrad = torch.zeros((self.cap_u, dim), dtype=torch.float32, device=dev)
@@ -411,9 +422,21 @@ class SparseChannel:
 
     # ------------------------------------------------------------------ helpers
     @property
-    def dedup_by(self) -> "SparseChannel":
-        """The channel whose dedup result ``off`` / ``uniq`` / ``inv`` are: another one after a shared pull."""
-        return self if self._dedup_by is None else self._dedup_by()
+    def off(self) -> torch.Tensor:
+        return self.dedup.off
+
+    @property
+    def uniq(self) -> torch.Tensor:
+        return self.dedup.uniq
+
+    @property
+    def inv(self) -> torch.Tensor:
+        return self.dedup.inv
+
+    @property
+    def lookups(self) -> int:
+        """How many dedups this channel has run (shared ones are another channel's)."""
+        return self._own.runs
 
     @property
     def rows_recv(self) -> torch.Tensor:
@@ -442,14 +465,10 @@ class SparseChannel:
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
         # the other channel's unique ids must fit this one's buffers
         share = (share_from is not None and share_from.salt == self.salt and share_from.world == self.world
-                 and share_from.dedup_by.cap_u <= min(self.cap_u, self.cap_s))
-        if share:
-            self.off, self.uniq, self.inv = share_from.off, share_from.uniq, share_from.inv
-            self._dedup_by = weakref.ref(share_from.dedup_by)
-        else:
-            self._dedup_by = None
-            self.lookups += 1
-            self.off, self.uniq, self.inv = self._own_off, self._own_uniq, self._own_inv
+                 and share_from.dedup.cap_u <= min(self.cap_u, self.cap_s))
+        self.dedup = share_from.dedup if share else self._own
+        if not share:
+            self._own.runs += 1
         if self.world == 1:
             # nobody to exchange with: the dedup's second kernel also finds the rows
             if share:
@@ -580,11 +599,11 @@ class SparseChannel:
         if grads.dtype != torch.float32 or not grads.is_contiguous():
             grads = grads.to(torch.float32).contiguous()
         if self.world == 1:
-            by = self.dedup_by
+            by = self.dedup
             if self._bag_of is None and bag_offsets is not None:
                 self._bag_of = torch.zeros(self.cap_u, dtype=torch.int32, device=self.table.device)
-            C.local_push(self.table.host(), grads, self.inv, by.slot_of, by.win, n, bag_offsets, weights, mean, bag_mean,
-                         by.ctrl, self.multi, self._bag_of, self.ugrad, self.off, self.slot_cache, self.table.optim, lr)
+            C.local_push(self.table.host(), grads, by.inv, by.first, by.win, n, bag_offsets, weights, mean, bag_mean,
+                         by.ctrl, self.multi, self._bag_of, self.ugrad, by.off, self.slot_cache, self.table.optim, lr)
             self.launches += 2  # scatter, update
         else:
             C.push_scatter(grads, self.inv, n, dim, bag_offsets, weights, mean, bag_mean, self.ugrad)

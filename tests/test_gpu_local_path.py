@@ -244,3 +244,22 @@ def test_tables_that_share_a_dedup(between):
     for t, d in ((a, 16), (b, 1)):
         rows, found = eng.sparse[t].lookup(every)
         assert torch.equal(rows[found.bool()], (3 - count).expand(-1, d)[found.bool()])
+
+
+def test_a_shared_dedup_outlives_the_channel_that_ran_it():
+    from kraken_b200.parallel.sparse_shard import GpuSparseTable, SparseChannel
+    dev = torch.device("cuda", torch.cuda.current_device())
+    lr = torch.ones(1, device=dev)
+    tables = [GpuSparseTable(k, f"t{k}", 8, kk.InitializerType.kConstant, {"value": "3"}, kk.OptimType.kSGD, {}, 0, 1 << 10, 1,
+                             dev) for k in range(2)]
+    first, second = (SparseChannel(t, 0, 1, 256) for t in tables)
+    ids = torch.tensor([5, 6, 5, 7], device=dev)
+    first.pull(ids)
+    _, ticket = second.pull(ids, share_from=first)
+    del first
+    second.push(torch.ones(4, 8, device=dev), lr, ticket=ticket)
+    _, ticket = second.pull(ids, share_from=second)
+    second.push(torch.ones(4, 8, device=dev), lr, ticket=ticket)
+    rows, found = tables[1].lookup(torch.tensor([5, 6, 7], device=dev))
+    assert bool(found.bool().all()) and torch.equal(rows[:, 0].cpu(), torch.tensor([-1.0, 1.0, 1.0]))
+    second.check()

@@ -463,9 +463,10 @@ class SparseChannel:
             raise C.KrakenError(f"table {self.table.name!r}: {n} ids in one call exceed the channel capacity "
                                 f"{self.cap}; raise max_ids_per_call")
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
-        # the other channel's unique ids must fit this one's buffers
+        # the other channel's unique ids must fit this one's buffers; the bound for one owner is looked after by the kernels
+        # behind, for shared ids as for a dedup of its own
         share = (share_from is not None and share_from.salt == self.salt and share_from.world == self.world
-                 and share_from.dedup.cap_u <= min(self.cap_u, self.cap_s))
+                 and share_from.dedup.cap_u <= self.cap_u)
         self.dedup = share_from.dedup if share else self._own
         if not share:
             self._own.runs += 1

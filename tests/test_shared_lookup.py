@@ -1,0 +1,51 @@
+"""When a channel's lookup uses another channel's dedup, on stand-ins for the kernels."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from kraken_b200.parallel import sparse_shard
+from kraken_b200.parallel.sparse_shard import Dedup, SparseChannel
+
+
+class Kernels:
+    KrakenError = RuntimeError
+
+    def __init__(self):
+        self.called = []
+
+    def __getattr__(self, name):
+        return lambda *a, **k: self.called.append(name)
+
+
+def channel(world, cap_u, cap_s, salt=0):
+    ch = object.__new__(SparseChannel)
+    own = Dedup(cap_u, *(torch.zeros(1) for _ in range(6)))
+    ch.__dict__.update(world=world, owner_world=world, cap=1000, cap_u=cap_u, cap_s=cap_s, salt=salt, spin=1, serial=0,
+                       launches=0, hbits=4, lbits=4, ctrl=torch.zeros(8), cnt=None, slot_of=None, lset=None, pos=None,
+                       win=None, slot_cache=None, lay=None, arena=SimpleNamespace(heap=None), _hkeys=torch.zeros(1),
+                       table=SimpleNamespace(name="t", host=lambda: None), _own=own, dedup=own, _wait=0)
+    return ch
+
+
+# (ranks, bounds on the unique ids of the channel that has looked up and of the one that follows, bound per owner, shared)
+@pytest.mark.parametrize("world,first,second,per_owner,shared", [
+    (1, 500, 500, 500, True), (4, 500, 500, 300, True), (4, 500, 600, 300, True), (1, 500, 500, 300, True),
+    (4, 501, 500, 500, False), (1, 501, 500, 500, False)])
+def test_bounds_that_let_a_dedup_be_shared(monkeypatch, world, first, second, per_owner, shared):
+    a, b = channel(world, first, per_owner), channel(world, second, per_owner)
+    kernels = Kernels()
+    monkeypatch.setattr(sparse_shard, "C", kernels)
+    ids = torch.arange(10)
+    a._lookup_phase(ids, True)
+    kernels.called.clear()
+    b._lookup_phase(ids, True, share_from=a)
+    ran = "local_lookup" in kernels.called or "dedup_bucketize" in kernels.called
+    assert ran == (not shared) and b.dedup is (a.dedup if shared else b._own) and b.lookups == (0 if shared else 1)
+
+
+def test_another_owner_salt_needs_a_dedup_of_its_own(monkeypatch):
+    monkeypatch.setattr(sparse_shard, "C", Kernels())
+    a, b = channel(4, 500, 500, salt=1), channel(4, 500, 500, salt=2)
+    b._lookup_phase(torch.arange(10), True, share_from=a)
+    assert b.dedup is b._own

@@ -515,13 +515,13 @@ class SparseChannel:
         occurrence -> unique map [n], ticket).  The rows belong to the channel and are
         overwritten by its next pull; a consumer kernel reads them through the map.
 
-        ``in_place`` (honoured on single-GPU jobs): no copy of the rows is made; the first result is
+        ``in_place`` (honoured on single-GPU jobs without a bound per owner of their own): no copy of the rows is made; the first result is
         the table's value slab and ``ticket.slots[u]`` is the slab row of unique entry ``u``.
         Worth it for small batches only: a consumer that visits every occurrence then reads
         scattered table rows instead of a compact buffer that fits in L2."""
         ids = ids.reshape(-1)
         n = self._lookup_phase(ids, insert=True, share_from=share_from)
-        if in_place and self.world == 1:
+        if in_place and self.world == 1 and self.cap_s >= self.cap_u:  # every unique id has an entry in slot_cache
             return self.table.val, self.inv, Ticket(self, self.serial, n, None, None, False, None, self.slot_cache)
         if self.world == 1:
             C.local_gather(self.table.host(), self.off, self.slot_cache, n, self.rows_recv)

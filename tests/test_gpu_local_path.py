@@ -112,6 +112,28 @@ def test_ids_beyond_the_unique_limit_are_reported():
     kk.native.engine().check()
 
 
+# More unique ids than the bound for one owner, which a job of one GPU can set too: reported, and no consumer is handed
+# slots that do not cover them all.
+def test_ids_beyond_the_limit_per_owner_are_reported():
+    kk.initialize("gpu", table_capacity=1 << 12, max_ids_per_call=4096, max_unique_per_call=1000, max_per_owner_per_call=100)
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    a, b = (kk.register_sparse_table(n, d, torch.float32, kk.InitializerType.kConstant, {"value": "3"})
+            for n, d in (("a", 16), ("b", 1)))
+    eng = kk.native.engine()
+    for n in (100, 101, 900):
+        ids = torch.arange(n, device=DEV)
+        for t, share, d in ((a, None, 16), (b, a, 1)):
+            rows, inv, ticket = eng.pull_sparse_unique(t, ids, share_with=share, in_place=True)
+            assert ticket.slots is None or ticket.slots.numel() >= n
+            got = rows[inv[:n].long()]
+            assert got.shape == (n, d) and int((got == 3).all(1).sum()) == min(n, 100)  # the others read as zeros
+            if n > 100:
+                with pytest.raises(kk.KrakenError):
+                    eng.channels[t].check()
+            eng.push_sparse_accumulated(t, ticket)
+        eng.check()
+
+
 # The first occurrence of an id is updated from the caller's gradients, the others from their sum; widths on both sides
 # of the line below which every gradient is summed (8), with bags (weights, mean, empty ones) and without, and further
 # pushes of the same shape in which other ids are the ones that repeat.

@@ -298,6 +298,7 @@ class GpuEngine(Engine):
         if self.nccl:
             self._ensure_room(table_id, idx.numel())
             rows = self._nccl_channel(table_id, idx.numel()).pull(idx)
+            self._looked_up()
             self._nccl_ids = {**getattr(self, "_nccl_ids", {}), table_id: (indices, *self._sig(indices), idx)}
             return rows.view(*indices.shape, info.dimension)
         ch = self._channel(table_id, idx.numel())
@@ -727,6 +728,7 @@ class GpuEngine(Engine):
         hit the probe limit and come back as kTableFull).  Decided on a host-side upper bound of the row counts.  When a
         table is within two calls of its limit, the counters of all tables are sampled in one asynchronous copy behind
         the lookup (``_looked_up``), so that a call waits for the device only if the bound passes the limit all the same."""
+        self._sample_next = False  # a call that raised before its ``_looked_up`` leaves nothing to this one
         if torch.cuda.is_current_stream_capturing():
             return
         want = []

@@ -59,6 +59,29 @@ def test_imported_rows_count_while_a_sample_is_in_flight():
     assert eng.counters.poll(wait=True) and eng.sparse[t].rows_bound() == 2000
 
 
+def test_a_refused_lookup_leaves_no_sample_for_a_captured_one():
+    """The sample's copy and event belong to the call that decided on them: in a graph they would be replayed, and the event
+    could not be asked for any more."""
+    kk.initialize("gpu", table_capacity=1 << 10)
+    eng = kk.native.engine()
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    t = kk.register_sparse_table("t", 4, torch.float32, kk.InitializerType.kConstant, {"value": "1"})
+    ids = torch.arange(500, device=DEV)
+    kk.pull_sparse_table(t, ids)
+    eng.counters.poll(wait=True)
+    with pytest.raises(kk.KrakenError, match="exceed the channel capacity"):
+        kk.pull_sparse_table(t, torch.arange(5000, device=DEV))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        rows = kk.pull_sparse_table(t, ids)
+    graph.replay()
+    assert torch.equal(rows, torch.ones(500, 4, device=DEV))
+    for _ in range(3):
+        eng.end_step()
+        torch.cuda.synchronize()
+    assert eng.sparse[t].sampled_rows == 500
+
+
 def test_an_engine_that_is_let_go_is_freed_at_once():
     """Tables and exchange buffers are gigabytes: nothing may keep them until the garbage collector looks for cycles."""
     import gc

@@ -47,6 +47,7 @@ class RowCounters:
         self.banks = []            # (int32 [BANK] device tensor, its copy to the host); tables hold one-element views
         self.tables = []
         self._marks = None         # ``added`` of every table when the sample in flight was taken
+        self.moves = 0             # how often one of the tables has been reallocated
 
     def attach(self, table) -> torch.Tensor:
         k = len(self.tables)
@@ -272,6 +273,7 @@ class GpuSparseTable:
         old = self.export()
         self.size.zero_()
         self._alloc(need_bits)
+        self.counters.moves += 1
         C.table_import(self._host, old["ids"], old["vals"],
                        *[old["states"].get(int(self.optim_info["slab_state_types"][k])) if self.slabs[k] is not None
                          else None for k in range(3)],

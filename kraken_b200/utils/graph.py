@@ -15,8 +15,9 @@ step does on the host is not part of a graph, so after every replay
 ``GraphedStep`` runs it itself: ``optimizer.host_step()`` when an optimizer was
 given (learning-rate schedule into the engine's device-side value), else the
 engine's ``end_step()`` - table growth and the kernels' error words.  When a
-table had to be reallocated the captured graphs hold stale pointers and are
-captured again before the next replay.  DCT's periodic threshold refresh is
+table had to be reallocated, there or by an eager lookup or an import between
+two replays, the captured graphs hold stale pointers and are captured again
+before the next replay.  DCT's periodic threshold refresh is
 not capturable.  Every rank of a multi-GPU job captures its own graph and
 replays in lockstep; the cross-GPU waits inside the kernels stay bounded.
 """
@@ -65,6 +66,19 @@ class GraphedStep:
             self.static_outs.append(out)
             torch.cuda.synchronize(self.device)
         self.graph, self.static_out = self.graphs[0], self.static_outs[0]
+        self._moves = self._table_moves()
+
+    @staticmethod
+    def _table_moves() -> int:
+        """How often the tables that the graphs hold pointers to have been reallocated."""
+        from ..pytorch import native
+        counters = getattr(native.engine(), "counters", None) if native.is_initialized() else None
+        return counters.moves if counters is not None else 0
+
+    def _before_replay(self) -> None:
+        if self._table_moves() != self._moves:
+            self.recaptures += 1
+            self._capture()
 
     def _after_replay(self) -> None:
         """Host-side work of a step (see the module text); rebuilds the graphs after a table grew."""
@@ -80,6 +94,7 @@ class GraphedStep:
     def __call__(self, *inputs: torch.Tensor):
         for s, t in zip(self.static_in, inputs):
             s.copy_(t, non_blocking=True)
+        self._before_replay()
         self.graph.replay()
         out = self.static_out
         self._after_replay()
@@ -91,6 +106,7 @@ class GraphedStep:
 
     def replay(self, slot: int = 0):
         """Replays the graph of ``slot`` on whatever its input buffers hold now."""
+        self._before_replay()
         self.graphs[slot].replay()
         out = self.static_outs[slot]
         self._after_replay()

@@ -119,6 +119,41 @@ def test_graphed_step_grows_tables_and_follows_the_lr_schedule():
     assert bool(found.all()) and bool((rows[:512 * 2] < 0).all())
 
 
+@pytest.mark.parametrize("by", ["lookup", "import"])
+def test_replays_follow_a_table_that_grew_between_them(by):
+    """A captured step, then an eager lookup or an import that makes the table grow, then the step again: it is captured anew
+    and works on the table that is there."""
+    from kraken_b200.utils.graph import GraphedStep
+    kk.initialize("gpu", table_capacity=1 << 10, max_ids_per_call=4096)
+    emb = kk.Embedding(4, initializer=kk.ConstantInitializer(1.0), name="g")
+    opt = kk.Optimizer("m", emb.named_parameters(), 0.5, kk.SGD())
+    eng = kk.native.engine()
+
+    def train(ids):
+        loss = emb(ids).sum()
+        loss.backward()
+        opt.step()
+        return loss.detach()
+
+    ids = torch.arange(64, device=DEV)
+    step = GraphedStep(train, (ids,), warmup=1, optimizer=opt)
+    step(ids)
+    table = eng.sparse[emb.sparse_table.table_id()]
+    capacity = table.capacity
+    if by == "lookup":
+        kk.pull_sparse_table(emb.sparse_table.table_id(), torch.arange(1000, 4000, device=DEV))
+    else:
+        table.import_rows(torch.arange(1000, 4000, device=DEV), torch.ones(3000, 4, device=DEV))
+    assert table.capacity > capacity and step.recaptures == 0
+    losses = [float(step(ids)) for _ in range(3)]
+    # 64 rows of 4 ones, less 0.5 after the warm-up step and after every replay (whose housekeeping may grow it once more)
+    assert step.recaptures >= 1 and losses == [256.0 * (1 - 0.5 * k) for k in (2, 3, 4)]
+    rows, found = table.lookup(ids)
+    assert bool(found.bool().all()) and torch.equal(rows, torch.full_like(rows, 1 - 0.5 * 5))
+    assert table.num_rows() == 64 + 3000
+    eng.check()
+
+
 def test_bf16_step_tracks_the_fp32_step_on_the_teacher_task():
     """The benchmark's fused bf16 step and the all-fp32 step, same model, same batches, 300 Adam steps:
     held-out loss and AUC must agree closely (the reference computes in fp32, kraken/t/math.cc:20-76)."""

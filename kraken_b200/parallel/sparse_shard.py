@@ -37,8 +37,9 @@ def _next_pow2_bits(n: int) -> int:
 class RowCounters:
     """Row counters of a rank's tables, side by side in device memory, so that the host learns how full ALL of them are
     with one asynchronous copy.  ``added`` of a table counts, on the host, the rows that the calls so far may have
-    created; a sample remembers it, so that ``bound(table)`` - the sampled rows plus what was added since - never lies
-    below the number of rows that the enqueued calls can lead to."""
+    created; a sample remembers it, so that the table's ``rows_bound()`` - the sampled rows plus what was added since -
+    does not lie below the number of rows that the enqueued calls can lead to.  That holds for lookups that the sample's
+    stream is ordered behind; a graph that is replayed without ``GraphedStep`` counts from the next sample on."""
 
     BANK = 256
 
@@ -48,6 +49,9 @@ class RowCounters:
         self.tables = []
         self._marks = None         # ``added`` of every table when the sample in flight was taken
         self.moves = 0             # how often one of the tables has been reallocated
+        # (table, rows) of lookups that are captured instead of run, where a GraphedStep collects them; it adds them to
+        # ``added`` with every replay
+        self.captured = None
 
     def attach(self, table) -> torch.Tensor:
         k = len(self.tables)
@@ -319,8 +323,8 @@ class GpuSparseTable:
 
 
 class Dedup:
-    """Buffers that the dedup of a channel leaves behind.  Channels that look the same ids up share the object, and keep it
-    when the channel that ran the dedup goes; it does not refer to any of them."""
+    """Buffers that the dedup of a channel leaves behind.  Channels that look the same ids up share the object, and keep
+    it when the channel that ran the dedup goes; it does not refer to any of them."""
 
     __slots__ = ("cap_u", "off", "uniq", "inv", "first", "win", "ctrl", "runs")
 

@@ -729,8 +729,6 @@ class GpuEngine(Engine):
         table is within two calls of its limit, the counters of all tables are sampled in one asynchronous copy behind
         the lookup (``_looked_up``), so that a call waits for the device only if the bound passes the limit all the same."""
         self._sample_next = False  # a call that raised before its ``_looked_up`` leaves nothing to this one
-        if torch.cuda.is_current_stream_capturing():
-            return
         want = []
         for table_id, n_ids in zip(table_ids, counts):
             t = self.sparse[table_id]
@@ -743,6 +741,10 @@ class GpuEngine(Engine):
                 n_ids = min(n_ids, ch.cap_u)
                 inflow = min(self.world * ch.cap_s, 2 * n_ids) if self.world > 1 else n_ids
             want.append((t, inflow))
+        if torch.cuda.is_current_stream_capturing():
+            if self.counters.captured is not None:  # nothing runs now, the replays count
+                self.counters.captured += want
+            return
         self._sample_next = any(t.rows_bound() + 2 * inflow > 0.6 * t.capacity for t, inflow in want)
         if self._sample_next:
             self.counters.poll()

@@ -11,18 +11,20 @@ once and replayed: ``GraphedStep`` does that.
     loss = step(dense, ids, labels)      # copies the inputs into static buffers and replays
 
 The captured function must run the same kernel sequence every step.  What a
-step does on the host is not part of a graph, so after every replay
-``GraphedStep`` runs it itself: ``optimizer.host_step()`` when an optimizer was
-given (learning-rate schedule into the engine's device-side value), else the
-engine's ``end_step()`` - table growth and the kernels' error words.  When a
-table had to be reallocated, there or by an eager lookup or an import between
-two replays, the captured graphs hold stale pointers and are captured again
-before the next replay.  DCT's periodic threshold refresh is
-not capturable.  Every rank of a multi-GPU job captures its own graph and
-replays in lockstep; the cross-GPU waits inside the kernels stay bounded.
+step does on the host is not part of a graph, so ``GraphedStep`` does it
+itself.  With every replay it counts the rows that the captured lookups may
+create, and after it come ``optimizer.host_step()`` when an optimizer was given
+(learning-rate schedule into the engine's device-side value), else the engine's
+``end_step()`` - table growth and the kernels' error words.  When a table had
+to be reallocated, there or by an eager lookup or an import between two
+replays, the captured graphs hold stale pointers and are captured again before
+the next replay.  DCT's periodic threshold refresh is not capturable.  Every
+rank of a multi-GPU job captures its own graph and replays in lockstep; the
+cross-GPU waits inside the kernels stay bounded.
 """
 from __future__ import annotations
 
+import weakref
 from typing import Callable, Sequence
 
 import torch
@@ -57,28 +59,43 @@ class GraphedStep:
 
     def _capture(self) -> None:
         torch.cuda.synchronize(self.device)
-        self.graphs, self.static_outs = [], []
+        self.graphs, self.static_outs, self._lookups = [], [], []
+        counters = self._counters()
         for k in range(self.slots):
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, pool=self.graphs[0].pool() if self.graphs else None):
-                out = self.fn(*self.static_ins[k])
+            lookups = []
+            if counters is not None:
+                counters.captured = lookups
+            try:
+                with torch.cuda.graph(g, pool=self.graphs[0].pool() if self.graphs else None):
+                    out = self.fn(*self.static_ins[k])
+            finally:
+                if counters is not None:
+                    counters.captured = None
             self.graphs.append(g)
             self.static_outs.append(out)
+            # an engine's tables may go before the step does
+            self._lookups.append([(weakref.ref(table), rows) for table, rows in lookups])
             torch.cuda.synchronize(self.device)
         self.graph, self.static_out = self.graphs[0], self.static_outs[0]
         self._moves = self._table_moves()
 
     @staticmethod
-    def _table_moves() -> int:
-        """How often the tables that the graphs hold pointers to have been reallocated."""
+    def _counters():
         from ..pytorch import native
-        counters = getattr(native.engine(), "counters", None) if native.is_initialized() else None
+        return getattr(native.engine(), "counters", None) if native.is_initialized() else None
+
+    def _table_moves(self) -> int:
+        """How often the tables that the graphs hold pointers to have been reallocated."""
+        counters = self._counters()
         return counters.moves if counters is not None else 0
 
-    def _before_replay(self) -> None:
+    def _before_replay(self, slot: int = 0) -> None:
         if self._table_moves() != self._moves:
             self.recaptures += 1
             self._capture()
+        for table, rows in self._lookups[slot]:
+            table().added += rows
 
     def _after_replay(self) -> None:
         """Host-side work of a step (see the module text); rebuilds the graphs after a table grew."""
@@ -106,7 +123,7 @@ class GraphedStep:
 
     def replay(self, slot: int = 0):
         """Replays the graph of ``slot`` on whatever its input buffers hold now."""
-        self._before_replay()
+        self._before_replay(slot)
         self.graphs[slot].replay()
         out = self.static_outs[slot]
         self._after_replay()

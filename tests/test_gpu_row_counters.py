@@ -59,6 +59,31 @@ def test_imported_rows_count_while_a_sample_is_in_flight():
     assert eng.counters.poll(wait=True) and eng.sparse[t].rows_bound() == 2000
 
 
+def test_replays_count_the_rows_they_may_create():
+    """Replays create rows that no eager call announced; a sample of the counters may be many replays old when the host runs
+    ahead, so it is held back here.  The eager lookup behind them then grows the table in time."""
+    from kraken_b200.utils.graph import GraphedStep
+    kk.initialize("gpu", table_capacity=1 << 12, max_ids_per_call=1024)
+    eng = kk.native.engine()
+    emb = kk.Embedding(4, initializer=kk.ConstantInitializer(1.0), name="t")
+    kk.Optimizer("m", emb.named_parameters(), 0.5, kk.SGD())
+    ids = torch.arange(400, device=DEV)
+    step = GraphedStep(lambda x: emb(x).sum().detach(), (ids,), warmup=1)
+    t = emb.sparse_table.table_id()
+    table = eng.sparse[t]
+    eng.counters.poll(wait=True)
+    eng.counters.start()
+    eng.counters.poll = lambda wait=False: False          # "not landed yet"
+    for k in range(1, 5):
+        step(ids + 400 * k)
+        assert table.rows_bound() >= 400 * (k + 1)
+    del eng.counters.poll
+    kk.pull_sparse_table(t, torch.arange(10_000, 11_000, device=DEV))
+    assert table.num_rows() == 400 * 5 + 1000 and table.num_rows() <= 0.6 * table.capacity and step.recaptures == 0
+    assert float(step(ids)) == 1600.0 and step.recaptures == 1
+    eng.check()
+
+
 def test_a_refused_lookup_leaves_no_sample_for_a_captured_one():
     """The sample's copy and event belong to the call that decided on them: in a graph they would be replayed, and the event
     could not be asked for any more."""

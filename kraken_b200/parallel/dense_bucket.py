@@ -121,20 +121,15 @@ class DenseBucket:
         the updated parameters in every rank's ``param`` buffer."""
         if self.dct:
             refresh = self.dct_step % self.life_span == 0
+            keep = self._dct_keep() if refresh else {}
             self.dct_step += 1
             if refresh or self.world > 1:
                 C.dct_accumulate(self.grad, self.residual)
                 self.launches += 1
-            if refresh:
-                for idx, tid in enumerate(self.table_ids):
-                    off, numel = self.offsets[tid]
-                    if numel < DCT_MIN_SIZE:
-                        continue  # tau stays 0: the table travels whole
-                    k = int(numel * (1.0 - self.eta))
-                    if k < 1:
-                        raise C.KrakenError("DCT keeps no element: eta too close to 1")
-                    C.dct_select_tau(self.grad[off:off + numel], k, self.hist, self.prefix, self.tau[idx:idx + 1])
-                    self.launches += 9
+            for idx, k in keep.items():
+                off, numel = self.offsets[self.table_ids[idx]]
+                C.dct_select_tau(self.grad[off:off + numel], k, self.hist, self.prefix, self.tau[idx:idx + 1])
+                self.launches += 9
             if self.world == 1:
                 C.dense_step_dct(self.bases, self.rank, self.lay, self.ctrl, self.n_pad, self.state[0], self.state[1],
                                  self.state[2], self.residual, self.tau, not refresh, self.chunk_table, self.table_steps,
@@ -148,6 +143,18 @@ class DenseBucket:
                      float(grad_scale), self.dct, self.spin)
         # between GPUs: rendezvous, (COO gather,) update, wait for the owners, zero; one GPU: update
         self.launches += (4 if self.world > 1 else 1) + (1 if self.dct else 0)
+
+    def _dct_keep(self) -> Dict[int, int]:
+        """How many elements of which table (by position) its new threshold lets pass; a table that is not named travels
+        whole (its tau stays 0).  Raises before the step has changed anything."""
+        keep = {}
+        for idx, tid in enumerate(self.table_ids):
+            numel = self.offsets[tid][1]
+            if numel >= DCT_MIN_SIZE:
+                keep[idx] = int(numel * (1.0 - self.eta))
+                if keep[idx] < 1:
+                    raise C.KrakenError("DCT keeps no element: eta too close to 1")
+        return keep
 
     def check(self) -> None:
         code = int(self.ctrl[3].item())

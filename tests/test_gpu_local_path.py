@@ -236,6 +236,20 @@ def test_dct_step_matches_the_cpu_compressor(optim, conf):
     kk.native.engine().check()
 
 
+def test_dct_that_keeps_nothing_is_refused_at_every_step():
+    kk.initialize("gpu", emitter_type=kk.EmitterType.kDCT, life_span=4, eta=0.999)
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    kk.update_lr(0.5)
+    t = kk.register_dense_table("w", torch.ones(300))
+    kk.push_dense_table(t, torch.ones(300, device=DEV))
+    for _ in range(3):
+        with pytest.raises(kk.KrakenError, match="keeps no element"):
+            kk.pull_dense_table(t)
+    bucket = kk.native.engine().bucket
+    assert torch.equal(bucket.param_view(t, (300,)), torch.ones(300, device=DEV))
+    assert torch.equal(bucket.grad_view(t, (300,)), torch.ones(300, device=DEV))
+
+
 # Two tables that share one dedup, with another lookup of the first between pull and push of the second: the second's
 # ticket is out of date then and its ids are resolved again.
 # A third case has the second table's buffers smaller than the first's: it runs its own dedup.

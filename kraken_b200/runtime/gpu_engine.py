@@ -393,7 +393,7 @@ class GpuEngine(Engine):
             flat = [self._prep_ids(indices[p]).reshape(-1) for p in pos]
             counts = [int(f.numel()) for f in flat]
             ch = self._group_channel(tids, sum(counts))
-            self._ensure_rooms(tids, counts)
+            self._ensure_rooms(tids, counts, [None] * len(tids))
             with self._region("pull"):
                 rows, ticket = ch.pull(torch.cat(flat), counts)
             self._looked_up()
@@ -474,7 +474,7 @@ class GpuEngine(Engine):
             bag_mean = torch.cat([torch.full((bags[k],), 1 if means[p] else 0, dtype=torch.uint8, device=self.device)
                                   for k, p in enumerate(pos)])
             ch = self._group_channel(tids, sum(counts))
-            self._ensure_rooms(tids, counts)
+            self._ensure_rooms(tids, counts, [None] * len(tids))
             with self._region("pull"):
                 rows, ticket = ch.pull(torch.cat(vals), counts, bag_offsets=torch.cat(offs).contiguous(),
                                        weights=weights, bag_mean=bag_mean, patch_value=patch)
@@ -720,19 +720,19 @@ class GpuEngine(Engine):
 
     def _ensure_room(self, table_id: int, n_ids: int) -> None:
         """``_ensure_rooms`` for one table."""
-        self._ensure_rooms((table_id,), (n_ids,))
+        self._ensure_rooms((table_id,), (n_ids,), (self.channels.get(table_id),))
 
-    def _ensure_rooms(self, table_ids: Sequence[int], counts: Sequence[int]) -> None:
+    def _ensure_rooms(self, table_ids: Sequence[int], counts: Sequence[int], channels) -> None:
         """Makes sure the shards can take the rows that a lookup of ``counts`` ids may create BEFORE its kernels run
         (growth by ``end_step`` reacts one step late: a first batch larger than the free slots would otherwise
         hit the probe limit and come back as kTableFull).  Decided on a host-side upper bound of the row counts.  When a
         table is within two calls of its limit, the counters of all tables are sampled in one asynchronous copy behind
-        the lookup (``_looked_up``), so that a call waits for the device only if the bound passes the limit all the same."""
+        the lookup (``_looked_up``), so that a call waits for the device only if the bound passes the limit all the same.
+        ``channels``: what the lookup of each table goes through, None for a combined one or one over collectives."""
         self._sample_next = False  # a call that raised before its ``_looked_up`` leaves nothing to this one
         want = []
-        for table_id, n_ids in zip(table_ids, counts):
+        for table_id, n_ids, ch in zip(table_ids, counts, channels):
             t = self.sparse[table_id]
-            ch = self.channels.get(table_id)
             inflow = n_ids * self.world  # worst case: every rank's ids of this call belong to this shard
             if ch is not None:
                 # no more than the exchange buffers admit (world x cap_s), and with a uniform owner hash about

@@ -47,6 +47,22 @@ def test_tables_grow_before_they_are_full(combined, end_step):
         assert bool(found.bool().all()) and torch.equal(rows, (1 - times)[:, None].expand(-1, 4))
 
 
+def test_a_combined_lookup_is_not_bounded_by_the_tables_own_buffers():
+    kk.initialize("gpu", table_capacity=1 << 10)
+    eng = kk.native.engine()
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    tids = [kk.register_sparse_table(f"t{k}", 4, torch.float32, kk.InitializerType.kConstant, {"value": "1"})
+            for k in range(2)]
+    for t in tids:
+        kk.pull_sparse_table(t, torch.arange(10, device=DEV))  # buffers for 1024 ids
+    ids = [torch.arange(5000, device=DEV)] * 2
+    rows = kk.combine_pull_sparse_table(tids, ids)
+    eng.check()
+    for t, r in zip(tids, rows):
+        assert torch.equal(r, torch.ones(5000, 4, device=DEV))
+        assert eng.sparse[t].num_rows() == 5000 <= eng.sparse[t].rows_bound() and eng.sparse[t].capacity > 5000 / 0.6
+
+
 def test_imported_rows_count_while_a_sample_is_in_flight():
     kk.initialize("gpu", table_capacity=1 << 12)
     eng = kk.native.engine()

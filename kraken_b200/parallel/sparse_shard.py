@@ -34,6 +34,15 @@ def _next_pow2_bits(n: int) -> int:
     return max(4, int(math.ceil(math.log2(max(2, n)))))
 
 
+def _rows_of_gradients(grads: torch.Tensor, dim: int) -> torch.Tensor:
+    """``grads`` as the kernels read them: float32 rows back to back on a 16-byte boundary.  A slice of a flat gradient
+    (what autograd hands back for one part of a concatenation) can be contiguous and start anywhere."""
+    grads = grads.reshape(-1, dim)
+    if grads.dtype != torch.float32 or not grads.is_contiguous():
+        grads = grads.to(torch.float32).contiguous()
+    return grads if grads.data_ptr() % 16 == 0 else grads.clone()
+
+
 class RowCounters:
     """Row counters of a rank's tables, side by side in device memory, so that the host learns how full ALL of them are
     with one asynchronous copy.  ``added`` of a table counts, on the host, the rows that the calls so far may have
@@ -602,9 +611,7 @@ class SparseChannel:
                 raise C.KrakenError("push without a current ticket needs the ids")
             n = self._lookup_phase(ids.reshape(-1), insert=False)
         dim = self.table.dim
-        grads = grads.reshape(-1, dim)
-        if grads.dtype != torch.float32 or not grads.is_contiguous():
-            grads = grads.to(torch.float32).contiguous()
+        grads = _rows_of_gradients(grads, dim)
         if self.world == 1:
             by = self.dedup
             if self._bag_of is None and bag_offsets is not None:
@@ -779,9 +786,7 @@ class GroupChannel:
                 raise C.KrakenError("a combined push without a current ticket needs the ids")
             n = self._lookup_phase(ids_cat.reshape(-1), counts, insert=False)
         h, lay, ctrl = self.arena.heap, self.lay, self.ctrl
-        grads = grads_cat.reshape(-1, self.dim)
-        if grads.dtype != torch.float32 or not grads.is_contiguous():
-            grads = grads.to(torch.float32).contiguous()
+        grads = _rows_of_gradients(grads_cat, self.dim)
         C.push_scatter(grads, self.inv, n, self.dim, bag_offsets, weights, False, bag_mean, self.ugrad)
         C.push_dispatch(h, lay, ctrl, self.ugrad, self.off, n, self.dim)
         C.group_push_apply(h, lay, ctrl, self.table_views, self.dim, self.slot_cache, self.ttab, self.tables[0].optim,

@@ -50,6 +50,36 @@ def test_push_updates_rows_as_the_cpu_shard(optim, conf, dim, ids):
     assert float(ch.ugrad.abs().max()) == 0.0  # zero again for the next step
 
 
+# Gradients that are a part of a flat tensor: contiguous, but on any 4-byte boundary.
+@pytest.mark.parametrize("dim", [4, 6, 64])
+@pytest.mark.parametrize("at", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("combined", [False, True])
+def test_push_of_gradients_that_start_anywhere(dim, at, combined):
+    kk.initialize("gpu", table_capacity=1 << 10)
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    kk.update_lr(1.0)
+    tids = [kk.register_sparse_table(f"e{k}", dim, torch.float32, kk.InitializerType.kConstant, {"value": "1"})
+            for k in range(2)]
+    ids = torch.arange(50, device=DEV)
+    g = torch.randn(at + 50 * dim, device=DEV)[at:].view(50, dim)
+    assert g.is_contiguous()
+    if combined:
+        kk.combine_pull_sparse_table(tids, [ids, ids])
+        eng = kk.native.engine()
+        ch, = eng.group_channels.values()
+        both = torch.randn(at + 100 * dim, device=DEV)[at:].view(100, dim)
+        ch.push(both, eng.lr_dev, ticket=eng.group_tickets.pop(tuple(tids))[0])
+        wants = both.split(50)
+    else:
+        for t in tids:
+            kk.pull_sparse_table(t, ids)
+            kk.push_sparse_table(t, ids, g)
+        wants = (g, g)
+    kk.native.engine().check()
+    for t, want in zip(tids, wants):
+        assert torch.equal(kk.pull_sparse_table(t, ids), 1 - want)
+
+
 def test_push_drops_the_gradient_of_an_unknown_id():
     t, _ = make(8, kk.OptimType.kSGD, {})
     known = torch.arange(4, device=DEV)

@@ -251,6 +251,8 @@ class _FusedMLP(torch.autograd.Function):
                 counters.add()
                 C.linear_wgrad(dh, acts[i], _grad_target(ws[i]), st, _grad_target(bs[i]))
                 dh.record_stream(side)
+                if _deferred_join:  # nobody waits for this stream before the graph lets go of the layer's input
+                    acts[i].record_stream(side)
             _notify((ws[i], bs[i]), side)
             dh = dprev
         if _deferred_join:

@@ -88,3 +88,32 @@ def test_bias_gradient_is_right_beside_heavy_memory_traffic():
     for db in dbs:
         # 65536 float32 additions of values of magnitude 1 in blocks: sums of ~256, roundings of 2^-24 of them
         assert float((db.double() - want).abs().max()) < 2e-3
+
+
+def test_inputs_of_unjoined_weight_gradients_are_not_given_away():
+    """With the join deferred the weight gradients may still wait on their stream when the backward pass has returned: the
+    memory of the activations they read must not go to the next allocation of the main stream."""
+    from kraken_b200.models import MLP
+    from kraken_b200.ops import mlp as fused
+    torch.manual_seed(1)
+    model = MLP(64, [128, 64, 1]).to(DEV)
+    for p in model.parameters():
+        p.grad = torch.zeros_like(p)
+    rows = 1 << 16
+    model(torch.randn(rows, 64, device=DEV).to(torch.bfloat16)).sum().backward()
+    torch.cuda.synchronize()
+    fused.set_deferred_join(True)
+    try:
+        x = torch.randn(rows, 64, device=DEV).to(torch.bfloat16)
+        want = x.data_ptr()
+        side = fused._side_stream(x.device)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(400_000_000)  # about 0.2 s
+        model(x).sum().backward()
+        del x
+        held = [torch.empty(rows, 64, dtype=torch.bfloat16, device=DEV) for _ in range(4)]
+        assert not side.query() and want not in [h.data_ptr() for h in held]
+        torch.cuda.current_stream().wait_stream(fused.take_pending_side_stream(held[0].device))
+    finally:
+        fused.set_deferred_join(False)
+    torch.cuda.synchronize()

@@ -284,6 +284,9 @@ struct SymHeap {
   }
 };
 
+// A channel of one rank has no inboxes and goes through the local_* calls.
+void need_peers(const SymHeap& h, const char* what) { TORCH_CHECK(h.world > 1, what, ": between GPUs only"); }
+
 // A small device buffer's contents on their way to pinned host memory: start() enqueues the copy on the current
 // stream, ready() asks without waiting whether it has landed.
 struct AsyncRead {
@@ -1303,6 +1306,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     cu::DedupScratch sc{hkeys.data_ptr(), ptr<int>(slot_of), hbits};
     if (heap != nullptr && lay != nullptr && ctrl.has_value()) {
       // with a channel: the dedup's second kernel also dispatches the unique ids to their owners
+      need_peers(*heap, "dedup_bucketize with a channel");
       cu::dedup_bucketize_dispatch(ptr<int64_t>(ids), n, world, owner_world, salt, sc, ptr<int>(cnt), ptr<int>(off),
                                    ptr<int64_t>(uniq), ptr<int>(inv), cap_u, ptr<int>(status), heap->View(), *lay,
                                    ctrl_ptr(*ctrl), cur_stream());
@@ -1316,18 +1320,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
      py::arg("ctrl") = py::none(), py::arg("owner_world") = 0);
   m.def("pull_dispatch", [](const SymHeap& h, const cu::ChanLayout& lay, const torch::Tensor& ctrl,
                             const torch::Tensor& uniq, const torch::Tensor& off, int max_n) {
+    need_peers(h, "pull_dispatch");
     cu::pull_dispatch(h.View(), lay, ctrl_ptr(ctrl), ptr<int64_t>(uniq), ptr<int>(off),
                       max_n, cur_stream());
     check_launch("pull_dispatch");
   });
   m.def("pull_probe", [](const SymHeap& h, const cu::ChanLayout& lay, const torch::Tensor& ctrl,
                          const cu::TableHost& table, const torch::Tensor& slot_cache, bool insert, uint32_t spin) {
+    need_peers(h, "pull_probe");
     cu::pull_probe(h.View(), lay, ctrl_ptr(ctrl), table, ptr<int>(slot_cache), insert,
                    spin, cur_stream());
     check_launch("pull_probe");
   });
   m.def("pull_gather", [](const SymHeap& h, const cu::ChanLayout& lay, const torch::Tensor& ctrl,
                           const cu::TableHost& table, const torch::Tensor& slot_cache) {
+    need_peers(h, "pull_gather");
     cu::pull_gather(h.View(), lay, ctrl_ptr(ctrl), table, ptr<int>(slot_cache),
                     cur_stream());
     check_launch("pull_gather");
@@ -1367,6 +1374,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                          const cu::TableHost& table, const torch::Tensor& slot_cache, const OptimPOD& optim,
                          const torch::Tensor& lr, uint32_t spin) {
     need_cuda(lr, "lr", torch::kFloat32);
+    need_peers(h, "push_apply");
     cu::push_apply(h.View(), lay, ctrl_ptr(ctrl), table, ptr<int>(slot_cache), optim,
                    ptr<float>(lr), spin, cur_stream());
     check_launch("push_apply");

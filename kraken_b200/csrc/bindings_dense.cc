@@ -226,17 +226,6 @@ void bind_dense(py::module_& m) {
                         dxp, lddx, dw.data_ptr<float>(), optr<float>(db), cur_stream());
     check_launch("rowdot_backward");
   });
-  m.def("cast_w_wt", [](const torch::Tensor& w) {
-    TORCH_CHECK(w.is_cuda() && w.scalar_type() == torch::kFloat32 && w.dim() == 2 && w.is_contiguous(),
-                "w must be a contiguous 2-D CUDA f32 tensor");
-    const int N = w.size(0), K = w.size(1);
-    torch::Tensor w16 = torch::empty({N, K}, w.options().dtype(torch::kBFloat16));
-    torch::Tensor wt16 = torch::empty({K, N}, w.options().dtype(torch::kBFloat16));
-    cu::cast_w_wt(w.data_ptr<float>(), N, K, reinterpret_cast<__nv_bfloat16*>(w16.data_ptr()),
-                  reinterpret_cast<__nv_bfloat16*>(wt16.data_ptr()), cur_stream());
-    check_launch("cast_w_wt");
-    return std::make_pair(w16, wt16);
-  });
   // All matrices in as few launches as possible, their bf16 copies (and transposes) in ONE buffer, which is returned
   // with the views so that a caller on another stream has one tensor to record.
   m.def("cast_weights", [](const std::vector<torch::Tensor>& ws, bool transpose) {

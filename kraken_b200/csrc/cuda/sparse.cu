@@ -147,9 +147,7 @@ dedup_finalize_kernel(const int64_t* __restrict__ ids, int n, int world, int own
   if (DISPATCH && blockIdx.x == 0 && threadIdx.x < world) {
     const int o = threadIdx.x;
     const int lo = min(s_off[o], cap_u), hi = min(s_off[o + 1], cap_u);
-    const int2 m = make_int2(min(hi - lo, lay.capS), lo);
-    sym.at<int2>(o, lay.inbox_meta)[sym.rank] = m;
-    if (o == sym.rank) ctrl->snap[o] = m;  // single-GPU jobs launch no request wait
+    sym.at<int2>(o, lay.inbox_meta)[sym.rank] = make_int2(min(hi - lo, lay.capS), lo);
   }
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
@@ -210,7 +208,6 @@ pull_dispatch_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, const int64_t* __restr
     int c = s_off[o + 1] - s_off[o];
     if (c > lay.capS) c = lay.capS;
     sym.at<int2>(o, lay.inbox_meta)[sym.rank] = make_int2(c, s_off[o]);
-    if (o == sym.rank) ctrl->snap[o] = make_int2(c, s_off[o]);
   }
   if (last_block_done(&ctrl->done[0])) {
     const uint32_t e = ctrl->pull_epoch + 1;
@@ -445,7 +442,7 @@ push_dispatch_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, float* ugrad, const in
   }
 }
 
-// Owner side, world > 1: several sources may have sent a row for the same
+// Owner side: several sources may have sent a row for the same
 // slot.  The first entry to claim the slot this epoch becomes its leader and
 // the others add their row into the leader's inbox row.
 template <int VEC>
@@ -521,7 +518,7 @@ push_update_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, TableView t, const int* 
       const unsigned entry = static_cast<unsigned>(s) * lay.capS + r;
       const int slot = slot_cache[entry];
       if (slot < 0) continue;
-      if (sym.world > 1 && t.lead[slot] != ((static_cast<unsigned long long>(epoch) << 32) | entry)) continue;
+      if (t.lead[slot] != ((static_cast<unsigned long long>(epoch) << 32) | entry)) continue;
       // Lane 0 of the row owns the step counter: it reads, bumps and shares it.
       int step_i = 1;
       if (t.steps) {
@@ -688,10 +685,10 @@ void push_apply(SymHost sym, ChanLayout lay, Ctrl* ctrl, TableHost table, const 
   const TableView t = to_view(table);
   launch_wait(s, lay, ctrl, kWaitPush, spin_limit, stream);
   if (g.vec == 4) {
-    if (sym.world > 1) launch_pdl(push_merge_kernel<4>, dim3(grid), dim3(kThreads), 0, stream, s, lay, ctrl, t, slot_cache, g.chunks, g.lpr);
+    launch_pdl(push_merge_kernel<4>, dim3(grid), dim3(kThreads), 0, stream, s, lay, ctrl, t, slot_cache, g.chunks, g.lpr);
     launch_update<4>(grid, stream, s, lay, ctrl, t, slot_cache, optim, lr, g.chunks, g.lpr);
   } else {
-    if (sym.world > 1) launch_pdl(push_merge_kernel<1>, dim3(grid), dim3(kThreads), 0, stream, s, lay, ctrl, t, slot_cache, g.chunks, g.lpr);
+    launch_pdl(push_merge_kernel<1>, dim3(grid), dim3(kThreads), 0, stream, s, lay, ctrl, t, slot_cache, g.chunks, g.lpr);
     launch_update<1>(grid, stream, s, lay, ctrl, t, slot_cache, optim, lr, g.chunks, g.lpr);
   }
 }

@@ -305,13 +305,6 @@ class GpuSparseTable:
         self._rows_seen = rows
         return rows + 2 * pace > max_load * self.capacity and self.reserve(int((rows + 2 * pace) * 2))
 
-    def poll_growth(self, max_load: float = 0.6) -> bool:
-        """Non-blocking load-factor check of a table by itself: looks at the row counter copied out during the
-        previous call and starts the next copy.  Call between steps."""
-        grew = self.counters.poll() and self.grow_for_pace(max_load)
-        self.counters.start()
-        return grew
-
     def evict(self, min_steps: int) -> int:
         """Drops the rows updated fewer than ``min_steps`` times by rebuilding the
         table from the survivors; returns how many rows were dropped."""

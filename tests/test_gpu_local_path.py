@@ -92,10 +92,10 @@ def test_push_drops_the_gradient_of_an_unknown_id():
     assert float(kk.native.engine().channels[t].ugrad.abs().max()) == 0.0
 
 
-# Id counts around the threads of a block (256), around the point where a thread takes four ids (two full waves of
-# blocks: 606208), and with heavy repetition; rows that exist, rows that are created, and both.
-@pytest.mark.parametrize("n,space", [(1, 1), (255, 300), (256, 256), (257, 40), (5003, 4000), (606207, 500_000),
-                                     (606208, 500_000), (700_001, 9)])
+# Id counts around the threads of a block (256), around the grid that fills the chip, from which on a launch is not made
+# early (592 blocks: 151297 ids), far above it, and with heavy repetition; rows that exist, rows that are created, and both.
+@pytest.mark.parametrize("n,space", [(1, 1), (255, 300), (256, 256), (257, 40), (5003, 4000), (151_296, 100_000),
+                                     (151_297, 100_000), (606207, 500_000), (606208, 500_000), (700_001, 9)])
 def test_lookup_numbers_every_id_once_and_finds_its_row(n, space):
     t, shard = make(4, kk.OptimType.kSGD, {}, capacity=1 << 21, max_ids_per_call=800_000)
     torch.manual_seed(n)
@@ -200,6 +200,40 @@ def test_push_of_ids_that_occur_once_and_of_ids_that_repeat(dim, bags):
     # three Adagrad updates of at most 0.05 / sqrt(0.1) * |g|, their sums of up to 41 terms in another order
     assert torch.allclose(kk.pull_sparse_table(t, every.to(DEV)).cpu(), shard.pull_sparse(t, every), atol=2e-4)
     assert float(eng.channels[t].ugrad.abs().max()) == 0.0
+
+
+# Row counts around the launch lines of the update: a row of 64 floats has 16 threads, so a block takes 8 rows; launches of
+# fewer than 1184 blocks are made early, and beyond 11840 blocks (94720 rows) a block takes further rows.  The same for the
+# segment sum with 16 rows a block: 592 and 2368 blocks (9472 and 37888 rows).
+@pytest.mark.parametrize("rows", [9464, 9465, 9473, 37889, 94720, 94721, 200_003])
+@pytest.mark.parametrize("bags", [False, True])
+def test_push_around_the_launch_lines(rows, bags):
+    n = rows + rows // 3
+    t, shard = make(64, kk.OptimType.kAdam, {"eps": "0.01"}, capacity=1 << 19, max_ids_per_call=n)
+    torch.manual_seed(rows)
+    eng = kk.native.engine()
+    ids = torch.cat([torch.arange(rows), torch.randint(0, rows, (n - rows,))])[torch.randperm(n)]
+    uniq, inv = C.cpu_dedup(ids)
+    shard.pull_sparse(t, uniq)
+    for _ in range(2):
+        if bags:
+            off = torch.cat([torch.arange(0, n, 3), torch.tensor([n])])
+            _, ticket = eng.pull_sparse_pooled(t, ids.to(DEV), off.to(DEV))
+            gb = torch.randn(off.numel() - 1, 64)
+            eng.push_sparse_pooled(t, ticket, gb.to(DEV), ids.to(DEV))
+            g = gb.repeat_interleave(off[1:] - off[:-1], 0)
+        else:
+            kk.pull_sparse_table(t, ids.to(DEV))
+            g = torch.randn(n, 64)
+            kk.push_sparse_table(t, ids.to(DEV), g.to(DEV))
+        assert shard.push_sparse(t, uniq, C.cpu_segment_sum(g, inv, uniq.numel()), 0.05) == 0
+    eng.check()
+    got, found = eng.sparse[t].lookup(uniq.to(DEV))
+    assert bool(found.bool().all())
+    want = shard.pull_sparse(t, uniq)
+    # rows of ~0.5 from a float32 Box-Muller: 1e-5; sums of up to ~6 values of ~1 in another order: 1e-6 each, of which an
+    # update passes on at most 0.05 / eps = 5 times that where a sum is near zero, and far less elsewhere
+    assert torch.allclose(got.cpu(), want, atol=2e-5)
 
 
 # Offsets that leave ids out in front of the first bag, behind the last, or altogether, after pushes of more bags: such an

@@ -1394,8 +1394,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                 "dedup outputs too small");
     TORCH_CHECK(cnt.numel() >= 1 && off.numel() >= 2, "cnt/off too small");
     c10::cuda::CUDAGuard guard(ids.device());
-    cu::local_lookup(ptr<int64_t>(ids), n, cu::LocalScratch{ptr<int>(set), ptr<int>(first), ptr<int>(pos), ptr<int>(win), hbits}, ptr<int>(cnt), ptr<int>(off), ptr<int64_t>(uniq), ptr<int>(inv), cap_u, table, ptr<int>(slot_cache),
-                     static_cast<int>(slot_cache.numel()), insert, ctrl_ptr(ctrl), cur_stream());
+    const cu::LocalScratch sc{ptr<int>(set), ptr<int>(first), ptr<int>(pos), ptr<int>(win), hbits};
+    cu::local_lookup(ptr<int64_t>(ids), n, sc, ptr<int>(cnt), ptr<int>(off), ptr<int64_t>(uniq), ptr<int>(inv), cap_u, table,
+                     ptr<int>(slot_cache), static_cast<int>(slot_cache.numel()), insert, ctrl_ptr(ctrl), cur_stream());
     check_launch("local_lookup");
   });
   m.def("local_probe", [](const torch::Tensor& uniq, const torch::Tensor& off, int max_n, const cu::TableHost& table,

@@ -183,7 +183,8 @@ void bind_dense(py::module_& m) {
     const int M = dy.size(0), N = dy.size(1), K = x.size(1);
     TORCH_CHECK(x.size(0) == M && dw.size(0) == N && dw.size(1) == K, "linear_wgrad: shape mismatch");
     const int rc = cu::linear_wgrad(bf(dy), dy.stride(0), bf(x), x.stride(0), dw.data_ptr<float>(), dw.stride(0),
-                                    db.has_value() ? db->data_ptr<float>() : nullptr, M, N, K, status.data_ptr<int>(), cur_stream());
+                                    db.has_value() ? db->data_ptr<float>() : nullptr, M, N, K, status.data_ptr<int>(),
+                                    cur_stream());
     TORCH_CHECK(rc == 0, "linear_wgrad: cannot encode the TMA descriptors (pitches must be multiples of 8)");
   }, py::arg("dy"), py::arg("x"), py::arg("dw"), py::arg("status"), py::arg("db") = py::none());
   m.def("gemm_set_tuning", &cu::gemm_set_tuning, py::arg("variant") = 0, py::arg("n_tiles") = 0);

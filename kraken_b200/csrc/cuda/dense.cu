@@ -177,7 +177,8 @@ dense_step_kernel(Sym sym, DenseLayout lay, DenseCtrl* ctrl, long long n_pad, fl
       if (kS0) a0[u] = *reinterpret_cast<const float4*>(s0 + li[u]);
       if (kS1) a1[u] = *reinterpret_cast<const float4*>(s1 + li[u]);
       if (kS2) a2[u] = *reinterpret_cast<const float4*>(s2 + li[u]);
-      if (DCT) e[u] = dct.add ? __ldcs(reinterpret_cast<const float4*>(dct.residual + li[u])) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (DCT)
+        e[u] = dct.add ? __ldcs(reinterpret_cast<const float4*>(dct.residual + li[u])) : make_float4(0.f, 0.f, 0.f, 0.f);
       if (MULTI && use_coo) {
         g[u] = *reinterpret_cast<const float4*>(acc + li[u]);
       } else if (!MULTI) {

@@ -518,7 +518,9 @@ push_update_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, TableView t, const int* 
       const unsigned entry = static_cast<unsigned>(s) * lay.capS + r;
       const int slot = slot_cache[entry];
       if (slot < 0) continue;
-      if (t.lead[slot] != ((static_cast<unsigned long long>(epoch) << 32) | entry)) continue;
+      // (with the count of ranks in the condition, as a table of one rank has no `lead`, Adam's variant fits 64 registers;
+      // without it ptxas spills 4 bytes)
+      if (sym.world > 1 && t.lead[slot] != ((static_cast<unsigned long long>(epoch) << 32) | entry)) continue;
       // Lane 0 of the row owns the step counter: it reads, bumps and shares it.
       int step_i = 1;
       if (t.steps) {

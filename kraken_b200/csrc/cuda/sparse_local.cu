@@ -53,13 +53,15 @@ struct DirectSource {
 // threads of a block, one 16-byte chunk each (a row width like 20 floats leaves no lane idle, as a power-of-two group
 // per row would); the threads of a row may sit in two warps, so its step counter is read by all of them before the
 // block barrier and written behind it.  What is known of the next row is fetched one pass ahead.  Nine blocks of 128
-// threads per SM hold 56 registers a thread without spills; eight of them were 3 to 6 % slower, four or five blocks of
-// 256 threads up to 25 %.
+// threads per SM leave 56 registers a thread, which holds every variant but Adam of 4-float chunks with direct gradients
+// (4 bytes spilled with rows, 12 with bags); eight of them were 3 to 6 % slower, four or five blocks of 256 threads up to
+// 25 %.
 //
 // FROM: with kFromRows and kFromBags the gradient of every id's first occurrence is read from the caller's gradients
-// (`so`); `ugrad` holds the sum of the others, which is not read where there are none.  2.3 M rows of 64 floats, Adagrad: 853 us with two
-// kernels, 590 us with one that reads and clears every sum, 500 us so, of 460 us at the copy rate.  A first occurrence
-// outside every bag has no gradient: the row is updated with the sum of the others, or with zeros.
+// (`so`); `ugrad` holds the sum of the others, which is not read where there are none.  2.3 M rows of 64 floats,
+// Adagrad: 853 us with two kernels, 590 us with one that reads and clears every sum, 500 us so, of 460 us at the copy
+// rate.  A first occurrence outside every bag has no gradient: the row is updated with the sum of the others, or with
+// zeros.
 constexpr int kUpdateThreads = 128;
 enum GradSource { kFromSum = 0, kFromRows = 1, kFromBags = 2 };
 
@@ -85,7 +87,7 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
   int u = blockIdx.x * rows + r;
   // what is known of a row before its data: its slot, the row of `grads`, whether there is a sum of others
   auto slot_of = [&](int v) { return active && v < limit ? slot_cache[v] : -1; };
-  auto src_of = [&](int v) { 
+  auto src_of = [&](int v) {
     if (FROM == kFromSum || !active || v >= U) return 0;
     return FROM == kFromBags ? so.bag_of[v] : so.win[v];
   };
@@ -154,8 +156,8 @@ void launch_local_update(int grid, cudaStream_t stream, const TableView& t, floa
                          const int* slot_cache, const DirectSource& so, const OptimPOD& optim, const float* lr, int cap_s,
                          int chunks, int tpr) {
   auto go = [&](auto kernel) {
-    launch_pdl_if(grid < 2 * kFullGrid, kernel, dim3(grid), dim3(kUpdateThreads), 0, stream, t, ugrad, off, slot_cache, so, optim, lr,
-                  cap_s, chunks, tpr);
+    launch_pdl_if(grid < 2 * kFullGrid, kernel, dim3(grid), dim3(kUpdateThreads), 0, stream, t, ugrad, off, slot_cache, so,
+                  optim, lr, cap_s, chunks, tpr);
   };
   switch (optim.type) {
     case 0: go(local_update_kernel<VEC, 0, FROM>); break;
@@ -340,8 +342,8 @@ __device__ __forceinline__ void init_created(const TableView& t, unsigned todo, 
 
 // Second kernel, with the table probe: every occurrence learns its unique id's number; the winner also writes the
 // unique list, empties the set's entry, and finds (or, with `insert`, claims and initialises) the row.  The block that
-// finishes last zeroes `cnt` for the next call and counts the lookup.  The ids do not pass through the inbox, and no block ends on a
-// system-scope fence.
+// finishes last zeroes `cnt` for the next call and counts the lookup.  The ids do not pass through the inbox, and no
+// block ends on a system-scope fence.
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 local_resolve_kernel(const int64_t* __restrict__ ids, int n, int* __restrict__ set, const int* __restrict__ first,
@@ -617,8 +619,8 @@ void local_push(TableHost table, const LocalPush& p, float* ugrad, const int* of
     return;
   }
   DirectSource so{};
-  so.grads = p.grads, so.bag_offsets = p.bag_offsets, so.nbags = p.nbags, so.weights = p.weights, so.bag_mean = p.bag_mean;
-  so.mean = p.mean ? 1 : 0;
+  so.grads = p.grads, so.bag_offsets = p.bag_offsets, so.nbags = p.nbags;
+  so.weights = p.weights, so.bag_mean = p.bag_mean, so.mean = p.mean ? 1 : 0;
   so.win = p.win, so.multi = p.multi, so.epoch = &p.lookup->pull_epoch;
   so.bag_of = p.bag_of;
   const RowGeom g = row_geom(table.dim);

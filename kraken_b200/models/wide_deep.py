@@ -86,8 +86,8 @@ class MultiHotWideAndDeep(torch.nn.Module):
         if hasattr(eng, "pull_sparse_pooled"):
             # both tables look the same ids up: where the wide one's lookup is known to be that, its dedup serves both
             share = self.wide.embedding.sparse_table.table_id() if self._wide_is_one_lookup(bags) else None
-            pooled = _PooledLookup.apply(self.deep.sparse_table, bags.values(), bags.offsets(), self.field_is_mean.repeat(B),
-                                         share)
+            pooled = _PooledLookup.apply(self.deep.sparse_table, bags.values(), bags.offsets(),
+                                         self.field_is_mean.repeat(B), share)
         else:
             emb = self.deep(bags.values())
             off = bags.offsets()
@@ -112,8 +112,8 @@ class MultiHotWideAndDeep(torch.nn.Module):
 
 
 class _PooledLookup(torch.autograd.Function):
-    """Fused bag lookup with a per-bag sum / mean switch (GPU engine).  ``share_with``: id of a table that has just looked
-    the same ids up, whose dedup is used again."""
+    """Fused bag lookup with a per-bag sum / mean switch (GPU engine).  ``share_with``: id of a table that has just
+    looked the same ids up, whose dedup is used again."""
 
     @staticmethod
     def forward(ctx, sparse_table, values, offsets, bag_mean, share_with):

@@ -448,7 +448,8 @@ class SparseChannel:
 
     @property
     def rows_recv(self) -> torch.Tensor:
-        """The rows of the latest ``pull_unique``: the buffer peers write, or, on one GPU, a local one made on first use."""
+        """The rows of the latest ``pull_unique``: the buffer peers write, or, on one GPU, a local one made on first
+        use."""
         if self._rows_recv is None:
             self._rows_recv = torch.zeros((self.cap_u, self.table.dim), dtype=torch.float32, device=self.table.device)
         return self._rows_recv
@@ -471,8 +472,8 @@ class SparseChannel:
             raise C.KrakenError(f"table {self.table.name!r}: {n} ids in one call exceed the channel capacity "
                                 f"{self.cap}; raise max_ids_per_call")
         h, lay, ctrl, tbl = self.arena.heap, self.lay, self.ctrl, self.table.host()
-        # the other channel's unique ids must fit this one's buffers; the bound for one owner is looked after by the kernels
-        # behind, for shared ids as for a dedup of its own
+        # the other channel's unique ids must fit this one's buffers; the bound for one owner is looked after by the
+        # kernels behind, for shared ids as for a dedup of its own
         share = (share_from is not None and share_from.salt == self.salt and share_from.world == self.world
                  and share_from.dedup.cap_u <= self.cap_u)
         self.dedup = share_from.dedup if share else self._own
@@ -523,8 +524,8 @@ class SparseChannel:
         occurrence -> unique map [n], ticket).  The rows belong to the channel and are
         overwritten by its next pull; a consumer kernel reads them through the map.
 
-        ``in_place`` (honoured on single-GPU jobs without a bound per owner of their own): no copy of the rows is made; the first result is
-        the table's value slab and ``ticket.slots[u]`` is the slab row of unique entry ``u``.
+        ``in_place`` (honoured on single-GPU jobs without a bound per owner of their own): no copy of the rows is
+        made; the first result is the table's value slab and ``ticket.slots[u]`` is the slab row of unique entry ``u``.
         Worth it for small batches only: a consumer that visits every occurrence then reads
         scattered table rows instead of a compact buffer that fits in L2."""
         ids = ids.reshape(-1)

@@ -572,8 +572,10 @@ class GpuEngine(Engine):
             self._nccl_channel(table_id, idx.numel()).push(idx, grad.detach().to(self.device), self.lr_dev)
             return
         ticket = self._recall(table_id, indices)
-        idx = None if ticket is not None else self._prep_ids(indices)
         ch = self._channel(table_id, indices.numel())
+        if ticket is not None and not ticket.current(ch):
+            ticket = None  # another kind of lookup has used the channel since
+        idx = None if ticket is not None else self._prep_ids(indices)
         g = grad.detach()
         if g.device != self.device:
             g = g.to(self.device)

@@ -28,6 +28,31 @@ def test_first_pull_larger_than_the_table_grows_it_first():
     assert eng.sparse[t].num_rows() == 20_000 and eng.sparse[t].capacity >= 20_000 / 0.6
 
 
+@pytest.mark.parametrize("between", ["pooled", "unique", "push"])
+def test_push_after_another_kind_of_lookup_of_the_table(between):
+    """The plain pull's ticket is out of date when the table has been looked up for bags or in place since; its ids are
+    resolved again."""
+    kk.initialize("gpu", table_capacity=1 << 10)
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    kk.update_lr(1.0)
+    eng = kk.native.engine()
+    t = kk.register_sparse_table("e", 8, torch.float32, kk.InitializerType.kConstant, {"value": "1"})
+    ids, others = torch.arange(6, device=DEV), torch.arange(4, 20, device=DEV)
+    kk.pull_sparse_table(t, ids)
+    if between == "pooled":
+        eng.pull_sparse_pooled(t, others, torch.tensor([0, 8, 16], device=DEV))
+    elif between == "unique":
+        eng.pull_sparse_unique(t, others)
+    else:
+        kk.pull_sparse_table(t, ids)
+        _, ticket = eng.pull_sparse_pooled(t, others, torch.tensor([0, 8, 16], device=DEV))
+        eng.push_sparse_pooled(t, ticket, torch.zeros(2, 8, device=DEV), others)
+    kk.push_sparse_table(t, ids, torch.ones(6, 8, device=DEV))
+    rows, found = eng.sparse[t].lookup(torch.arange(20, device=DEV))
+    assert bool(found.bool().all()) and rows[:, 0].tolist() == [0.0] * 6 + [1.0] * 14
+    eng.check()
+
+
 def test_long_id_stream_runs_as_several_rounds():
     """With ``long_id_streams`` a call longer than the exchange buffers (1000 ids here) is served in rounds
     through the same buffers, as the reference's emitter takes a request of any length

@@ -476,28 +476,28 @@ class SparseChannel:
         # kernels behind, for shared ids as for a dedup of its own
         share = (share_from is not None and share_from.salt == self.salt and share_from.world == self.world
                  and share_from.dedup.cap_u <= self.cap_u)
-        self.dedup = share_from.dedup if share else self._own
+        d = self.dedup = share_from.dedup if share else self._own
         if not share:
-            self._own.runs += 1
+            d.runs += 1
         if self.world == 1:
             # nobody to exchange with: the dedup's second kernel also finds the rows
             if share:
-                C.local_probe(self.uniq, self.off, n, tbl, self.slot_cache, insert, ctrl)
+                C.local_probe(d.uniq, d.off, n, tbl, self.slot_cache, insert, ctrl)
                 self.launches += 1
             else:
-                C.local_lookup(ids, self.lset, self.slot_of, self.pos, self.win, self.lbits, self.cnt, self.off,
-                               self.uniq, self.inv, self.cap_u, tbl, self.slot_cache, insert, ctrl)
+                C.local_lookup(ids, self.lset, d.first, self.pos, d.win, self.lbits, self.cnt, d.off, d.uniq, d.inv,
+                               self.cap_u, tbl, self.slot_cache, insert, ctrl)
                 self.launches += 2
             self.serial += 1
             self.last_n = n
             return n
         if share:
-            C.pull_dispatch(h, lay, ctrl, self.uniq, self.off, n)
+            C.pull_dispatch(h, lay, ctrl, d.uniq, d.off, n)
             self.launches += 1
         else:
             # the dedup's second kernel also sends the unique ids to their owners' inboxes
             C.dedup_bucketize(ids, self.world, self.salt, self.hkeys, self.slot_of, self.hbits,
-                              self.cnt, self.off, self.uniq, self.inv, self.ctrl[4:5], self.cap_u, h, lay, ctrl,
+                              self.cnt, d.off, d.uniq, d.inv, self.ctrl[4:5], self.cap_u, h, lay, ctrl,
                               self.owner_world)
             self.launches += 2
         C.pull_probe(h, lay, ctrl, tbl, self.slot_cache, insert, self.spin)
@@ -579,7 +579,7 @@ class SparseChannel:
         if out is None:
             out = torch.empty((rows, dim), dtype=torch.float32, device=self.table.device)
         if self.world == 1:  # the rows are read where they are
-            C.local_combine(tbl, self.inv, self.slot_cache, n, bag_offsets, weights, mean, bag_mean, patch_value, out)
+            C.local_combine(tbl, self.dedup.inv, self.slot_cache, n, bag_offsets, weights, mean, bag_mean, patch_value, out)
             self.launches += 1
         else:
             C.pull_gather(h, lay, ctrl, tbl, self.slot_cache)

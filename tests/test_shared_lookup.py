@@ -12,10 +12,13 @@ class Kernels:
     KrakenError = RuntimeError
 
     def __init__(self):
-        self.called = []
+        self.called, self.args = [], {}
 
     def __getattr__(self, name):
-        return lambda *a, **k: self.called.append(name)
+        def call(*args, **kwargs):
+            self.called.append(name)
+            self.args[name] = args
+        return call
 
 
 def channel(world, cap_u, cap_s, salt=0):
@@ -24,7 +27,8 @@ def channel(world, cap_u, cap_s, salt=0):
     ch.__dict__.update(world=world, owner_world=world, cap=1000, cap_u=cap_u, cap_s=cap_s, salt=salt, spin=1, serial=0,
                        launches=0, hbits=4, lbits=4, ctrl=torch.zeros(8), cnt=None, slot_of=None, lset=None, pos=None,
                        win=None, slot_cache=None, lay=None, arena=SimpleNamespace(heap=None), _hkeys=torch.zeros(1),
-                       table=SimpleNamespace(name="t", host=lambda: None), _own=own, dedup=own, _wait=0)
+                       table=SimpleNamespace(name="t", host=lambda: None, dim=4, device="cpu", optim=None), _own=own,
+                       dedup=own, _wait=int(world > 1), ugrad=torch.zeros(cap_u, 4), multi=None, _bag_of=None)
     return ch
 
 
@@ -49,3 +53,33 @@ def test_another_owner_salt_needs_a_dedup_of_its_own(monkeypatch):
     a, b = channel(4, 500, 500, salt=1), channel(4, 500, 500, salt=2)
     b._lookup_phase(torch.arange(10), True, share_from=a)
     assert b.dedup is b._own
+
+
+def given(kernels, name, tensor):
+    return any(a is tensor for a in kernels.args[name])
+
+
+# Pooled lookups of one id list for two tables, then their pushes, in both orders: every kernel gets the buffers of the one
+# dedup; once those have been written again, the push of the table that shared them resolves its ids.
+@pytest.mark.parametrize("world", [1, 4])
+@pytest.mark.parametrize("sharer_first", [False, True])
+def test_pooled_lookups_and_pushes_of_a_shared_dedup(monkeypatch, world, sharer_first):
+    a, b = channel(world, 500, 500), channel(world, 500, 500)
+    kernels = Kernels()
+    monkeypatch.setattr(sparse_shard, "C", kernels)
+    ids, off, lr = torch.arange(10), torch.tensor([0, 4, 10]), torch.ones(1)
+    combine, scatter = ("local_combine", "local_push") if world == 1 else ("pull_combine", "push_scatter")
+    _, ta = a.pull(ids, bag_offsets=off)
+    _, tb = b.pull(ids, bag_offsets=off, share_from=a)
+    assert given(kernels, combine, a.inv) and kernels.called.count("local_lookup") + kernels.called.count("dedup_bucketize") == 1
+    kernels.called.clear()
+    for ch, ticket in ((b, tb), (a, ta)) if sharer_first else ((a, ta), (b, tb)):
+        ch.push(torch.zeros(2, 4), lr, ticket=ticket)
+        assert given(kernels, scatter, a.inv) and given(kernels, "local_push" if world == 1 else "push_dispatch", a.off)
+    assert "local_lookup" not in kernels.called and "dedup_bucketize" not in kernels.called
+    a.pull(ids, bag_offsets=off)
+    _, tb = b.pull(ids, bag_offsets=off, share_from=a)
+    a.pull(ids + 5, bag_offsets=off)
+    kernels.called.clear()
+    b.push(torch.zeros(2, 4), lr, ticket=tb, ids=ids, bag_offsets=off)
+    assert ("local_lookup" if world == 1 else "dedup_bucketize") in kernels.called and given(kernels, scatter, b._own.inv)

@@ -35,12 +35,13 @@ def _next_pow2_bits(n: int) -> int:
 
 
 def _rows_of_gradients(grads: torch.Tensor, dim: int) -> torch.Tensor:
-    """``grads`` as the kernels read them: float32 rows back to back on a 16-byte boundary.  A slice of a flat gradient
-    (what autograd hands back for one part of a concatenation) can be contiguous and start anywhere."""
+    """``grads`` as the kernels read them: float32 rows back to back, and on a 16-byte boundary where they go by four
+    floats.  A slice of a flat gradient (what autograd hands back for one part of a concatenation) can be contiguous and
+    start anywhere."""
     grads = grads.reshape(-1, dim)
     if grads.dtype != torch.float32 or not grads.is_contiguous():
         grads = grads.to(torch.float32).contiguous()
-    return grads if grads.data_ptr() % 16 == 0 else grads.clone()
+    return grads if dim % 4 or grads.data_ptr() % 16 == 0 else grads.clone()
 
 
 class RowCounters:
@@ -341,11 +342,13 @@ class Ticket:
     """Identifies one pull so that the matching push can reuse its dedup result
     and the slots the owners resolved."""
 
-    __slots__ = ("channel", "serial", "n", "bag_offsets", "weights", "mean", "bag_mean", "slots", "dedup", "runs")
+    __slots__ = ("channel", "serial", "n", "bag_offsets", "weights", "mean", "bag_mean", "slots", "dedup", "runs",
+                 "generation")
 
     def __init__(self, channel, serial, n, bag_offsets, weights, mean, bag_mean, slots=None):
-        self.dedup = getattr(channel, "dedup", None)  # after a shared pull it can be run again by another channel
-        self.runs = self.dedup.runs if self.dedup is not None else 0
+        self.dedup = dedup = channel.dedup  # after a shared pull it can be run again by another channel
+        self.runs = dedup.runs
+        self.generation = channel.generation  # of the tables whose slots the owners have resolved
         self.slots = slots  # in-place pulls: table slot of every unique entry (rows are the table's value slab)
         self.channel = channel
         self.serial = serial
@@ -357,8 +360,7 @@ class Ticket:
 
     def current(self, channel) -> bool:
         """Whether ``channel``'s buffers still hold what this pull left in them."""
-        return (self.channel is channel and self.serial == channel.serial
-                and (self.dedup is None or self.runs == self.dedup.runs))
+        return self.channel is channel and self.serial == channel.serial and self.runs == self.dedup.runs
 
 
 class SparseChannel:
@@ -540,11 +542,27 @@ class SparseChannel:
         self.launches += 1 + self._wait
         return self.rows_recv, self.inv, Ticket(self, self.serial, n, None, None, False, None)
 
+    @property
+    def generation(self) -> int:
+        return self.table.generation
+
+    def _refresh_slots(self, ticket: Ticket) -> None:
+        """Resolves the slots of the ticket's pull again, for a shard that has been reallocated since (another lookup of
+        the table, a combined one say, or an import made it grow).  Concerns this rank alone: the ids that peers have
+        asked for stay in its inbox until they have passed the push that follows."""
+        if self.world == 1:
+            C.local_probe(self.uniq, self.off, ticket.n, self.table.host(), self.slot_cache, False, self.ctrl)
+        else:
+            C.pull_probe(self.arena.heap, self.lay, self.ctrl, self.table.host(), self.slot_cache, False, self.spin)
+        self.launches += 1 + self._wait
+
     def push_accumulated(self, lr: torch.Tensor, ticket: Ticket) -> None:
         """Push for gradients that a fused kernel has already summed per unique id into
         ``self.ugrad`` (the pull's ticket must still be current)."""
         if not ticket.current(self):
             raise C.KrakenError("push_accumulated needs the ticket of this channel's latest pull")
+        if ticket.generation != self.table.generation:
+            self._refresh_slots(ticket)
         self._apply_accumulated(lr, ticket.n)
         self.serial += 1
 
@@ -600,6 +618,8 @@ class SparseChannel:
         if ticket is not None and ticket.current(self):
             n = ticket.n
             bag_offsets, weights, mean, bag_mean = ticket.bag_offsets, ticket.weights, ticket.mean, ticket.bag_mean
+            if ticket.generation != self.table.generation:
+                self._refresh_slots(ticket)
         else:
             if ids is None:
                 raise C.KrakenError("push without a current ticket needs the ids")
@@ -657,6 +677,7 @@ class GroupChannel:
         self.cap_u = int(max_unique) if max_unique and max_unique < max_ids else int(max_ids)
         dev = self.tables[0].device
         self.device = dev
+        self._counters = list({id(t.counters): t.counters for t in self.tables}.values())
         T, dim = self.T, self.dim
 
         lay = Layout()
@@ -688,6 +709,7 @@ class GroupChannel:
         self.slot_cache = torch.full((world * self.cap_u,), -1, dtype=torch.int32, device=dev)
         self.ttab = torch.zeros(world * self.cap_u, dtype=torch.int16, device=dev)
         self.ugrad = torch.zeros((self.cap_u, dim), dtype=torch.float32, device=dev)
+        self.dedup = Dedup(self.cap_u, self.off, self.uniq, self.inv, None, None, self.ctrl)  # not shared
         self.hkeys = None           # dedup scratch, one region per table, sized on first use
         self._shape_sig = None      # ids per table of the call the descriptors were built for
         self._views_sig = None      # generations of the tables the device-side descriptors describe
@@ -731,6 +753,11 @@ class GroupChannel:
             self.table_views.copy_(host)   # same device buffer: launches captured in a CUDA graph stay valid
         self._views_sig = sig
 
+    @property
+    def generation(self) -> int:
+        """Changes whenever one of the tables (or of their engine's) is reallocated."""
+        return sum(c.moves for c in self._counters)
+
     # ------------------------------------------------------------------ exchange
     def _lookup_phase(self, ids_cat: torch.Tensor, counts, insert: bool) -> int:
         n = int(ids_cat.numel())
@@ -743,12 +770,15 @@ class GroupChannel:
         C.group_dedup_dispatch(ids_cat, self.occ_start, self.region_base, self.region_bits, self.salts, self.world,
                                self.hkeys, self.slot_of, self.cnt, self.off, self.uniq, self.inv, self.ctrl[4:5],
                                self.cap_u, h, lay, ctrl, self.owner_world)
-        C.group_probe(h, lay, ctrl, self.table_views, self.T, self.dim, self.snap_t, self.slot_cache, self.ttab,
-                      insert, self.spin)
+        self._probe(insert)
         self.launches += 5  # memset is not counted: insert, finalize + dispatch, request wait, probe (+ init)
         self.serial += 1
         self.last_n = n
         return n
+
+    def _probe(self, insert: bool) -> None:
+        C.group_probe(self.arena.heap, self.lay, self.ctrl, self.table_views, self.T, self.dim, self.snap_t,
+                      self.slot_cache, self.ttab, insert, self.spin)
 
     def pull(self, ids_cat: torch.Tensor, counts, bag_offsets: Optional[torch.Tensor] = None,
              weights: Optional[torch.Tensor] = None, bag_mean: Optional[torch.Tensor] = None,
@@ -772,9 +802,13 @@ class GroupChannel:
         dedup result and the owners' slots are reused; otherwise the ids are looked up again (an id a table
         does not hold is kSparseIdNotExist)."""
         bag_offsets = weights = bag_mean = None
-        if ticket is not None and ticket.channel is self and ticket.serial == self.serial:
+        if ticket is not None and ticket.current(self):
             n = ticket.n
             bag_offsets, weights, bag_mean = ticket.bag_offsets, ticket.weights, ticket.bag_mean
+            if ticket.generation != self.generation:  # as SparseChannel._refresh_slots
+                self._refresh_views()
+                self._probe(insert=False)
+                self.launches += 2
         else:
             if ids_cat is None or counts is None:
                 raise C.KrakenError("a combined push without a current ticket needs the ids")

@@ -573,7 +573,7 @@ class GpuEngine(Engine):
             return
         ticket = self._recall(table_id, indices)
         ch = self._channel(table_id, indices.numel())
-        if ticket is not None and not ticket.current(ch):
+        if ticket is not None and ticket.serial != ch.serial:
             ticket = None  # another kind of lookup has used the channel since
         idx = None if ticket is not None else self._prep_ids(indices)
         g = grad.detach()
@@ -732,7 +732,7 @@ class GpuEngine(Engine):
         the lookup (``_looked_up``), so that a call waits for the device only if the bound passes the limit all the same.
         ``channels``: what the lookup of each table goes through, None for a combined one or one over collectives."""
         self._sample_next = False  # a call that raised before its ``_looked_up`` leaves nothing to this one
-        want = []
+        want, near = [], False
         for table_id, n_ids, ch in zip(table_ids, counts, channels):
             t = self.sparse[table_id]
             inflow = n_ids * self.world  # worst case: every rank's ids of this call belong to this shard
@@ -743,12 +743,13 @@ class GpuEngine(Engine):
                 n_ids = min(n_ids, ch.cap_u)
                 inflow = min(self.world * ch.cap_s, 2 * n_ids) if self.world > 1 else n_ids
             want.append((t, inflow))
+            near = near or t.rows_bound() + 2 * inflow > 0.6 * t.capacity
         if torch.cuda.is_current_stream_capturing():
             if self.counters.captured is not None:  # nothing runs now, the replays count
                 self.counters.captured += want
             return
-        self._sample_next = any(t.rows_bound() + 2 * inflow > 0.6 * t.capacity for t, inflow in want)
-        if self._sample_next:
+        self._sample_next = near
+        if near:
             self.counters.poll()
             for _ in range(2):  # the sample that is waited for first may be an older one
                 if any(t.rows_bound() + inflow > 0.6 * t.capacity for t, inflow in want):

@@ -53,6 +53,44 @@ def test_push_after_another_kind_of_lookup_of_the_table(between):
     eng.check()
 
 
+def _lookup_then_grow(kind):
+    """Looks ids up, makes the table grow through another path, and returns the table and a function that pushes ones."""
+    kk.initialize("gpu", table_capacity=1 << 10, max_ids_per_call=4096)
+    kk.init_model("m", kk.OptimType.kSGD, {})
+    kk.update_lr(1.0)
+    eng = kk.native.engine()
+    tids = [kk.register_sparse_table(f"t{k}", 8, torch.float32, kk.InitializerType.kConstant, {"value": "1"})
+            for k in range(2)]
+    ids, many = torch.arange(6, device=DEV), torch.arange(1000, 4000, device=DEV)
+    ones = torch.ones(6, 8, device=DEV)
+    table = eng.sparse[tids[0]]
+    before = table.capacity
+    if kind == "combined":
+        kk.combine_pull_sparse_table(tids, [ids, ids])
+        kk.pull_sparse_table(tids[0], many)
+        push = lambda: kk.combine_push_sparse_table(tids, [ids, ids], [ones, ones])
+    elif kind == "plain":
+        kk.pull_sparse_table(tids[0], ids)
+        kk.combine_pull_sparse_table(tids, [many, many])
+        push = lambda: kk.push_sparse_table(tids[0], ids, ones)
+    else:
+        _, inv, ticket = eng.pull_sparse_unique(tids[0], ids, in_place=True)
+        kk.combine_pull_sparse_table(tids, [many, many])
+        eng.grad_accumulator(tids[0]).index_add_(0, inv[:6].long(), ones)
+        push = lambda: eng.push_sparse_accumulated(tids[0], ticket)
+    assert table.capacity > before
+    return table, push
+
+
+@pytest.mark.parametrize("kind", ["plain", "accumulated", "combined"])
+def test_push_to_a_table_that_grew_since_its_lookup(kind):
+    table, push = _lookup_then_grow(kind)
+    push()
+    kk.native.engine().check()
+    rows, found = table.lookup(torch.cat([torch.arange(6, device=DEV), torch.arange(1000, 4000, device=DEV)]))
+    assert bool(found.bool().all()) and rows[:, 0].tolist() == [0.0] * 6 + [1.0] * 3000
+
+
 def test_long_id_stream_runs_as_several_rounds():
     """With ``long_id_streams`` a call longer than the exchange buffers (1000 ids here) is served in rounds
     through the same buffers, as the reference's emitter takes a request of any length

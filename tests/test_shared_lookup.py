@@ -27,7 +27,8 @@ def channel(world, cap_u, cap_s, salt=0):
     ch.__dict__.update(world=world, owner_world=world, cap=1000, cap_u=cap_u, cap_s=cap_s, salt=salt, spin=1, serial=0,
                        launches=0, hbits=4, lbits=4, ctrl=torch.zeros(8), cnt=None, slot_of=None, lset=None, pos=None,
                        win=None, slot_cache=None, lay=None, arena=SimpleNamespace(heap=None), _hkeys=torch.zeros(1),
-                       table=SimpleNamespace(name="t", host=lambda: None, dim=4, device="cpu", optim=None), _own=own,
+                       table=SimpleNamespace(name="t", host=lambda: None, dim=4, device="cpu", optim=None,
+                                             generation=1), _own=own,
                        dedup=own, _wait=int(world > 1), ugrad=torch.zeros(cap_u, 4), multi=None, _bag_of=None)
     return ch
 
@@ -83,3 +84,25 @@ def test_pooled_lookups_and_pushes_of_a_shared_dedup(monkeypatch, world, sharer_
     kernels.called.clear()
     b.push(torch.zeros(2, 4), lr, ticket=tb, ids=ids, bag_offsets=off)
     assert ("local_lookup" if world == 1 else "dedup_bucketize") in kernels.called and given(kernels, scatter, b._own.inv)
+
+
+# A shard that was reallocated between a pull and its push: the slots are resolved again, by this rank alone.
+@pytest.mark.parametrize("world", [1, 4])
+@pytest.mark.parametrize("accumulated", [False, True])
+def test_push_after_the_shard_was_reallocated(monkeypatch, world, accumulated):
+    ch = channel(world, 500, 500)
+    kernels = Kernels()
+    monkeypatch.setattr(sparse_shard, "C", kernels)
+    probe = "local_probe" if world == 1 else "pull_probe"
+    for moved in (False, True):
+        _, ticket = ch.pull(torch.arange(10))
+        if moved:
+            ch.table.generation += 1
+        kernels.called.clear()
+        if accumulated:
+            ch.push_accumulated(torch.ones(1), ticket)
+        else:
+            ch.push(torch.zeros(10, 4), torch.ones(1), ticket=ticket)
+        assert (probe in kernels.called) == moved and "dedup_bucketize" not in kernels.called
+        if moved:
+            assert kernels.called[0] == probe and kernels.args[probe][5] is False

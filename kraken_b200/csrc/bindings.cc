@@ -330,15 +330,36 @@ struct AsyncRead {
   }
 };
 
+// Rows of floats at any pitch, each row contiguous.
+void need_rows(const torch::Tensor& t, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.dim() == 2 &&
+                  (t.size(1) == 1 || t.stride(1) == 1) && t.stride(0) >= t.size(1),
+              name, " must be a CUDA float32 matrix with contiguous rows");
+}
+
 cu::TableHost make_table(const torch::Tensor& keys, const torch::Tensor& val, const c10::optional<torch::Tensor>& s0,
                          const c10::optional<torch::Tensor>& s1, const c10::optional<torch::Tensor>& s2,
                          const c10::optional<torch::Tensor>& steps, const c10::optional<torch::Tensor>& lead,
                          const torch::Tensor& size, const torch::Tensor& status, uint32_t bits, int dim, int init_type,
                          float init_a, float init_b, uint64_t seed_key) {
   need_cuda(keys, "keys", torch::kInt64);
-  need_cuda(val, "val", torch::kFloat32);
   TORCH_CHECK(keys.numel() == (1ll << bits), "keys must have 1 << bits elements");
-  TORCH_CHECK(val.numel() == keys.numel() * dim, "val must be [cap, dim]");
+  // value and state rows of a slot may be parts of one record, so they share a pitch
+  auto rows = [&](const torch::Tensor& x, const char* what) {
+    need_rows(x, what);
+    TORCH_CHECK(x.size(0) == keys.numel() && x.size(1) == dim && x.stride(0) == val.stride(0) &&
+                    (dim % 4 != 0 || (x.stride(0) % 4 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0)),
+                what, " must be [cap, dim] with the pitch of the values");
+  };
+  rows(val, "val");
+  for (const auto* s : {&s0, &s1, &s2}) {
+    if (s->has_value()) rows(**s, "state");
+  }
+  if (steps.has_value()) {
+    TORCH_CHECK(steps->is_cuda() && steps->scalar_type() == torch::kInt32 && steps->dim() == 1 &&
+                    steps->numel() == keys.numel() && steps->stride(0) >= 1,
+                "steps must be CUDA int32 [cap]");
+  }
   cu::TableHost t{};
   t.keys = keys.data_ptr();
   t.val = ptr<float>(val);
@@ -351,6 +372,8 @@ cu::TableHost make_table(const torch::Tensor& keys, const torch::Tensor& val, co
   t.status = ptr<int>(status);
   t.bits = bits;
   t.dim = dim;
+  t.pitch = static_cast<int>(val.stride(0));
+  t.step_pitch = steps.has_value() ? static_cast<int>(steps->stride(0)) : 0;
   t.init.type = static_cast<uint8_t>(init_type);
   t.init.a = init_a;
   t.init.b = init_b;
@@ -1538,19 +1561,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            const c10::optional<torch::Tensor>& inv1, const torch::Tensor& dense, int B, int F, int D,
            const torch::Tensor& x, const torch::Tensor& fm_logit, const c10::optional<torch::Tensor>& slots2,
            const c10::optional<torch::Tensor>& slots1, const c10::optional<torch::Tensor>& ssum) {
-          need_cuda(rows2, "rows2", torch::kFloat32);
+          need_rows(rows2, "rows2");
           need_cuda(dense, "dense", torch::kFloat32);
           need_cuda(x, "x", torch::kBFloat16);
           need_cuda(fm_logit, "fm_logit", torch::kFloat32);
           const int RD = rows2.size(1), ND = dense.size(1), ldx = x.size(1);
-          TORCH_CHECK(D % 4 == 0 && RD % 4 == 0 && RD >= D, "row widths must be multiples of 4");
+          TORCH_CHECK(D % 4 == 0 && RD % 4 == 0 && RD >= D && rows2.stride(0) % 4 == 0,
+                      "row widths and pitches must be multiples of 4");
           TORCH_CHECK(((D / 4) & (D / 4 - 1)) == 0 && D <= 128, "D / 4 must be a power of two, D <= 128");
           if (ssum.has_value()) {
             need_cuda(*ssum, "ssum", torch::kFloat32);
             TORCH_CHECK(ssum->numel() == static_cast<int64_t>(B) * D, "ssum must be [B, D]");
           }
           if (rows1.has_value()) {
-            need_cuda(*rows1, "rows1", torch::kFloat32);
+            need_rows(*rows1, "rows1");
             TORCH_CHECK(rows1->size(1) == 1 && inv1.has_value() && inv1->numel() >= static_cast<int64_t>(B) * F,
                         "first-order table must have dim 1 and its own occurrence map");
           } else {
@@ -1560,7 +1584,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           TORCH_CHECK(x.size(0) == B && ldx >= F * D + ND && ldx % 4 == 0 && dense.size(0) == B && fm_logit.numel() == B,
                       "deepfm_pack_forward: shape mismatch");
           cu::deepfm_pack_forward(ptr<float>(rows2), ptr<int>(inv2), optr<int>(slots2), optr<float>(rows1), optr<int>(inv1),
-                                  optr<int>(slots1), ptr<float>(dense), B, F, D, RD, ND, reinterpret_cast<__nv_bfloat16*>(x.data_ptr()), ldx,
+                                  optr<int>(slots1), ptr<float>(dense), B, F, D, static_cast<int>(rows2.stride(0)),
+                                  rows1.has_value() ? static_cast<int>(rows1->stride(0)) : 0, ND, reinterpret_cast<__nv_bfloat16*>(x.data_ptr()), ldx,
                                   ptr<float>(fm_logit), optr<float>(ssum), cur_stream());
           check_launch("deepfm_pack_forward");
         },
@@ -1572,14 +1597,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            const c10::optional<torch::Tensor>& dx, const torch::Tensor& dlogit, int B, int F, int D,
            const torch::Tensor& ugrad2, const c10::optional<torch::Tensor>& ugrad1,
            const c10::optional<torch::Tensor>& slots2, const torch::Tensor& ssum) {
-          need_cuda(rows2, "rows2", torch::kFloat32);
+          need_rows(rows2, "rows2");
           need_cuda(ssum, "ssum", torch::kFloat32);
           TORCH_CHECK(ssum.numel() == static_cast<int64_t>(B) * D && ((D / 4) & (D / 4 - 1)) == 0 && D <= 128,
                       "ssum must be [B, D] with D / 4 a power of two");
           need_cuda(dlogit, "dlogit", torch::kFloat32);
           need_cuda(ugrad2, "ugrad2", torch::kFloat32);
           const int RD = rows2.size(1);
-          TORCH_CHECK(ugrad2.size(1) == RD && D % 4 == 0 && RD % 4 == 0, "gradient buffer must match the row width");
+          TORCH_CHECK(ugrad2.size(1) == RD && D % 4 == 0 && RD % 4 == 0 && rows2.stride(0) % 4 == 0, "gradient buffer must match the row width");
           if (ugrad1.has_value()) {
             need_cuda(*ugrad1, "ugrad1", torch::kFloat32);
             TORCH_CHECK(inv1.has_value(), "separate first-order table needs its occurrence map");
@@ -1596,7 +1621,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           }
           TORCH_CHECK(dlogit.numel() == B, "deepfm_pack_backward: shape mismatch");
           cu::deepfm_pack_backward(ptr<float>(rows2), ptr<int>(inv2), optr<int>(slots2), optr<int>(inv1), dxp, lddx,
-                                   ptr<float>(dlogit), ptr<float>(ssum), B, F, D, RD, ptr<float>(ugrad2),
+                                   ptr<float>(dlogit), ptr<float>(ssum), B, F, D, static_cast<int>(rows2.stride(0)), RD, ptr<float>(ugrad2),
                                    optr<float>(ugrad1), cur_stream());
           check_launch("deepfm_pack_backward");
         },

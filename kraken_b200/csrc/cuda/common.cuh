@@ -34,14 +34,16 @@ struct Sym {
 // are never deleted on the training path; eviction rebuilds the table).
 struct TableView {
   unsigned long long* keys;  // [cap], kEmptyKey = free
-  float* val;                // [cap, dim]
-  float* s[3];               // optimizer state slabs [cap, dim] or nullptr
-  int* steps;                // [cap] or nullptr
+  float* val;                // value rows of `dim` floats, one every `pitch` floats
+  float* s[3];               // optimizer state rows, one every `pitch` floats, or nullptr
+  int* steps;                // step counters, one every `step_pitch` ints, or nullptr
   unsigned long long* lead;  // [cap] (push epoch << 32 | entry) or nullptr when world == 1
   int* size;                 // number of occupied slots
   int* status;               // first error code wins
   uint32_t bits;             // cap = 1 << bits
   int dim;
+  int pitch;
+  int step_pitch;
   InitPOD init;
   uint64_t seed_key;
 };

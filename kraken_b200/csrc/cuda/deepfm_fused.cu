@@ -35,6 +35,7 @@ __device__ __forceinline__ size_t row_of(const int* __restrict__ slots, int u) {
   return static_cast<size_t>(s < 0 ? 0 : s);
 }
 
+// P2 and P1 are the pitches of rows2 and rows1 in floats: the row width for gathered rows, the tables' pitch in place.
 // Lanes per sample = (D / 4) x G: lane (g, c) owns dims [4c, 4c + 4) of the fields g, g + G, ...
 // Splitting the fields over G lane groups (a power of two) multiplies the number of independent
 // row loads in flight; the per-sample sums are combined with shuffles and the forward pass leaves
@@ -43,7 +44,7 @@ __global__ void __launch_bounds__(kThreads)
 deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restrict__ inv2,
                            const int* __restrict__ slots2, const float* __restrict__ rows1,
                            const int* __restrict__ inv1, const int* __restrict__ slots1,
-                           const float* __restrict__ dense, int B, int F, int D, int RD, int ND, int lpr, int G,
+                           const float* __restrict__ dense, int B, int F, int D, int P2, int P1, int ND, int lpr, int G,
                            __nv_bfloat16* __restrict__ x, int ldx, float* __restrict__ fm_logit,
                            float* __restrict__ ssum) {
   pdl_enter();
@@ -64,7 +65,7 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
       __nv_bfloat16* xr = x + static_cast<size_t>(b) * ldx;
 #pragma unroll 4
       for (int f = fg; f < F; f += G) {
-        const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, i2[f]) * RD) + c);
+        const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, i2[f]) * P2) + c);
         s.x += e.x, s.y += e.y, s.z += e.z, s.w += e.w;
         q.x += e.x * e.x, q.y += e.y * e.y, q.z += e.z * e.z, q.w += e.w * e.w;
         __nv_bfloat162 lo = __floats2bfloat162_rn(e.x, e.y), hi = __floats2bfloat162_rn(e.z, e.w);
@@ -76,10 +77,10 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
       // first-order weights, dense features and the zero pad, spread over the sample's lanes
       if (rows1 != nullptr) {
         const int* i1 = inv1 + static_cast<size_t>(b) * F;
-        for (int f = lane; f < F; f += lpr) part += __ldcg(rows1 + row_of(slots1, i1[f]));
+        for (int f = lane; f < F; f += lpr) part += __ldcg(rows1 + row_of(slots1, i1[f]) * P1);
       } else {
         // folded layout: column D of the same row is the field's first-order weight
-        for (int f = lane; f < F; f += lpr) part += __ldcg(rows2 + row_of(slots2, i2[f]) * RD + D);
+        for (int f = lane; f < F; f += lpr) part += __ldcg(rows2 + row_of(slots2, i2[f]) * P2 + D);
       }
       const int base = F * D;
       for (int j = lane; base + j < ldx; j += lpr)
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(kThreads)
 deepfm_pack_backward_kernel(const float* __restrict__ rows2, const int* __restrict__ inv2,
                             const int* __restrict__ slots2, const int* __restrict__ inv1,
                             const __nv_bfloat16* __restrict__ dx, int lddx, const float* __restrict__ dlogit,
-                            const float* __restrict__ ssum, int B, int F, int D, int RD, int lpr, int G,
+                            const float* __restrict__ ssum, int B, int F, int D, int P2, int RD, int lpr, int G,
                             float* ugrad2, float* ugrad1) {
   pdl_enter();
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -122,7 +123,7 @@ deepfm_pack_backward_kernel(const float* __restrict__ rows2, const int* __restri
 #pragma unroll 4
     for (int f = fg; f < F; f += G) {
       const int u = i2[f];
-      const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, u) * RD) + c);
+      const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, u) * P2) + c);
       float4 d = make_float4(g * (s.x - e.x), g * (s.y - e.y), g * (s.z - e.z), g * (s.w - e.w));
       if (dxr) {
         const uint2 p = *reinterpret_cast<const uint2*>(dxr + f * D + c * 4);
@@ -167,26 +168,26 @@ int grid_for(long long rows, int lpr) {
 }  // namespace
 
 void deepfm_pack_forward(const float* rows2, const int* inv2, const int* slots2, const float* rows1, const int* inv1,
-                         const int* slots1, const float* dense, int B, int F, int D, int RD, int ND, __nv_bfloat16* x,
+                         const int* slots1, const float* dense, int B, int F, int D, int P2, int P1, int ND, __nv_bfloat16* x,
                          int ldx, float* fm_logit, float* ssum, cudaStream_t stream) {
   if (B <= 0) return;
   const int chunks = D / 4;
   const int G = field_groups(chunks);
   const int lpr = chunks * G;
   launch_pdl(deepfm_pack_forward_kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, rows1, inv1, slots1, dense,
-                                                                        B, F, D, RD, ND, lpr, G, x, ldx, fm_logit, ssum);
+                                                                        B, F, D, P2, P1, ND, lpr, G, x, ldx, fm_logit, ssum);
 }
 
 void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2, const int* inv1,
                           const __nv_bfloat16* dx, int lddx,
-                          const float* dlogit, const float* ssum, int B, int F, int D, int RD, float* ugrad2,
+                          const float* dlogit, const float* ssum, int B, int F, int D, int P2, int RD, float* ugrad2,
                           float* ugrad1, cudaStream_t stream) {
   if (B <= 0) return;
   const int chunks = D / 4;
   const int G = field_groups(chunks);
   const int lpr = chunks * G;
   launch_pdl(deepfm_pack_backward_kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, inv1, dx, lddx, dlogit,
-                                                                         ssum, B, F, D, RD, lpr, G, ugrad2, ugrad1);
+                                                                         ssum, B, F, D, P2, RD, lpr, G, ugrad2, ugrad1);
 }
 
 }  // namespace cu

@@ -259,7 +259,7 @@ pull_probe_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, TableView t, int* slot_ca
         const int r_slot = __shfl_sync(0xffffffffu, slot, src < 0 ? 0 : src);
         const uint64_t r_id = __shfl_sync(0xffffffffu, id, src < 0 ? 0 : src);
         if (src >= 0) {
-          float* row = t.val + static_cast<size_t>(r_slot) * t.dim;
+          float* row = t.val + static_cast<size_t>(r_slot) * t.pitch;
           for (int c = lane % lpr; c < chunks; c += lpr) {
             float q[4];
             if (VEC == 4) {
@@ -308,7 +308,7 @@ pull_gather_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, TableView t, const int* 
         typename V::T v[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u)
-          v[u] = slot[u] < 0 ? V::zero() : V::ld(t.val + static_cast<size_t>(slot[u]) * t.dim + c * VEC);
+          v[u] = slot[u] < 0 ? V::zero() : V::ld(t.val + static_cast<size_t>(slot[u]) * t.pitch + c * VEC);
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
           const int ru = r + u * row_stride;
@@ -525,14 +525,15 @@ push_update_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, TableView t, const int* 
       int step_i = 1;
       if (t.steps) {
         if (lane == 0) {
-          step_i = t.steps[slot] + 1;
-          t.steps[slot] = step_i;
+          int* const counter = t.steps + static_cast<size_t>(slot) * t.step_pitch;
+          step_i = *counter + 1;
+          *counter = step_i;
         }
         step_i = __shfl_sync(group_mask, step_i, (threadIdx.x & 31) / lpr * lpr);
       }
       const int64_t step = step_i;
       const AdamBias ab = optim.type == 1 ? AdamBiasAt(optim, step) : AdamBias{1.f, 1.f};
-      const size_t row = static_cast<size_t>(slot) * t.dim;
+      const size_t row = static_cast<size_t>(slot) * t.pitch;
       for (int c = lane; c < chunks; c += lpr) {
         float g[VEC], w[VEC], a0[VEC], a1[VEC], a2[VEC];
         *reinterpret_cast<typename V::T*>(g) = V::ldcg(inbox + static_cast<size_t>(entry) * t.dim + c * VEC);

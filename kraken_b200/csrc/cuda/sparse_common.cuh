@@ -32,6 +32,8 @@ inline TableView to_view(const TableHost& h) {
   t.status = h.status;
   t.bits = h.bits;
   t.dim = h.dim;
+  t.pitch = h.pitch;
+  t.step_pitch = h.step_pitch;
   t.init = h.init;
   t.seed_key = h.seed_key;
   return t;

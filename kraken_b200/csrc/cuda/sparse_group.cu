@@ -249,7 +249,7 @@ group_probe_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, const TableView* __restr
         const uint64_t r_id = __shfl_sync(0xffffffffu, id, src < 0 ? 0 : src);
         if (src >= 0) {
           const TableView& tb = tv[r_t];
-          float* row = tb.val + static_cast<size_t>(r_slot) * tb.dim;
+          float* row = tb.val + static_cast<size_t>(r_slot) * tb.pitch;
           for (int c = lane % lpr; c < chunks; c += lpr) {
             float q[4];
             if (VEC == 4) {
@@ -291,7 +291,9 @@ group_gather_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, const TableView* __rest
         src[u] = nullptr;
         if (ru < m.x) {
           const int slot = slot_cache[e0 + ru];
-          if (slot >= 0) src[u] = tv[ttab[e0 + ru]].val + static_cast<size_t>(slot) * dim;
+          if (slot < 0) continue;
+          const TableView& t = tv[ttab[e0 + ru]];
+          src[u] = t.val + static_cast<size_t>(slot) * t.pitch;
         }
       }
       for (int c = lane; c < chunks; c += lpr) {
@@ -387,14 +389,15 @@ group_push_update_kernel(Sym sym, ChanLayout lay, Ctrl* ctrl, const TableView* _
       int step_i = 1;
       if (t.steps) {
         if (lane == 0) {
-          step_i = t.steps[slot] + 1;
-          t.steps[slot] = step_i;
+          int* const counter = t.steps + static_cast<size_t>(slot) * t.step_pitch;
+          step_i = *counter + 1;
+          *counter = step_i;
         }
         step_i = __shfl_sync(group_mask, step_i, (threadIdx.x & 31) / lpr * lpr);
       }
       const int64_t step = step_i;
       const AdamBias ab = optim.type == 1 ? AdamBiasAt(optim, step) : AdamBias{1.f, 1.f};
-      const size_t row = static_cast<size_t>(slot) * dim;
+      const size_t row = static_cast<size_t>(slot) * t.pitch;
       for (int c = lane; c < chunks; c += lpr) {
         float g[VEC], w[VEC], a0[VEC], a1[VEC], a2[VEC];
         *reinterpret_cast<typename V::T*>(g) = V::ldcg(inbox + static_cast<size_t>(entry) * dim + c * VEC);

@@ -26,6 +26,8 @@ TableView to_view(const TableHost& h) {
   t.status = h.status;
   t.bits = h.bits;
   t.dim = h.dim;
+  t.pitch = h.pitch;
+  t.step_pitch = h.step_pitch;
   t.init = h.init;
   t.seed_key = h.seed_key;
   return t;
@@ -36,7 +38,7 @@ __global__ void table_clear_kernel(TableView t) {
   for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < cap;
        i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
     t.keys[i] = kEmptyKey;
-    if (t.steps) t.steps[i] = 0;
+    if (t.steps) t.steps[i * t.step_pitch] = 0;
     if (t.lead) t.lead[i] = 0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *t.size = 0;
@@ -73,14 +75,14 @@ __global__ void table_import_kernel(TableView t, const int64_t* __restrict__ ids
       if (found < 0) {
         set_status(t.status, err::kTableFull);
       } else {
-        const size_t dst = static_cast<size_t>(found) * t.dim, src = static_cast<size_t>(i) * t.dim;
+        const size_t dst = static_cast<size_t>(found) * t.pitch, src = static_cast<size_t>(i) * t.dim;
         for (int j = 0; j < t.dim; ++j) {
           t.val[dst + j] = vals[src + j];
           if (t.s[0] && s0) t.s[0][dst + j] = s0[src + j];
           if (t.s[1] && s1) t.s[1][dst + j] = s1[src + j];
           if (t.s[2] && s2) t.s[2][dst + j] = s2[src + j];
         }
-        if (t.steps && steps) t.steps[found] = steps[i];
+        if (t.steps && steps) t.steps[static_cast<size_t>(found) * t.step_pitch] = steps[i];
       }
     }
     count_created(t, created);
@@ -94,7 +96,7 @@ __global__ void table_lookup_kernel(TableView t, const int64_t* __restrict__ ids
   const int slot = table_find_or_insert(t, static_cast<uint64_t>(ids[i]), false, &created);
   found[i] = slot >= 0;
   for (int j = 0; j < t.dim; ++j)
-    rows[static_cast<size_t>(i) * t.dim + j] = slot >= 0 ? t.val[static_cast<size_t>(slot) * t.dim + j] : 0.f;
+    rows[static_cast<size_t>(i) * t.dim + j] = slot >= 0 ? t.val[static_cast<size_t>(slot) * t.pitch + j] : 0.f;
 }
 
 __global__ void table_export_kernel(TableView t, int filter_mode, uint64_t salt, int world, int rank, int min_steps,
@@ -112,7 +114,7 @@ __global__ void table_export_kernel(TableView t, int filter_mode, uint64_t salt,
         switch (filter_mode) {
           case 1: take = static_cast<int>(OwnerOf(salt, k, world)) == rank; break;
           case 2: take = static_cast<int>(OwnerOf(salt, k, world)) != rank; break;
-          case 3: take = t.steps ? t.steps[slot] >= min_steps : true; break;
+          case 3: take = t.steps ? t.steps[slot * t.step_pitch] >= min_steps : true; break;
           case 4: take = static_cast<int>(k % static_cast<unsigned long long>(world)) == rank; break;  // id % world == rank
           default: take = true;
         }
@@ -128,14 +130,14 @@ __global__ void table_export_kernel(TableView t, int filter_mode, uint64_t salt,
       const int pos = warp_base + __popc(m & ((1u << lane) - 1));
       if (pos < out_cap) {
         out_ids[pos] = static_cast<int64_t>(k);
-        const size_t src = slot * t.dim, dst = static_cast<size_t>(pos) * t.dim;
+        const size_t src = slot * t.pitch, dst = static_cast<size_t>(pos) * t.dim;
         for (int j = 0; j < t.dim; ++j) {
           out_vals[dst + j] = t.val[src + j];
           if (out_s0 && t.s[0]) out_s0[dst + j] = t.s[0][src + j];
           if (out_s1 && t.s[1]) out_s1[dst + j] = t.s[1][src + j];
           if (out_s2 && t.s[2]) out_s2[dst + j] = t.s[2][src + j];
         }
-        if (out_steps) out_steps[pos] = t.steps ? t.steps[slot] : 0;
+        if (out_steps) out_steps[pos] = t.steps ? t.steps[slot * t.step_pitch] : 0;
       }
     }
   }

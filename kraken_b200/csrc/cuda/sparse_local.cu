@@ -259,13 +259,15 @@ __device__ __forceinline__ uint64_t canonical_id(uint64_t id) { return id == kEm
 // before, 185 us now; 1.7 M ids, 0.55 M distinct: 102 and 58 us.
 
 // First kernel: every occurrence finds or claims its id's entry; the winner numbers the id.  first[i] = the winner's
-// index for the others, ~entry for the winner itself; pos[i] = the number, written by winners only.  One id per thread:
+// index for the others, ~entry for the winner itself; pos[i] = the number, written by winners only, like the unique list
+// and win.  One id per thread:
 // two or four were slower (3.4 M ids: 80, 85 and 107 us), the claims of a thread wait for one another.  The first look
 // at an entry may be a stale one from L1, where the entries of frequent ids stay: an entry only ever goes from free to
 // claimed within a launch, and a claim is made by compare-and-swap.
 __global__ void __launch_bounds__(kThreads)
 local_insert_kernel(const int64_t* __restrict__ ids, int n, int* set, uint32_t hbits, int* __restrict__ first,
-                    int* __restrict__ pos, int* cnt, int* status) {
+                    int* __restrict__ pos, int* cnt, int64_t* __restrict__ uniq, int* __restrict__ win, int cap_u,
+                    int* status) {
   pdl_enter();
   constexpr int kWarps = kThreads / 32;
   __shared__ int s_cnt[kWarps];
@@ -273,8 +275,9 @@ local_insert_kernel(const int64_t* __restrict__ ids, int n, int* set, uint32_t h
   const int i = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t mask = static_cast<uint32_t>((1ull << hbits) - 1);
   bool won = false;
+  uint64_t id = 0;
   if (i < n) {
-    uint64_t id = static_cast<uint64_t>(ids[i]);
+    id = static_cast<uint64_t>(ids[i]);
     if (id == kEmptyKey) set_status(status, err::kBadArgument);  // reserved: reported, then treated as its neighbour
     id = canonical_id(id);
     uint32_t slot = static_cast<uint32_t>(SlotHash(id ^ kDedupSalt, hbits));
@@ -309,7 +312,14 @@ local_insert_kernel(const int64_t* __restrict__ ids, int n, int* set, uint32_t h
     for (int w = 0; w < kWarps; ++w) s_cnt[w] += start;
   }
   __syncthreads();
-  if (won) pos[i] = s_cnt[warp] + __popc(winners & ((1u << lane) - 1u));
+  if (won) {
+    const int u = s_cnt[warp] + __popc(winners & ((1u << lane) - 1u));
+    pos[i] = u;
+    if (u < cap_u) {
+      uniq[u] = static_cast<int64_t>(id);
+      win[u] = i;
+    }
+  }
 }
 
 // Rows that the warp's lanes have just created (bit set in `todo`, slot and id per lane), initialised by the whole
@@ -342,21 +352,23 @@ __device__ __forceinline__ void init_created(const TableView& t, unsigned todo, 
   }
 }
 
-// Second kernel, with the table probe: every occurrence learns its unique id's number; the winner also writes the
-// unique list, empties the set's entry, and finds (or, with `insert`, claims and initialises) the row.  The block that
-// finishes last zeroes `cnt` for the next call and counts the lookup.  The ids do not pass through the inbox, and no
-// block ends on a system-scope fence.
+// Second kernel, with the table probe: every occurrence learns its unique id's number, a winner empties its entry of the
+// set, and thread u finds (or, with `insert`, claims and initialises) the row of unique id u.  The probe is the long chain
+// of this kernel, a random access to HBM or more; as the winner's own work it held every warp with a winner among its lanes
+// (nearly all of them, where a third of the occurrences win), over unique ids it is done by full warps and by no more of
+// them than there are ids: 8.6 M ids, 3.2 M distinct, 211 us before and 167 us so; 3.4 M, 2.3 M distinct, 112 and 103 us.
+// The block that finishes last zeroes `cnt` for the next call and counts the lookup.  The ids do not pass through the inbox,
+// and no block ends on a system-scope fence.
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
-local_resolve_kernel(const int64_t* __restrict__ ids, int n, int* __restrict__ set, const int* __restrict__ first,
-                     const int* __restrict__ pos, int* cnt, int* off, int64_t* __restrict__ uniq, int* __restrict__ inv,
-                     int* __restrict__ win, int cap_u, TableView t, int* __restrict__ slot_cache, int cap_s, int insert,
+local_resolve_kernel(int n, int* __restrict__ set, const int* __restrict__ first, const int* __restrict__ pos, int* cnt,
+                     int* off, const int64_t* __restrict__ uniq, int* __restrict__ inv, int cap_u, TableView t, int* __restrict__ slot_cache, int cap_s, int insert,
                      uint32_t* epoch, uint32_t* done, int* status, int chunks, int lpr) {
   pdl_enter();
+  const int U = *cnt;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     // more unique ids than the channel's buffers hold: reported and clamped, so that no later kernel indexes
     // past a buffer (the step's result is then invalid, not its memory)
-    const int U = *cnt;
     if (U > cap_u || U > cap_s) set_status(status, err::kInboxOverflow);
     off[0] = 0;
     off[1] = min(U, cap_u);
@@ -369,28 +381,21 @@ local_resolve_kernel(const int64_t* __restrict__ ids, int n, int* __restrict__ s
     const int f = first[i];
     const int u = pos[f < 0 ? i : f];
     inv[i] = u < cap_u ? u : 0;
-    if (f < 0) {
-      id = canonical_id(static_cast<uint64_t>(ids[i]));
-      set[~f] = -1;  // leave the set empty for the next call
-      if (u < cap_u) {
-        uniq[u] = static_cast<int64_t>(id);
-        win[u] = i;
-        if (u < cap_s) {
-          slot = table_find_or_insert(t, id, insert != 0, &created);
-          if (slot < 0 && !insert) set_status(status, err::kSparseIdNotExist);
-          slot_cache[u] = slot;
-        }
-      }
-    }
+    if (f < 0) set[~f] = -1;  // leave the set empty for the next call
+  }
+  if (i < min(U, min(cap_u, cap_s))) {
+    id = static_cast<uint64_t>(uniq[i]);
+    slot = table_find_or_insert(t, id, insert != 0, &created);
+    if (slot < 0 && !insert) set_status(status, err::kSparseIdNotExist);
+    slot_cache[i] = slot;
   }
   const unsigned todo = __ballot_sync(0xffffffffu, created);
   if (todo) {
     if ((threadIdx.x & 31) == __ffs(todo) - 1) atomicAdd(t.size, __popc(todo));
     init_created<VEC>(t, todo, slot, id, chunks, lpr);
   }
+  __syncthreads();  // every thread of the block has read the count, so the last block to arrive may clear it
   if (threadIdx.x == 0) {
-    // block 0 has read the count before it arrives here, so the last to arrive may clear it
-    if (blockIdx.x == 0) __threadfence();
     if (atomicAdd(done, 1u) == gridDim.x - 1) {
       *done = 0;
       *cnt = 0;
@@ -546,10 +551,10 @@ void local_lookup(const int64_t* ids, int n, LocalScratch sc, int* cnt, int* off
   const dim3 grid((n + kThreads - 1) / kThreads);
   const bool early = grid.x < kFullGrid;
   launch_pdl_if(early, local_insert_kernel, grid, dim3(kThreads), 0, stream, ids, n, sc.set, sc.hbits, sc.first, sc.pos, cnt,
-                &ctrl->status);
+                uniq, sc.win, cap_u, &ctrl->status);
   auto kernel = g.vec == 4 ? local_resolve_kernel<4> : local_resolve_kernel<1>;
-  launch_pdl_if(early, kernel, grid, dim3(kThreads), 0, stream, ids, n, sc.set, static_cast<const int*>(sc.first),
-                static_cast<const int*>(sc.pos), cnt, off, uniq, inv, sc.win, cap_u, to_view(table), slot_cache, cap_s,
+  launch_pdl_if(early, kernel, grid, dim3(kThreads), 0, stream, n, sc.set, static_cast<const int*>(sc.first),
+                static_cast<const int*>(sc.pos), cnt, off, static_cast<const int64_t*>(uniq), inv, cap_u, to_view(table), slot_cache, cap_s,
                 insert ? 1 : 0, &ctrl->pull_epoch, &ctrl->done[0], &ctrl->status, g.chunks, g.lpr);
 }
 

@@ -227,6 +227,48 @@ void bind_dense(py::module_& m) {
                         dxp, lddx, dw.data_ptr<float>(), optr<float>(db), cur_stream());
     check_launch("rowdot_backward");
   });
+  m.def("head_supported", [](const torch::Tensor& x, const torch::Tensor& w, const c10::optional<torch::Tensor>& dw) {
+    return x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2 && x.stride(1) == 1 && w.is_cuda() &&
+           w.scalar_type() == torch::kFloat32 && w.dim() == 2 && w.is_contiguous() && w.size(1) == x.size(1) &&
+           cu::head_supported(x.data_ptr(), x.stride(0), w.data_ptr(), x.size(1), w.size(0)) &&
+           (!dw.has_value() || (dw->is_cuda() && dw->scalar_type() == torch::kFloat32 && dw->is_contiguous() &&
+                                dw->numel() == w.numel() && reinterpret_cast<uintptr_t>(dw->data_ptr()) % 16 == 0));
+  }, py::arg("x"), py::arg("w"), py::arg("dw") = py::none());
+  m.def("head_forward", [bf](const torch::Tensor& x, const torch::Tensor& w, const torch::Tensor& bias, const torch::Tensor& y) {
+    TORCH_CHECK(cu::head_supported(x.data_ptr(), x.stride(0), w.data_ptr(), x.size(1), w.size(0)) && w.size(1) == x.size(1),
+                "head_forward: unsupported operands");
+    TORCH_CHECK(y.is_cuda() && y.scalar_type() == torch::kFloat32 && y.is_contiguous() &&
+                    y.numel() == x.size(0) * w.size(0) && bias.is_cuda() && bias.is_contiguous() &&
+                    bias.scalar_type() == torch::kFloat32 && bias.numel() == w.size(0),
+                "head_forward: shape mismatch");
+    cu::head_forward(bf(x), x.stride(0), w.data_ptr<float>(), bias.data_ptr<float>(), x.size(0), x.size(1), w.size(0),
+                     y.data_ptr<float>(), cur_stream());
+    check_launch("head_forward");
+  });
+  m.def("head_backward", [bf](const torch::Tensor& x, const torch::Tensor& w, const torch::Tensor& g, bool relu_mask,
+                              const c10::optional<torch::Tensor>& dx, const torch::Tensor& dw, const torch::Tensor& db) {
+    TORCH_CHECK(cu::head_supported(x.data_ptr(), x.stride(0), w.data_ptr(), x.size(1), w.size(0)) && w.size(1) == x.size(1),
+                "head_backward: unsupported operands");
+    TORCH_CHECK(g.is_cuda() && g.scalar_type() == torch::kFloat32 && g.is_contiguous() && g.numel() == x.size(0) * w.size(0),
+                "g must be a contiguous CUDA f32 [M, classes]");
+    TORCH_CHECK(dw.scalar_type() == torch::kFloat32 && dw.is_contiguous() && dw.numel() == w.numel() &&
+                    reinterpret_cast<uintptr_t>(dw.data_ptr()) % 16 == 0 && db.scalar_type() == torch::kFloat32 &&
+                    db.is_contiguous() && db.numel() == w.size(0),
+                "bad dw / db");
+    __nv_bfloat16* dxp = nullptr;
+    int lddx = 0;
+    if (dx.has_value()) {
+      TORCH_CHECK(dx->is_cuda() && dx->scalar_type() == torch::kBFloat16 && dx->dim() == 2 && dx->stride(1) == 1 &&
+                      dx->size(0) == x.size(0) && dx->size(1) == x.size(1) && dx->stride(0) % 4 == 0 &&
+                      reinterpret_cast<uintptr_t>(dx->data_ptr()) % 8 == 0,
+                  "bad dx");
+      dxp = reinterpret_cast<__nv_bfloat16*>(dx->data_ptr());
+      lddx = dx->stride(0);
+    }
+    cu::head_backward(bf(x), x.stride(0), w.data_ptr<float>(), g.data_ptr<float>(), x.size(0), x.size(1), w.size(0),
+                      relu_mask, dxp, lddx, dw.data_ptr<float>(), db.data_ptr<float>(), cur_stream());
+    check_launch("head_backward");
+  });
   // All matrices in as few launches as possible, their bf16 copies (and transposes) in ONE buffer, which is returned
   // with the views so that a caller on another stream has one tensor to record.
   m.def("cast_weights", [](const std::vector<torch::Tensor>& ws, bool transpose) {

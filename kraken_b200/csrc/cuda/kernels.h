@@ -269,6 +269,15 @@ void cast_weights(CastBatch b, cudaStream_t stream);
 void rowdot_forward(const __nv_bfloat16* x, int ldx, const float* w, const float* bias, const float* addend, int M,
                     int K, float* y, cudaStream_t stream);
 // Its backward: dx (optional, bf16, optionally masked by x > 0), dw[K] += ..., db[0] += sum(dy).
+// Linear layer with up to kMaxHead outputs on bf16 activations, everything else fp32: y [M, classes] = x w^T + bias, and its
+// backward (dw and db are added to, dx may be null).  head_supported: whether the kernels take these operands.
+constexpr int kMaxHead = 16;
+bool head_supported(const void* x, int ldx, const void* w, int K, int classes);
+void head_forward(const __nv_bfloat16* x, int ldx, const float* w, const float* bias, int M, int K, int classes, float* y,
+                  cudaStream_t stream);
+void head_backward(const __nv_bfloat16* x, int ldx, const float* w, const float* g, int M, int K, int classes,
+                   bool relu_mask, __nv_bfloat16* dx, int lddx, float* dw, float* db, cudaStream_t stream);
+
 void rowdot_backward(const __nv_bfloat16* x, int ldx, const float* w, const float* dy, int M, int K, bool relu_mask,
                      __nv_bfloat16* dx, int lddx, float* dw, float* db, cudaStream_t stream);
 

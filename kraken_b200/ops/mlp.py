@@ -121,7 +121,8 @@ def check_gemm_status(device: torch.device) -> None:
 def supported(in_features: int, sizes: Sequence[int]) -> bool:
     """Whether the hidden layers meet the TMA pitch rule (widths in multiples of 8 elements).
     The last layer may have any width: 1 runs as a row-dot kernel, a multiple of 8 on the
-    tensor cores, anything else (a 10-class head, say) as a small fp32 matmul."""
+    tensor cores, another one up to 16 (a 10-class head, say) in fp32 kernels of its own,
+    anything else as a small fp32 matmul of the library."""
     dims = [in_features] + list(sizes)
     return len(sizes) >= 1 and all(d % 8 == 0 for d in dims[:-1])
 
@@ -171,8 +172,12 @@ class _FusedMLP(torch.autograd.Function):
             counters.add()
             C.linear_forward(h, wl.to(torch.bfloat16), bl, False, y, st)
             out = y.float()
+        elif C.head_supported(h, wl) and bl.is_contiguous():
+            out = torch.empty((M, wl.shape[0]), dtype=torch.float32, device=dev)
+            counters.add()
+            C.head_forward(h, wl, bl, out)
         else:
-            out = torch.addmm(bl, h.float(), wl.t())  # narrow odd-width head: library fp32 matmul
+            out = torch.addmm(bl, h.float(), wl.t())  # wider odd-width head: library fp32 matmul
         if addend is not None:
             out = out + addend.reshape(M, 1).to(out.dtype)
         ctx.acts, ctx.ws, ctx.bs, ctx.n_layers, ctx.wts, ctx.masks = acts, ws, bs, n_layers, wts, masks
@@ -202,6 +207,11 @@ class _FusedMLP(torch.autograd.Function):
             counters.add()
             C.rowdot_backward(h_last, wl.detach().reshape(-1).contiguous(), dy, L > 1, dh,
                               _grad_target(wl).view(-1), _grad_target(bs[-1]))
+        elif (wl.shape[0] % 8 != 0 and C.head_supported(h_last, wl.detach(), _grad_target(wl))
+              and _grad_target(bs[-1]).is_contiguous()):
+            dh = torch.empty_like(h_last) if need_dx_last else None
+            counters.add()
+            C.head_backward(h_last, wl.detach(), gout.float().contiguous(), L > 1, dh, _grad_target(wl), _grad_target(bs[-1]))
         elif wl.shape[0] % 8 != 0:
             g32 = gout.float()
             h32 = h_last.float()

@@ -330,6 +330,9 @@ struct AsyncRead {
   }
 };
 
+// Rows narrower than this are not pooled into an MLP input: their pushes sum every gradient in float32.
+constexpr int kMinPooledInput = 8;
+
 // Rows of floats at any pitch, each row contiguous.
 void need_rows(const torch::Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.dim() == 2 &&
@@ -1450,6 +1453,26 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                             patch_value, ptr<float>(out), cur_stream());
           check_launch("local_combine");
         });
+  m.def("local_combine_input",
+        [](const cu::TableHost& table, const torch::Tensor& inv, const torch::Tensor& slot_cache,
+           const torch::Tensor& bag_offsets, const c10::optional<torch::Tensor>& bag_mean, float patch_value, int fields,
+           const torch::Tensor& dense, const torch::Tensor& x) {
+          const int k = static_cast<int>(bag_offsets.numel()) - 1;
+          need_cuda(x, "x", torch::kBFloat16);
+          need_cuda(dense, "dense", torch::kFloat32);
+          TORCH_CHECK(table.dim % 4 == 0 && table.dim >= kMinPooledInput && fields > 0 && k % fields == 0,
+                      "bags must be whole samples of rows of a multiple of 4 floats, ", kMinPooledInput, " at least");
+          TORCH_CHECK(x.dim() == 2 && dense.dim() == 2 && x.size(0) == k / fields && dense.size(0) == k / fields &&
+                          x.size(1) % 4 == 0 && x.size(1) >= fields * table.dim + dense.size(1) &&
+                          reinterpret_cast<uintptr_t>(x.data_ptr()) % 8 == 0,
+                      "local_combine_input: shape mismatch");
+          const cu::PooledInput in{reinterpret_cast<__nv_bfloat16*>(x.data_ptr()), static_cast<int>(x.size(1)), fields,
+                                   ptr<float>(dense), static_cast<int>(dense.size(1))};
+          cu::local_combine_input(table, ptr<int>(inv), ptr<int>(slot_cache), static_cast<int>(slot_cache.numel()),
+                                  ptr<int64_t>(bag_offsets), k, optr<uint8_t>(bag_mean), patch_value, in, cur_stream());
+          check_launch("local_combine_input");
+        });
+  m.attr("MIN_POOLED_INPUT") = kMinPooledInput;
   m.def("local_push_update", [](const cu::TableHost& table, const torch::Tensor& ugrad, const torch::Tensor& off,
                                 const torch::Tensor& slot_cache, int max_n, const OptimPOD& optim,
                                 const torch::Tensor& lr) {
@@ -1466,24 +1489,38 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            const c10::optional<torch::Tensor>& weights, bool mean, const c10::optional<torch::Tensor>& bag_mean,
            const torch::Tensor& lookup_ctrl, const torch::Tensor& multi, const c10::optional<torch::Tensor>& bag_of,
            const torch::Tensor& ugrad, const torch::Tensor& off, const torch::Tensor& slot_cache, const OptimPOD& optim,
-           const torch::Tensor& lr) {
-          need_cuda(grads, "grads", torch::kFloat32);
+           const torch::Tensor& lr, int fields) {
+          const bool half = fields > 0;  // the gradient of local_combine_input's x
+          need_cuda(grads, "grads", half ? torch::kBFloat16 : torch::kFloat32);
           need_cuda(ugrad, "ugrad", torch::kFloat32);
           need_cuda(lr, "lr", torch::kFloat32);
           const int k = bag_offsets.has_value() ? static_cast<int>(bag_offsets->numel()) - 1 : 0;
-          TORCH_CHECK(grads.numel() == static_cast<int64_t>(bag_offsets.has_value() ? k : n) * table.dim,
-                      "grads has the wrong size");
+          if (half) {
+            TORCH_CHECK(grads.dim() == 2 && bag_offsets.has_value() && !weights.has_value() && table.dim % 4 == 0 &&
+                            table.dim >= kMinPooledInput && grads.size(0) * fields == k && grads.size(1) % 4 == 0 &&
+                            grads.size(1) >= fields * table.dim && reinterpret_cast<uintptr_t>(grads.data_ptr()) % 8 == 0,
+                        "grads is not the gradient of a pooled MLP input");
+          } else {
+            TORCH_CHECK(grads.numel() == static_cast<int64_t>(bag_offsets.has_value() ? k : n) * table.dim,
+                        "grads has the wrong size");
+          }
           TORCH_CHECK(ugrad.dim() == 2 && ugrad.size(1) == table.dim && inv.numel() >= n && first.numel() >= n &&
                           multi.numel() >= ugrad.size(0) &&
-                          (!bag_offsets.has_value() || (bag_of.has_value() && bag_of->numel() >= ugrad.size(0))),
+                          (!bag_offsets.has_value() || (bag_of.has_value() && bag_of->is_contiguous() && bag_of->numel() >= 2 * ugrad.size(0))),
                       "the lookup's buffers do not fit this channel");
-          cu::LocalPush p{ptr<float>(grads), ptr<int>(inv), ptr<int>(first), ptr<int>(win), optr<int64_t>(bag_offsets), k,
+          cu::LocalPush p{half ? nullptr : ptr<float>(grads),
+                          half ? reinterpret_cast<const __nv_bfloat16*>(grads.data_ptr()) : nullptr,
+                          half ? static_cast<int>(grads.size(1)) : 0, fields, ptr<int>(inv), ptr<int>(first), ptr<int>(win), optr<int64_t>(bag_offsets), k,
                           optr<float>(weights), mean, optr<uint8_t>(bag_mean), ctrl_ptr(lookup_ctrl),
                           reinterpret_cast<uint32_t*>(ptr<int>(multi)), optr<int>(bag_of)};
           cu::local_push(table, p, ptr<float>(ugrad), ptr<int>(off), ptr<int>(slot_cache), n,
                          static_cast<int>(slot_cache.numel()), optim, ptr<float>(lr), cur_stream());
           check_launch("local_push");
-        });
+        },
+        py::arg("table"), py::arg("grads"), py::arg("inv"), py::arg("first"), py::arg("win"), py::arg("n"),
+        py::arg("bag_offsets"), py::arg("weights"), py::arg("mean"), py::arg("bag_mean"), py::arg("lookup_ctrl"),
+        py::arg("multi"), py::arg("bag_of"), py::arg("ugrad"), py::arg("off"), py::arg("slot_cache"), py::arg("optim"),
+        py::arg("lr"), py::arg("fields") = 0);
 
   // ---------------- one exchange for several tables of one row width
   m.def("group_table_views", [](const std::vector<cu::TableHost>& tables) {

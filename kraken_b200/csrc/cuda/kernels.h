@@ -141,6 +141,18 @@ void local_gather(TableHost table, const int* off, const int* slot_cache, int ma
 void local_combine(TableHost table, const int* inv, const int* slot_cache, int n, int cap_s, const int64_t* bag_offsets,
                    int k, const float* weights, bool mean, const uint8_t* bag_mean, float patch_value, float* out,
                    cudaStream_t stream);
+// local_combine of bags into the input of an MLP: bag b = field b % fields of sample b / fields.  x [k / fields, ldx] bf16
+// receives the pooled rows of a sample's fields back to back (4 floats at a time: dim % 4 == 0, ldx % 4 == 0), behind them
+// its nd dense features and zeros.
+struct PooledInput {
+  __nv_bfloat16* x;
+  int ldx;
+  int fields;
+  const float* dense;
+  int nd;
+};
+void local_combine_input(TableHost table, const int* inv, const int* slot_cache, int cap_s, const int64_t* bag_offsets, int k,
+                         const uint8_t* bag_mean, float patch_value, const PooledInput& in, cudaStream_t stream);
 // push_dispatch + push_apply without the inbox: updates the rows of the U = off[1] unique ids of the lookup from
 // ugrad and zeroes it.  slot_cache[u] is the row of unique id u (u < cap_s); max_n bounds U.
 void local_push_update(TableHost table, float* ugrad, const int* off, const int* slot_cache, int max_n, int cap_s,
@@ -150,6 +162,8 @@ void local_push_update(TableHost table, float* ugrad, const int* off, const int*
 // into ugrad but read from `grads` by the update.
 struct LocalPush {
   const float* grads;          // [n, dim], or [nbags, dim] with bag_offsets
+  const __nv_bfloat16* grads16;  // instead of them, for bags: gradient of the x of local_combine_input
+  int ld16, fields;
   const int* inv;              // inv, first and win are the lookup's
   const int* first;
   const int* win;
@@ -160,7 +174,7 @@ struct LocalPush {
   const uint8_t* bag_mean;
   const Ctrl* lookup;          // control block of the channel that did the dedup
   uint32_t* multi;             // [cap_u] of this channel: number of the last lookup in which the id occurred more than once
-  int* bag_of;                 // [cap_u] scratch (bags only)
+  int* bag_of;                 // [cap_u][2] scratch (bags only)
 };
 void local_push(TableHost table, const LocalPush& p, float* ugrad, const int* off, const int* slot_cache, int n, int cap_s,
                 OptimPOD optim, const float* lr, cudaStream_t stream);

@@ -3,6 +3,8 @@
 // With one rank there is nobody to exchange with: the rank that looks ids up owns every row.  The
 // kernels of sparse.cu would still move every row through the channel's inboxes, because that is what
 // peers read and write; these move each row once.
+#include <cuda_bf16.h>
+
 #include "sparse_common.cuh"
 
 namespace kb {
@@ -25,22 +27,42 @@ constexpr int kDirectDim = 8;
 // Where the update finds the gradient of every id's first occurrence.
 struct DirectSource {
   const float* grads;          // [n, dim], or [bags, dim]
+  const __nv_bfloat16* grads16;  // of bags that were pooled into an MLP input: bag b = field b % fields of row b / fields
+  int ld16, fields;
   const int64_t* bag_offsets;  // null: one gradient row per occurrence
   int nbags;
   const float* weights;        // per occurrence of a bag, or null
   const uint8_t* bag_mean;
   int mean;
   const int* win;              // unique id -> its first occurrence
-  // Unique id -> the bag of its first occurrence (null without bags).  Occurrences may lie outside every bag (offsets
-  // that start behind the first id or end before the last); the entry of such an id is what an earlier push left there,
-  // of ANY number of bags, and holds only if that bag is one of this push and contains the occurrence.
-  const int* bag_of;
+  // Unique id -> {bag of its first occurrence, factor of that bag's gradient as bits of a float} (null without bags); bag -1
+  // where the occurrence lies outside every bag (offsets that start behind the first id or end before the last).  Every push
+  // writes the entries of all of its unique ids.
+  const int2* bag_of;
   const uint32_t* multi;       // == *epoch: the id occurs more than once
   const uint32_t* epoch;       // number of the lookup
   __device__ __forceinline__ float bag_scale(int b) const {
     const int64_t len = bag_offsets[b + 1] - bag_offsets[b];
     const bool is_mean = bag_mean ? bag_mean[b] != 0 : mean != 0;
     return is_mean && len > 0 ? 1.f / static_cast<float>(len) : 1.f;
+  }
+  // where the gradient of row `i` begins, and VEC elements of it
+  template <bool B16>
+  __device__ __forceinline__ size_t row(int i, int dim) const {
+    if (!B16) return static_cast<size_t>(i) * dim;
+    const int sample = i / fields;
+    return static_cast<size_t>(sample) * ld16 + (i - sample * fields) * dim;
+  }
+  template <int VEC, bool B16>
+  __device__ __forceinline__ typename Vec<VEC>::T ldcg(size_t at) const {
+    if constexpr (B16) {
+      static_assert(VEC == 4, "bf16 gradients go by four");
+      const uint2 v = __ldcg(reinterpret_cast<const uint2*>(grads16 + at));
+      return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xFFFF0000u), __uint_as_float(v.y << 16),
+                         __uint_as_float(v.y & 0xFFFF0000u));
+    } else {
+      return Vec<VEC>::ldcg(grads + at);
+    }
   }
 };
 
@@ -64,7 +86,7 @@ struct DirectSource {
 // rate.  A first occurrence outside every bag has no gradient: the row is updated with the sum of the others, or with
 // zeros.
 constexpr int kUpdateThreads = 128;
-enum GradSource { kFromSum = 0, kFromRows = 1, kFromBags = 2 };
+enum GradSource { kFromSum = 0, kFromRows = 1, kFromBags = 2, kFromBags16 = 3 };
 
 template <int VEC, int OPT, int FROM>
 __global__ void __launch_bounds__(kUpdateThreads, 9)
@@ -73,6 +95,7 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
                     const float* __restrict__ lr_ptr, int cap_s, int chunks, int tpr) {
   pdl_enter();
   using V = Vec<VEC>;
+  constexpr bool kBags = FROM == kFromBags || FROM == kFromBags16, kHalf = FROM == kFromBags16;
   const uint32_t now = FROM != kFromSum ? *so.epoch : 0;
   OptimPOD optim = optim_in;
   optim.type = OPT;
@@ -88,28 +111,25 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
   int u = blockIdx.x * rows + r;
   // what is known of a row before its data: its slot, the row of `grads`, whether there is a sum of others
   auto slot_of = [&](int v) { return active && v < limit ? slot_cache[v] : -1; };
+  // (one 8-byte entry: from win, the offsets, the means and the weights it was seven loads of each of a row's threads, and the
+  // multi-hot step, 3.2 M rows of 64 floats, took 2590 us instead of 2345)
   auto src_of = [&](int v) {
-    if (FROM == kFromSum || !active || v >= U) return 0;
-    return FROM == kFromBags ? so.bag_of[v] : so.win[v];
+    if (FROM == kFromSum || !active || v >= U) return make_int2(0, 0);
+    return kBags ? so.bag_of[v] : make_int2(so.win[v], 0);
   };
   auto many_of = [&](int v) { return active && v < U && (FROM == kFromSum || so.multi[v] == now); };
-  int slot = slot_of(u), from = src_of(u);
+  int slot = slot_of(u);
+  int2 from = src_of(u);
   bool many = many_of(u);
   for (int base = blockIdx.x * rows; base < U; base += stride, u += stride) {
-    const int next = slot_of(u + stride), next_from = src_of(u + stride);
+    const int next = slot_of(u + stride);
+    const int2 next_from = src_of(u + stride);
     const bool next_many = many_of(u + stride);
     const bool mine = active && u < U;
     float* const gu = ugrad + static_cast<size_t>(u) * t.dim;
-    const float* const gd = so.grads + static_cast<size_t>(from) * t.dim;
-    float scale = 1.f, weight = 1.f;
-    const bool in_grads = FROM == kFromRows || (FROM == kFromBags && from < so.nbags);
-    bool direct = in_grads;
-    if (FROM == kFromBags && mine && in_grads) {
-      const int i = so.win[u];
-      direct = so.bag_offsets[from] <= i && i < so.bag_offsets[from + 1];
-      scale = so.bag_scale(from);
-      if (so.weights) weight = so.weights[i];
-    }
+    const bool direct = FROM == kFromRows || (kBags && static_cast<unsigned>(from.x) < static_cast<unsigned>(so.nbags));
+    const size_t gd = FROM != kFromSum && direct ? so.template row<kHalf>(from.x, t.dim) : 0;
+    const float scale = __int_as_float(from.y);
     const size_t row = static_cast<size_t>(slot < 0 ? 0 : slot) * t.pitch;
     int* const counter = t.steps + static_cast<size_t>(slot < 0 ? 0 : slot) * t.step_pitch;
     // an id that was not found (reported by the lookup) has no row: its gradient is dropped
@@ -119,7 +139,7 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
     float g[VEC], d[VEC], w[VEC], a0[VEC], a1[VEC], a2[VEC];
     auto load = [&](int c) {
       *reinterpret_cast<typename V::T*>(g) = many ? V::ldcg(gu + c * VEC) : V::zero();
-      if (FROM != kFromSum) *reinterpret_cast<typename V::T*>(d) = in_grads ? V::ldcg(gd + c * VEC) : V::zero();
+      if (FROM != kFromSum) *reinterpret_cast<typename V::T*>(d) = direct ? so.template ldcg<VEC, kHalf>(gd + c * VEC) : V::zero();
       *reinterpret_cast<typename V::T*>(w) = V::ld(t.val + row + c * VEC);
       if (t.s[0]) *reinterpret_cast<typename V::T*>(a0) = V::ld(t.s[0] + row + c * VEC);
       if (t.s[1]) *reinterpret_cast<typename V::T*>(a1) = V::ld(t.s[1] + row + c * VEC);
@@ -137,7 +157,7 @@ local_update_kernel(TableView t, float* __restrict__ ugrad, const int* __restric
         if (c != c0) load(c);
         if (FROM != kFromSum && direct) {
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) g[e] += FROM == kFromBags ? d[e] * scale * weight : d[e];
+          for (int e = 0; e < VEC; ++e) g[e] += kBags ? d[e] * scale : d[e];
         }
 #pragma unroll
         for (int e = 0; e < VEC; ++e) UpdateElem(optim, lr, g[e], step, ab, w[e], a0[e], a1[e], a2[e]);
@@ -209,23 +229,30 @@ local_scatter_kernel(const int* __restrict__ inv, const int* __restrict__ first,
   }
 }
 
-template <int VEC>
+template <int VEC, bool B16>
 __global__ void __launch_bounds__(kThreads)
 local_bag_scatter_kernel(const int* __restrict__ inv, const int* __restrict__ first, DirectSource so, uint32_t* multi,
-                         int* __restrict__ bag_of, int nbags, int dim, int chunks, int tpr, float* ugrad) {
+                         int2* __restrict__ bag_of, int n, int nbags, int dim, int chunks, int tpr, float* ugrad) {
   pdl_enter();
   using V = Vec<VEC>;
   constexpr int kUnroll = 4;
   const uint32_t now = *so.epoch;
   const int rows = kThreads / tpr;
   const int g = threadIdx.x / tpr, c0 = threadIdx.x - g * tpr;
+  // ids in front of the first bag and behind the last: their first occurrences have no gradient
+  const int head = static_cast<int>(min(static_cast<int64_t>(n), so.bag_offsets[0]));
+  const int tail = static_cast<int>(max(static_cast<int64_t>(0), so.bag_offsets[nbags]));
+  for (int j = blockIdx.x * kThreads + threadIdx.x; j < head || j < n - tail; j += gridDim.x * kThreads) {
+    if (j < head && first[j] < 0) bag_of[inv[j]] = make_int2(-1, 0);
+    if (j < n - tail && first[tail + j] < 0) bag_of[inv[tail + j]] = make_int2(-1, 0);
+  }
   if (g >= rows) return;
   for (int b = blockIdx.x * rows + g; b < nbags; b += gridDim.x * rows) {
-    const int64_t lo = so.bag_offsets[b], hi = so.bag_offsets[b + 1];
+    const int lo = static_cast<int>(so.bag_offsets[b]), hi = static_cast<int>(so.bag_offsets[b + 1]);
     const float scale = so.bag_scale(b);
     for (int c = c0; c < chunks; c += tpr) {
-      const typename V::T v = V::scale(V::ld(so.grads + static_cast<size_t>(b) * dim + c * VEC), scale);
-      for (int64_t i0 = lo; i0 < hi; i0 += kUnroll) {
+      const typename V::T v = V::scale(so.template ldcg<VEC, B16>(so.template row<B16>(b, dim) + c * VEC), scale);
+      for (int i0 = lo; i0 < hi; i0 += kUnroll) {
         int u[kUnroll], f[kUnroll];
 #pragma unroll
         for (int q = 0; q < kUnroll; ++q) {
@@ -239,7 +266,7 @@ local_bag_scatter_kernel(const int* __restrict__ inv, const int* __restrict__ fi
             V::red(ugrad + static_cast<size_t>(u[q]) * dim + c * VEC, so.weights ? V::scale(v, so.weights[i0 + q]) : v);
             if (c == 0) multi[u[q]] = now;
           } else if (c == 0) {
-            bag_of[u[q]] = b;
+            bag_of[u[q]] = make_int2(b, __float_as_int(so.weights ? scale * so.weights[i0 + q] : scale));
           }
         }
       }
@@ -499,12 +526,16 @@ local_expand_kernel(TableView t, const int* __restrict__ inv, const int* __restr
 }
 
 // out[b] = pooled rows of bag b, read from the table where they are; four rows of a bag in flight per thread.  The
-// sum runs in the order of the occurrences, as in pull_combine_kernel.
-template <int VEC>
-__global__ void __launch_bounds__(kThreads)
+// sum runs in the order of the occurrences, as in pull_combine_kernel.  What it waits for is rows, so six blocks of it
+// are resident; five were a quarter slower (8.6 M rows of 64 floats: 305 and 392 us).
+//
+// INPUT: the pooled rows go out as what the first layer of an MLP reads (`in`), rounded here as its own conversion would
+// round them; the threads of a sample's last field also write its dense features and the zeros behind them.
+template <int VEC, bool INPUT>
+__global__ void __launch_bounds__(kThreads, VEC == 4 ? 6 : 8)
 local_pool_kernel(TableView t, const int* __restrict__ inv, const int* __restrict__ slot_cache, int cap_s, int chunks,
                   int tpr, const int64_t* __restrict__ bag_offsets, int nbags, const float* __restrict__ weights, int mean,
-                  const uint8_t* __restrict__ bag_mean, float patch_value, float* __restrict__ out) {
+                  const uint8_t* __restrict__ bag_mean, float patch_value, float* __restrict__ out, PooledInput in) {
   pdl_enter();
   using V = Vec<VEC>;
   constexpr int kUnroll = 4;
@@ -512,11 +543,11 @@ local_pool_kernel(TableView t, const int* __restrict__ inv, const int* __restric
   const int g = threadIdx.x / tpr, c0 = threadIdx.x - g * tpr;
   if (g >= rows) return;
   for (int b = blockIdx.x * rows + g; b < nbags; b += gridDim.x * rows) {
-    const int64_t lo = bag_offsets[b], hi = bag_offsets[b + 1];
+    const int lo = static_cast<int>(bag_offsets[b]), hi = static_cast<int>(bag_offsets[b + 1]);  // ids of a call: an int
     const bool is_mean = bag_mean ? bag_mean[b] != 0 : mean != 0;
     for (int c = c0; c < chunks; c += tpr) {
       typename V::T acc = V::zero();
-      for (int64_t r = lo; r < hi; r += kUnroll) {
+      for (int r = lo; r < hi; r += kUnroll) {
         int slot[kUnroll];
         typename V::T v[kUnroll];
 #pragma unroll
@@ -534,7 +565,23 @@ local_pool_kernel(TableView t, const int* __restrict__ inv, const int* __restric
         acc = V::fill(patch_value);
       else if (is_mean)
         acc = V::scale(acc, 1.f / static_cast<float>(hi - lo));
-      V::st(out + static_cast<size_t>(b) * t.dim + c * VEC, acc);
+      if constexpr (INPUT) {
+        const int sample = b / in.fields;
+        const __nv_bfloat162 lo2 = __floats2bfloat162_rn(acc.x, acc.y), hi2 = __floats2bfloat162_rn(acc.z, acc.w);
+        uint2 packed;
+        packed.x = *reinterpret_cast<const uint32_t*>(&lo2);
+        packed.y = *reinterpret_cast<const uint32_t*>(&hi2);
+        *reinterpret_cast<uint2*>(in.x + static_cast<size_t>(sample) * in.ldx + (b - sample * in.fields) * t.dim + c * VEC) =
+            packed;
+      } else {
+        V::st(out + static_cast<size_t>(b) * t.dim + c * VEC, acc);
+      }
+    }
+    if (INPUT && b % in.fields == in.fields - 1) {
+      const int sample = b / in.fields, base = in.fields * t.dim;
+      for (int j = c0; base + j < in.ldx; j += tpr)
+        in.x[static_cast<size_t>(sample) * in.ldx + base + j] =
+            __float2bfloat16(j < in.nd ? in.dense[static_cast<size_t>(sample) * in.nd + j] : 0.f);
     }
   }
 }
@@ -590,10 +637,21 @@ void local_combine(TableHost table, const int* inv, const int* slot_cache, int n
     launch_pdl_if(early, kernel, dim3(grid), dim3(kThreads), 0, stream, to_view(table), inv, slot_cache, cap_s, n, g.chunks,
                   tpr, out);
   } else {
-    auto kernel = g.vec == 4 ? local_pool_kernel<4> : local_pool_kernel<1>;
+    auto kernel = g.vec == 4 ? local_pool_kernel<4, false> : local_pool_kernel<1, false>;
     launch_pdl_if(early, kernel, dim3(grid), dim3(kThreads), 0, stream, to_view(table), inv, slot_cache, cap_s, g.chunks, tpr,
-                  bag_offsets, k, weights, mean ? 1 : 0, bag_mean, patch_value, out);
+                  bag_offsets, k, weights, mean ? 1 : 0, bag_mean, patch_value, out, PooledInput{});
   }
+}
+
+void local_combine_input(TableHost table, const int* inv, const int* slot_cache, int cap_s, const int64_t* bag_offsets, int k,
+                         const uint8_t* bag_mean, float patch_value, const PooledInput& in, cudaStream_t stream) {
+  if (k <= 0) return;
+  const RowGeom g = row_geom(table.dim);
+  const int tpr = g.chunks < kThreads ? g.chunks : kThreads;
+  const int grid = grid_for(k, kThreads / tpr, 148 * 16);
+  launch_pdl_if(grid < kFullGrid, local_pool_kernel<4, true>, dim3(grid), dim3(kThreads), 0, stream, to_view(table), inv,
+                slot_cache, cap_s, g.chunks, tpr, bag_offsets, k, static_cast<const float*>(nullptr), 0, bag_mean,
+                patch_value, static_cast<float*>(nullptr), in);
 }
 
 namespace {
@@ -604,10 +662,10 @@ void update_all(TableHost table, float* ugrad, const int* off, const int* slot_c
   const int tpr = g.chunks < kUpdateThreads ? g.chunks : kUpdateThreads;
   const int grid = grid_for(max_n, kUpdateThreads / tpr, 148 * 80);
   const TableView t = to_view(table);
-  if (g.vec == 4)
+  if (FROM == kFromBags16 || g.vec == 4)
     launch_local_update<4, FROM>(grid, stream, t, ugrad, off, slot_cache, so, optim, lr, cap_s, g.chunks, tpr);
   else
-    launch_local_update<1, FROM>(grid, stream, t, ugrad, off, slot_cache, so, optim, lr, cap_s, g.chunks, tpr);
+    launch_local_update<FROM == kFromBags16 ? 4 : 1, FROM>(grid, stream, t, ugrad, off, slot_cache, so, optim, lr, cap_s, g.chunks, tpr);
 }
 }  // namespace
 
@@ -626,24 +684,29 @@ void local_push(TableHost table, const LocalPush& p, float* ugrad, const int* of
     return;
   }
   DirectSource so{};
-  so.grads = p.grads, so.bag_offsets = p.bag_offsets, so.nbags = p.nbags;
+  so.grads = p.grads, so.grads16 = p.grads16, so.ld16 = p.ld16, so.fields = p.fields;
+  so.bag_offsets = p.bag_offsets, so.nbags = p.nbags;
   so.weights = p.weights, so.bag_mean = p.bag_mean, so.mean = p.mean ? 1 : 0;
   so.win = p.win, so.multi = p.multi, so.epoch = &p.lookup->pull_epoch;
-  so.bag_of = p.bag_of;
+  so.bag_of = reinterpret_cast<const int2*>(p.bag_of);
   const RowGeom g = row_geom(table.dim);
   const int tpr = g.chunks < kThreads ? g.chunks : kThreads;
   const int grid = grid_for(bags ? p.nbags : n, kThreads / tpr, 148 * 16);
   if (bags) {
-    auto kernel = g.vec == 4 ? local_bag_scatter_kernel<4> : local_bag_scatter_kernel<1>;
+    auto kernel = p.grads16 != nullptr ? local_bag_scatter_kernel<4, true>
+                  : g.vec == 4         ? local_bag_scatter_kernel<4, false>
+                                       : local_bag_scatter_kernel<1, false>;
     if (p.nbags > 0)
-      launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, p.inv, p.first, so, p.multi, p.bag_of,
-                    p.nbags, table.dim, g.chunks, tpr, ugrad);
+      launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, p.inv, p.first, so, p.multi,
+                    reinterpret_cast<int2*>(p.bag_of), n, p.nbags, table.dim, g.chunks, tpr, ugrad);
   } else {
     auto kernel = g.vec == 4 ? local_scatter_kernel<4> : local_scatter_kernel<1>;
     launch_pdl_if(grid < kFullGrid, kernel, dim3(grid), dim3(kThreads), 0, stream, p.inv, p.first, so, p.multi, n, table.dim,
                   g.chunks, tpr, ugrad);
   }
-  if (bags)
+  if (p.grads16 != nullptr)
+    update_all<kFromBags16>(table, ugrad, off, slot_cache, so, n, cap_s, optim, lr, stream);
+  else if (bags)
     update_all<kFromBags>(table, ugrad, off, slot_cache, so, n, cap_s, optim, lr, stream);
   else
     update_all<kFromRows>(table, ugrad, off, slot_cache, so, n, cap_s, optim, lr, stream);

@@ -57,6 +57,18 @@ class WideAndDeep(torch.nn.Module):
         return wide + self.mlp(torch.cat(parts, dim=1)).squeeze(-1) + self.bias
 
 
+def _stock(module, cls) -> bool:
+    """Whether calling ``module`` runs ``cls.forward`` and nothing else: the class itself, no hooks."""
+    return (type(module) is cls and "forward" not in vars(module) and not module._forward_pre_hooks
+            and not module._forward_hooks and not module._backward_hooks and not module._backward_pre_hooks
+            and not _has_any_global_hook())
+
+
+def _stock_mlp(mlp) -> bool:
+    """Whether ``mlp`` takes a bfloat16 input as it takes the float32 one that it would round."""
+    return _stock(mlp, MLP) and mlp.use_tensor_cores and mlp.layers[0].weight.is_cuda
+
+
 class MultiHotWideAndDeep(torch.nn.Module):
     """``forward(dense, bags)`` with ``bags`` = one JaggedTensor whose bags are laid out
     sample-major, field-minor: bag ``b * num_fields + f`` holds sample b's ids of field f."""
@@ -86,6 +98,10 @@ class MultiHotWideAndDeep(torch.nn.Module):
         if hasattr(eng, "pull_sparse_pooled"):
             # both tables look the same ids up: where the wide one's lookup is known to be that, its dedup serves both
             share = self.wide.embedding.sparse_table.table_id() if self._wide_is_one_lookup(bags) else None
+            if self._pools_into_mlp(eng, dense, B):
+                x = _PooledInput.apply(self.deep.sparse_table, bags.values(), bags.offsets(), self.field_is_mean.repeat(B),
+                                       dense, self.num_fields, self.mlp_in, share)
+                return wide + self.mlp(x, input_grad_cols=self.num_fields * self.dim).squeeze(-1) + self.bias
             pooled = _PooledLookup.apply(self.deep.sparse_table, bags.values(), bags.offsets(),
                                          self.field_is_mean.repeat(B), share)
         else:
@@ -102,6 +118,13 @@ class MultiHotWideAndDeep(torch.nn.Module):
             parts.append(torch.zeros(B, pad, dtype=pooled.dtype, device=pooled.device))
         return wide + self.mlp(torch.cat(parts, dim=1)).squeeze(-1) + self.bias
 
+    def _pools_into_mlp(self, eng, dense: torch.Tensor, samples: int) -> bool:
+        """Whether the lookup can write the MLP's input itself: what stands between them is the stock module without
+        hooks on the tensor cores, and nothing else wants the float32 input or its gradient."""
+        return (hasattr(eng, "pools_into_input") and eng.pools_into_input(self.deep.sparse_table.table_id())
+                and _stock_mlp(self.mlp) and dense.dtype == torch.float32 and not dense.requires_grad and dense.dim() == 2
+                and dense.shape[0] == samples and dense.shape[1] <= self.mlp_in - self.num_fields * self.dim)
+
     def _wide_is_one_lookup(self, bags: kk.JaggedTensor) -> bool:
         """Whether calling ``self.wide`` on ``bags`` has been one fused lookup of exactly their ids, with nothing behind
         it: the module as it was made, without hooks that might change the ids or look others up, on the fused path."""
@@ -109,6 +132,27 @@ class MultiHotWideAndDeep(torch.nn.Module):
         return (type(w) is kk.JaggedEmbedding and type(w.embedding) is kk.Embedding and "forward" not in vars(w)
                 and not w._forward_pre_hooks and not w._forward_hooks and not _has_any_global_hook()
                 and w.fused(bags))
+
+
+class _PooledInput(torch.autograd.Function):
+    """Fused bag lookup that ends in the bfloat16 input of the MLP: pooled rows, dense features, zeros (one GPU).  The
+    MLP would round its input to bfloat16 and hands back a bfloat16 gradient in any case; as float32 both crossed memory
+    three times more, in a concatenation and conversions (4096 samples of 100 fields x 64: 210 us of a step of 2800)."""
+
+    @staticmethod
+    def forward(ctx, sparse_table, values, offsets, bag_mean, dense, fields, width, share_with):
+        from ..pytorch import native
+        eng = native.engine()
+        tid = sparse_table.table_id()
+        x, ticket = eng.pull_sparse_input(tid, values, offsets, bag_mean, dense, fields, width, share_with=share_with)
+        ctx.state = (eng, tid, ticket, values, fields)
+        return x
+
+    @staticmethod
+    def backward(ctx, grad):
+        eng, tid, ticket, values, fields = ctx.state
+        eng.push_sparse_pooled(tid, ticket, grad, values, fields=fields)
+        return None, None, None, None, None, None, None, None
 
 
 class _PooledLookup(torch.autograd.Function):

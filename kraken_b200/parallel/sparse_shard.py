@@ -630,15 +630,28 @@ class SparseChannel:
             self.launches += 3  # gather, response wait, combine
         return out, Ticket(self, self.serial, n, bag_offsets, weights, mean, bag_mean)
 
+    def pull_input(self, ids: torch.Tensor, bag_offsets: torch.Tensor, bag_mean: torch.Tensor, dense: torch.Tensor,
+                   fields: int, width: int, share_from: Optional["SparseChannel"] = None):
+        """``pull`` of bags that an MLP takes in next (one GPU): returns (x, ticket), x [bags / fields, width] bfloat16 =
+        the pooled rows of a sample's ``fields`` bags side by side, its ``dense`` features, zeros.  The pooled rows do not
+        exist in float32, and its gradient goes to ``push(..., fields=fields)`` as it is."""
+        n = self._lookup_phase(ids.reshape(-1), insert=True, share_from=share_from)
+        samples = (int(bag_offsets.numel()) - 1) // fields
+        x = torch.empty((samples, width), dtype=torch.bfloat16, device=self.table.device)
+        C.local_combine_input(self.table.host(), self.dedup.inv, self.slot_cache, bag_offsets, bag_mean, 0.0, fields, dense, x)
+        self.launches += 1
+        return x, Ticket(self, self.serial, n, bag_offsets, None, False, bag_mean)
+
     # ------------------------------------------------------------------ push
     def push(self, grads: torch.Tensor, lr: torch.Tensor, ticket: Optional[Ticket] = None,
              ids: Optional[torch.Tensor] = None, bag_offsets: Optional[torch.Tensor] = None,
              weights: Optional[torch.Tensor] = None, mean: bool = False,
-             bag_mean: Optional[torch.Tensor] = None) -> None:
+             bag_mean: Optional[torch.Tensor] = None, fields: int = 0) -> None:
         """Sums the gradients of duplicate ids, sends them to the owners and runs
         the optimizer there.  With the ticket of the latest pull of this channel
         the dedup result and the owners' slots are reused; otherwise ``ids`` are
-        looked up again (an id the table does not hold is kSparseIdNotExist)."""
+        looked up again (an id the table does not hold is kSparseIdNotExist).
+        ``fields``: ``grads`` is the gradient of the x that ``pull_input`` returned."""
         if ticket is not None and ticket.current(self):
             n = ticket.n
             bag_offsets, weights, mean, bag_mean = ticket.bag_offsets, ticket.weights, ticket.mean, ticket.bag_mean
@@ -649,13 +662,18 @@ class SparseChannel:
                 raise C.KrakenError("push without a current ticket needs the ids")
             n = self._lookup_phase(ids.reshape(-1), insert=False)
         dim = self.table.dim
-        grads = _rows_of_gradients(grads, dim)
+        if fields:
+            grads = grads.contiguous()
+            if grads.data_ptr() % 8:
+                grads = grads.clone()
+        else:
+            grads = _rows_of_gradients(grads, dim)
         if self.world == 1:
             by = self.dedup
             if self._bag_of is None and bag_offsets is not None:
-                self._bag_of = torch.zeros(self.cap_u, dtype=torch.int32, device=self.table.device)
+                self._bag_of = torch.zeros((self.cap_u, 2), dtype=torch.int32, device=self.table.device)
             C.local_push(self.table.host(), grads, by.inv, by.first, by.win, n, bag_offsets, weights, mean, bag_mean,
-                         by.ctrl, self.multi, self._bag_of, self.ugrad, by.off, self.slot_cache, self.table.optim, lr)
+                         by.ctrl, self.multi, self._bag_of, self.ugrad, by.off, self.slot_cache, self.table.optim, lr, fields)
             self.launches += 2  # scatter, update
         else:
             C.push_scatter(grads, self.inv, n, dim, bag_offsets, weights, mean, bag_mean, self.ugrad)

@@ -531,12 +531,32 @@ class GpuEngine(Engine):
         self._looked_up()
         return out
 
+    def pools_into_input(self, table_id: int) -> bool:
+        """Whether ``pull_sparse_input`` takes this table."""
+        dim = self._table(table_id, "sparse").dimension
+        return self.world == 1 and dim % 4 == 0 and dim >= C.MIN_POOLED_INPUT
+
+    def pull_sparse_input(self, table_id: int, values: torch.Tensor, offsets: torch.Tensor, bag_mean: torch.Tensor,
+                          dense: torch.Tensor, fields: int, width: int, share_with: Optional[int] = None):
+        """``pull_sparse_pooled`` straight into the bfloat16 input of an MLP, ``SparseChannel.pull_input``: returns (x,
+        ticket).  ``push_sparse_pooled(..., fields=fields)`` takes the gradient of x."""
+        idx = self._prep_ids(values)
+        off = offsets.detach().to(self.device, torch.int64).contiguous()
+        bm = bag_mean.detach().to(self.device, torch.uint8).contiguous()
+        dense = dense.detach().to(self.device, torch.float32).contiguous()
+        ch = self._channel(table_id, idx.numel())
+        self._ensure_room(table_id, idx.numel())
+        share = self.channels.get(share_with) if share_with is not None else None
+        out = ch.pull_input(idx, off, bm, dense, fields, width, share_from=share)
+        self._looked_up()
+        return out
+
     def push_sparse_pooled(self, table_id: int, ticket: Ticket, grads: torch.Tensor,
-                           values: Optional[torch.Tensor] = None) -> None:
+                           values: Optional[torch.Tensor] = None, fields: int = 0) -> None:
         ch = self.channels[table_id]
         ids = self._prep_ids(values) if values is not None else None
         ch.push(grads, self.lr_dev, ticket=ticket, ids=ids, bag_offsets=ticket.bag_offsets, weights=ticket.weights,
-                mean=ticket.mean, bag_mean=ticket.bag_mean)
+                mean=ticket.mean, bag_mean=ticket.bag_mean, fields=fields)
 
     def pull_sparse_unique(self, table_id: int, indices: torch.Tensor, share_with: Optional[int] = None,
                            in_place: bool = False):

@@ -43,7 +43,8 @@ int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int 
                  int M, int N, int K, int* status, cudaStream_t stream);
 
 // Knobs for measurements.  variant: 0 = chosen from the shape, 1 = weight-resident CTA pair
-// (cta_group::2), 2 = weight-resident single CTA, 3 = one output tile per CTA.  n_tiles: column
+// (cta_group::2), 2 = weight-resident single CTA, 3 = one output tile per CTA, 4 = weight gradients on
+// CTA pairs (the rest as 3).  n_tiles: column
 // tiles of the resident variants (0 = chosen from the shape).
 void gemm_set_tuning(int variant, int n_tiles);
 

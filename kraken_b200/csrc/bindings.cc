@@ -1588,6 +1588,41 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     check_launch("group_push_apply");
   });
 
+  // dst[i].copy_(src[i], non_blocking=True) for every i, those that are plain copies on this device in one launch.
+  m.def("copy_batch", [](const std::vector<torch::Tensor>& dst, const std::vector<torch::Tensor>& src) {
+    TORCH_CHECK(dst.size() == src.size(), "one source per destination is needed");
+    cu::CopyBatch b{};
+    auto flush = [&] {
+      if (b.n == 1) {  // nothing to save
+        CUDA_OK(cudaMemcpyAsync(b.dst[0], b.src[0], b.bytes[0], cudaMemcpyDeviceToDevice, cur_stream()));
+      } else if (b.n > 1) {
+        cu::copy_batch(b, cur_stream());
+        check_launch("copy_batch");
+      }
+      b.n = 0;
+    };
+    for (size_t i = 0; i < dst.size(); ++i) {
+      const torch::Tensor &d = dst[i], &s = src[i];
+      const bool plain = d.is_cuda() && d.device() == s.device() && d.get_device() == c10::cuda::current_device() &&
+                         d.scalar_type() == s.scalar_type() && d.sizes() == s.sizes() && d.is_contiguous() &&
+                         s.is_contiguous() && !d.requires_grad() && !s.requires_grad() && !s.is_neg() && !s.is_conj() &&
+                         !d.is_neg() && !d.is_conj();
+      if (!plain) {
+        flush();  // in the order they were named
+        torch::Tensor(d).copy_(s, true);
+        continue;
+      }
+      if (d.numel() == 0) continue;
+      b.src[b.n] = static_cast<const char*>(s.data_ptr());
+      b.dst[b.n] = static_cast<char*>(d.data_ptr());
+      b.bytes[b.n] = static_cast<long long>(d.nbytes());
+      ++b.n;
+      d.unsafeGetTensorImpl()->bump_version();
+      if (b.n == cu::CopyBatch::kMax) flush();
+    }
+    flush();
+  });
+
   // ---------------- fused DeepFM front end
   m.def("pull_wait", [](const SymHeap& h, const cu::ChanLayout& lay, const torch::Tensor& ctrl, uint32_t spin) {
     cu::pull_wait(h.View(), lay, ctrl_ptr(ctrl), spin, cur_stream());

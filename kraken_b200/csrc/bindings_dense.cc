@@ -143,7 +143,8 @@ void bind_dense(py::module_& m) {
      py::arg("mask_out") = py::none());
   m.def("linear_dgrad", [bf, need_bf16](const torch::Tensor& dy, const torch::Tensor& wt,
                                         const c10::optional<torch::Tensor>& h, const torch::Tensor& dx,
-                                        const torch::Tensor& status, const c10::optional<torch::Tensor>& mask) {
+                                        const torch::Tensor& status, const c10::optional<torch::Tensor>& mask,
+                                        int zero_cols) {
     need_bf16(dy, "dy");
     need_bf16(wt, "wt");
     need_bf16(dx, "dx");
@@ -167,10 +168,11 @@ void bind_dense(py::module_& m) {
       ldm = mask->stride(0);
     }
     const int rc = cu::linear_dgrad(bf(dy), dy.stride(0), bf(wt), wt.stride(0), hp, ldh, mp, ldm,
-                                    reinterpret_cast<__nv_bfloat16*>(dx.data_ptr()), dx.stride(0), M, N, K,
+                                    reinterpret_cast<__nv_bfloat16*>(dx.data_ptr()), dx.stride(0), M, N, K, zero_cols,
                                     status.data_ptr<int>(), cur_stream());
     TORCH_CHECK(rc == 0, "linear_dgrad: cannot encode the TMA descriptors (pitches must be multiples of 8)");
-  }, py::arg("dy"), py::arg("wt"), py::arg("h"), py::arg("dx"), py::arg("status"), py::arg("mask") = py::none());
+  }, py::arg("dy"), py::arg("wt"), py::arg("h"), py::arg("dx"), py::arg("status"), py::arg("mask") = py::none(),
+     py::arg("zero_cols") = 0);
   m.def("linear_wgrad", [bf, need_bf16](const torch::Tensor& dy, const torch::Tensor& x, const torch::Tensor& dw,
                                         const torch::Tensor& status, const c10::optional<torch::Tensor>& db) {
     need_bf16(dy, "dy");

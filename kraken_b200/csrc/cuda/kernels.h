@@ -263,6 +263,16 @@ void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2
                           const __nv_bfloat16* dx, int lddx, const float* dlogit, const float* ssum, int B, int F, int D,
                           int P2, int RD, float* ugrad2, float* ugrad1, cudaStream_t stream);
 
+// Several buffers copied in one launch; any sizes and alignments.
+struct CopyBatch {
+  static constexpr int kMax = 8;
+  int n;
+  const char* src[kMax];
+  char* dst[kMax];
+  long long bytes[kMax], first[kMax];  // first: filled by the call
+};
+void copy_batch(CopyBatch b, cudaStream_t stream);
+
 // bf16 copy [N, K] and bf16 transpose [K, N] of an fp32 weight matrix [N, K], one pass.
 void cast_w_wt(const float* w, int N, int K, __nv_bfloat16* w16, __nv_bfloat16* wt16, cudaStream_t stream);
 

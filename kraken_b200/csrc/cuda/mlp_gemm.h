@@ -5,6 +5,7 @@
 //
 //   linear_forward   Y[M,N]  = act(X[M,K] * W[N,K]^T + bias)         bf16 out
 //   linear_dgrad     dX[M,K] = (dY[M,N] * Wt[K,N]^T) .* (H > 0)       bf16 out, Wt = W^T stored [K,N]
+//                    and zero_cols (a multiple of 8) columns of zeros behind the K of dX
 //   linear_wgrad     dW[N,K] += dY[M,N]^T * X[M,K]                    fp32 red-add, split over M;
 //                    db[N] += column sums of dY in the same pass (db may be null)
 //
@@ -36,8 +37,8 @@ int linear_forward(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, int 
                    cudaStream_t stream);
 
 int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int ldwt, const __nv_bfloat16* H,
-                 int ldh, const uint16_t* mask, int ldm, __nv_bfloat16* dX, int lddx, int M, int N, int K, int* status,
-                 cudaStream_t stream);
+                 int ldh, const uint16_t* mask, int ldm, __nv_bfloat16* dX, int lddx, int M, int N, int K, int zero_cols,
+                 int* status, cudaStream_t stream);
 
 int linear_wgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* X, int ldx, float* dW, int lddw, float* db,
                  int M, int N, int K, int* status, cudaStream_t stream);

@@ -437,6 +437,46 @@ rowdot_backward_wide_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const 
   }
 }
 
+// Buffers of a step's inputs, one launch for all of them: as copies of their own, each of two microseconds and its gap, they
+// stood in front of every replay of a captured step (three of a DeepFM batch
+// of 8192: 6.7 us, 3.3 so; of 65536: 12.4 and 8.2).  Thread t takes 16-byte piece
+// t of the buffers laid end to end; what is left of a buffer, or one that is not on 16 bytes, goes by bytes.
+__global__ void __launch_bounds__(kThreads)
+copy_batch_kernel(CopyBatch b, long long pieces) {
+  pdl_enter();
+  constexpr int kUnroll = 4;
+  const long long stride = static_cast<long long>(gridDim.x) * kThreads;
+  for (long long p0 = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; p0 < pieces; p0 += stride * kUnroll) {
+    uint4 v[kUnroll];
+    const char* s[kUnroll];
+    char* d[kUnroll];
+    int left[kUnroll];  // bytes of the piece, 0 for none
+#pragma unroll
+    for (int q = 0; q < kUnroll; ++q) {
+      const long long p = p0 + q * stride;
+      left[q] = 0;
+      if (p >= pieces) continue;
+      int l = 0;
+      while (l + 1 < b.n && p >= b.first[l + 1]) ++l;
+      const long long at = (p - b.first[l]) * 16;
+      s[q] = b.src[l] + at;
+      d[q] = b.dst[l] + at;
+      left[q] = static_cast<int>(min(16ll, b.bytes[l] - at));
+      if (left[q] == 16 && ((reinterpret_cast<uintptr_t>(s[q]) | reinterpret_cast<uintptr_t>(d[q])) & 15) == 0) {
+        left[q] = 17;  // one load and one store
+        v[q] = __ldcs(reinterpret_cast<const uint4*>(s[q]));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kUnroll; ++q) {
+      if (left[q] == 17)
+        *reinterpret_cast<uint4*>(d[q]) = v[q];
+      else
+        for (int j = 0; j < left[q]; ++j) d[q][j] = s[q][j];
+    }
+  }
+}
+
 // fp32 weight [N, K] -> bf16 copy [N, K] and bf16 transpose [K, N] in one pass (the forward and
 // the input-gradient GEMMs want the two layouts).
 __global__ void __launch_bounds__(256)
@@ -509,6 +549,18 @@ cast_weights_kernel(CastBatch b) {
 }
 
 }  // namespace
+
+void copy_batch(CopyBatch b, cudaStream_t stream) {
+  long long pieces = 0;
+  for (int l = 0; l < b.n; ++l) {
+    b.first[l] = pieces;
+    pieces += (b.bytes[l] + 15) / 16;
+  }
+  if (pieces <= 0) return;
+  long long grid = (pieces + 4 * kThreads - 1) / (4 * kThreads);
+  if (grid > 148 * 8) grid = 148 * 8;
+  launch_pdl(copy_batch_kernel, dim3(static_cast<unsigned>(grid)), dim3(kThreads), 0, stream, b, pieces);
+}
 
 void cast_weights(CastBatch b, cudaStream_t stream) {
   int tiles = 0;

@@ -252,8 +252,7 @@ class _FusedMLP(torch.autograd.Function):
                 cols = ctx.input_grad_cols if (i == 0 and ctx.input_grad_cols) else dprev.shape[1]
                 if cols < dprev.shape[1]:
                     # only the leading columns of the input need a gradient (the rest are constants)
-                    dprev[:, cols:].zero_()
-                    C.linear_dgrad(dh, wt16[:cols], None, dprev[:, :cols], st)
+                    C.linear_dgrad(dh, wt16[:cols], None, dprev[:, :cols], st, None, dprev.shape[1] - cols)
                 else:
                     C.linear_dgrad(dh, wt16, None, dprev, st, ctx.masks[i])
             side.wait_event(ready)

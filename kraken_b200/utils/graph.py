@@ -29,6 +29,8 @@ from typing import Callable, Sequence
 
 import torch
 
+from .._native import C
+
 
 class GraphedStep:
     def __init__(self, fn: Callable, example_inputs: Sequence[torch.Tensor], warmup: int = 3,
@@ -109,8 +111,8 @@ class GraphedStep:
             self._capture()
 
     def __call__(self, *inputs: torch.Tensor):
-        for s, t in zip(self.static_in, inputs):
-            s.copy_(t, non_blocking=True)
+        n = min(len(self.static_in), len(inputs))
+        C.copy_batch(self.static_in[:n], list(inputs[:n]))
         self._before_replay()
         self.graph.replay()
         out = self.static_out

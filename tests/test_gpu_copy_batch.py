@@ -1,0 +1,33 @@
+"""Several buffers copied in one launch (B200 only)."""
+import pytest
+import torch
+
+from kraken_b200._native import C
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# Sizes around a 16-byte piece, a block and the grid; buffers on any byte; more of them than one launch takes.
+@pytest.mark.parametrize("sizes", [[1, 15], [16, 17, 31], [4095, 4096, 4097], [0, 5, 0], [1 << 20, 3, (1 << 22) + 1],
+                                   list(range(1, 20)), [7]])
+@pytest.mark.parametrize("at", [0, 1, 8])
+def test_bytes(sizes, at):
+    g = torch.Generator(device=DEV).manual_seed(len(sizes) + at)
+    src = [torch.randint(0, 256, (n + at,), dtype=torch.uint8, device=DEV, generator=g)[at:] for n in sizes]
+    room = [torch.zeros(n + 32, dtype=torch.uint8, device=DEV) for n in sizes]
+    C.copy_batch([r[16:16 + n] for r, n in zip(room, sizes)], src)
+    for r, s, n in zip(room, src, sizes):
+        assert torch.equal(r[16:16 + n], s) and not bool(r[:16].any()) and not bool(r[16 + n:].any())
+
+
+def test_what_is_not_a_plain_copy_is_copied_as_torch_does():
+    src = [torch.arange(12, device=DEV).view(3, 4).t(), torch.arange(5), torch.ones(3, device=DEV, dtype=torch.float64),
+           torch.full((1,), 2.0, device=DEV), torch.arange(6.0, device=DEV)]
+    dst = [torch.zeros(4, 3, dtype=torch.int64, device=DEV), torch.zeros(5, dtype=torch.int64, device=DEV),
+           torch.zeros(3, device=DEV), torch.zeros(4, device=DEV), torch.zeros(6, device=DEV)]
+    C.copy_batch(dst, src)
+    for d, s in zip(dst, src):
+        assert torch.equal(d, torch.zeros_like(d).copy_(s))
+    with pytest.raises(RuntimeError):
+        C.copy_batch(dst, src[:-1])

@@ -87,3 +87,15 @@ def test_weight_gradient(M, N, K, bias, variant):
     check(db[:N], 1 + 2 * d.sum(0) if bias else torch.ones(N, device=DEV).double(), 1 + 2 * d.abs().sum(0), M + 200, 0)
     assert bool((dw[N:] == 1).all()) and bool((dw[:, K:] == 1).all()) and db[N].item() == 1
     assert status.item() == 0
+
+
+@pytest.mark.parametrize("M", [1, 70, 4096, 40001])   # one tile per CTA, and the persistent kernel
+def test_columns_without_a_gradient_are_cleared(M):
+    torch.manual_seed(M)
+    dy, w = rnd(M, 400), rnd(400, 416, scale=0.1)
+    dx = torch.full((M + 1, 440), 7.0, device=DEV, dtype=torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    C.linear_dgrad(dy, w.t().contiguous(), None, dx[:M, :416], status, None, 16)
+    check(dx[:M, :416], dy.double() @ w.double(), dy.double().abs() @ w.double().abs(), 400, 2 ** -8)
+    assert bool((dx[:M, 416:432] == 0).all()) and bool((dx[:M, 432:] == 7).all()) and bool((dx[M] == 7).all())
+    assert status.item() == 0

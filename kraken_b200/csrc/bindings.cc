@@ -1632,7 +1632,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         [](const torch::Tensor& rows2, const torch::Tensor& inv2, const c10::optional<torch::Tensor>& rows1,
            const c10::optional<torch::Tensor>& inv1, const torch::Tensor& dense, int B, int F, int D,
            const torch::Tensor& x, const torch::Tensor& fm_logit, const c10::optional<torch::Tensor>& slots2,
-           const c10::optional<torch::Tensor>& slots1, const c10::optional<torch::Tensor>& ssum) {
+           const c10::optional<torch::Tensor>& slots1, const c10::optional<torch::Tensor>& ssum, bool fm) {
           need_rows(rows2, "rows2");
           need_cuda(dense, "dense", torch::kFloat32);
           need_cuda(x, "x", torch::kBFloat16);
@@ -1658,21 +1658,23 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           cu::deepfm_pack_forward(ptr<float>(rows2), ptr<int>(inv2), optr<int>(slots2), optr<float>(rows1), optr<int>(inv1),
                                   optr<int>(slots1), ptr<float>(dense), B, F, D, static_cast<int>(rows2.stride(0)),
                                   rows1.has_value() ? static_cast<int>(rows1->stride(0)) : 0, ND, reinterpret_cast<__nv_bfloat16*>(x.data_ptr()), ldx,
-                                  ptr<float>(fm_logit), optr<float>(ssum), cur_stream());
+                                  ptr<float>(fm_logit), optr<float>(ssum), fm, cur_stream());
           check_launch("deepfm_pack_forward");
         },
         py::arg("rows2"), py::arg("inv2"), py::arg("rows1"), py::arg("inv1"), py::arg("dense"), py::arg("B"), py::arg("F"),
         py::arg("D"), py::arg("x"), py::arg("fm_logit"), py::arg("slots2") = py::none(), py::arg("slots1") = py::none(),
-        py::arg("ssum") = py::none());
+        py::arg("ssum") = py::none(), py::arg("fm") = true);
   m.def("deepfm_pack_backward",
         [](const torch::Tensor& rows2, const torch::Tensor& inv2, const c10::optional<torch::Tensor>& inv1,
            const c10::optional<torch::Tensor>& dx, const torch::Tensor& dlogit, int B, int F, int D,
            const torch::Tensor& ugrad2, const c10::optional<torch::Tensor>& ugrad1,
-           const c10::optional<torch::Tensor>& slots2, const torch::Tensor& ssum) {
+           const c10::optional<torch::Tensor>& slots2, const c10::optional<torch::Tensor>& ssum) {
           need_rows(rows2, "rows2");
-          need_cuda(ssum, "ssum", torch::kFloat32);
-          TORCH_CHECK(ssum.numel() == static_cast<int64_t>(B) * D && ((D / 4) & (D / 4 - 1)) == 0 && D <= 128,
-                      "ssum must be [B, D] with D / 4 a power of two");
+          TORCH_CHECK(((D / 4) & (D / 4 - 1)) == 0 && D <= 128, "D / 4 must be a power of two, D <= 128");
+          if (ssum.has_value()) {
+            need_cuda(*ssum, "ssum", torch::kFloat32);
+            TORCH_CHECK(ssum->numel() == static_cast<int64_t>(B) * D, "ssum must be [B, D]");
+          }
           need_cuda(dlogit, "dlogit", torch::kFloat32);
           need_cuda(ugrad2, "ugrad2", torch::kFloat32);
           const int RD = rows2.size(1);
@@ -1693,7 +1695,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           }
           TORCH_CHECK(dlogit.numel() == B, "deepfm_pack_backward: shape mismatch");
           cu::deepfm_pack_backward(ptr<float>(rows2), ptr<int>(inv2), optr<int>(slots2), optr<int>(inv1), dxp, lddx,
-                                   ptr<float>(dlogit), ptr<float>(ssum), B, F, D, static_cast<int>(rows2.stride(0)), RD, ptr<float>(ugrad2),
+                                   ptr<float>(dlogit), optr<float>(ssum), B, F, D, static_cast<int>(rows2.stride(0)), RD, ptr<float>(ugrad2),
                                    optr<float>(ugrad1), cur_stream());
           check_launch("deepfm_pack_backward");
         },

@@ -40,6 +40,8 @@ __device__ __forceinline__ size_t row_of(const int* __restrict__ slots, int u) {
 // Splitting the fields over G lane groups (a power of two) multiplies the number of independent
 // row loads in flight; the per-sample sums are combined with shuffles and the forward pass leaves
 // S[b, :] = sum_f e_f for the backward pass, whose lanes then need nothing from each other.
+// FM false (Wide&Deep): the logit is sum_f w_f alone, and the backward pass needs neither the rows nor ssum.
+template <bool FM>
 __global__ void __launch_bounds__(kThreads)
 deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restrict__ inv2,
                            const int* __restrict__ slots2, const float* __restrict__ rows1,
@@ -66,8 +68,10 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
 #pragma unroll 4
       for (int f = fg; f < F; f += G) {
         const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, i2[f]) * P2) + c);
-        s.x += e.x, s.y += e.y, s.z += e.z, s.w += e.w;
-        q.x += e.x * e.x, q.y += e.y * e.y, q.z += e.z * e.z, q.w += e.w * e.w;
+        if (FM) {
+          s.x += e.x, s.y += e.y, s.z += e.z, s.w += e.w;
+          q.x += e.x * e.x, q.y += e.y * e.y, q.z += e.z * e.z, q.w += e.w * e.w;
+        }
         __nv_bfloat162 lo = __floats2bfloat162_rn(e.x, e.y), hi = __floats2bfloat162_rn(e.z, e.w);
         uint2 packed;
         packed.x = *reinterpret_cast<uint32_t*>(&lo);
@@ -87,13 +91,13 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
         xr[base + j] = __float2bfloat16(j < ND ? dense[static_cast<size_t>(b) * ND + j] : 0.f);
     }
     // sums over the field groups of the same chunk (lanes c, c + chunks, c + 2 chunks, ...)
-    for (int o = chunks; o < lpr; o <<= 1) {
+    for (int o = chunks; FM && o < lpr; o <<= 1) {
       s.x += __shfl_xor_sync(group_mask, s.x, o), s.y += __shfl_xor_sync(group_mask, s.y, o);
       s.z += __shfl_xor_sync(group_mask, s.z, o), s.w += __shfl_xor_sync(group_mask, s.w, o);
       q.x += __shfl_xor_sync(group_mask, q.x, o), q.y += __shfl_xor_sync(group_mask, q.y, o);
       q.z += __shfl_xor_sync(group_mask, q.z, o), q.w += __shfl_xor_sync(group_mask, q.w, o);
     }
-    if (b < B && fg == 0) {
+    if (FM && b < B && fg == 0) {
       part += 0.5f * (s.x * s.x - q.x + s.y * s.y - q.y + s.z * s.z - q.z + s.w * s.w - q.w);
       if (ssum != nullptr) *reinterpret_cast<float4*>(ssum + static_cast<size_t>(b) * D + c * 4) = s;
     }
@@ -102,6 +106,7 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
   }
 }
 
+template <bool FM>
 __global__ void __launch_bounds__(kThreads)
 deepfm_pack_backward_kernel(const float* __restrict__ rows2, const int* __restrict__ inv2,
                             const int* __restrict__ slots2, const int* __restrict__ inv1,
@@ -119,12 +124,16 @@ deepfm_pack_backward_kernel(const float* __restrict__ rows2, const int* __restri
     const int* i2 = inv2 + static_cast<size_t>(b) * F;
     const float g = dlogit[b];
     const __nv_bfloat16* dxr = dx ? dx + static_cast<size_t>(b) * lddx : nullptr;
-    const float4 s = *reinterpret_cast<const float4*>(ssum + static_cast<size_t>(b) * D + c * 4);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (FM) s = *reinterpret_cast<const float4*>(ssum + static_cast<size_t>(b) * D + c * 4);
 #pragma unroll 4
     for (int f = fg; f < F; f += G) {
       const int u = i2[f];
-      const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, u) * P2) + c);
-      float4 d = make_float4(g * (s.x - e.x), g * (s.y - e.y), g * (s.z - e.z), g * (s.w - e.w));
+      float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (FM) {
+        const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, u) * P2) + c);
+        d = make_float4(g * (s.x - e.x), g * (s.y - e.y), g * (s.z - e.z), g * (s.w - e.w));
+      }
       if (dxr) {
         const uint2 p = *reinterpret_cast<const uint2*>(dxr + f * D + c * 4);
         const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&p.x);
@@ -169,12 +178,13 @@ int grid_for(long long rows, int lpr) {
 
 void deepfm_pack_forward(const float* rows2, const int* inv2, const int* slots2, const float* rows1, const int* inv1,
                          const int* slots1, const float* dense, int B, int F, int D, int P2, int P1, int ND, __nv_bfloat16* x,
-                         int ldx, float* fm_logit, float* ssum, cudaStream_t stream) {
+                         int ldx, float* fm_logit, float* ssum, bool fm, cudaStream_t stream) {
   if (B <= 0) return;
   const int chunks = D / 4;
   const int G = field_groups(chunks);
   const int lpr = chunks * G;
-  launch_pdl(deepfm_pack_forward_kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, rows1, inv1, slots1, dense,
+  auto kernel = fm ? deepfm_pack_forward_kernel<true> : deepfm_pack_forward_kernel<false>;
+  launch_pdl(kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, rows1, inv1, slots1, dense,
                                                                         B, F, D, P2, P1, ND, lpr, G, x, ldx, fm_logit, ssum);
 }
 
@@ -186,7 +196,8 @@ void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2
   const int chunks = D / 4;
   const int G = field_groups(chunks);
   const int lpr = chunks * G;
-  launch_pdl(deepfm_pack_backward_kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, inv1, dx, lddx, dlogit,
+  auto kernel = ssum != nullptr ? deepfm_pack_backward_kernel<true> : deepfm_pack_backward_kernel<false>;
+  launch_pdl(kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, inv1, dx, lddx, dlogit,
                                                                          ssum, B, F, D, P2, RD, lpr, G, ugrad2, ugrad1);
 }
 

@@ -256,7 +256,8 @@ void pull_wait(SymHost sym, ChanLayout lay, Ctrl* ctrl, uint32_t spin_limit, cud
 // row slots[u] (the in-place path of single-GPU jobs).
 void deepfm_pack_forward(const float* rows2, const int* inv2, const int* slots2, const float* rows1, const int* inv1,
                          const int* slots1, const float* dense, int B, int F, int D, int P2, int P1, int ND,
-                         __nv_bfloat16* x, int ldx, float* fm_logit, float* ssum, cudaStream_t stream);
+                         __nv_bfloat16* x, int ldx, float* fm_logit, float* ssum, bool fm, cudaStream_t stream);
+// fm false leaves the second-order term out (Wide&Deep); its backward takes a null ssum.
 // Adds each occurrence's gradient into ugrad2 [*, RD] / ugrad1 [*, 1] (per unique id).  dx may be null;
 // ugrad1 == nullptr: the first-order gradient goes to column D of ugrad2.
 void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2, const int* inv1,

@@ -19,6 +19,8 @@ import torch
 from torch.nn.modules.module import _has_any_global_hook
 
 from .. import pytorch as kk
+from .._native import C
+from ..ops import counters
 from .mlp import MLP
 
 
@@ -46,6 +48,11 @@ class WideAndDeep(torch.nn.Module):
         if self.both is not None:
             w, e = self.both([ids, ids])
             wide = w.sum(dim=(1, 2))
+        elif self._fused_ok(dense, ids):
+            prepared = self.mlp.prepare()  # weight casts run beside the sparse pull
+            x, wide = _WideDeepFront.apply(self.deep.sparse_table, self.wide.sparse_table, dense, ids, self.mlp_in, self.dim)
+            return self.mlp(x, input_grad_cols=self.num_fields * self.dim, addend=wide,
+                            prepared=prepared).squeeze(-1) + self.bias
         else:
             wide = self.wide(ids).sum(dim=(1, 2))
             e = self.deep(ids)
@@ -55,6 +62,23 @@ class WideAndDeep(torch.nn.Module):
             parts.append(torch.zeros(dense.shape[0], self.mlp_in - e.shape[1] * e.shape[2] - dense.shape[1],
                                      dtype=e.dtype, device=e.device))
         return wide + self.mlp(torch.cat(parts, dim=1)).squeeze(-1) + self.bias
+
+    def _fused_ok(self, dense: torch.Tensor, ids: torch.Tensor) -> bool:
+        """Whether one dedup and one kernel can stand for the two lookups, their sum and the concatenation: one GPU, the
+        stock modules without hooks, tables that are float32 and trained alike, and a float32 batch without gradient."""
+        from ..pytorch import native
+        if not ids.is_cuda or ids.dim() != 2 or ids.shape[1] != self.num_fields or not native.is_initialized():
+            return False
+        eng = native.engine()
+        chunks = self.dim // 4
+        tables = (self.wide.sparse_table, self.deep.sparse_table)
+        return (hasattr(eng, "pull_sparse_unique") and eng.world == 1 and not eng.cfg.long_id_streams
+                and self.dim % 4 == 0 and chunks & (chunks - 1) == 0 and self.dim <= 128
+                and all(_stock(m, kk.Embedding) for m in (self.wide, self.deep)) and _stock_mlp(self.mlp)
+                and all(t.dtype() == torch.float32 and t.table_id() is not None
+                        and (t.requires_grad or not torch.is_grad_enabled()) for t in tables)
+                and dense.dtype == torch.float32 and not dense.requires_grad and dense.dim() == 2
+                and dense.shape[0] == ids.shape[0] and dense.shape[1] <= self.mlp_in - self.num_fields * self.dim)
 
 
 def _stock(module, cls) -> bool:
@@ -67,6 +91,46 @@ def _stock(module, cls) -> bool:
 def _stock_mlp(mlp) -> bool:
     """Whether ``mlp`` takes a bfloat16 input as it takes the float32 one that it would round."""
     return _stock(mlp, MLP) and mlp.use_tensor_cores and mlp.layers[0].weight.is_cuda
+
+
+class _WideDeepFront(torch.autograd.Function):
+    """Both lookups with one dedup -> pack kernel -> (bf16 MLP input, sum of the wide weights); the backward kernel adds
+    every occurrence's gradient into the push buffers.  What DeepFM's front end does, without the second-order term.  Of the
+    38 kernels of a step by modules, a dozen moved the rows from one to the next."""
+
+    @staticmethod
+    def forward(ctx, deep_table, wide_table, dense, ids, width, dim):
+        from ..pytorch import native
+        eng = native.engine()
+        id2, id1 = deep_table.table_id(), wide_table.table_id()
+        B, F = ids.shape
+        in_place = ids.numel() <= (1 << 19)  # as DeepFM
+        rows2, inv2, t2 = eng.pull_sparse_unique(id2, ids, in_place=in_place)
+        rows1, inv1, t1 = eng.pull_sparse_unique(id1, ids, share_with=id2, in_place=in_place)
+        x = torch.empty((B, width), dtype=torch.bfloat16, device=rows2.device)
+        wide = torch.empty(B, dtype=torch.float32, device=rows2.device)
+        dense = dense.to(rows2.device).contiguous()
+        counters.add()
+        C.deepfm_pack_forward(rows2, inv2, rows1, inv1, dense, B, F, dim, x, wide, t2.slots, t1.slots, fm=False)
+        ctx.state = (eng, id1, id2, rows2, inv2, inv1, t1, t2, dim, ids)
+        return x, wide
+
+    @staticmethod
+    def backward(ctx, dx, dwide):
+        eng, id1, id2, rows2, inv2, inv1, t1, t2, dim, ids = ctx.state
+        B, F = ids.shape
+        dwide = dwide.float().contiguous()
+        if not (t1.current(eng.channels[id1]) and t2.current(eng.channels[id2])):
+            # another lookup has used the channels since: the gradients go out by id
+            eng.push_sparse_table(id2, ids, dx[:, :F * dim].float().reshape(B, F, dim))
+            eng.push_sparse_table(id1, ids, dwide.view(B, 1, 1).expand(B, F, 1).contiguous())
+            return None, None, None, None, None, None
+        counters.add()
+        C.deepfm_pack_backward(rows2, inv2, inv1, dx.contiguous(), dwide, B, F, dim, eng.grad_accumulator(id2),
+                               eng.grad_accumulator(id1), t2.slots, None)
+        eng.push_sparse_accumulated(id1, t1)
+        eng.push_sparse_accumulated(id2, t2)
+        return None, None, None, None, None, None
 
 
 class MultiHotWideAndDeep(torch.nn.Module):

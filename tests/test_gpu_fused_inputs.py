@@ -3,7 +3,7 @@ import pytest
 import torch
 
 import kraken_b200.pytorch as kk
-from kraken_b200.models import MultiHotWideAndDeep
+from kraken_b200.models import MultiHotWideAndDeep, WideAndDeep
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -14,9 +14,15 @@ def multihot(dim):
     return MultiHotWideAndDeep(num_fields=FIELDS, num_dense=3, dim=dim, hidden=(32, 16), mean_fields=(1, 4))
 
 
+def wide_deep(dim):
+    return WideAndDeep(num_fields=FIELDS, num_dense=3, dim=dim, hidden=(32, 16))
+
+
 def batch(kind, seed):
     g = torch.Generator().manual_seed(seed)
     dense = torch.randn(BATCH, 3, generator=g).to(DEV)
+    if kind is wide_deep:
+        return dense, torch.randint(0, SPACE, (BATCH, FIELDS), generator=g).to(DEV)
     lens = torch.randint(0, 6, (BATCH * FIELDS,), generator=g)
     off = torch.cat([torch.zeros(1, dtype=torch.int64), lens.cumsum(0)])
     ids = torch.randint(0, SPACE, (int(off[-1]),), generator=g)
@@ -63,10 +69,10 @@ def same(a, b):
         assert float((x - y).norm()) <= 2e-3 * float(y.norm()) + 1e-6
 
 
-@pytest.mark.parametrize("kind,dims", [(multihot, (4, 8, 12, 16, 64, 6))])  # 4 and 6: the general path on both sides
+@pytest.mark.parametrize("kind,dims", [(multihot, (4, 8, 12, 16, 64, 6)), (wide_deep, (4, 8, 16, 64, 12, 6))])
 @pytest.mark.parametrize("optim", [kk.SGD(), kk.Adagrad(initial_accumulator_value=0.1)], ids=["sgd", "adagrad"])
 def test_trains_as_the_modules_by_themselves(kind, dims, optim):
-    for dim in dims:
+    for dim in dims:  # among them widths that only the general path takes
         fused, general = (train(kind, dim, optim, g) for g in (False, True))
         assert torch.allclose(fused[0][0], general[0][0], rtol=1e-4, atol=1e-5)   # one step: nothing to amplify
         for a, b in zip(fused[:3], general[:3]):
@@ -75,9 +81,16 @@ def test_trains_as_the_modules_by_themselves(kind, dims, optim):
             assert fused[3]   # one dedup for both tables
 
 
-@pytest.mark.parametrize("kind", [multihot])
+@pytest.mark.parametrize("kind", [multihot, wide_deep])
 @pytest.mark.parametrize("order", ["two forwards", "scoring between"])
 def test_backward_of_a_lookup_that_is_not_the_latest(kind, order):
     fused, general = (train(kind, 8, kk.SGD(), g, order=order) for g in (False, True))
+    for a, b in zip(fused[:3], general[:3]):
+        same(a, b)
+
+
+@pytest.mark.parametrize("freeze", [(0,), (1,), (0, 1)])
+def test_a_frozen_table_keeps_its_rows(freeze):
+    fused, general = (train(wide_deep, 8, kk.SGD(), g, freeze=freeze) for g in (False, True))
     for a, b in zip(fused[:3], general[:3]):
         same(a, b)

@@ -1523,6 +1523,56 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("lr"), py::arg("fields") = 0);
 
   // ---------------- one exchange for several tables of one row width
+  // What a combined call does per table on the host, for all of its tables at once.
+  m.def("signatures", [](const std::vector<torch::Tensor>& ts) {
+    std::vector<std::tuple<uintptr_t, int64_t, int64_t>> out;
+    out.reserve(ts.size());
+    for (const auto& t : ts) out.emplace_back(reinterpret_cast<uintptr_t>(t.data_ptr()), t.numel(), t._version());
+    return out;
+  });
+  // Ids of several tables back to back and how many each has, or None if one of them is not int64 on `device`.
+  m.def("concat_ids", [](const std::vector<torch::Tensor>& ids, int device) -> py::object {
+    std::vector<torch::Tensor> flat;
+    std::vector<int64_t> counts;
+    for (const auto& t : ids) {
+      if (!t.is_cuda() || t.get_device() != device || t.scalar_type() != torch::kInt64) return py::none();
+      flat.push_back(t.dim() == 1 ? t : t.reshape({-1}));
+      counts.push_back(t.numel());
+    }
+    return py::make_tuple(torch::cat(flat), counts);
+  });
+  // The rows of a combined lookup per table, in the shape of its ids.
+  m.def("split_rows", [](const torch::Tensor& rows, const std::vector<torch::Tensor>& ids) {
+    std::vector<int64_t> counts;
+    for (const auto& t : ids) counts.push_back(t.numel());
+    std::vector<torch::Tensor> out = rows.split_with_sizes(counts);
+    for (size_t i = 0; i < ids.size(); ++i) {
+      if (ids[i].dim() == 1) continue;
+      std::vector<int64_t> shape = ids[i].sizes().vec();
+      shape.push_back(rows.size(1));
+      out[i] = out[i].view(shape);
+    }
+    return out;
+  });
+  // Gradients of several tables back to back, float32 on `device`; a missing one counts as zeros.
+  m.def("concat_grads", [](const std::vector<c10::optional<torch::Tensor>>& grads, const std::vector<torch::Tensor>& ids,
+                           int64_t dim, int device) {
+    const auto options = torch::TensorOptions().dtype(torch::kFloat32).device(torch::kCUDA, device);
+    std::vector<torch::Tensor> parts;
+    TORCH_CHECK(grads.size() == ids.size(), "one gradient per table is needed");
+    for (size_t i = 0; i < grads.size(); ++i) {
+      const int64_t n = ids[i].numel();
+      if (!grads[i].has_value() || !grads[i]->defined()) {
+        parts.push_back(torch::zeros({n, dim}, options));
+        continue;
+      }
+      if (grads[i]->numel() != n * dim) throw KrakenError(err::kBadArgument, "gradient shape must be indices.shape + [dimension]");
+      torch::Tensor g = grads[i]->requires_grad() ? grads[i]->detach() : *grads[i];
+      if (g.device() != options.device() || g.scalar_type() != torch::kFloat32) g = g.to(options.device(), torch::kFloat32);
+      parts.push_back(g.dim() == 2 && g.size(0) == n ? g : g.reshape({n, dim}));
+    }
+    return torch::cat(parts);
+  });
   m.def("group_table_views", [](const std::vector<cu::TableHost>& tables) {
     // the tables' device-side descriptors as one CPU byte tensor; the caller copies it to the device
     const int T = static_cast<int>(tables.size());

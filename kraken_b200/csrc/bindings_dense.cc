@@ -1,4 +1,7 @@
 // Bindings of the dense-parameter path (fused dense step, DCT compression).
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/stl.h>
 #include <torch/extension.h>
@@ -30,6 +33,75 @@ cu::SymHost sym_from(const std::vector<uintptr_t>& bases, int rank) {
   s.rank = rank;
   s.world = static_cast<int>(bases.size());
   return s;
+}
+
+// All matrices in as few launches as possible, their bf16 copies (and transposes) in ONE buffer, which is returned
+// with the views so that a caller on another stream has one tensor to record.
+std::tuple<std::vector<torch::Tensor>, std::vector<torch::Tensor>, torch::Tensor> cast_weights(
+    const std::vector<torch::Tensor>& ws, bool transpose) {
+  int64_t total = 0;
+  auto room = [](int64_t n) { return (n + 63) / 64 * 64; };
+  std::vector<torch::Tensor> rows;  // a copy of those that are not stored row by row
+  for (const auto& w : ws) rows.push_back(w.contiguous());
+  for (const auto& w : rows) {
+    TORCH_CHECK(w.is_cuda() && w.scalar_type() == torch::kFloat32 && w.dim() == 2,
+                "weights must be 2-D CUDA f32 tensors");
+    total += room(w.numel()) * (transpose ? 2 : 1);
+  }
+  std::vector<torch::Tensor> w16s, wt16s;
+  if (ws.empty()) return {w16s, wt16s, torch::Tensor()};
+  torch::Tensor buf = torch::empty({total}, ws[0].options().dtype(torch::kBFloat16));
+  __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(buf.data_ptr());
+  cu::CastBatch batch{};
+  int64_t at = 0;
+  for (const auto& w : rows) {
+    const int N = w.size(0), K = w.size(1);
+    w16s.push_back(buf.narrow(0, at, w.numel()).view({N, K}));
+    __nv_bfloat16* const w16 = base + at;
+    at += room(w.numel());
+    __nv_bfloat16* wt16 = nullptr;
+    if (transpose) {
+      wt16s.push_back(buf.narrow(0, at, w.numel()).view({K, N}));
+      wt16 = base + at;
+      at += room(w.numel());
+    }
+    const float* src = w.data_ptr<float>();
+    if (N % 8 != 0 || K % 8 != 0 || reinterpret_cast<uintptr_t>(src) % 16 != 0) {
+      torch::Tensor spare;
+      if (wt16 == nullptr) {
+        spare = torch::empty({w.numel()}, buf.options());
+        wt16 = reinterpret_cast<__nv_bfloat16*>(spare.data_ptr());
+      }
+      cu::cast_w_wt(src, N, K, w16, wt16, cur_stream());
+      continue;
+    }
+    const int l = batch.layers++;
+    batch.w[l] = src, batch.w16[l] = w16, batch.wt16[l] = wt16, batch.N[l] = N, batch.K[l] = K;
+    if (batch.layers == cu::CastBatch::kMax) {
+      cu::cast_weights(batch, cur_stream());
+      batch.layers = 0;
+    }
+  }
+  if (batch.layers > 0) cu::cast_weights(batch, cur_stream());
+  check_launch("cast_weights");
+  return {w16s, wt16s, buf};
+}
+
+struct StreamEvent {
+  at::cuda::CUDAEvent event;
+  void Wait() { event.block(c10::cuda::getCurrentCUDAStream()); }
+};
+
+// `later` waits for what `earlier` has been given so far.
+void join(const c10::cuda::CUDAStream& earlier, const c10::cuda::CUDAStream& later) {
+  at::cuda::CUDAEvent e;
+  e.record(earlier);
+  e.block(later);
+}
+
+// The caching allocator keeps `t`'s memory until `stream` has passed this point.
+void on_stream(const torch::Tensor& t, const c10::cuda::CUDAStream& stream) {
+  c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
 }
 
 }  // namespace
@@ -271,52 +343,108 @@ void bind_dense(py::module_& m) {
                       relu_mask, dxp, lddx, dw.data_ptr<float>(), db.data_ptr<float>(), cur_stream());
     check_launch("head_backward");
   });
-  // All matrices in as few launches as possible, their bf16 copies (and transposes) in ONE buffer, which is returned
-  // with the views so that a caller on another stream has one tensor to record.
-  m.def("cast_weights", [](const std::vector<torch::Tensor>& ws, bool transpose) {
-    int64_t total = 0;
-    auto room = [](int64_t n) { return (n + 63) / 64 * 64; };
-    for (const auto& w : ws) {
-      TORCH_CHECK(w.is_cuda() && w.scalar_type() == torch::kFloat32 && w.dim() == 2 && w.is_contiguous(),
-                  "weights must be contiguous 2-D CUDA f32 tensors");
-      total += room(w.numel()) * (transpose ? 2 : 1);
+  m.def("cast_weights", &cast_weights);
+  // The casts on stream `side` beside whatever the current stream does next; `wait` of the event orders a stream behind them.
+  py::class_<StreamEvent>(m, "StreamEvent").def("wait", &StreamEvent::Wait);
+  m.def("prepare_weights", [](const std::vector<torch::Tensor>& ws, bool transpose, int64_t id, int64_t index, int64_t type) {
+    TORCH_CHECK(!ws.empty(), "no weights");
+    const c10::cuda::CUDAGuard device(ws[0].device());
+    const auto main = c10::cuda::getCurrentCUDAStream();
+    const auto side = c10::cuda::CUDAStream::unpack3(id, index, static_cast<c10::DeviceType>(type));
+    join(main, side);
+    auto event = std::make_unique<StreamEvent>();
+    std::tuple<std::vector<torch::Tensor>, std::vector<torch::Tensor>, torch::Tensor> cast;
+    {
+      const c10::cuda::CUDAStreamGuard on(side);
+      cast = cast_weights(ws, transpose);
+      if (std::get<2>(cast).defined()) on_stream(std::get<2>(cast), main);
+      event->event.record(side);
     }
-    std::vector<torch::Tensor> w16s, wt16s;
-    if (ws.empty()) return std::make_tuple(w16s, wt16s, torch::Tensor());
-    torch::Tensor buf = torch::empty({total}, ws[0].options().dtype(torch::kBFloat16));
-    __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(buf.data_ptr());
-    cu::CastBatch batch{};
-    int64_t at = 0;
-    for (const auto& w : ws) {
+    return py::make_tuple(std::get<0>(cast), std::get<1>(cast), std::move(event));
+  });
+  // The hidden layers of an MLP, every one Linear + ReLU: returns [x, h1, h2, ...] and, with `masks`, the ReLU bits of the
+  // h's (see linear_forward).
+  m.def("mlp_hidden_forward", [bf, need_bf16](const torch::Tensor& x, const std::vector<torch::Tensor>& ws,
+                                              const std::vector<torch::Tensor>& bs, const torch::Tensor& status, bool masks) {
+    need_bf16(x, "x");
+    TORCH_CHECK(bs.size() >= ws.size(), "a bias per layer is needed");
+    const c10::cuda::CUDAGuard device(x.device());
+    std::vector<torch::Tensor> acts{x}, bits;
+    const int M = x.size(0);
+    for (size_t i = 0; i < ws.size(); ++i) {
+      const torch::Tensor h = acts.back(), w = ws[i], bias = bs[i].contiguous();
+      need_bf16(w, "w");
       const int N = w.size(0), K = w.size(1);
-      w16s.push_back(buf.narrow(0, at, w.numel()).view({N, K}));
-      __nv_bfloat16* const w16 = base + at;
-      at += room(w.numel());
-      __nv_bfloat16* wt16 = nullptr;
-      if (transpose) {
-        wt16s.push_back(buf.narrow(0, at, w.numel()).view({K, N}));
-        wt16 = base + at;
-        at += room(w.numel());
-      }
-      const float* src = w.data_ptr<float>();
-      if (N % 8 != 0 || K % 8 != 0 || reinterpret_cast<uintptr_t>(src) % 16 != 0) {
-        torch::Tensor spare;
-        if (wt16 == nullptr) {
-          spare = torch::empty({w.numel()}, buf.options());
-          wt16 = reinterpret_cast<__nv_bfloat16*>(spare.data_ptr());
-        }
-        cu::cast_w_wt(src, N, K, w16, wt16, cur_stream());
-        continue;
-      }
-      const int l = batch.layers++;
-      batch.w[l] = src, batch.w16[l] = w16, batch.wt16[l] = wt16, batch.N[l] = N, batch.K[l] = K;
-      if (batch.layers == cu::CastBatch::kMax) {
-        cu::cast_weights(batch, cur_stream());
-        batch.layers = 0;
-      }
+      TORCH_CHECK(h.size(1) == K && bias.is_cuda() && bias.scalar_type() == torch::kFloat32 && bias.numel() == N,
+                  "mlp_hidden_forward: shape mismatch");
+      torch::Tensor y = torch::empty({M, N}, x.options());
+      torch::Tensor mask;
+      if (masks) mask = torch::empty({(N + 15) / 16, (M + 63) / 64 * 64}, x.options().dtype(torch::kInt16));
+      const int rc = cu::linear_forward(bf(h), h.stride(0), bf(w), w.stride(0), bias.data_ptr<float>(),
+                                        reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), y.stride(0), M, N, K, true,
+                                        masks ? reinterpret_cast<uint16_t*>(mask.data_ptr()) : nullptr,
+                                        masks ? static_cast<int>(mask.stride(0)) : 0, status.data_ptr<int>(), cur_stream());
+      TORCH_CHECK(rc == 0, "linear_forward: cannot encode the TMA descriptors (pitches must be multiples of 8)");
+      acts.push_back(y);
+      if (masks) bits.push_back(mask);
     }
-    if (batch.layers > 0) cu::cast_weights(batch, cur_stream());
-    check_launch("cast_weights");
-    return std::make_tuple(w16s, wt16s, buf);
+    return std::make_pair(acts, bits);
+  });
+  // Their backward.  dh: gradient of acts.back() with its ReLU mask applied.  The chain dh_L -> dh_{L-1} -> ... is serial and
+  // runs on the current stream; a layer's weight and bias gradients only need that layer's dh and run on stream `side`,
+  // behind it (in a graph capture this becomes a parallel branch).  `input_cols` > 0: only the leading columns of x want a
+  // gradient, the rest are zeros.  on_ready(i), if given, is called when everything that writes layer i's gradients is
+  // enqueued.  Unless `deferred`, the current stream waits for `side` at the end.  Returns the gradient of x or None.
+  m.def("mlp_hidden_backward", [bf, need_bf16](torch::Tensor dh, const std::vector<torch::Tensor>& acts,
+                                               const std::vector<torch::Tensor>& masks,
+                                               const std::vector<torch::Tensor>& wts, const std::vector<torch::Tensor>& dws,
+                                               const std::vector<torch::Tensor>& dbs, const torch::Tensor& status,
+                                               bool x_needs_grad, int input_cols, int64_t id, int64_t index, int64_t type,
+                                               bool deferred, const py::object& on_ready) -> py::object {
+    const int L = static_cast<int>(dws.size());
+    need_bf16(dh, "dh");
+    TORCH_CHECK(static_cast<int>(acts.size()) == L + 1 && static_cast<int>(masks.size()) >= L &&
+                    static_cast<int>(wts.size()) >= L && static_cast<int>(dbs.size()) >= L,
+                "mlp_hidden_backward: one tensor per layer is needed");
+    const c10::cuda::CUDAGuard device(dh.device());
+    const auto main = c10::cuda::getCurrentCUDAStream();
+    const auto side = c10::cuda::CUDAStream::unpack3(id, index, static_cast<c10::DeviceType>(type));
+    const int M = dh.size(0);
+    for (int i = L - 1; i >= 0; --i) {
+      at::cuda::CUDAEvent ready;
+      ready.record(main);
+      const torch::Tensor& h = acts[i];
+      const int N = dh.size(1), K = h.size(1);
+      torch::Tensor dprev;
+      if (i > 0 || x_needs_grad) {
+        // the chain first: it is what the rest of the backward pass waits for
+        need_bf16(wts[i], "wt");
+        TORCH_CHECK(wts[i].size(0) == K && wts[i].size(1) == N, "mlp_hidden_backward: weight shape");
+        dprev = torch::empty({M, K}, dh.options());
+        const int cols = i == 0 && input_cols > 0 && input_cols < K ? input_cols : K;  // behind them zeros
+        // masks[i - 1] holds the ReLU bits of h; the input of the MLP has none
+        const uint16_t* mask = i > 0 ? reinterpret_cast<const uint16_t*>(masks[i - 1].data_ptr()) : nullptr;
+        const int rc = cu::linear_dgrad(bf(dh), dh.stride(0), bf(wts[i]), wts[i].stride(0), nullptr, 0, mask,
+                                        i > 0 ? static_cast<int>(masks[i - 1].stride(0)) : 0,
+                                        reinterpret_cast<__nv_bfloat16*>(dprev.data_ptr()), K, M, N, cols, K - cols,
+                                        status.data_ptr<int>(), main.stream());
+        TORCH_CHECK(rc == 0, "linear_dgrad: cannot encode the TMA descriptors (pitches must be multiples of 8)");
+      }
+      ready.block(side);
+      const torch::Tensor &dw = dws[i], &db = dbs[i];
+      TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == torch::kFloat32 && dw.dim() == 2 && dw.stride(1) == 1 &&
+                      dw.size(0) == N && dw.size(1) == K && db.is_cuda() && db.scalar_type() == torch::kFloat32 &&
+                      db.is_contiguous() && db.numel() == N,
+                  "mlp_hidden_backward: gradient buffers must be f32 of the parameters' shapes");
+      const int rc = cu::linear_wgrad(bf(dh), dh.stride(0), bf(h), h.stride(0), dw.data_ptr<float>(), dw.stride(0),
+                                      db.data_ptr<float>(), M, N, K, status.data_ptr<int>(), side.stream());
+      TORCH_CHECK(rc == 0, "linear_wgrad: cannot encode the TMA descriptors (pitches must be multiples of 8)");
+      on_stream(dh, side);
+      if (deferred) on_stream(h, side);  // nobody waits for this stream before the graph lets go of the layer's input
+      if (!on_ready.is_none()) on_ready(i);
+      dh = dprev;
+    }
+    if (!deferred) join(side, main);
+    return dh.defined() ? py::cast(dh) : py::none();
   });
 }

@@ -1471,7 +1471,7 @@ int linear_forward(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, int 
   if (mask_out != nullptr && ldm < M) return -1;
   g.status = status;
   CUtensorMap ta, tb, td;
-  g.out_tma = g_variant < 2 && make_tmap_out(&td, Y, M, N, ldy) ? 1 : 0;
+  g.out_tma = g_variant < 2 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (ldy % 8) == 0 ? 1 : 0;
   const bool pair = (g_variant == 0 || g_variant == 1) && plan_pair(M, N, K, g.out_tma != 0, &g.BN, &g.stages);
   const bool resident = !pair && (g_variant == 0 || g_variant == 2) && plan_resident(M, N, K, &g.BN, &g.stages);
   if (!pair && !resident) g.BN = tile_bn(M, N);
@@ -1479,7 +1479,7 @@ int linear_forward(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, int 
   if ((ldy % 8) != 0 || !make_tmap(&ta, X, M, K, ldx, 64, kBM) ||
       !make_tmap(&tb, W, N, K, ldw, 64, pair ? g.BN / 2 : g.BN))
     return -1;
-  if (!g.out_tma) td = ta;  // a map that nothing reads
+  if (g.out_tma ? !make_tmap_out(&td, Y, M, N, ldy) : (td = ta, false)) return -1;  // or a map that nothing reads
   if (pair) return launch_pair<EPI_BIAS_ACT>(ta, tb, td, g, stream);
   if (resident) return launch_resident<EPI_BIAS_ACT>(ta, tb, g, stream);
   g.stages = one_wave_stages(M, N, K, g.BN);
@@ -1506,7 +1506,7 @@ int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int
   g.status = status;
   CUtensorMap ta, tb, td;
   // (with the activations instead of their bits the epilogue reads 16 columns of a row at a time and stores as it goes)
-  g.out_tma = g_variant < 2 && (H == nullptr || mask != nullptr) && make_tmap_out(&td, dX, M, K, lddx) ? 1 : 0;
+  g.out_tma = g_variant < 2 && (H == nullptr || mask != nullptr) && (reinterpret_cast<uintptr_t>(dX) & 15) == 0 && (lddx % 8) == 0 ? 1 : 0;
   const bool pair = (g_variant == 0 || g_variant == 1) && plan_pair(M, K, N, g.out_tma != 0, &g.BN, &g.stages);
   const bool resident = !pair && (g_variant == 0 || g_variant == 2) && plan_resident(M, K, N, &g.BN, &g.stages);
   if (!pair && !resident) g.BN = tile_bn(M, K);
@@ -1514,7 +1514,7 @@ int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int
   if ((lddx % 8) != 0 || (H && (ldh % 8) != 0) || !make_tmap(&ta, dY, M, N, lddy, 64, kBM) ||
       !make_tmap(&tb, Wt, K, N, ldwt, 64, pair ? g.BN / 2 : g.BN))
     return -1;
-  if (!g.out_tma) td = ta;  // a map that nothing reads
+  if (g.out_tma ? !make_tmap_out(&td, dX, M, K, lddx) : (td = ta, false)) return -1;  // or a map that nothing reads
   if (pair) return launch_pair<EPI_RELU_MASK>(ta, tb, td, g, stream);
   if (resident) return launch_resident<EPI_RELU_MASK>(ta, tb, g, stream);
   g.stages = one_wave_stages(M, K, N, g.BN);

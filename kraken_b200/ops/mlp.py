@@ -15,6 +15,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from .._native import C
+from ..utils.profiler import engine_region
 from . import counters
 
 _status = {}
@@ -35,9 +36,8 @@ def set_grad_ready_callback(fn) -> None:
 
 
 def _notify(params, stream) -> None:
-    if _grad_ready is not None:
-        for p in params:
-            _grad_ready(p, stream)
+    for p in params:
+        _grad_ready(p, stream)
 
 
 def set_deferred_join(on: bool) -> None:
@@ -71,6 +71,11 @@ def _side_stream(device: torch.device) -> torch.cuda.Stream:
 
 
 
+def _ids(stream: torch.cuda.Stream):
+    """A stream as the native side takes it."""
+    return stream.stream_id, stream.device_index, stream.device_type
+
+
 class PreparedWeights:
     """bf16 copies of the hidden layers' weights, cast on the side stream: as they are and, for a forward pass that a
     backward pass will follow, transposed (``wt16s`` is empty otherwise)."""
@@ -81,7 +86,7 @@ class PreparedWeights:
 
 def _cast(weights: Sequence[torch.Tensor], transpose: bool):
     counters.add()
-    return C.cast_weights([w.detach().contiguous() for w in weights], transpose)
+    return C.cast_weights(weights, transpose)
 
 
 def prepare_weights(weights: Sequence[torch.Tensor]) -> PreparedWeights:
@@ -89,17 +94,8 @@ def prepare_weights(weights: Sequence[torch.Tensor]) -> PreparedWeights:
     at once.  A model calls this before work that does not depend on the weights (the sparse
     pull of a recommender), hands the result to ``fused_mlp(prepared=...)``, and the casts run
     beside that work instead of in front of the first GEMM."""
-    dev = weights[0].device
-    main = torch.cuda.current_stream(dev)
-    side = _side_stream(dev)
-    side.wait_stream(main)
-    with torch.cuda.stream(side):
-        w16s, wt16s, buf = _cast(weights[:-1], torch.is_grad_enabled())
-        if buf is not None:
-            buf.record_stream(main)
-        event = torch.cuda.Event()
-        event.record(side)
-    return PreparedWeights(w16s, wt16s, event)
+    counters.add()
+    return PreparedWeights(*C.prepare_weights(weights[:-1], torch.is_grad_enabled(), *_ids(_side_stream(weights[0].device))))
 
 
 def gemm_status(device: torch.device) -> torch.Tensor:
@@ -140,25 +136,18 @@ class _FusedMLP(torch.autograd.Function):
         ws, bs = params[:n_layers], params[n_layers:]
         dev = x.device
         if prepared is not None and (prepared.wt16s or not with_grad):
-            torch.cuda.current_stream(dev).wait_event(prepared.event)
+            prepared.event.wait()
             w16s, wts = prepared.w16s, prepared.wt16s
         else:
             w16s, wts, _ = _cast(ws[:-1], with_grad)
         st = gemm_status(dev)
         h = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
-        acts = [h]
         M = h.shape[0]
-        masks = [None]  # masks[i] belongs to acts[i]; the MLP input has none
-        for i in range(n_layers - 1):
-            w16 = w16s[i]
-            y = torch.empty((M, w16.shape[0]), dtype=torch.bfloat16, device=dev)
-            # one bit per output (> 0): the next layer's input gradient masks with it instead of re-reading y
-            mask = torch.empty(((w16.shape[0] + 15) // 16, (M + 63) // 64 * 64), dtype=torch.int16, device=dev)
-            counters.add()
-            C.linear_forward(h, w16, bs[i].detach(), True, y, st, mask)
-            acts.append(y)
-            masks.append(mask)
-            h = y
+        # masks[i] is one bit per element of acts[i + 1] (> 0): the next layer's input gradient masks with it instead of
+        # re-reading the activations
+        counters.add(n_layers - 1)
+        acts, masks = C.mlp_hidden_forward(h, w16s, bs[:-1], st, with_grad)
+        h = acts[-1]
         wl, bl = ws[-1].detach(), bs[-1].detach()
         if wl.shape[0] == 1:
             out = torch.empty(M, dtype=torch.float32, device=dev)
@@ -188,7 +177,6 @@ class _FusedMLP(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, gout):
-        from ..utils.profiler import engine_region
         with engine_region("mlp_bwd"):
             return _FusedMLP._backward(ctx, gout)
 
@@ -233,41 +221,20 @@ class _FusedMLP(torch.autograd.Function):
                 counters.add()
                 C.linear_dgrad(dy16, wl.detach().t().contiguous().to(torch.bfloat16), None, dh, st,
                                ctx.masks[-1] if L > 1 else None)
-        _notify((wl, bs[-1]), torch.cuda.current_stream(dev))
-        # The chain dh_L -> dh_{L-1} -> ... is serial; each layer's weight and bias gradients only
-        # need that layer's dh, so they run on a second stream beside the chain and are joined at
-        # the end (in a CUDA-graph capture this becomes a parallel branch).
-        main = torch.cuda.current_stream(dev)
+        if _grad_ready is not None:
+            _notify((wl, bs[-1]), torch.cuda.current_stream(dev))
         side = _side_stream(dev)
-        for i in range(L - 2, -1, -1):
-            # dh is d(loss)/d(acts[i + 1]) with layer i's ReLU mask already applied
-            ready = torch.cuda.Event()
-            ready.record(main)
-            dprev = None
-            if i > 0 or ctx.x_needs_grad:
-                # the chain first: it is what the rest of the backward pass waits for
-                dprev = torch.empty_like(acts[i])
-                wt16 = ctx.wts[i]
-                counters.add()
-                cols = ctx.input_grad_cols if (i == 0 and ctx.input_grad_cols) else dprev.shape[1]
-                if cols < dprev.shape[1]:
-                    # only the leading columns of the input need a gradient (the rest are constants)
-                    C.linear_dgrad(dh, wt16[:cols], None, dprev[:, :cols], st, None, dprev.shape[1] - cols)
-                else:
-                    C.linear_dgrad(dh, wt16, None, dprev, st, ctx.masks[i])
-            side.wait_event(ready)
-            with torch.cuda.stream(side):
-                counters.add()
-                C.linear_wgrad(dh, acts[i], _grad_target(ws[i]), st, _grad_target(bs[i]))
-                dh.record_stream(side)
-                if _deferred_join:  # nobody waits for this stream before the graph lets go of the layer's input
-                    acts[i].record_stream(side)
-            _notify((ws[i], bs[i]), side)
-            dh = dprev
+        if L > 1:
+            counters.add(2 * (L - 1) - (0 if ctx.x_needs_grad else 1))
+            ready = None
+            if _grad_ready is not None:
+                def ready(i):
+                    _notify((ws[i], bs[i]), side)
+            dh = C.mlp_hidden_backward(dh, acts, ctx.masks, ctx.wts, [_grad_target(w) for w in ws[:-1]],
+                                       [_grad_target(b) for b in bs[:-1]], st, ctx.x_needs_grad,
+                                       ctx.input_grad_cols or 0, *_ids(side), _deferred_join, ready)
         if _deferred_join:
             _pending_join.add((dev.type, dev.index))
-        else:
-            main.wait_stream(side)
         dx = None
         if ctx.x_needs_grad and dh is not None:
             dx = dh if ctx.x_dtype == torch.bfloat16 else dh.to(ctx.x_dtype)
@@ -283,7 +250,6 @@ def fused_mlp(x: torch.Tensor, weights: List[torch.Tensor], biases: List[torch.T
     (a multiple of 8, 0 = all) limits the input gradient to the leading columns of x.
     ``addend`` [M] (single-output heads) is added to the output inside the head kernel.
     ``prepared`` is the result of an earlier ``prepare_weights`` call on the same weights."""
-    from ..utils.profiler import engine_region
     with engine_region("mlp_fwd"):
         if addend is not None and weights[-1].shape[0] != 1:
             raise ValueError("addend needs a single-output head")

@@ -151,6 +151,7 @@ class GpuSparseTable:
         dev = self.device
         info = self.optim_info
         self.bits = bits
+        self.limit = 0.6 * cap    # rows beyond which a lookup makes the table grow first
         self.keys = torch.full((cap,), _EMPTY, dtype=torch.int64, device=dev)
         used = self.dim * (1 + sum(info["slabs"]))
         pitch = record_pitch(self.dim, used, info["needs_steps"])

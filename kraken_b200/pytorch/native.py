@@ -165,7 +165,10 @@ def pull_sparse_table(table_id: int, indices: torch.Tensor) -> torch.Tensor:
 
 
 def combine_pull_sparse_table(table_ids: Sequence[int], indices: Sequence[torch.Tensor]) -> List[torch.Tensor]:
-    outs = engine().combine_pull_sparse_table(list(table_ids), list(indices))
+    eng = engine()
+    outs = eng.combine_pull_sparse_table(list(table_ids), list(indices))
+    if hasattr(eng, "plain_float32") and eng.plain_float32(table_ids):
+        return outs
     return [_as_registered(i, t) for i, t in zip(table_ids, outs)]
 
 

@@ -8,6 +8,7 @@ here synchronises the host: errors are collected from device status words by
 """
 from __future__ import annotations
 
+import contextlib
 import os
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -21,6 +22,8 @@ from ..parallel.sparse_shard import GpuSparseTable, GroupChannel, RowCounters, S
 from ..utils import profiler as _profiler
 from .engine import Engine, EngineConfig, TableInfo
 
+_NO_REGION = contextlib.nullcontext()
+
 
 class GpuEngine(Engine):
     def __init__(self, cfg: EngineConfig, rank: int = 0, world: int = 1, group=None,
@@ -30,8 +33,11 @@ class GpuEngine(Engine):
             raise RuntimeError("the GPU engine needs a CUDA device")
         self.device = device or torch.device("cuda", torch.cuda.current_device())
         torch.cuda.set_device(self.device)
+        if self.device.index is None:
+            self.device = torch.device("cuda", torch.cuda.current_device())
         self.lr_dev = torch.zeros(1, dtype=torch.float32, device=self.device)
         self._lr_host = torch.zeros(1, dtype=torch.float32).pin_memory()
+        self._lr_sent: Optional[float] = None   # what lr_dev was last set from (a float32 need not compare equal to it)
         self.sparse: Dict[int, GpuSparseTable] = {}
         self.counters = RowCounters(self.device)
         self._sample_next = False
@@ -39,6 +45,7 @@ class GpuEngine(Engine):
         self.tickets: Dict[int, Tuple[Ticket, int, int, int]] = {}
         self.group_channels: Dict[Tuple[int, ...], GroupChannel] = {}
         self.group_tickets: Dict[Tuple[int, ...], tuple] = {}
+        self._classes: Dict[Tuple[int, ...], Optional[Dict[int, List[int]]]] = {}   # see _dim_classes
         self.owner_world = world   # sparse rows live on ranks 0 .. owner_world - 1; reshard() changes it
         self.dense_init: Dict[int, torch.Tensor] = {}
         self.bucket: Optional[BucketSet] = None
@@ -54,12 +61,13 @@ class GpuEngine(Engine):
         self.nccl = cfg.exchange == "nccl" and world > 1
         self.nccl_channels: Dict[int, NcclSparseChannel] = {}
         from ..ops import mlp as fused_mlp
+        self._fused_mlp = fused_mlp
         fused_mlp.set_deferred_join(bool(cfg.overlap_dense_step) and not self.nccl)
 
     # ------------------------------------------------------------------ registry hooks
     def _on_update_lr(self) -> None:
-        if float(self._lr_host[0]) != self.lr or self._steps == 0:
-            self._lr_host[0] = self.lr
+        if self._lr_sent != self.lr or self._steps == 0:
+            self._lr_host[0] = self._lr_sent = self.lr
             self.lr_dev.copy_(self._lr_host, non_blocking=True)
 
     def _on_register_dense(self, info: TableInfo, val: torch.Tensor) -> None:
@@ -187,18 +195,16 @@ class GpuEngine(Engine):
             if self.nccl:
                 for g in b.grads():
                     dist.all_reduce(g, group=self.group)
-            from ..ops import mlp as fused_mlp
-            side = fused_mlp.take_pending_side_stream(self.device) if not self.nccl else None
-            main = torch.cuda.current_stream(self.device)
+            side = self._fused_mlp.take_pending_side_stream(self.device) if not self.nccl else None
             if side is not None:
                 # the MLP backward left its weight gradients on this stream: step (what is left) there, then join
                 with torch.cuda.stream(side):
                     b.step(self.lr_dev)
-                main.wait_stream(side)
+                torch.cuda.current_stream(self.device).wait_stream(side)
             else:
                 b.step(self.lr_dev)
             if getattr(self, "_comm_used", False):
-                main.wait_stream(self._comm_stream)  # buckets that were stepped during the backward pass
+                torch.cuda.current_stream(self.device).wait_stream(self._comm_stream)  # buckets that were stepped during the backward pass
                 self._comm_used = False
         self._bucket_ready.clear()
         self._dense_pending = False
@@ -207,12 +213,11 @@ class GpuEngine(Engine):
     def _region(self, name: str):
         """Phase bracket: CUDA-event timing when KRAKEN_PROFILE is set, an NVTX range when KRAKEN_NVTX=1
         (for timeline tools), nothing otherwise."""
-        import contextlib
         if self.profiler is not None:
             return self.profiler.region(name)
         if self._nvtx:
             return torch.cuda.nvtx.range(f"kraken.{name}")
-        return contextlib.nullcontext()
+        return _NO_REGION
 
     def metrics(self) -> dict:
         """Counters of the shards (synchronises): rows and load factor per sparse table and, where
@@ -368,12 +373,17 @@ class GpuEngine(Engine):
     def _dim_classes(self, table_ids: Sequence[int]):
         """Positions of ``table_ids`` grouped by row width, in first-appearance order; None when a table is
         named twice (each call then goes through its own exchange)."""
-        if len(set(table_ids)) != len(table_ids):
-            return None
-        classes: Dict[int, List[int]] = {}
-        for pos, t in enumerate(table_ids):
-            classes.setdefault(self._table(t, "sparse").dimension, []).append(pos)
-        return classes
+        key = tuple(table_ids)
+        if key not in self._classes:  # a registered table keeps its width
+            classes: Optional[Dict[int, List[int]]] = None
+            if len(set(key)) == len(key):
+                classes = {}
+                for pos, t in enumerate(key):
+                    classes.setdefault(self._table(t, "sparse").dimension, []).append(pos)
+            if len(self._classes) >= 64:
+                self._classes.clear()
+            self._classes[key] = classes
+        return self._classes[key]
 
     def combine_pull_sparse_table(self, table_ids: Sequence[int], indices: Sequence[torch.Tensor]) -> List[torch.Tensor]:
         """All tables of one row width share ONE exchange (dedup keyed by (table, id), one dispatch, one
@@ -390,17 +400,27 @@ class GpuEngine(Engine):
                 out[pos[0]] = self.pull_sparse_table(table_ids[pos[0]], indices[pos[0]])
                 continue
             tids = tuple(int(table_ids[p]) for p in pos)
-            flat = [self._prep_ids(indices[p]).reshape(-1) for p in pos]
-            counts = [int(f.numel()) for f in flat]
+            mine = [indices[p] for p in pos]
+            flat, counts = self._concat_ids(mine)
             ch = self._group_channel(tids, sum(counts))
             self._ensure_rooms(tids, counts, [None] * len(tids))
             with self._region("pull"):
-                rows, ticket = ch.pull(torch.cat(flat), counts)
+                rows, ticket = ch.pull(flat, counts)
             self._looked_up()
-            self.group_tickets[tids] = (ticket, [indices[p] for p in pos], [self._sig(indices[p]) for p in pos])
-            for p, part in zip(pos, rows.split(counts)):
-                out[p] = part.view(*indices[p].shape, dim)
+            self.group_tickets[tids] = (ticket, mine, C.signatures(mine))
+            for p, part in zip(pos, C.split_rows(rows, mine)):
+                out[p] = part
         return out
+
+    def plain_float32(self, table_ids: Sequence[int]) -> bool:
+        """Whether every one of these tables is registered as what the shards hold."""
+        tables = self.tables
+        return all(tables[t].dtype is torch.float32 for t in table_ids)
+
+    def _concat_ids(self, indices: Sequence[torch.Tensor]):
+        """The ids of several tables back to back on this device, and how many each table has."""
+        done = C.concat_ids(indices, self.device.index)
+        return done if done is not None else C.concat_ids([self._prep_ids(t) for t in indices], self.device.index)
 
     def combine_push_sparse_table(self, table_ids: Sequence[int], indices: Sequence[torch.Tensor],
                                   grads: Sequence[torch.Tensor]) -> None:
@@ -414,22 +434,17 @@ class GpuEngine(Engine):
                 self.push_sparse_table(table_ids[pos[0]], indices[pos[0]], grads[pos[0]])
                 continue
             tids = tuple(int(table_ids[p]) for p in pos)
-            grads = list(grads)
-            for p in pos:
-                if grads[p] is None:  # an output autograd never used
-                    grads[p] = torch.zeros((int(indices[p].numel()), dim), dtype=torch.float32, device=self.device)
-                if grads[p].numel() != indices[p].numel() * dim:
-                    raise C.KrakenError("gradient shape must be indices.shape + [dimension]")
+            mine = [indices[p] for p in pos]
+            g = C.concat_grads([grads[p] for p in pos], mine, dim, self.device.index)  # None: an output autograd never used
             saved = self.group_tickets.pop(tids, None)
-            ticket = saved[0] if saved is not None and saved[2] == [self._sig(indices[p]) for p in pos] else None
-            g = torch.cat([grads[p].detach().to(self.device, torch.float32).reshape(-1, dim) for p in pos])
-            ch = self._group_channel(tids, sum(int(indices[p].numel()) for p in pos))
+            ticket = saved[0] if saved is not None and saved[2] == C.signatures(mine) else None
+            ch = self._group_channel(tids, int(g.shape[0]))
             with self._region("push"):
                 if ticket is not None:
                     ch.push(g, self.lr_dev, ticket=ticket)
                 else:
-                    flat = [self._prep_ids(indices[p]).reshape(-1) for p in pos]
-                    ch.push(g, self.lr_dev, ids_cat=torch.cat(flat), counts=[int(f.numel()) for f in flat])
+                    flat, counts = self._concat_ids(mine)
+                    ch.push(g, self.lr_dev, ids_cat=flat, counts=counts)
 
     def combine_pull_sparse_pooled(self, table_ids: Sequence[int], inputs, means: Sequence[bool],
                                    patch_values: Sequence[float]):
@@ -753,17 +768,18 @@ class GpuEngine(Engine):
         ``channels``: what the lookup of each table goes through, None for a combined one or one over collectives."""
         self._sample_next = False  # a call that raised before its ``_looked_up`` leaves nothing to this one
         want, near = [], False
+        sparse, world = self.sparse, self.world
         for table_id, n_ids, ch in zip(table_ids, counts, channels):
-            t = self.sparse[table_id]
-            inflow = n_ids * self.world  # worst case: every rank's ids of this call belong to this shard
+            t = sparse[table_id]
+            inflow = n_ids * world  # worst case: every rank's ids of this call belong to this shard
             if ch is not None:
                 # no more than the exchange buffers admit (world x cap_s), and with a uniform owner hash about
                 # 1 / world of every rank's unique ids - twice that is reserved; a shard that still runs full
                 # reports kTableFull and is grown by end_step()
                 n_ids = min(n_ids, ch.cap_u)
-                inflow = min(self.world * ch.cap_s, 2 * n_ids) if self.world > 1 else n_ids
+                inflow = min(world * ch.cap_s, 2 * n_ids) if world > 1 else n_ids
             want.append((t, inflow))
-            near = near or t.rows_bound() + 2 * inflow > 0.6 * t.capacity
+            near = near or t.rows_bound() + 2 * inflow > t.limit
         if torch.cuda.is_current_stream_capturing():
             if self.counters.captured is not None:  # nothing runs now, the replays count
                 self.counters.captured += want
@@ -772,12 +788,18 @@ class GpuEngine(Engine):
         if near:
             self.counters.poll()
             for _ in range(2):  # the sample that is waited for first may be an older one
-                if any(t.rows_bound() + inflow > 0.6 * t.capacity for t, inflow in want):
-                    self.counters.start()
-                    self.counters.poll(wait=True)
+                full = False
+                for t, inflow in want:
+                    if t.rows_bound() + inflow > t.limit:
+                        full = True
+                        break
+                if not full:
+                    break
+                self.counters.start()
+                self.counters.poll(wait=True)
             for t, inflow in want:
                 hi = t.rows_bound() + inflow
-                if hi > 0.6 * t.capacity:
+                if hi > t.limit:
                     t.reserve(hi)
         for t, inflow in want:
             t.added += inflow

@@ -108,11 +108,17 @@ def from_env(rank: int = 0) -> Optional[StepProfiler]:
     return StepProfiler(path, rank)
 
 
+_native = None
+_NOTHING = contextlib.nullcontext()
+
+
 def engine_region(name: str):
     """Region of the process-global engine's profiler, or a no-op when profiling is off."""
-    from ..pytorch import native
-    if native.is_initialized():
-        prof = getattr(native.engine(), "profiler", None)
+    global _native
+    if _native is None:  # imported on first use: the engine imports this module
+        from ..pytorch import native as _native
+    if _native.is_initialized():
+        prof = getattr(_native.engine(), "profiler", None)
         if prof is not None:
             return prof.region(name)
-    return contextlib.nullcontext()
+    return _NOTHING

@@ -969,7 +969,7 @@ __device__ __forceinline__ int boxes_inside(int begin, int width, int limit) {
   return inside <= 0 ? 0 : (inside + 63) / 64;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairWgradThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairWgradThreads, 2)
 gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmD, const __grid_constant__ GemmArgs g) {
   extern __shared__ uint8_t smem_raw[];

@@ -141,6 +141,8 @@ bce_kernel(const float* __restrict__ logits, const float* __restrict__ labels, i
 }
 
 // ---- Linear layer with a single output (the MLP's logit head): y[m] = x[m, :] . w + b
+// Bound by memory: x is read once, 65536 x 400 in 16.5 us (3.2 TB/s, from L2 and DRAM).  Four rows a warp with 16-byte loads
+// took 18.2 us (a row of 400 fills 50 lanes of 64), and 3.2 us for 2.7 at 4096 rows, which leave such warps too few.
 __global__ void __launch_bounds__(kThreads)
 rowdot_forward_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* __restrict__ w,
                       const float* __restrict__ bias, const float* __restrict__ addend, int M, int K,
@@ -168,44 +170,6 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
   for (int q = 0; q < 4; ++q) {
     f[2 * q] = __uint_as_float(w[q] << 16);
     f[2 * q + 1] = __uint_as_float(w[q] & 0xFFFF0000u);
-  }
-}
-
-// The same for K % 8 == 0 and 16-byte aligned rows.  Bound by memory: x is read once.  A warp has four rows in flight and
-// a lane reads 16 bytes of each, where the kernel above waits for 4-byte loads of one row.
-__global__ void __launch_bounds__(kThreads)
-rowdot_forward_wide_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* __restrict__ w,
-                           const float* __restrict__ bias, const float* __restrict__ addend, int M, int K,
-                           float* __restrict__ y) {
-  pdl_enter();
-  constexpr int kRows = 4;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int m0 = warp * kRows; m0 < M; m0 += nwarps * kRows) {
-    float acc[kRows] = {0.f, 0.f, 0.f, 0.f};
-    for (int k = lane * 8; k < K; k += 256) {
-      uint4 v[kRows];
-#pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        v[r] = m0 + r < M ? __ldcg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(m0 + r) * ldx + k))
-                          : make_uint4(0, 0, 0, 0);
-      const float4 wa = *reinterpret_cast<const float4*>(w + k), wb = *reinterpret_cast<const float4*>(w + k + 4);
-#pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        float f[8];
-        unpack8(v[r], f);
-        acc[r] += f[0] * wa.x + f[1] * wa.y + f[2] * wa.z + f[3] * wa.w;
-        acc[r] += f[4] * wb.x + f[5] * wb.y + f[6] * wb.z + f[7] * wb.w;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < kRows; ++r)
-      for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
-    if (lane < kRows && m0 + lane < M) {
-      const float a = lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3];
-      y[m0 + lane] = a + (bias ? bias[0] : 0.f) + (addend ? addend[m0 + lane] : 0.f);
-    }
   }
 }
 
@@ -610,14 +574,6 @@ void bce_forward_backward(const float* logits, const float* labels, int n, float
 void rowdot_forward(const __nv_bfloat16* x, int ldx, const float* w, const float* bias, const float* addend, int M,
                     int K, float* y, cudaStream_t stream) {
   if (M <= 0) return;
-  const bool wide = K % 8 == 0 && ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
-                    (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  if (wide) {
-    int grid = (M + 4 * (kThreads / 32) - 1) / (4 * (kThreads / 32));
-    if (grid > 148 * 8) grid = 148 * 8;
-    launch_pdl(rowdot_forward_wide_kernel, dim3(grid), dim3(kThreads), 0, stream, x, ldx, w, bias, addend, M, K, y);
-    return;
-  }
   int grid = (M * 32 + kThreads - 1) / kThreads;
   if (grid > 148 * 8) grid = 148 * 8;
   launch_pdl(rowdot_forward_kernel, dim3(grid), dim3(kThreads), 0, stream, x, ldx, w, bias, addend, M, K, y);

@@ -15,6 +15,8 @@
 // Reference model math: examples/DeepFM/model/DeepFM.py:87-125 (torch CPU ops).
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -24,6 +26,9 @@ namespace cu {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kForwardBlocks = 4;   // a multiprocessor: 64 registers a thread
+constexpr int kBatch = 7;           // row loads of a lane in flight in the forward pass: as many as those registers hold
+constexpr int kBackwardBlocks = 6;
 
 // Row index of unique entry `u`: the entry itself when the rows were gathered into a receive
 // buffer, or the table slot the owner resolved for it when the kernel reads the table in place
@@ -35,26 +40,38 @@ __device__ __forceinline__ size_t row_of(const int* __restrict__ slots, int u) {
   return static_cast<size_t>(s < 0 ? 0 : s);
 }
 
+// Field groups per sample: as many as keep (D / 4) x G lanes within a quarter warp.
+constexpr int field_groups(int chunks) {
+  int g = 1;
+  while (chunks * g * 2 <= 16) g <<= 1;
+  return g;
+}
+
 // P2 and P1 are the pitches of rows2 and rows1 in floats: the row width for gathered rows, the tables' pitch in place.
 // Lanes per sample = (D / 4) x G: lane (g, c) owns dims [4c, 4c + 4) of the fields g, g + G, ...
 // Splitting the fields over G lane groups (a power of two) multiplies the number of independent
 // row loads in flight; the per-sample sums are combined with shuffles and the forward pass leaves
 // S[b, :] = sum_f e_f for the backward pass, whose lanes then need nothing from each other.
+// The forward pass is bound by the latency of its loads, entry -> slot -> row, not by bandwidth.  So a lane fetches the entries
+// of two of 2 x lpr fields, reads their first-order weights, and the lane groups get theirs by shuffles: kBatch rows of each
+// lane are in flight together.  65536 samples of 26 fields of dim 16, rows in L2: 36.8 us (5.2 TB/s of rows and x); 50.2 us
+// with the entries loaded where they are used, four fields unrolled and the rest one after the other.  Four rows in flight
+// take 39.1 us, eight 42.5 (they spill), seven with 5 blocks and spills 64; with the sizes as arguments of the kernel 43.8.
 // FM false (Wide&Deep): the logit is sum_f w_f alone, and the backward pass needs neither the rows nor ssum.
-template <bool FM>
-__global__ void __launch_bounds__(kThreads)
+template <bool FM, int chunks>
+__global__ void __launch_bounds__(kThreads, kForwardBlocks)
 deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restrict__ inv2,
                            const int* __restrict__ slots2, const float* __restrict__ rows1,
                            const int* __restrict__ inv1, const int* __restrict__ slots1,
-                           const float* __restrict__ dense, int B, int F, int D, int P2, int P1, int ND, int lpr, int G,
+                           const float* __restrict__ dense, int B, int F, int P2, int P1, int ND,
                            __nv_bfloat16* __restrict__ x, int ldx, float* __restrict__ fm_logit,
                            float* __restrict__ ssum) {
   pdl_enter();
+  constexpr int D = 4 * chunks, G = field_groups(chunks), lpr = chunks * G;
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = gtid % lpr;
   const int stride = (gridDim.x * blockDim.x) / lpr;
   const unsigned group_mask = (lpr == 32 ? 0xffffffffu : ((1u << lpr) - 1u)) << ((threadIdx.x & 31) / lpr * lpr);
-  const int chunks = D / 4;
   const int c = lane % chunks;   // chunks * G == lpr
   const int fg = lane / chunks;
   const int rounds = (B + stride - 1) / stride;
@@ -62,30 +79,60 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
     const int b = gtid / lpr + it * stride;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f), q = s;
     float part = 0.f;
-    if (b < B) {
+    const int fields = b < B ? F : 0;
+    __nv_bfloat16* xr = x + static_cast<size_t>(b) * ldx;
+    for (int base = 0; base < F; base += 2 * lpr) {
+      const int f0 = base + lane, f1 = f0 + lpr;
       const int* i2 = inv2 + static_cast<size_t>(b) * F;
-      __nv_bfloat16* xr = x + static_cast<size_t>(b) * ldx;
-#pragma unroll 4
-      for (int f = fg; f < F; f += G) {
-        const float4 e = __ldcg(reinterpret_cast<const float4*>(rows2 + row_of(slots2, i2[f]) * P2) + c);
-        if (FM) {
-          s.x += e.x, s.y += e.y, s.z += e.z, s.w += e.w;
-          q.x += e.x * e.x, q.y += e.y * e.y, q.z += e.z * e.z, q.w += e.w * e.w;
-        }
-        __nv_bfloat162 lo = __floats2bfloat162_rn(e.x, e.y), hi = __floats2bfloat162_rn(e.z, e.w);
-        uint2 packed;
-        packed.x = *reinterpret_cast<uint32_t*>(&lo);
-        packed.y = *reinterpret_cast<uint32_t*>(&hi);
-        *reinterpret_cast<uint2*>(xr + f * D + c * 4) = packed;
-      }
-      // first-order weights, dense features and the zero pad, spread over the sample's lanes
+      int r0 = 0, r1 = 0;
+      if (f0 < fields) r0 = i2[f0];
+      if (f1 < fields) r1 = i2[f1];
+      float w0 = 0.f, w1 = 0.f;
       if (rows1 != nullptr) {
         const int* i1 = inv1 + static_cast<size_t>(b) * F;
-        for (int f = lane; f < F; f += lpr) part += __ldcg(rows1 + row_of(slots1, i1[f]) * P1);
-      } else {
-        // folded layout: column D of the same row is the field's first-order weight
-        for (int f = lane; f < F; f += lpr) part += __ldcg(rows2 + row_of(slots2, i2[f]) * P2 + D);
+        int u0 = 0, u1 = 0;
+        if (f0 < fields) u0 = i1[f0];
+        if (f1 < fields) u1 = i1[f1];
+        if (f0 < fields) w0 = __ldcg(rows1 + row_of(slots1, u0) * P1);
+        if (f1 < fields) w1 = __ldcg(rows1 + row_of(slots1, u1) * P1);
       }
+      if (slots2 != nullptr) {
+        if (f0 < fields) r0 = static_cast<int>(row_of(slots2, r0));
+        if (f1 < fields) r1 = static_cast<int>(row_of(slots2, r1));
+      }
+      if (rows1 == nullptr) {
+        // folded layout: column D of the same row is the field's first-order weight
+        if (f0 < fields) w0 = __ldcg(rows2 + static_cast<size_t>(r0) * P2 + D);
+        if (f1 < fields) w1 = __ldcg(rows2 + static_cast<size_t>(r1) * P2 + D);
+      }
+      for (int j = 0; j < 2 * chunks && base + j * G < F; j += kBatch) {
+        float4 e[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int k = (j + i) * G + fg;  // field of the 2 x lpr
+          const int row = __shfl_sync(group_mask, j + i < chunks ? r0 : r1, k & (lpr - 1), lpr);
+          e[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (j + i < 2 * chunks && base + k < fields)
+            e[i] = __ldcg(reinterpret_cast<const float4*>(rows2 + static_cast<size_t>(row) * P2) + c);
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int k = (j + i) * G + fg;
+          if (FM) {
+            s.x += e[i].x, s.y += e[i].y, s.z += e[i].z, s.w += e[i].w;
+            q.x += e[i].x * e[i].x, q.y += e[i].y * e[i].y, q.z += e[i].z * e[i].z, q.w += e[i].w * e[i].w;
+          }
+          __nv_bfloat162 lo = __floats2bfloat162_rn(e[i].x, e[i].y), hi = __floats2bfloat162_rn(e[i].z, e[i].w);
+          uint2 packed;
+          packed.x = *reinterpret_cast<uint32_t*>(&lo);
+          packed.y = *reinterpret_cast<uint32_t*>(&hi);
+          if (j + i < 2 * chunks && base + k < fields) *reinterpret_cast<uint2*>(xr + (base + k) * D + c * 4) = packed;
+        }
+      }
+      part += w0 + w1;
+    }
+    if (b < B) {
+      // dense features and the zero pad, spread over the sample's lanes
       const int base = F * D;
       for (int j = lane; base + j < ldx; j += lpr)
         xr[base + j] = __float2bfloat16(j < ND ? dense[static_cast<size_t>(b) * ND + j] : 0.f);
@@ -106,18 +153,23 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
   }
 }
 
-template <bool FM>
-__global__ void __launch_bounds__(kThreads)
+// Bound by the reductions: those on one row are serialised in L2 (about 2.6 ns each), and the top id of a skewed field has
+// thousands.  65536 samples of 26 fields: 50.3 us for uniform ids, 90.4 for Zipf(1.1) ids, whose top ids come 5550 times; 52.1
+// and 92.9 us with the sizes as arguments, 57 for uniform ids at 4 blocks.  With the forward pass's batches uniform ids took
+// 70 us: the blocks in flight matter more.  Sums of the block's repeated ids first (counts and lists in shared memory) took 83
+// us for Zipf ids, but 70 for uniform ones.
+template <bool FM, int chunks>
+__global__ void __launch_bounds__(kThreads, kBackwardBlocks)
 deepfm_pack_backward_kernel(const float* __restrict__ rows2, const int* __restrict__ inv2,
                             const int* __restrict__ slots2, const int* __restrict__ inv1,
                             const __nv_bfloat16* __restrict__ dx, int lddx, const float* __restrict__ dlogit,
-                            const float* __restrict__ ssum, int B, int F, int D, int P2, int RD, int lpr, int G,
+                            const float* __restrict__ ssum, int B, int F, int P2, int RD,
                             float* ugrad2, float* ugrad1) {
   pdl_enter();
+  constexpr int D = 4 * chunks, G = field_groups(chunks), lpr = chunks * G;
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = gtid % lpr;
   const int stride = (gridDim.x * blockDim.x) / lpr;
-  const int chunks = D / 4;
   const int c = lane % chunks;
   const int fg = lane / chunks;
   for (int b = gtid / lpr; b < B; b += stride) {
@@ -160,18 +212,24 @@ Sym to_sym(const SymHost& h) {
   return s;
 }
 
-// Field groups per sample: as many as keep (D / 4) x G lanes within a quarter warp.
-int field_groups(int chunks) {
-  int g = 1;
-  while (chunks * g * 2 <= 16) g <<= 1;
-  return g;
-}
-
 int grid_for(long long rows, int lpr) {
   long long g = (rows * lpr + kThreads - 1) / kThreads;
   if (g < 1) g = 1;
   if (g > 148 * 16) g = 148 * 16;
   return static_cast<int>(g);
+}
+
+// Calls f with the chunk count as a compile-time constant; D is 4 .. 128, D / 4 a power of two (the bindings check it).
+template <typename Fn>
+void by_chunks(int D, Fn f) {
+  switch (D / 4) {
+    case 1: return f(std::integral_constant<int, 1>());
+    case 2: return f(std::integral_constant<int, 2>());
+    case 4: return f(std::integral_constant<int, 4>());
+    case 8: return f(std::integral_constant<int, 8>());
+    case 16: return f(std::integral_constant<int, 16>());
+    case 32: return f(std::integral_constant<int, 32>());
+  }
 }
 
 }  // namespace
@@ -180,12 +238,12 @@ void deepfm_pack_forward(const float* rows2, const int* inv2, const int* slots2,
                          const int* slots1, const float* dense, int B, int F, int D, int P2, int P1, int ND, __nv_bfloat16* x,
                          int ldx, float* fm_logit, float* ssum, bool fm, cudaStream_t stream) {
   if (B <= 0) return;
-  const int chunks = D / 4;
-  const int G = field_groups(chunks);
-  const int lpr = chunks * G;
-  auto kernel = fm ? deepfm_pack_forward_kernel<true> : deepfm_pack_forward_kernel<false>;
-  launch_pdl(kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, rows1, inv1, slots1, dense,
-                                                                        B, F, D, P2, P1, ND, lpr, G, x, ldx, fm_logit, ssum);
+  by_chunks(D, [&](auto n) {
+    constexpr int chunks = decltype(n)::value;
+    auto kernel = fm ? deepfm_pack_forward_kernel<true, chunks> : deepfm_pack_forward_kernel<false, chunks>;
+    launch_pdl(kernel, dim3(grid_for(B, chunks * field_groups(chunks))), dim3(kThreads), 0, stream, rows2, inv2, slots2,
+               rows1, inv1, slots1, dense, B, F, P2, P1, ND, x, ldx, fm_logit, ssum);
+  });
 }
 
 void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2, const int* inv1,
@@ -193,12 +251,12 @@ void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2
                           const float* dlogit, const float* ssum, int B, int F, int D, int P2, int RD, float* ugrad2,
                           float* ugrad1, cudaStream_t stream) {
   if (B <= 0) return;
-  const int chunks = D / 4;
-  const int G = field_groups(chunks);
-  const int lpr = chunks * G;
-  auto kernel = ssum != nullptr ? deepfm_pack_backward_kernel<true> : deepfm_pack_backward_kernel<false>;
-  launch_pdl(kernel, dim3(grid_for(B, lpr)), dim3(kThreads), 0, stream, rows2, inv2, slots2, inv1, dx, lddx, dlogit,
-                                                                         ssum, B, F, D, P2, RD, lpr, G, ugrad2, ugrad1);
+  by_chunks(D, [&](auto n) {
+    constexpr int chunks = decltype(n)::value;
+    auto kernel = ssum != nullptr ? deepfm_pack_backward_kernel<true, chunks> : deepfm_pack_backward_kernel<false, chunks>;
+    launch_pdl(kernel, dim3(grid_for(B, chunks * field_groups(chunks))), dim3(kThreads), 0, stream, rows2, inv2, slots2,
+               inv1, dx, lddx, dlogit, ssum, B, F, P2, RD, ugrad2, ugrad1);
+  });
 }
 
 }  // namespace cu

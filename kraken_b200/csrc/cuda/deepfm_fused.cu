@@ -28,7 +28,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kForwardBlocks = 4;   // a multiprocessor: 64 registers a thread
 constexpr int kBatch = 7;           // row loads of a lane in flight in the forward pass: as many as those registers hold
-constexpr int kBackwardBlocks = 6;
+constexpr int kBackwardBlocks = 5;
 
 // Row index of unique entry `u`: the entry itself when the rows were gathered into a receive
 // buffer, or the table slot the owner resolved for it when the kernel reads the table in place
@@ -154,10 +154,11 @@ deepfm_pack_forward_kernel(const float* __restrict__ rows2, const int* __restric
 }
 
 // Bound by the reductions: those on one row are serialised in L2 (about 2.6 ns each), and the top id of a skewed field has
-// thousands.  65536 samples of 26 fields: 50.3 us for uniform ids, 90.4 for Zipf(1.1) ids, whose top ids come 5550 times; 52.1
-// and 92.9 us with the sizes as arguments, 57 for uniform ids at 4 blocks.  With the forward pass's batches uniform ids took
-// 70 us: the blocks in flight matter more.  Sums of the block's repeated ids first (counts and lists in shared memory) took 83
-// us for Zipf ids, but 70 for uniform ones.
+// thousands.  65536 samples of 26 fields of dim 16: 52.1 us for uniform ids, 90.0 for Zipf(1.1) ids, whose top ids come 5550
+// times; 52.1 and 92.9 us with the sizes as arguments.  Over 500 .. 32768 samples of 10 .. 39 fields of 4 .. 64 floats it
+// takes 0.93 of the time of that form; with 4, 6 or 7 blocks a multiprocessor 0.96 to 0.97.  With the forward pass's batches
+// uniform ids took 70 us: the blocks in flight matter more.  Sums of the block's repeated ids first (counts and lists in
+// shared memory) took 83 us for Zipf ids, but 70 for uniform ones.
 template <bool FM, int chunks>
 __global__ void __launch_bounds__(kThreads, kBackwardBlocks)
 deepfm_pack_backward_kernel(const float* __restrict__ rows2, const int* __restrict__ inv2,

@@ -1761,6 +1761,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
 
   // ---------------- table maintenance
+  m.def("fill_records", [](const torch::Tensor& records, int at, int dim, float value) {
+    need_cuda(records, "records", torch::kFloat32);
+    TORCH_CHECK(records.dim() == 2 && at >= 0 && dim >= 0 && at + dim <= records.size(1) &&
+                    reinterpret_cast<uintptr_t>(records.data_ptr()) % 16 == 0,
+                "records must be a matrix on a 16-byte boundary that has the columns");
+    const c10::cuda::CUDAGuard device(records.device());
+    cu::fill_records(ptr<float>(records), records.numel(), static_cast<int>(records.size(1)), at, dim, value, cur_stream());
+    check_launch("fill_records");
+  });
   m.def("table_clear", [](const cu::TableHost& t) {
     cu::table_clear(t, cur_stream());
     check_launch("table_clear");

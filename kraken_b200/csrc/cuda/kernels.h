@@ -219,6 +219,7 @@ void group_push_apply(SymHost sym, ChanLayout lay, Ctrl* ctrl, const void* table
 void owner_of(const int64_t* ids, int n, uint64_t salt, int world, int* owners, cudaStream_t stream);
 
 // ---- table maintenance ----
+void fill_records(float* records, long long floats, int pitch, int at, int dim, float value, cudaStream_t stream);
 void table_clear(TableHost table, cudaStream_t stream);
 // Inserts rows with given values and states (any of s0..s2 / steps may be null).
 void table_import(TableHost table, const int64_t* ids, const float* vals, const float* s0, const float* s1,

@@ -155,15 +155,14 @@ class GpuSparseTable:
         self.keys = torch.full((cap,), _EMPTY, dtype=torch.int64, device=dev)
         used = self.dim * (1 + sum(info["slabs"]))
         pitch = record_pitch(self.dim, used, info["needs_steps"])
-        record = torch.zeros((cap, pitch), dtype=torch.float32, device=dev)
+        record = self._record = torch.empty((cap, pitch), dtype=torch.float32, device=dev)
+        self._reset_records()
         self.val = record[:, :self.dim]
         self.slabs, at = [], self.dim
         for k in range(3):
             if info["slabs"][k]:
                 self.slabs.append(record[:, at:at + self.dim])
                 at += self.dim
-                if info["type"] == 0 and k == 0 and info["initial_accumulator_value"]:
-                    self.slabs[k].fill_(info["initial_accumulator_value"])
             else:
                 self.slabs.append(None)
         self.steps = None
@@ -174,6 +173,14 @@ class GpuSparseTable:
         self._host = C.make_table(self.keys, self.val, self.slabs[0], self.slabs[1], self.slabs[2], self.steps,
                                   self.lead, self.size, self.status, bits, self.dim, self.init[0], self.init[1],
                                   self.init[2], self.seed_key)
+
+    def _reset_records(self) -> None:
+        """Zeros in every record but for Adagrad's accumulators (the first state), which start at their initial value."""
+        info = self.optim_info
+        if info["type"] == 0 and info["slabs"][0] and info["initial_accumulator_value"]:
+            C.fill_records(self._record, self.dim, self.dim, info["initial_accumulator_value"])
+        else:
+            self._record.zero_()
 
     @property
     def capacity(self) -> int:
@@ -337,11 +344,7 @@ class GpuSparseTable:
         before = self.num_rows()
         keep = self.export(filter_mode=3, min_steps=min_steps)
         C.table_clear(self._host)
-        self.val.zero_()
-        for k, s in enumerate(self.slabs):
-            if s is not None:
-                s.fill_(self.optim_info["initial_accumulator_value"] if (self.optim_info["type"] == 0 and k == 0)
-                        else 0.0)
+        self._reset_records()
         self.import_rows(keep["ids"], keep["vals"], keep["states"], keep["states_i"])
         return before - int(keep["ids"].numel())
 

@@ -58,3 +58,18 @@ def test_parts_of_a_record_keep_apart(optim, conf, dim):
     for k, s in enumerate(table.slabs):
         assert s is None or bool((s[free] == (fill if k == 0 else 0.0)).all())
     assert table.steps is None or bool((table.steps[free] == 0).all())
+
+
+# Pitches that are no multiple of the four floats of a thread's store, records larger than one; totals with a rest.
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,pitch,at,dim", [(1, 1, 0, 1), (3, 1, 0, 0), (5, 3, 1, 2), (7, 5, 2, 1), (333, 30, 10, 10),
+                                               (1000, 128, 64, 64), (300_001, 7, 3, 3)])
+def test_records_are_filled_by_column(rows, pitch, at, dim):
+    from kraken_b200._native import C
+    records = torch.full((rows, pitch), 7.0, device="cuda")
+    C.fill_records(records, at, dim, 0.1)
+    want = torch.zeros(rows, pitch, device="cuda")
+    want[:, at:at + dim] = 0.1
+    assert torch.equal(records, want)
+    with pytest.raises(RuntimeError):
+        C.fill_records(records, at, pitch - at + 1, 0.1)

@@ -37,7 +37,7 @@ class GpuEngine(Engine):
             self.device = torch.device("cuda", torch.cuda.current_device())
         self.lr_dev = torch.zeros(1, dtype=torch.float32, device=self.device)
         self._lr_host = torch.zeros(1, dtype=torch.float32).pin_memory()
-        self._lr_sent: Optional[float] = None   # what lr_dev was last set from (a float32 need not compare equal to it)
+        self._lr_sent: Optional[float] = None   # what lr_dev was last set from (a float32 need not compare equal to it); None: not known
         self.sparse: Dict[int, GpuSparseTable] = {}
         self.counters = RowCounters(self.device)
         self._sample_next = False
@@ -67,7 +67,9 @@ class GpuEngine(Engine):
     # ------------------------------------------------------------------ registry hooks
     def _on_update_lr(self) -> None:
         if self._lr_sent != self.lr or self._steps == 0:
-            self._lr_host[0] = self._lr_sent = self.lr
+            # in a capture the copy is only recorded: until that graph is replayed lr_dev holds what it held
+            self._lr_sent = None if torch.cuda.is_current_stream_capturing() else self.lr
+            self._lr_host[0] = self.lr
             self.lr_dev.copy_(self._lr_host, non_blocking=True)
 
     def _on_register_dense(self, info: TableInfo, val: torch.Tensor) -> None:

@@ -67,10 +67,17 @@ class GpuEngine(Engine):
     # ------------------------------------------------------------------ registry hooks
     def _on_update_lr(self) -> None:
         if self._lr_sent != self.lr or self._steps == 0:
-            # in a capture the copy is only recorded: until that graph is replayed lr_dev holds what it held
-            self._lr_sent = None if torch.cuda.is_current_stream_capturing() else self.lr
             self._lr_host[0] = self.lr
-            self.lr_dev.copy_(self._lr_host, non_blocking=True)
+            if torch.cuda.is_current_stream_capturing():
+                # only recorded: until that graph is replayed lr_dev holds what it held.  A replay takes the latest rate;
+                # the host may be ahead of it, but then it has enqueued a fill behind it, too.
+                self._lr_sent = None
+                self.lr_dev.copy_(self._lr_host, non_blocking=True)
+            else:
+                # as an argument of the kernel: a copy reads the host's word when it runs, and by then the host may have
+                # written the rate of a later step there
+                self._lr_sent = self.lr
+                self.lr_dev.fill_(self.lr)
 
     def _on_register_dense(self, info: TableInfo, val: torch.Tensor) -> None:
         v = val.detach().to(self.device, torch.float32).contiguous().clone()

@@ -38,3 +38,15 @@ def test_a_rate_that_changed_during_a_capture_reaches_what_follows(rate, replaye
     before = table.lookup(ids)[0].clone()
     train(ids)
     assert torch.allclose(before - table.lookup(ids)[0], torch.full_like(before, rate * 0.25), rtol=1e-4)
+
+
+def test_a_step_has_its_own_rate_when_the_host_runs_ahead():
+    kk.initialize("gpu", table_capacity=1 << 10, seed=2)
+    eng = kk.native.engine()
+    kk.update_lr(1.0)
+    seen = []
+    torch.cuda._sleep(200_000_000)   # a tenth of a second in which the host enqueues everything below
+    for k in range(20):
+        kk.update_lr(0.1 * 0.9 ** k)
+        seen.append(eng.lr_dev.clone())   # what a kernel enqueued here reads
+    assert [float(s) for s in seen] == pytest.approx([0.1 * 0.9 ** k for k in range(20)])

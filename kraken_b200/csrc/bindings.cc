@@ -1638,7 +1638,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     check_launch("group_push_apply");
   });
 
-  // dst[i].copy_(src[i], non_blocking=True) for every i, those that are plain copies on this device in one launch.
+  // dst[i].copy_(src[i], non_blocking=True) for every i, in the order in which they are named; plain copies on this device
+  // go in one launch.  A launch copies its buffers side by side, so one whose memory another's copy writes, or that writes
+  // memory which another's copy reads, waits for the next.
   m.def("copy_batch", [](const std::vector<torch::Tensor>& dst, const std::vector<torch::Tensor>& src) {
     TORCH_CHECK(dst.size() == src.size(), "one source per destination is needed");
     cu::CopyBatch b{};
@@ -1651,21 +1653,39 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       }
       b.n = 0;
     };
+    auto apart = [](const char* p, long long n, const char* q, long long m) {
+      const uintptr_t x = reinterpret_cast<uintptr_t>(p), y = reinterpret_cast<uintptr_t>(q);
+      return x + n <= y || y + m <= x;
+    };
     for (size_t i = 0; i < dst.size(); ++i) {
       const torch::Tensor &d = dst[i], &s = src[i];
-      const bool plain = d.is_cuda() && d.device() == s.device() && d.get_device() == c10::cuda::current_device() &&
-                         d.scalar_type() == s.scalar_type() && d.sizes() == s.sizes() && d.is_contiguous() &&
-                         s.is_contiguous() && !d.requires_grad() && !s.requires_grad() && !s.is_neg() && !s.is_conj() &&
-                         !d.is_neg() && !d.is_conj();
+      bool plain = d.is_cuda() && d.device() == s.device() && d.get_device() == c10::cuda::current_device() &&
+                   d.scalar_type() == s.scalar_type() && d.sizes() == s.sizes() && d.is_contiguous() && s.is_contiguous() &&
+                   !d.requires_grad() && !s.requires_grad() && !s.is_neg() && !s.is_conj() && !d.is_neg() && !d.is_conj();
+      const char* from = nullptr;
+      char* to = nullptr;
+      long long bytes = 0;
+      if (plain) {
+        from = static_cast<const char*>(s.data_ptr()), to = static_cast<char*>(d.data_ptr());
+        bytes = static_cast<long long>(d.nbytes());
+        if (bytes == 0 || from == to) continue;
+        plain = apart(from, bytes, to, bytes);  // else copy_ refuses it
+      }
       if (!plain) {
-        flush();  // in the order they were named
+        flush();
         torch::Tensor(d).copy_(s, true);
         continue;
       }
-      if (d.numel() == 0) continue;
-      b.src[b.n] = static_cast<const char*>(s.data_ptr());
-      b.dst[b.n] = static_cast<char*>(d.data_ptr());
-      b.bytes[b.n] = static_cast<long long>(d.nbytes());
+      for (int l = 0; l < b.n; ++l) {
+        if (apart(to, bytes, b.dst[l], b.bytes[l]) && apart(to, bytes, b.src[l], b.bytes[l]) &&
+            apart(from, bytes, b.dst[l], b.bytes[l]))
+          continue;
+        flush();
+        break;
+      }
+      b.src[b.n] = from;
+      b.dst[b.n] = to;
+      b.bytes[b.n] = bytes;
       ++b.n;
       d.unsafeGetTensorImpl()->bump_version();
       if (b.n == cu::CopyBatch::kMax) flush();

@@ -31,3 +31,28 @@ def test_what_is_not_a_plain_copy_is_copied_as_torch_does():
         assert torch.equal(d, torch.zeros_like(d).copy_(s))
     with pytest.raises(RuntimeError):
         C.copy_batch(dst, src[:-1])
+
+
+def test_buffers_that_overlap_are_copied_in_the_order_they_are_named():
+    """A step whose inputs are its own earlier inputs: what the first copies wrote is what the later ones read."""
+    n = 1 << 22
+    def buffers():
+        return [torch.full((n,), float(k), device=DEV) for k in range(4)]
+    pairs = [lambda a, b, c, d: ([b, c, d], [a, b, c]),             # every one gets the first one's values
+             lambda a, b, c, d: ([d, c, b], [c, b, a]),             # shifted by one
+             lambda a, b, c, d: ([a, b], [b, a]),
+             lambda a, b, c, d: ([a, b, a], [b, c, d]),             # written twice
+             lambda a, b, c, d: ([a[n // 2:], b[:n // 2 + 5]], [c[n // 2:], a[n // 2 - 5:]]),
+             lambda a, b, c, d: ([a[1:n // 2], c], [b[1:n // 2], a]),
+             lambda a, b, c, d: ([a, b, c], [a, b, d])]             # onto itself
+    for make in pairs:
+        for _ in range(5):
+            got, want = buffers(), buffers()
+            C.copy_batch(*make(*got))
+            for t, s in zip(*make(*want)):
+                t.copy_(s)
+            assert all(torch.equal(x, y) for x, y in zip(got, want))
+    a = torch.arange(64.0, device=DEV)
+    for t, s in ((a[:48], a[16:]), (a[16:], a[:48])):
+        with pytest.raises(RuntimeError):   # as copy_ itself: a part of what is read is written
+            C.copy_batch([t, torch.empty(3, device=DEV)], [s, torch.ones(3, device=DEV)])

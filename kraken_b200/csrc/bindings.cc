@@ -1683,10 +1683,17 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         flush();
         break;
       }
-      b.src[b.n] = from;
-      b.dst[b.n] = to;
-      b.bytes[b.n] = bytes;
-      ++b.n;
+      // Off 16 bytes the kernel goes by words or pairs of them: two buffers of 4 MB on any float took 8.6 us, 8.3 as copies of
+      // their own, of 64 MB 111 and 49, of 256 KB 2.7 and 6.2.
+      const uintptr_t both = reinterpret_cast<uintptr_t>(from) | reinterpret_cast<uintptr_t>(to);
+      if (both % 4 != 0 || (both % 16 != 0 && bytes >= 4 << 20)) {
+        CUDA_OK(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, cur_stream()));
+      } else {
+        b.src[b.n] = from;
+        b.dst[b.n] = to;
+        b.bytes[b.n] = bytes;
+        ++b.n;
+      }
       d.unsafeGetTensorImpl()->bump_version();
       if (b.n == cu::CopyBatch::kMax) flush();
     }

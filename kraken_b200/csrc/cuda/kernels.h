@@ -265,13 +265,14 @@ void deepfm_pack_backward(const float* rows2, const int* inv2, const int* slots2
                           const __nv_bfloat16* dx, int lddx, const float* dlogit, const float* ssum, int B, int F, int D,
                           int P2, int RD, float* ugrad2, float* ugrad1, cudaStream_t stream);
 
-// Several buffers copied in one launch; any sizes and alignments.
+// Several buffers copied in one launch; any sizes, on 4-byte boundaries.
 struct CopyBatch {
   static constexpr int kMax = 8;
   int n;
   const char* src[kMax];
   char* dst[kMax];
-  long long bytes[kMax], first[kMax];  // first: filled by the call
+  long long bytes[kMax], first[kMax];  // first, shift: filled by the call
+  int shift[kMax];
 };
 void copy_batch(CopyBatch b, cudaStream_t stream);
 

@@ -402,9 +402,9 @@ rowdot_backward_wide_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const 
 }
 
 // Buffers of a step's inputs, one launch for all of them: as copies of their own, each of two microseconds and its gap, they
-// stood in front of every replay of a captured step (three of a DeepFM batch
-// of 8192: 6.7 us, 3.3 so; of 65536: 12.4 and 8.2).  Thread t takes 16-byte piece
-// t of the buffers laid end to end; what is left of a buffer, or one that is not on 16 bytes, goes by bytes.
+// stood in front of every replay of a captured step (three of a DeepFM batch of 8192: 6.7 us, 3.3 so; of 65536: 12.4 and
+// 8.2).  Thread t takes piece t of the buffers laid end to end; a buffer goes in pieces of the 16, 8 or 4 bytes that both of
+// its addresses are aligned to (a batch sliced out of a larger tensor may start on any float), the rest of it by bytes.
 __global__ void __launch_bounds__(kThreads)
 copy_batch_kernel(CopyBatch b, long long pieces) {
   pdl_enter();
@@ -414,7 +414,7 @@ copy_batch_kernel(CopyBatch b, long long pieces) {
     uint4 v[kUnroll];
     const char* s[kUnroll];
     char* d[kUnroll];
-    int left[kUnroll];  // bytes of the piece, 0 for none
+    int size[kUnroll], left[kUnroll];  // bytes of a whole piece and of this one, 0 for none
 #pragma unroll
     for (int q = 0; q < kUnroll; ++q) {
       const long long p = p0 + q * stride;
@@ -422,21 +422,30 @@ copy_batch_kernel(CopyBatch b, long long pieces) {
       if (p >= pieces) continue;
       int l = 0;
       while (l + 1 < b.n && p >= b.first[l + 1]) ++l;
-      const long long at = (p - b.first[l]) * 16;
+      const long long at = (p - b.first[l]) << b.shift[l];
       s[q] = b.src[l] + at;
       d[q] = b.dst[l] + at;
-      left[q] = static_cast<int>(min(16ll, b.bytes[l] - at));
-      if (left[q] == 16 && ((reinterpret_cast<uintptr_t>(s[q]) | reinterpret_cast<uintptr_t>(d[q])) & 15) == 0) {
-        left[q] = 17;  // one load and one store
+      size[q] = 1 << b.shift[l];
+      left[q] = static_cast<int>(min(static_cast<long long>(size[q]), b.bytes[l] - at));
+      if (left[q] < size[q]) continue;
+      if (size[q] == 16)
         v[q] = __ldcs(reinterpret_cast<const uint4*>(s[q]));
-      }
+      else if (size[q] == 8)
+        *reinterpret_cast<uint2*>(&v[q]) = __ldcs(reinterpret_cast<const uint2*>(s[q]));
+      else
+        v[q].x = __ldcs(reinterpret_cast<const uint32_t*>(s[q]));
     }
 #pragma unroll
     for (int q = 0; q < kUnroll; ++q) {
-      if (left[q] == 17)
-        *reinterpret_cast<uint4*>(d[q]) = v[q];
-      else
+      if (left[q] == 0) continue;
+      if (left[q] < size[q])
         for (int j = 0; j < left[q]; ++j) d[q][j] = s[q][j];
+      else if (size[q] == 16)
+        *reinterpret_cast<uint4*>(d[q]) = v[q];
+      else if (size[q] == 8)
+        *reinterpret_cast<uint2*>(d[q]) = make_uint2(v[q].x, v[q].y);
+      else
+        *reinterpret_cast<uint32_t*>(d[q]) = v[q].x;
     }
   }
 }
@@ -517,8 +526,10 @@ cast_weights_kernel(CastBatch b) {
 void copy_batch(CopyBatch b, cudaStream_t stream) {
   long long pieces = 0;
   for (int l = 0; l < b.n; ++l) {
+    const uintptr_t both = reinterpret_cast<uintptr_t>(b.src[l]) | reinterpret_cast<uintptr_t>(b.dst[l]);
+    b.shift[l] = both % 16 == 0 ? 4 : both % 8 == 0 ? 3 : 2;
     b.first[l] = pieces;
-    pieces += (b.bytes[l] + 15) / 16;
+    pieces += (b.bytes[l] + (1 << b.shift[l]) - 1) >> b.shift[l];
   }
   if (pieces <= 0) return;
   long long grid = (pieces + 4 * kThreads - 1) / (4 * kThreads);

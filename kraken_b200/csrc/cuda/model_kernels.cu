@@ -245,14 +245,14 @@ head_backward_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* 
                      __nv_bfloat16* __restrict__ dx, int lddx, float* dw, float* db) {
   pdl_enter();
   __shared__ float s_g[kHeadStep][C];
-  const int r0 = blockIdx.y * kHeadStep;
+  const int r0 = blockIdx.x * kHeadStep;
   const int rows = min(kHeadStep, M - r0);
   for (int i = threadIdx.x; i < kHeadStep * C; i += kHeadThreads) {
     const int r = i / C, c = i - r * C;
     s_g[r][c] = r < rows && c < classes ? g[static_cast<size_t>(r0 + r) * classes + c] : 0.f;
   }
   __syncthreads();
-  const int k = (blockIdx.x * kHeadThreads + threadIdx.x) * 4;
+  const int k = (blockIdx.y * kHeadThreads + threadIdx.x) * 4;
   if (k < K) {
     float wk[C][4], acc[C][4];
 #pragma unroll
@@ -298,7 +298,7 @@ head_backward_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* 
     for (int c = 0; c < C; ++c)
       if (c < classes) red_add_v4(dw + static_cast<size_t>(c) * K + k, make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]));
   }
-  if (blockIdx.x == 0 && threadIdx.x < classes) {
+  if (blockIdx.y == 0 && threadIdx.x < classes) {
     float s = 0.f;
     for (int r = 0; r < rows; ++r) s += s_g[r][threadIdx.x];
     atomicAdd(db + threadIdx.x, s);
@@ -626,7 +626,7 @@ void head_backward(const __nv_bfloat16* x, int ldx, const float* w, const float*
   if (M <= 0) return;
   auto kernel = classes <= 4 ? head_backward_kernel<4> : classes <= 8 ? head_backward_kernel<8>
                 : classes <= 12 ? head_backward_kernel<12> : head_backward_kernel<16>;
-  const dim3 grid((K / 4 + kHeadThreads - 1) / kHeadThreads, (M + kHeadStep - 1) / kHeadStep);
+  const dim3 grid((M + kHeadStep - 1) / kHeadStep, (K / 4 + kHeadThreads - 1) / kHeadThreads);  // y ends at 65535
   launch_pdl(kernel, grid, dim3(kHeadThreads), 0, stream, x, ldx, w, g, M, K, classes, relu_mask ? 1 : 0, dx, lddx, dw, db);
 }
 

@@ -67,3 +67,20 @@ def test_operands_the_kernels_do_not_take():
     assert not C.head_supported(x[:, 1:9], torch.zeros(10, 8, device=DEV))         # rows off a 16-byte boundary
     assert not C.head_supported(x, torch.zeros(161, device=DEV)[1:].view(10, 16))  # weights off a 16-byte boundary
     assert not C.head_supported(x, w, torch.zeros(16, 10, device=DEV).t())         # gradient buffer with another stride
+
+
+def test_more_rows_than_a_grid_is_high():
+    """65535 blocks of rows and one more, in the direction of a grid that ends there."""
+    M, K, classes = 65535 * 32 + 7, 8, 3
+    torch.manual_seed(0)
+    x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    w, b, g = torch.randn(classes, K, device=DEV), torch.randn(classes, device=DEV), torch.randn(M, classes, device=DEV)
+    y, dx, dw, db = torch.empty(M, classes, device=DEV), torch.empty_like(x), torch.zeros_like(w), torch.zeros_like(b)
+    C.head_forward(x, w, b, y)
+    C.head_backward(x, w, g, False, dx, dw, db)
+    xd, wd, gd = x.double(), w.double(), g.double()
+    close(y, (xd @ wd.t() + b.double(), xd.abs() @ wd.abs().t() + b.double().abs()), K + 1)
+    close(dw, (gd.t() @ xd, gd.abs().t() @ xd.abs()), M)
+    close(db, (gd.sum(0), gd.abs().sum(0)), M)
+    want = gd @ wd
+    assert bool(((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -20 * (gd.abs() @ wd.abs())).all())

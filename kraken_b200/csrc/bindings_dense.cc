@@ -339,8 +339,12 @@ void bind_dense(py::module_& m) {
       dxp = reinterpret_cast<__nv_bfloat16*>(dx->data_ptr());
       lddx = dx->stride(0);
     }
+    torch::Tensor part;  // on this stream, like the kernels that write and read it
+    const size_t floats = cu::head_part_floats(x.size(0), x.size(1), w.size(0));
+    if (floats > 0) part = torch::empty({static_cast<int64_t>(floats)}, g.options());
     cu::head_backward(bf(x), x.stride(0), w.data_ptr<float>(), g.data_ptr<float>(), x.size(0), x.size(1), w.size(0),
-                      relu_mask, dxp, lddx, dw.data_ptr<float>(), db.data_ptr<float>(), cur_stream());
+                      relu_mask, dxp, lddx, dw.data_ptr<float>(), db.data_ptr<float>(),
+                      floats > 0 ? part.data_ptr<float>() : nullptr, cur_stream());
     check_launch("head_backward");
   });
   m.def("cast_weights", &cast_weights);

@@ -302,8 +302,10 @@ constexpr int kMaxHead = 16;
 bool head_supported(const void* x, int ldx, const void* w, int K, int classes);
 void head_forward(const __nv_bfloat16* x, int ldx, const float* w, const float* bias, int M, int K, int classes, float* y,
                   cudaStream_t stream);
+// The same operands give the same bits.  part: scratch of head_part_floats floats (none: 0).
+size_t head_part_floats(int M, int K, int classes);
 void head_backward(const __nv_bfloat16* x, int ldx, const float* w, const float* g, int M, int K, int classes,
-                   bool relu_mask, __nv_bfloat16* dx, int lddx, float* dw, float* db, cudaStream_t stream);
+                   bool relu_mask, __nv_bfloat16* dx, int lddx, float* dw, float* db, float* part, cudaStream_t stream);
 
 void rowdot_backward(const __nv_bfloat16* x, int ldx, const float* w, const float* dy, int M, int K, bool relu_mask,
                      __nv_bfloat16* dx, int lddx, float* dw, float* db, cudaStream_t stream);

@@ -234,34 +234,47 @@ head_forward_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* _
 
 // Its backward in one pass over the activations: dw[c, k] += sum_m g[m, c] x[m, k], db[c] += sum_m g[m, c] and
 // dx[m, k] = (sum_c g[m, c] w[c, k]) * (x[m, k] > 0 if relu_mask), rounded to bf16.  A thread owns four columns - their C
-// weights and C weight gradients live in its registers - and walks the rows of its block, whose g sits in shared memory.
+// weights and C weight gradients live in its registers - and walks the rows of its block's range, whose g pass through
+// shared memory.  The sums of the ranges are left in `part` [ranges][classes * K], behind them [ranges][classes] of db, and
+// head_sum_kernel adds them up in the order of the ranges: reductions into dw added them in the order in which blocks
+// arrived, and a training step that starts from the same state did not repeat bit for bit.  A single range (null part) adds
+// to dw and db itself.  1024 rows of 4096 columns, 10 classes: 14.3 us with reductions, 16.8 so, 2.5 of them the second
+// kernel; 65536 x 1024: 161 and 120 us; 65536 x 4096: 596 and 425.
 constexpr int kHeadThreads = 128;
-constexpr int kHeadStep = 32;  // rows of a block
+constexpr int kHeadStep = 64;   // rows of g in shared memory
+constexpr int kHeadRange = 32;  // rows of a range at least
+
+// Blocks of a multiprocessor: as many as 61, 94, 126 and 162 registers a thread leave room for.
+constexpr int head_blocks(int classes) { return classes <= 4 ? 8 : classes <= 8 ? 5 : classes <= 12 ? 4 : 3; }
 
 template <int C>
-__global__ void __launch_bounds__(kHeadThreads)
+__global__ void __launch_bounds__(kHeadThreads, head_blocks(C))
 head_backward_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* __restrict__ w,
-                     const float* __restrict__ g, int M, int K, int classes, int relu_mask,
-                     __nv_bfloat16* __restrict__ dx, int lddx, float* dw, float* db) {
+                     const float* __restrict__ g, int M, int K, int classes, int relu_mask, int range,
+                     __nv_bfloat16* __restrict__ dx, int lddx, float* dw, float* db, float* __restrict__ part) {
   pdl_enter();
   __shared__ float s_g[kHeadStep][C];
-  const int r0 = blockIdx.x * kHeadStep;
-  const int rows = min(kHeadStep, M - r0);
-  for (int i = threadIdx.x; i < kHeadStep * C; i += kHeadThreads) {
-    const int r = i / C, c = i - r * C;
-    s_g[r][c] = r < rows && c < classes ? g[static_cast<size_t>(r0 + r) * classes + c] : 0.f;
-  }
-  __syncthreads();
   const int k = (blockIdx.y * kHeadThreads + threadIdx.x) * 4;
-  if (k < K) {
-    float wk[C][4], acc[C][4];
+  float wk[C][4], acc[C][4], sum_g = 0.f;
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const float4 v = c < classes ? *reinterpret_cast<const float4*>(w + static_cast<size_t>(c) * K + k)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
-      wk[c][0] = v.x, wk[c][1] = v.y, wk[c][2] = v.z, wk[c][3] = v.w;
-      acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f;
+  for (int c = 0; c < C; ++c) {
+    const float4 v = k < K && c < classes ? *reinterpret_cast<const float4*>(w + static_cast<size_t>(c) * K + k)
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+    wk[c][0] = v.x, wk[c][1] = v.y, wk[c][2] = v.z, wk[c][3] = v.w;
+    acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f;
+  }
+  const int begin = static_cast<int>(blockIdx.x) * range, end = min(M - begin, range) + begin;
+  for (int r0 = begin; r0 < end; r0 += kHeadStep) {
+    const int rows = min(kHeadStep, end - r0);
+    __syncthreads();  // the rows before these have been used
+    for (int i = threadIdx.x; i < rows * C; i += kHeadThreads) {
+      const int r = i / C, c = i - r * C;
+      s_g[r][c] = c < classes ? g[static_cast<size_t>(r0 + r) * classes + c] : 0.f;
     }
+    __syncthreads();
+    if (blockIdx.y == 0 && threadIdx.x < classes)
+      for (int r = 0; r < rows; ++r) sum_g += s_g[r][threadIdx.x];
+    if (k >= K) continue;
     constexpr int kAhead = 4;  // rows requested together
     for (int r = 0; r < rows; r += kAhead) {
       uint2 v[kAhead];
@@ -294,14 +307,64 @@ head_backward_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* 
             make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
       }
     }
+  }
+  const size_t n = static_cast<size_t>(classes) * K;
+  if (k < K) {
 #pragma unroll
-    for (int c = 0; c < C; ++c)
-      if (c < classes) red_add_v4(dw + static_cast<size_t>(c) * K + k, make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]));
+    for (int c = 0; c < C; ++c) {
+      if (c >= classes) break;
+      float4 v = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+      float4* const to = reinterpret_cast<float4*>((part ? part + blockIdx.x * n : dw) + static_cast<size_t>(c) * K + k);
+      if (part == nullptr) {
+        const float4 o = *to;
+        v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+      }
+      *to = v;
+    }
   }
   if (blockIdx.y == 0 && threadIdx.x < classes) {
-    float s = 0.f;
-    for (int r = 0; r < rows; ++r) s += s_g[r][threadIdx.x];
-    atomicAdd(db + threadIdx.x, s);
+    if (part == nullptr)
+      db[threadIdx.x] += sum_g;
+    else
+      part[gridDim.x * n + static_cast<size_t>(blockIdx.x) * classes + threadIdx.x] = sum_g;
+  }
+}
+
+// dw += and db += the sums of the ranges.  A block takes 32 times four floats of dw, its warps the ranges in turn (eight loads
+// of a lane in flight), and the first warp adds up what they have; the last block does db.
+constexpr int kHeadSumWarps = 32;  // of a block where there are many ranges, else a quarter of them
+
+__global__ void __launch_bounds__(32 * kHeadSumWarps)
+head_sum_kernel(const float* __restrict__ part, int ranges, size_t n, int classes, float* dw, float* db) {
+  pdl_enter();
+  __shared__ float4 s_sum[kHeadSumWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const bool bias = blockIdx.x == gridDim.x - 1;
+  const size_t at = (static_cast<size_t>(blockIdx.x) * 32 + lane) * 4;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (bias) {
+    if (lane < classes)
+      for (int r = warp; r < ranges; r += warps) a.x += part[ranges * n + static_cast<size_t>(r) * classes + lane];
+  } else if (at < n) {
+#pragma unroll 8
+    for (int r = warp; r < ranges; r += warps) {
+      const float4 v = *reinterpret_cast<const float4*>(part + r * n + at);
+      a.x += v.x, a.y += v.y, a.z += v.z, a.w += v.w;
+    }
+  }
+  s_sum[warp][lane] = a;
+  __syncthreads();
+  if (warp != 0) return;
+  for (int v = 1; v < warps; ++v) {
+    const float4 o = s_sum[v][lane];
+    a.x += o.x, a.y += o.y, a.z += o.z, a.w += o.w;
+  }
+  if (bias) {
+    if (lane < classes) db[lane] += a.x;
+  } else if (at < n) {
+    float4* const to = reinterpret_cast<float4*>(dw + at);
+    const float4 o = *to;
+    *to = make_float4(o.x + a.x, o.y + a.y, o.z + a.z, o.w + a.w);
   }
 }
 
@@ -621,13 +684,41 @@ void head_forward(const __nv_bfloat16* x, int ldx, const float* w, const float* 
   launch_pdl(kernel, dim3((M + kHeadRows - 1) / kHeadRows), dim3(kThreads), 0, stream, x, ldx, w, bias, M, K, classes, y);
 }
 
+// Rows of a range and how many there are: two waves of blocks, or as many as there are rows for.  (65536 x 1024, 3 classes:
+// 68 us; 81 with whole steps of rows a range, whose blocks are 1.15 waves; 91 with half a wave.)
+static int head_range(int M, int K, int classes, int* ranges) {
+  const int columns = (K / 4 + kHeadThreads - 1) / kHeadThreads, blocks = 148 * 2 * head_blocks(classes);
+  const int most = blocks < columns ? 1 : blocks / columns;
+  int range = ((M - 1) / most + 4) / 4 * 4;
+  if (range < kHeadRange) range = kHeadRange;
+  *ranges = (M - 1) / range + 1;
+  return range;
+}
+
+size_t head_part_floats(int M, int K, int classes) {
+  if (M <= 0) return 0;
+  int ranges;
+  head_range(M, K, classes, &ranges);
+  return ranges > 1 ? static_cast<size_t>(ranges) * classes * (static_cast<size_t>(K) + 1) : 0;
+}
+
 void head_backward(const __nv_bfloat16* x, int ldx, const float* w, const float* g, int M, int K, int classes,
-                   bool relu_mask, __nv_bfloat16* dx, int lddx, float* dw, float* db, cudaStream_t stream) {
+                   bool relu_mask, __nv_bfloat16* dx, int lddx, float* dw, float* db, float* part, cudaStream_t stream) {
   if (M <= 0) return;
   auto kernel = classes <= 4 ? head_backward_kernel<4> : classes <= 8 ? head_backward_kernel<8>
                 : classes <= 12 ? head_backward_kernel<12> : head_backward_kernel<16>;
-  const dim3 grid((M + kHeadStep - 1) / kHeadStep, (K / 4 + kHeadThreads - 1) / kHeadThreads);  // y ends at 65535
-  launch_pdl(kernel, grid, dim3(kHeadThreads), 0, stream, x, ldx, w, g, M, K, classes, relu_mask ? 1 : 0, dx, lddx, dw, db);
+  int ranges;
+  const int range = head_range(M, K, classes, &ranges);
+  if (ranges == 1) part = nullptr;
+  const dim3 grid(ranges, (K / 4 + kHeadThreads - 1) / kHeadThreads);  // y ends at 65535
+  launch_pdl(kernel, grid, dim3(kHeadThreads), 0, stream, x, ldx, w, g, M, K, classes, relu_mask ? 1 : 0, range, dx, lddx, dw,
+             db, part);
+  if (part != nullptr) {
+    const size_t n = static_cast<size_t>(classes) * K;
+    const int warps = ranges > 64 ? kHeadSumWarps : kHeadSumWarps / 4;
+    launch_pdl(head_sum_kernel, dim3(static_cast<unsigned>((n / 4 + 31) / 32 + 1)), dim3(32 * warps), 0, stream, part, ranges,
+               n, classes, dw, db);
+  }
 }
 
 void cast_w_wt(const float* w, int N, int K, __nv_bfloat16* w16, __nv_bfloat16* wt16, cudaStream_t stream) {

@@ -84,3 +84,18 @@ def test_more_rows_than_a_grid_is_high():
     close(db, (gd.sum(0), gd.abs().sum(0)), M)
     want = gd @ wd
     assert bool(((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -20 * (gd.abs() @ wd.abs())).all())
+
+
+# Blocks of one and of several row ranges, with a remainder; one range alone.
+@pytest.mark.parametrize("M,K,classes", [(20, 256, 10), (1000, 4096, 10), (40_003, 256, 3), (777, 520, 16)])
+def test_backward_repeats_bit_for_bit(M, K, classes):
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    w, g = torch.randn(classes, K, device=DEV), torch.randn(M, classes, device=DEV)
+    outs = []
+    for _ in range(10):
+        dx, dw, db = torch.empty_like(x), torch.ones_like(w), torch.ones(classes, device=DEV)
+        C.head_backward(x, w, g, True, dx, dw, db)
+        outs.append((dx, dw, db))
+    for o in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(o, outs[0]))

@@ -351,10 +351,9 @@ void bind_dense(py::module_& m) {
   // The casts on stream `side` beside whatever the current stream does next; `wait` of the event orders a stream behind them.
   py::class_<StreamEvent>(m, "StreamEvent").def("wait", &StreamEvent::Wait);
   m.def("prepare_weights", [](const std::vector<torch::Tensor>& ws, bool transpose, int64_t id, int64_t index, int64_t type) {
-    TORCH_CHECK(!ws.empty(), "no weights");
-    const c10::cuda::CUDAGuard device(ws[0].device());
-    const auto main = c10::cuda::getCurrentCUDAStream();
     const auto side = c10::cuda::CUDAStream::unpack3(id, index, static_cast<c10::DeviceType>(type));
+    const c10::cuda::CUDAGuard device(side.device());
+    const auto main = c10::cuda::getCurrentCUDAStream();
     join(main, side);
     auto event = std::make_unique<StreamEvent>();
     std::tuple<std::vector<torch::Tensor>, std::vector<torch::Tensor>, torch::Tensor> cast;

@@ -117,3 +117,15 @@ def test_inputs_of_unjoined_weight_gradients_are_not_given_away():
     finally:
         fused.set_deferred_join(False)
     torch.cuda.synchronize()
+
+
+def test_weights_of_a_single_layer_can_be_prepared():
+    """There is no hidden layer whose weights could be cast ahead: nothing is prepared, and nothing refused."""
+    from kraken_b200.ops import mlp as fused
+    torch.manual_seed(0)
+    x, w, b = torch.randn(33, 64, device=DEV), torch.randn(10, 64, device=DEV), torch.randn(10, device=DEV)
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad):
+            prepared = fused.prepare_weights([w])
+            assert list(prepared.w16s) == [] and list(prepared.wt16s) == []
+            assert torch.equal(fused.fused_mlp(x, [w], [b], prepared=prepared), fused.fused_mlp(x, [w], [b]))

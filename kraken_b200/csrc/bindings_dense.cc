@@ -207,9 +207,12 @@ void bind_dense(py::module_& m) {
       mp = reinterpret_cast<uint16_t*>(mask_out->data_ptr());
       ldm = mask_out->stride(0);
     }
-    const int rc = cu::linear_forward(bf(x), x.stride(0), bf(w), w.stride(0), optr<float>(bias),
+    c10::optional<torch::Tensor> b;
+    bool late = false;
+    if (bias.has_value() && bias->defined()) late = !bias->is_contiguous(), b = bias->contiguous();
+    const int rc = cu::linear_forward(bf(x), x.stride(0), bf(w), w.stride(0), optr<float>(b),
                                       reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), y.stride(0), M, N, K, relu, mp, ldm,
-                                      status.data_ptr<int>(), cur_stream());
+                                      status.data_ptr<int>(), late, cur_stream());
     TORCH_CHECK(rc == 0, "linear_forward: cannot encode the TMA descriptors (pitches must be multiples of 8)");
   }, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("relu"), py::arg("y"), py::arg("status"),
      py::arg("mask_out") = py::none());
@@ -386,7 +389,8 @@ void bind_dense(py::module_& m) {
       const int rc = cu::linear_forward(bf(h), h.stride(0), bf(w), w.stride(0), bias.data_ptr<float>(),
                                         reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), y.stride(0), M, N, K, true,
                                         masks ? reinterpret_cast<uint16_t*>(mask.data_ptr()) : nullptr,
-                                        masks ? static_cast<int>(mask.stride(0)) : 0, status.data_ptr<int>(), cur_stream());
+                                        masks ? static_cast<int>(mask.stride(0)) : 0, status.data_ptr<int>(),
+                                        !bs[i].is_contiguous(), cur_stream());
       TORCH_CHECK(rc == 0, "linear_forward: cannot encode the TMA descriptors (pitches must be multiples of 8)");
       acts.push_back(y);
       if (masks) bits.push_back(mask);

@@ -66,6 +66,7 @@ struct GemmArgs {
   int zero_cols;          // columns behind the N of `out` that are cleared, a multiple of 8 (EPI_RELU_MASK)
   float* col_sums;        // [M] += column sums of A, or null (EPI_RED_F32 with an MN-major A: the bias gradient)
   int* status;
+  int late;               // host: launched behind the kernel in front and not beside its end (what wrote the bias)
 };
 
 // Position in a ring of stages: the stage and the parity of the round through it.  The threads that issue copies and MMAs
@@ -1301,7 +1302,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
     attr_set = true;
   }
   dim3 grid((g.M + kBM - 1) / kBM, (g.N + g.BN - 1) / g.BN, splits);
-  launch_pdl(gemm_kernel<A_MN, B_MN, EPI>, grid, dim3(kTileThreads<B_MN>), smem, stream, ta, tb, td, g);
+  launch_pdl_if(g.late == 0, gemm_kernel<A_MN, B_MN, EPI>, grid, dim3(kTileThreads<B_MN>), smem, stream, ta, tb, td, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1380,7 +1381,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   }
   int pairs = 74 / n_tiles;
   if (pairs > m_tiles) pairs = m_tiles;
-  launch_pdl(gemm_pair_kernel<EPI>, dim3(2 * pairs, n_tiles), dim3(kThreads), smem, stream, ta, tb, td, g);
+  launch_pdl_if(g.late == 0, gemm_pair_kernel<EPI>, dim3(2 * pairs, n_tiles), dim3(kThreads), smem, stream, ta, tb, td, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1401,7 +1402,7 @@ int launch_resident(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs g, cu
   }
   int per_n = 148 / n_tiles;
   if (per_n > m_tiles) per_n = m_tiles;
-  launch_pdl(gemm_bres_kernel<EPI>, dim3(per_n, n_tiles), dim3(kThreads), smem, stream, ta, tb, g);
+  launch_pdl_if(g.late == 0, gemm_bres_kernel<EPI>, dim3(per_n, n_tiles), dim3(kThreads), smem, stream, ta, tb, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1457,8 +1458,9 @@ static int can_store_v8(const void* out, int ld) {
 
 int linear_forward(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, int ldw, const float* bias,
                    __nv_bfloat16* Y, int ldy, int M, int N, int K, bool relu, uint16_t* mask_out, int ldm, int* status,
-                   cudaStream_t stream) {
+                   bool late, cudaStream_t stream) {
   GemmArgs g{};
+  g.late = late ? 1 : 0;
   g.M = M, g.N = N, g.K = K;
   g.BN = pick_bn(N, 16);
   g.stages = 2;

@@ -32,9 +32,12 @@ namespace cu {
 // 32 rows of a warp write 64 contiguous bytes); the input gradient of the next layer then takes that
 // bit mask instead of re-reading the bf16 activations H, which cuts its extra read traffic
 // sixteen-fold.  Either may be null; with both null no mask is applied.
+//
+// linear_forward reads the bias before it waits for the kernel in front of it on the stream (that wait is for the
+// activations), unless `late`: what wrote the bias is the kernel in front.
 int linear_forward(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, int ldw, const float* bias,
                    __nv_bfloat16* Y, int ldy, int M, int N, int K, bool relu, uint16_t* mask_out, int ldm, int* status,
-                   cudaStream_t stream);
+                   bool late, cudaStream_t stream);
 
 int linear_dgrad(const __nv_bfloat16* dY, int lddy, const __nv_bfloat16* Wt, int ldwt, const __nv_bfloat16* H,
                  int ldh, const uint16_t* mask, int ldm, __nv_bfloat16* dX, int lddx, int M, int N, int K, int zero_cols,

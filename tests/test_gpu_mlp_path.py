@@ -129,3 +129,23 @@ def test_weights_of_a_single_layer_can_be_prepared():
             prepared = fused.prepare_weights([w])
             assert list(prepared.w16s) == [] and list(prepared.wt16s) == []
             assert torch.equal(fused.fused_mlp(x, [w], [b], prepared=prepared), fused.fused_mlp(x, [w], [b]))
+
+
+@pytest.mark.parametrize("M,sizes", [(200, (64, 48, 16)), (4096, (400, 400, 8)), (65536, (256, 128, 24)), (1024, (2048, 8))])
+def test_biases_that_are_not_stored_back_to_back(M, sizes):
+    """Each is copied in front of the kernel that adds it, and that kernel waits for the copy; through every plan of the
+    forward pass, the head among the layers."""
+    from kraken_b200.ops import mlp as fused
+    torch.manual_seed(M)
+    K = 432
+    x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    ws = [torch.randn(n, k, device=DEV) / k ** 0.5 for n, k in zip(sizes, (K,) + sizes[:-1])]
+    for _ in range(5):
+        bs = [torch.randn(n, 3, device=DEV)[:, 1] for n in sizes]
+        with torch.no_grad():
+            want = fused.fused_mlp(x, ws, [b.clone(memory_format=torch.contiguous_format) for b in bs])
+            assert torch.equal(fused.fused_mlp(x, ws, bs), want)
+    ws, bs = [w.requires_grad_() for w in ws], [b.requires_grad_() for b in bs]
+    fused.fused_mlp(x, ws, bs).sum().backward()
+    fused.check_gemm_status(x.device)
+    assert all(b.grad is not None and bool(b.grad.isfinite().all()) for b in bs)

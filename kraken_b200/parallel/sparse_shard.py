@@ -182,6 +182,11 @@ class GpuSparseTable:
         else:
             self._record.zero_()
 
+    def clear(self) -> None:
+        """No rows, every slot as a new table has it."""
+        C.table_clear(self._host)
+        self._reset_records()
+
     @property
     def capacity(self) -> int:
         return 1 << self.bits
@@ -343,8 +348,7 @@ class GpuSparseTable:
         table from the survivors; returns how many rows were dropped."""
         before = self.num_rows()
         keep = self.export(filter_mode=3, min_steps=min_steps)
-        C.table_clear(self._host)
-        self._reset_records()
+        self.clear()
         self.import_rows(keep["ids"], keep["vals"], keep["states"], keep["states_i"])
         return before - int(keep["ids"].numel())
 

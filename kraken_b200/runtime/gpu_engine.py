@@ -678,13 +678,7 @@ class GpuEngine(Engine):
             in_vals = a2a(away["vals"], t.dim)
             in_states = {k: a2a(away["states"][k], t.dim) for k in skeys}
             in_steps = {0: a2a(away["states_i"][0], 0)} if has_steps else {}
-            C.table_clear(t.host())
-            t.val.zero_()
-            for k, slab in enumerate(t.slabs):
-                if slab is not None:
-                    slab.fill_(t.optim_info["initial_accumulator_value"] if (t.optim_info["type"] == 0 and k == 0) else 0.0)
-            if t.steps is not None:
-                t.steps.zero_()
+            t.clear()
             t.import_rows(keep["ids"], keep["vals"], keep["states"], keep["states_i"])
             t.import_rows(in_ids, in_vals, in_states, in_steps)
         self.owner_world = owner_world

@@ -73,3 +73,30 @@ def test_records_are_filled_by_column(rows, pitch, at, dim):
     assert torch.equal(records, want)
     with pytest.raises(RuntimeError):
         C.fill_records(records, at, pitch - at + 1, 0.1)
+
+
+@pytest.mark.gpu
+def test_a_reshard_resets_records_in_one_pass(monkeypatch):
+    """Every part of a slot lies in one record, so what a reshard clears is cleared once and not by columns; rows that stay
+    keep their columns, free slots start as the optimizer starts them."""
+    kk.initialize("gpu", table_capacity=1 << 8)
+    kk.init_model("m", kk.OptimType.kAdagrad, {"initial_accumulator_value": "0.1"})
+    t = kk.register_sparse_table("e", 5, torch.float32, kk.InitializerType.kConstant, {"value": "0"})
+    eng = kk.native.engine()
+    table = eng.sparse[t]
+    torch.manual_seed(1)
+    ids = torch.randperm(1000)[:60].cuda()
+    state = int(table.optim_info["slab_state_types"][0])
+    cols = {"ids": ids, "vals": torch.randn(60, 5).cuda(), "states": {state: torch.rand(60, 5).cuda()}, "states_i": {}}
+    eng.import_sparse(t, cols)
+    resets = []
+    whole = table._reset_records
+    monkeypatch.setattr(table, "_reset_records", lambda: (resets.append(1), whole()))
+    eng.owner_world = 2   # as if another rank had held rows: all come back to this one
+    assert eng.reshard(1) == 0 and resets == [1]
+    out = eng.export_sparse(t)
+    a, b = out["ids"].argsort(), ids.argsort()
+    assert torch.equal(out["ids"][a], ids[b]) and torch.equal(out["vals"][a], cols["vals"][b])
+    assert torch.equal(out["states"][state][a], cols["states"][state][b])
+    free = table.keys == -1
+    assert bool((table.val[free] == 0).all()) and bool((table.slabs[0][free] == 0.1).all())

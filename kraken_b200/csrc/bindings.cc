@@ -217,6 +217,16 @@ ckpt::RowFilter make_filter(int mode, uint64_t salt, uint32_t world, uint32_t ra
 }
 
 // ------------------------------------------------------------------ symmetric heap
+// What an engine that is no longer used gives back has nothing to do with a graph that this thread happens to be capturing
+// when Python's collector comes to it; without this the calls would end that capture with an error.
+struct DuringCaptures {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  DuringCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~DuringCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  DuringCaptures(const DuringCaptures&) = delete;
+  DuringCaptures& operator=(const DuringCaptures&) = delete;
+};
+
 // One cudaMalloc'd arena per rank, exported with a CUDA IPC handle and mapped by
 // every peer of the same box.
 struct SymHeap {
@@ -260,6 +270,7 @@ struct SymHeap {
         opened[p] = false;
       }
     if (local) {
+      const DuringCaptures allowed;
       cudaFree(local);
       local = nullptr;
     }
@@ -305,6 +316,7 @@ struct AsyncRead {
   AsyncRead& operator=(const AsyncRead&) = delete;
   ~AsyncRead() {
     if (event) {
+      const DuringCaptures allowed;
       cudaEventSynchronize(event);  // a copy in flight still writes to `host`
       cudaEventDestroy(event);
     }

@@ -381,3 +381,27 @@ def test_streamed_save_and_chunked_load_round_trip_on_the_gpu_engine(tmp_path):
     w1 = kk.pull_sparse_table(t2, some)
     acc = 0.1 + g[:1000] ** 2 + 1.0
     assert torch.allclose(w0 - w1, 0.5 / (acc.sqrt() + 1e-10), rtol=1e-4, atol=1e-6)
+
+
+def test_an_engine_that_goes_during_a_capture_leaves_the_graph_alone():
+    """Python's collector may come to an earlier job's engine, its pending row count and its buffers, at any time."""
+    import gc
+    from kraken_b200.pytorch import native
+    x = torch.zeros(1 << 20, device=DEV)
+    x.add_(0)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        kk.initialize("gpu", table_capacity=1 << 12, max_ids_per_call=1024, seed=1, status_poll_interval=1)
+        emb = kk.Embedding(4, initializer=kk.ConstantInitializer(1.0), name="e")
+        opt = kk.Optimizer("m", emb.named_parameters(), 0.5, kk.Adam())
+        for k in range(3):
+            emb(torch.arange(64, device=DEV) + k).sum().backward()
+            opt.step()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            x.add_(1)
+            native._engine = None   # what a job that starts behind this one does
+            del emb, opt
+            gc.collect()
+        graph.replay()
+    assert bool((x == 3).all())

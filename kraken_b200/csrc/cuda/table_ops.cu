@@ -60,23 +60,30 @@ fill_records_kernel(float* __restrict__ records, long long floats, int pitch, in
   }
 }
 
-// Calls move(dst + j, src + j) for the floats of every lane's row (`mine`); by all lanes of the warp, which must be converged,
-// one row after the other where rows are long enough to fill them.  With a thread a row, 2.3 M rows of 64 floats with a state
-// took 2.9 ms to export and 3.5 ms to import, a sector for each float; 1.2 and 1.0 ms so.
-constexpr int kWarpRow = 8;
+// Calls move(dst + j, src + j) for the floats of every lane's row (`mine`); the warp must be converged.  Rows go in
+// turn to the groups of 8, 16 or 32 lanes that a warp is divided into.  600 k rows with one state, us to export and to
+// import: of 64 floats 857 and 1666 with a thread a row, a sector for each float, 311 and 310 so; of 8 floats 160 and 109 with
+// a thread a row, 212 and 125 with a warp a row, 146 and 83 so.
+constexpr int kGroupRow = 8;
 
 template <typename Move>
 __device__ __forceinline__ void move_rows(bool mine, size_t dst, size_t src, int dim, Move move) {
-  if (dim < kWarpRow) {
+  if (dim < kGroupRow) {
     if (mine)
       for (int j = 0; j < dim; ++j) move(dst + j, src + j);
     return;
   }
-  const int lane = threadIdx.x & 31;
-  for (unsigned left = __ballot_sync(0xffffffffu, mine); left; left &= left - 1) {
-    const int l = __ffs(left) - 1;
+  const int lane = threadIdx.x & 31, group = dim < 16 ? 8 : dim < 32 ? 16 : 32;
+  const int groups = 32 / group;
+  unsigned left = __ballot_sync(0xffffffffu, mine);
+  int rows = __popc(left);
+  for (int k = lane / group; k > 0; --k) left &= left - 1;
+  for (; rows > 0; rows -= groups) {
+    const int l = left ? __ffs(left) - 1 : 0;
     const size_t d = __shfl_sync(0xffffffffu, dst, l), s = __shfl_sync(0xffffffffu, src, l);
-    for (int j = lane; j < dim; j += 32) move(d + j, s + j);
+    if (left)
+      for (int j = lane & (group - 1); j < dim; j += group) move(d + j, s + j);
+    for (int k = 0; k < groups; ++k) left &= left - 1;
   }
 }
 
@@ -94,6 +101,7 @@ __global__ void table_clear_kernel(TableView t) {
 __global__ void table_import_kernel(TableView t, const int64_t* __restrict__ ids, const float* __restrict__ vals,
                                     const float* __restrict__ s0, const float* __restrict__ s1,
                                     const float* __restrict__ s2, const int* __restrict__ steps, int n) {
+  const bool on0 = t.s[0] && s0, on1 = t.s[1] && s1, on2 = t.s[2] && s2;
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
     bool created = false;
@@ -126,10 +134,11 @@ __global__ void table_import_kernel(TableView t, const int64_t* __restrict__ ids
     }
     move_rows(found >= 0, static_cast<size_t>(found < 0 ? 0 : found) * t.pitch, static_cast<size_t>(i) * t.dim, t.dim,
               [&](size_t d, size_t s) {
-                t.val[d] = vals[s];
-                if (t.s[0] && s0) t.s[0][d] = s0[s];
-                if (t.s[1] && s1) t.s[1][d] = s1[s];
-                if (t.s[2] && s2) t.s[2][d] = s2[s];
+                const float v = vals[s], a = on0 ? s0[s] : 0.f, b = on1 ? s1[s] : 0.f, c = on2 ? s2[s] : 0.f;
+                t.val[d] = v;
+                if (on0) t.s[0][d] = a;
+                if (on1) t.s[1][d] = b;
+                if (on2) t.s[2][d] = c;
               });
     count_created(t, created);
   }
@@ -149,6 +158,7 @@ __global__ void table_export_kernel(TableView t, int filter_mode, uint64_t salt,
                                     int64_t* out_ids, float* out_vals, float* out_s0, float* out_s1, float* out_s2,
                                     int* out_steps, int* out_count, int out_cap) {
   const uint64_t cap = 1ull << t.bits;
+  const bool on0 = out_s0 && t.s[0], on1 = out_s1 && t.s[1], on2 = out_s2 && t.s[2];
   for (uint64_t base = blockIdx.x * static_cast<uint64_t>(blockDim.x); base < cap;
        base += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
     const uint64_t slot = base + threadIdx.x;
@@ -179,10 +189,11 @@ __global__ void table_export_kernel(TableView t, int filter_mode, uint64_t salt,
       if (out_steps) out_steps[pos] = t.steps ? t.steps[slot * t.step_pitch] : 0;
     }
     move_rows(fits, static_cast<size_t>(fits ? pos : 0) * t.dim, slot * t.pitch, t.dim, [&](size_t d, size_t s) {
-      out_vals[d] = t.val[s];
-      if (out_s0 && t.s[0]) out_s0[d] = t.s[0][s];
-      if (out_s1 && t.s[1]) out_s1[d] = t.s[1][s];
-      if (out_s2 && t.s[2]) out_s2[d] = t.s[2][s];
+      const float v = t.val[s], a = on0 ? t.s[0][s] : 0.f, b = on1 ? t.s[1][s] : 0.f, c = on2 ? t.s[2][s] : 0.f;
+      out_vals[d] = v;
+      if (on0) out_s0[d] = a;
+      if (on1) out_s1[d] = b;
+      if (on2) out_s2[d] = c;
     });
   }
 }

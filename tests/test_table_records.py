@@ -100,3 +100,29 @@ def test_a_reshard_resets_records_in_one_pass(monkeypatch):
     assert torch.equal(out["states"][state][a], cols["states"][state][b])
     free = table.keys == -1
     assert bool((table.val[free] == 0).all()) and bool((table.slabs[0][free] == 0.1).all())
+
+
+# Row widths around the groups of lanes that move a row, rows around a warp's and a block's; some slots of a warp hold a row.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim", [7, 8, 9, 15, 16, 31, 32, 33])
+@pytest.mark.parametrize("rows", [1, 31, 33, 257])
+def test_rows_are_moved_whole(dim, rows):
+    kk.initialize("gpu", table_capacity=1 << 10)
+    kk.init_model("m", kk.OptimType.kAdam, {"amsgrad": "true"})
+    t = kk.register_sparse_table("e", dim, torch.float32, kk.InitializerType.kConstant, {"value": "0"})
+    eng = kk.native.engine()
+    table = eng.sparse[t]
+    torch.manual_seed(dim + rows)
+    ids = torch.randperm(100_000)[:rows].cuda()
+    states = {int(st): torch.randn(rows, dim).cuda() for st in table.optim_info["slab_state_types"]}
+    cols = {"ids": ids, "vals": torch.randn(rows, dim).cuda(), "states": states,
+            "states_i": {0: torch.randint(1, 1000, (rows,)).cuda()}}
+    eng.import_sparse(t, cols)
+    out, want = eng.export_sparse(t), ids.argsort()
+    got = out["ids"].argsort()
+    assert torch.equal(out["vals"][got], cols["vals"][want]) and torch.equal(out["states_i"][0][got], cols["states_i"][0][want])
+    assert all(torch.equal(out["states"][st][got], states[st][want]) for st in states)
+    half = table.export(filter_mode=3, min_steps=500)   # some rows of a warp only
+    kept = cols["states_i"][0][want] >= 500
+    got = half["ids"].argsort()
+    assert torch.equal(half["ids"][got], ids[want][kept]) and torch.equal(half["vals"][got], cols["vals"][want][kept])

@@ -48,7 +48,6 @@ struct GemmArgs {
   int BN;                 // tile width (multiple of 16; of 64 when B is MN-major)
   int stages;
   int kb_per_split;       // k-blocks per blockIdx.z, or per work item of the streaming variant
-  int subs;               // streaming variant: column sub-tiles of BN per work item
   int tiles_m, tiles_n;   // ... its grid of tiles, and the number of (tile, split) items
   int items;
   int relu;
@@ -931,13 +930,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // tiles of a CTA pair (cta_group::2; CTA r holds dY columns [m0 + r * 128, +128) and its half of the X columns of a sub-tile).
 // What bounded gemm_kernel here was its producer: a k-block of a 128 x 256 tile is six boxes of 64 x 64, 100 cycles each to
 // issue, and with the wait for the stage that is 800 cycles where the MMAs take 512; and it brings 48 KB in for them, which
-// is 10 TB/s over all SMs.  A pair needs 32 KB per CTA for the same products, and with `subs` = 2 - up to 512 columns in ONE
-// tile, all of tensor memory - 24 KB: dY crosses the fabric once and X once per 256 rows.  The boxes are issued by three warps:
+// is 10 TB/s over all SMs.  A pair needs 32 KB per CTA for the same products, and with two sub-tiles of 256 columns - 512 in
+// ONE tile, all of tensor memory - 24 KB: dY crosses the fabric once and X once per 256 rows.  The boxes are issued by three warps:
 // dY, and each sub-tile's half of X.  Batch 65536 of 400 x 432: 38.1 us there, 31.2 here, of which 16 are MMAs; 4096 x 4096 at
 // batch 1024 51 and 39.5.  What is left is the start, and the reductions of 37 partial sums into L2.
 //
-// A work item is a tile and a range of k-blocks; a pair takes items pair, pair + pairs, ...  With one sub-tile the two
-// accumulators alternate, so the epilogue of an item runs beside the MMAs of the next.  Warps 10-13 exist where the bias
+// A work item is a tile and a range of k-blocks; a pair takes items pair, pair + pairs, ...  Warps 10-13 exist where the bias
 // gradient is wanted: they add up the columns of the dY tiles of the items in the first column of tiles.  The byte counts of
 // both CTAs' copies complete on the even CTA's barriers, which only that CTA can wait on, so the summing warps of both take a
 // stage when its MMAs have read it (`landed`: the commit arrives in both CTAs), and they, not the commit, free it.  (Passing
@@ -945,6 +943,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 constexpr int kSumWarps = 4;
 constexpr int kProducers = 3;                              // warps 0, 14 and 15
 constexpr int kPairWgradThreads = kThreads + 32 * (kSumWarps + kProducers - 1);
+
+constexpr int kSubs = 2, kSubCols = 256;  // a tile: two MMAs of 256 rows x 256 columns
 
 struct Item {
   int m0, n0, kb0, kb1;
@@ -956,7 +956,7 @@ __device__ __forceinline__ Item item_at(const GemmArgs& g, int i, int total_kb) 
   const int tm = i % g.tiles_m, rest = i / g.tiles_m;
   const int tn = rest % g.tiles_n, split = rest / g.tiles_n;
   t.m0 = tm * 2 * kBM;
-  t.n0 = tn * g.BN * g.subs;
+  t.n0 = tn * kSubs * kSubCols;
   t.kb0 = split * g.kb_per_split;
   t.kb1 = min(total_kb, t.kb0 + g.kb_per_split);
   t.first_col = tn == 0;
@@ -975,15 +975,15 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                        const __grid_constant__ CUtensorMap tmD, const __grid_constant__ GemmArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int half_bn = g.BN / 2;
-  const uint32_t a_bytes = kBM * 128;
-  const uint32_t b_bytes = static_cast<uint32_t>(half_bn) * 128;  // this CTA's half of one sub-tile
-  const uint32_t stage_bytes = a_bytes + static_cast<uint32_t>(g.subs) * b_bytes;
+  constexpr int half_bn = kSubCols / 2;
+  constexpr uint32_t a_bytes = kBM * 128;
+  constexpr uint32_t b_bytes = half_bn * 128;  // this CTA's half of one sub-tile
+  constexpr uint32_t stage_bytes = a_bytes + kSubs * b_bytes;
   // boxes of the epilogue's TMA reductions: behind the ring, or, where every pair has one item, in it
   const bool in_ring = g.items <= static_cast<int>(gridDim.x >> 1);
   uint8_t* const staging = smem + (in_ring ? 0 : static_cast<size_t>(g.stages) * stage_bytes);
 
-  __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], landed_bar[kMaxStages], acc_full[2], acc_empty[2];
+  __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], landed_bar[kMaxStages], acc_full, acc_empty;
   __shared__ uint32_t tmem_slot;
   __shared__ float s_sum[kBM];
 
@@ -994,8 +994,6 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   const int pairs = gridDim.x >> 1;
   const int total_kb = (g.K + kBK - 1) / kBK;
   const bool sums = g.col_sums != nullptr;
-  const int bufs = g.subs == 1 ? 2 : 1;
-  constexpr uint32_t kAccCols = 256;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < g.stages; ++s) {
@@ -1003,10 +1001,8 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       tc::mbar_init(&empty_bar[s], sums ? kSumWarps : 1);
       tc::mbar_init(&landed_bar[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      tc::mbar_init(&acc_full[b], 1);
-      tc::mbar_init(&acc_empty[b], 2 * kEpiWarps);
-    }
+    tc::mbar_init(&acc_full, 1);
+    tc::mbar_init(&acc_empty, 2 * kEpiWarps);
     tc::fence_barrier_init();
     tc::prefetch_tmap(&tmA);
     tc::prefetch_tmap(&tmB);
@@ -1021,7 +1017,7 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   const uint32_t tmem_base = tmem_slot;
 
   const int producer = warp == 0 ? 0 : warp - (2 + kEpiWarps + kSumWarps) + 1;  // 0: dY, 1 and 2: sub-tiles of X
-  if ((warp == 0 || producer > 0) && lane == 0 && producer <= g.subs) {
+  if ((warp == 0 || producer > 0) && lane == 0) {
     // ---------------- producers (both CTAs)
     bool ok = true;
     int it = 0;
@@ -1032,11 +1028,11 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       uint32_t bytes = 0;  // of both CTAs' copies of a k-block
       for (int r = 0; r < 2; ++r) {
         bytes += boxes_inside(t.m0 + r * kBM, kBM, g.M) * 8192;
-        for (int u = 0; u < g.subs; ++u) bytes += boxes_inside(t.n0 + u * g.BN + r * half_bn, half_bn, g.N) * 8192;
+        for (int u = 0; u < kSubs; ++u) bytes += boxes_inside(t.n0 + u * kSubCols + r * half_bn, half_bn, g.N) * 8192;
       }
       const CUtensorMap* const tm = producer == 0 ? &tmA : &tmB;
       const int x0 = producer == 0 ? t.m0 + static_cast<int>(rank) * kBM
-                                   : t.n0 + (producer - 1) * g.BN + static_cast<int>(rank) * half_bn;
+                                   : t.n0 + (producer - 1) * kSubCols + static_cast<int>(rank) * half_bn;
       const int boxes = producer == 0 ? boxes_inside(x0, kBM, g.M) : boxes_inside(x0, half_bn, g.N);
       uint8_t* const base = smem + (producer == 0 ? 0 : a_bytes + (producer - 1) * b_bytes);
       for (int kb = t.kb0; kb < t.kb1; ++kb, ++it, ring.next(g.stages)) {
@@ -1055,7 +1051,7 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     }
   } else if (warp == 1 && lane == 0 && rank == 0) {
     // ---------------- MMA issuer (even CTA only)
-    const uint32_t idesc = tc::instr_desc_bf16(2 * kBM, g.BN, 1, 1);
+    const uint32_t idesc = tc::instr_desc_bf16(2 * kBM, kSubCols, 1, 1);
     bool ok = true, ready = false;
     int j = 0;
     Ring ring;
@@ -1063,14 +1059,11 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     uint64_t* const read_bar = sums ? landed_bar : empty_bar;
     for (int i = pair; i < g.items && ok; i += pairs, ++j) {
       const Item t = item_at(g, i, total_kb);
-      const int buf = bufs == 2 ? j & 1 : 0;
-      const uint32_t use = static_cast<uint32_t>(bufs == 2 ? j >> 1 : j);
-      if (use > 0) {
-        ok = tc::mbar_wait(&acc_empty[buf], (use - 1) & 1, kWaitLimit);
+      if (j > 0) {
+        ok = tc::mbar_wait(&acc_empty, static_cast<uint32_t>(j - 1) & 1, kWaitLimit);
         if (!ok) break;
         tc::fence_after_sync();
       }
-      const uint32_t d_tmem = tmem_base + buf * kAccCols;
       for (int kb = t.kb0; kb < t.kb1; ++kb, ring.next(g.stages)) {
         const int s = ring.s;
         if (!ready) ok = tc::mbar_wait(&full_bar[s], ring.parity, kWaitLimit);
@@ -1084,28 +1077,25 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           if (k == 2) ready = tc::mbar_test(&full_bar[ahead.s], ahead.parity);  // see Ring
           const uint64_t ad = ad0 + at + k * k_step<true>, bd = bd0 + at + k * k_step<true>;
           const uint32_t more = (kb > t.kb0 || k > 0) ? 1u : 0u;
-          tc::mma_bf16_pair(d_tmem, ad, bd, idesc, more);
-          if (g.subs == 2) tc::mma_bf16_pair(d_tmem + kAccCols, ad, bd + (b_bytes >> 4), idesc, more);
+          tc::mma_bf16_pair(tmem_base, ad, bd, idesc, more);
+          tc::mma_bf16_pair(tmem_base + kSubCols, ad, bd + (b_bytes >> 4), idesc, more);
         }
         tc::mma_commit_pair(&read_bar[s], 3);  // the stage has been read in both CTAs
       }
-      if (ok) tc::mma_commit_pair(&acc_full[buf], 3);
+      if (ok) tc::mma_commit_pair(&acc_full, 3);
     }
     if (!ok) atomicCAS(g.status, 0, err::kTimeout);
   } else if (warp >= 2 && warp < 2 + kEpiWarps) {
     // ---------------- epilogue (both CTAs, each on its own 128 rows)
     const int quarter = warp & 3;
-    const uint32_t lead_acc_empty[2] = {tc::map_to_cta(tc::smem_u32(&acc_empty[0]), 0),
-                                        tc::map_to_cta(tc::smem_u32(&acc_empty[1]), 0)};
+    const uint32_t lead_acc_empty = tc::map_to_cta(tc::smem_u32(&acc_empty), 0);
     int j = 0, turn = 0;
     for (int i = pair; i < g.items; i += pairs, ++j) {
       const Item t = item_at(g, i, total_kb);
-      const int buf = bufs == 2 ? j & 1 : 0;
-      const uint32_t use = static_cast<uint32_t>(bufs == 2 ? j >> 1 : j);
       const int row0 = t.m0 + static_cast<int>(rank) * kBM + quarter * 32;
       int c_begin, c_end;
-      epi_cols(min(g.BN * g.subs, (g.N - t.n0 + 63) / 64 * 64), warp - 2, &c_begin, &c_end);
-      const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[buf], use & 1, kWaitLimit));
+      epi_cols(min(kSubs * kSubCols, (g.N - t.n0 + 63) / 64 * 64), warp - 2, &c_begin, &c_end);
+      const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full, static_cast<uint32_t>(j) & 1, kWaitLimit));
       tc::fence_after_sync();
       if (in_ring && sums)  // the MMAs have read every stage, and so must the summing warps have
         asm volatile("bar.sync 3, %0;" ::"n"(32 * (kEpiWarps + kSumWarps)) : "memory");
@@ -1114,11 +1104,11 @@ gemm_pair_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         break;
       }
       epilogue_reduce(g, &tmD, staging + (warp - 2) * 8192,
-                      tmem_base + buf * kAccCols + (static_cast<uint32_t>(quarter * 32) << 16), row0, t.n0, c_begin, c_end,
+                      tmem_base + (static_cast<uint32_t>(quarter * 32) << 16), row0, t.n0, c_begin, c_end,
                       turn);
       tc::fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive_cluster(lead_acc_empty[buf]);
+      if (lane == 0) tc::mbar_arrive_cluster(lead_acc_empty);
     }
     if (lane == 0) tc::bulk_wait_all();
   } else if (warp >= 2 + kEpiWarps && warp < 2 + kEpiWarps + kSumWarps && sums) {
@@ -1406,17 +1396,16 @@ int launch_resident(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs g, cu
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// Plan of the CTA-pair weight gradient of an M x N matrix (N inputs): tiles of 256 x 512 (256 x 256 or x 128 for few inputs)
-// and as many ranges of the batch as give every pair one.  True where it is the faster one: rows and columns enough for the
+// Plan of the CTA-pair weight gradient of an M x N matrix (N inputs): tiles of 256 x 512 and as many ranges of the batch
+// as give every pair one.  True where it is the faster one: rows and columns enough for the
 // traffic that a pair saves, and tiles for every pair or ranges that are worth its longer start and its reductions.  Measured,
 // us as tiles per CTA / on pairs: batch 65536 of 400 x 432 38.0 / 30.9, 32768 (14 k-blocks) 22.8 / 20.9, 16384 (7) 15.1 / 15.7,
 // 65536 of 256 x 512 23.4 / 26.8; 4096 x 4096 at batch 1024 51.8 / 41.6, at 100 25.0 / 20.5; 1024 x 6416 at 1000 26.8 / 23.3;
 // 2048 x 2048 at 1024 (8) 15.0 / 16.4.
 bool plan_pair_wgrad(int M, int N, int K, GemmArgs* g, int* splits) {
   const int total_kb = (K + kBK - 1) / kBK;
-  g->BN = N <= 128 ? 128 : 256;
-  g->subs = N <= 256 ? 1 : 2;
-  const int tiles = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + g->BN * g->subs - 1) / (g->BN * g->subs));
+  constexpr int kCols = kSubs * kSubCols;
+  const int tiles = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + kCols - 1) / kCols);
   int n = tiles < 74 ? 74 / tiles : 1;
   if (n > total_kb) n = total_kb;
   g->kb_per_split = (total_kb + n - 1) / n;
@@ -1426,14 +1415,13 @@ bool plan_pair_wgrad(int M, int N, int K, GemmArgs* g, int* splits) {
 
 int launch_pair_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, GemmArgs g, int splits,
                       cudaStream_t stream) {
-  const size_t stage = kBM * 128 + static_cast<size_t>(g.subs) * (g.BN / 2) * 128;
+  constexpr size_t stage = kBM * 128 + kSubs * (kSubCols / 2) * 128;
   g.tiles_m = (g.M + 2 * kBM - 1) / (2 * kBM);
-  g.tiles_n = (g.N + g.BN * g.subs - 1) / (g.BN * g.subs);
+  g.tiles_n = (g.N + kSubs * kSubCols - 1) / (kSubs * kSubCols);
   g.items = g.tiles_m * g.tiles_n * splits;
   const size_t limit = 225 * 1024;
   const size_t staging = g.items <= 74 ? 0 : kEpiWarps * 8192;  // one item a pair: the epilogue uses the ring (64 KB or more)
-  g.stages = static_cast<int>((limit - 1024 - staging) / stage);
-  if (g.stages > kMaxStages) g.stages = kMaxStages;
+  g.stages = static_cast<int>((limit - 1024 - staging) / stage);  // 4, or 3
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(gemm_pair_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

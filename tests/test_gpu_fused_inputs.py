@@ -94,3 +94,30 @@ def test_a_frozen_table_keeps_its_rows(freeze):
     fused, general = (train(wide_deep, 8, kk.SGD(), g, freeze=freeze) for g in (False, True))
     for a, b in zip(fused[:3], general[:3]):
         same(a, b)
+
+
+def test_more_ids_than_are_read_in_place():
+    """Above half a million ids the rows of both tables are gathered first."""
+    n, space = (1 << 19) // FIELDS + 2, 20_000
+    assert n * FIELDS > 1 << 19
+    g = torch.Generator().manual_seed(1)
+    dense, ids = torch.randn(n, 3, generator=g).to(DEV), torch.randint(0, space, (n, FIELDS), generator=g).to(DEV)
+    results = []
+    for general in (False, True):
+        kk.initialize("gpu", table_capacity=1 << 16, max_ids_per_call=n * FIELDS, seed=5)
+        torch.manual_seed(2)
+        model = wide_deep(8).to(DEV)
+        opt = kk.Optimizer("m", model.named_parameters(), 0.05, kk.SGD())
+        if general:
+            model.mlp.register_forward_pre_hook(lambda m, i: None)
+        out = model(dense, ids)
+        (out * torch.linspace(-1, 1, n, device=DEV)).sum().backward()
+        opt.step()
+        eng = kk.native.engine()
+        eng.check()
+        every = torch.arange(space, device=DEV)
+        rows = [eng.sparse[t.table_id()].lookup(every)[0].clone() for t in (model.wide.sparse_table, model.deep.sparse_table)]
+        results.append((out.detach().clone(), *rows, *[p.detach().clone() for p in model.mlp.parameters()]))
+        kk.stop()
+    assert torch.allclose(results[0][0], results[1][0], rtol=1e-4, atol=1e-5)
+    same(results[0][1:], results[1][1:])

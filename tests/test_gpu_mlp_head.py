@@ -15,7 +15,7 @@ def close(got, want, terms):
     assert bool(((got.double() - value).abs() <= 2 ** -23 * (terms ** 0.5 + 4) * magnitude + 1e-30).all())
 
 
-# Rows around a warp's four, columns around a lane's eight and a warp's 256 of them.
+# Rows around a block's eight warps, a row each; columns around the 64 that a warp takes at a time.
 @pytest.mark.parametrize("M", [1, 3, 4, 5, 33, 1000])
 @pytest.mark.parametrize("K", [8, 248, 256, 264, 400])
 def test_single_output_forward(M, K):

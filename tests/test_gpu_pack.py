@@ -84,3 +84,44 @@ def test_backward(B, F, D, folded, fm, with_dx, slots):
     close(grad2[:, D: D + 1] if folded else grad1, at if folded else inv1.long().view(-1), first, first.abs())
     if folded:
         assert bool((grad2[:, D + 1:] == 0).all())
+
+
+# What Wide&Deep (fm False) and two-table DeepFM take with more ids than are read in place: gathered rows of two tables; and
+# rows that lie further apart than they are wide, the first-order ones as well.
+@pytest.mark.parametrize("B,F,D", [(33, 33, 4), (40, 26, 16), (9, 29, 16), (7, 31, 32), (19, 33, 64), (3, 65, 128)])
+@pytest.mark.parametrize("fm", [False, True])
+@pytest.mark.parametrize("slots,pitch", [(False, 0), (False, 8), (True, 12)])
+def test_two_tables(B, F, D, fm, slots, pitch):
+    inv, inv1, rows, first, slots2, slots1, e, w = problem(B, F, D, False, slots)
+    if pitch:
+        wide, narrow = torch.full((U, D + pitch), float("nan"), device=DEV), torch.full((U, pitch), float("nan"), device=DEV)
+        wide[:, :D], narrow[:, :1] = rows, first
+        rows, first = wide[:, :D], narrow[:, :1]
+    ldx = (F * D + 13 + 7) // 8 * 8
+    dense = torch.randn(B, 13, device=DEV)
+    x = torch.full((B, ldx), 7.0, device=DEV, dtype=torch.bfloat16)
+    logit, ssum = torch.empty(B, device=DEV), torch.empty(B, D, device=DEV)
+    C.deepfm_pack_forward(rows, inv, first, inv1, dense, B, F, D, x, logit, slots2, slots1, ssum if fm else None, fm)
+    want = torch.zeros(B, ldx, device=DEV, dtype=torch.float64)
+    want[:, : F * D], want[:, F * D: F * D + 13] = e.view(B, F * D), dense.double()
+    assert torch.equal(x, want.float().to(torch.bfloat16))
+    value, size = w.sum(1), w.abs().sum(1)
+    if fm:
+        s, q, sabs = e.sum(1), (e * e).sum(1), e.abs().sum(1)
+        value, size = value + 0.5 * (s * s - q).sum(1), size + (sabs * sabs).sum(1) + q.sum(1)
+    assert bool(((logit.double() - value).abs() <= (F + D + 8) * 2 ** -24 * size).all())   # as above
+
+    dx, dlogit = torch.randn(B, F * D + 4, device=DEV).to(torch.bfloat16), torch.randn(B, device=DEV)
+    grad2, grad1 = torch.zeros(U, D, device=DEV), torch.zeros(U, 1, device=DEV)
+    C.deepfm_pack_backward(rows, inv, inv1, dx, dlogit, B, F, D, grad2, grad1, slots2, ssum if fm else None)
+    terms = dx[:, : F * D].double().view(B, F, D)
+    size = terms.abs()
+    if fm:
+        g, s = dlogit.double().view(B, 1, 1), ssum.double().unsqueeze(1)
+        terms, size = terms + g * (s - e), size + 2 * g.abs() * (s.abs() + e.abs())
+    once = dlogit.double().view(B, 1, 1).expand(B, F, 1)
+    for got, at, terms, size in ((grad2, inv, terms, size), (grad1, inv1, once, once.abs())):
+        at, zeros = at.long().view(-1), torch.zeros(U, terms.size(2), device=DEV, dtype=torch.float64)
+        counts = torch.bincount(at, minlength=U).double().unsqueeze(1)
+        bound = 2 ** -23 * (2 * counts.sqrt() + 4) * zeros.index_add(0, at, size.reshape(B * F, -1))   # as above
+        assert bool(((got.double() - zeros.index_add(0, at, terms.reshape(B * F, -1))).abs() <= bound).all())

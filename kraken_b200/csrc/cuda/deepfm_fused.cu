@@ -27,7 +27,10 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kForwardBlocks = 4;   // a multiprocessor: 64 registers a thread
-constexpr int kBatch = 7;           // row loads of a lane in flight in the forward pass: as many as those registers hold
+// Row loads of a lane in flight in the forward pass.  With FM the 64 registers hold them for rows of 4, 8, 16 and 128 floats;
+// for 32 and 64 they spill 40 and 56 bytes.  Six there spill nothing and are better for 39 fields of 32 floats (32768 samples:
+// 39.4 us for 44.1), worse for 26 (29.9 for 28.9), the same within 5 % for 64 floats.
+constexpr int kBatch = 7;
 constexpr int kBackwardBlocks = 5;
 
 // Row index of unique entry `u`: the entry itself when the rows were gathered into a receive
@@ -40,7 +43,7 @@ __device__ __forceinline__ size_t row_of(const int* __restrict__ slots, int u) {
   return static_cast<size_t>(s < 0 ? 0 : s);
 }
 
-// Field groups per sample: as many as keep (D / 4) x G lanes within a quarter warp.
+// Field groups per sample: as many as keep (D / 4) x G lanes within half a warp; rows of 128 floats take a whole one.
 constexpr int field_groups(int chunks) {
   int g = 1;
   while (chunks * g * 2 <= 16) g <<= 1;

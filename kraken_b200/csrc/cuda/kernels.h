@@ -295,7 +295,6 @@ void cast_weights(CastBatch b, cudaStream_t stream);
 // y[m] = x[m, :] . w + bias[0] + addend[m]   (bias and addend optional).
 void rowdot_forward(const __nv_bfloat16* x, int ldx, const float* w, const float* bias, const float* addend, int M,
                     int K, float* y, cudaStream_t stream);
-// Its backward: dx (optional, bf16, optionally masked by x > 0), dw[K] += ..., db[0] += sum(dy).
 // Linear layer with up to kMaxHead outputs on bf16 activations, everything else fp32: y [M, classes] = x w^T + bias, and its
 // backward (dw and db are added to, dx may be null).  head_supported: whether the kernels take these operands.
 constexpr int kMaxHead = 16;
@@ -307,6 +306,7 @@ size_t head_part_floats(int M, int K, int classes);
 void head_backward(const __nv_bfloat16* x, int ldx, const float* w, const float* g, int M, int K, int classes,
                    bool relu_mask, __nv_bfloat16* dx, int lddx, float* dw, float* db, float* part, cudaStream_t stream);
 
+// Backward of rowdot_forward: dx (optional, bf16, optionally masked by x > 0), dw[K] += ..., db[0] += sum(dy).
 void rowdot_backward(const __nv_bfloat16* x, int ldx, const float* w, const float* dy, int M, int K, bool relu_mask,
                      __nv_bfloat16* dx, int lddx, float* dw, float* db, cudaStream_t stream);
 

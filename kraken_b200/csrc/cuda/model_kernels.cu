@@ -244,7 +244,7 @@ constexpr int kHeadThreads = 128;
 constexpr int kHeadStep = 64;   // rows of g in shared memory
 constexpr int kHeadRange = 32;  // rows of a range at least
 
-// Blocks of a multiprocessor: as many as 61, 94, 126 and 162 registers a thread leave room for.
+// Blocks of a multiprocessor: as many as 59, 92, 126 and 161 registers a thread leave room for.
 constexpr int head_blocks(int classes) { return classes <= 4 ? 8 : classes <= 8 ? 5 : classes <= 12 ? 4 : 3; }
 
 template <int C>

@@ -71,13 +71,13 @@ struct DirectSource {
 //
 // Bound by HBM: per row it must read the gradient, read and write value and state rows and write the zeros.  The
 // two-kernel form (push_dispatch into the inbox, push_update out of it) wrote and read every gradient row once more.
-// Measured for 0.55 M rows of 20 floats with Adam: 245 us before, 194 us so, 115 us since a row's state lies beside its
+// Measured for 0.55 M rows of 20 floats with Adam: 245 us before, 194 us so, 99 us since a row's state lies beside its
 // value.  A row is handled by `chunks` neighbouring
 // threads of a block, one 16-byte chunk each (a row width like 20 floats leaves no lane idle, as a power-of-two group
 // per row would); the threads of a row may sit in two warps, so its step counter is read by all of them before the
 // block barrier and written behind it.  What is known of the next row is fetched one pass ahead.  Nine blocks of 128
-// threads per SM leave 56 registers a thread, which holds every variant but Adam of 4-float chunks with direct gradients
-// (4 bytes spilled with rows, 12 with bags); eight of them were 3 to 6 % slower, four or five blocks of 256 threads up to
+// threads per SM leave 56 registers a thread, which holds every variant but those of 4-float chunks with direct gradients for
+// Adam (4 bytes spilled with rows, 20 with bags, 16 with bf16 ones) and RMSprop (4 with bags); eight of them were 3 to 6 % slower, four or five blocks of 256 threads up to
 // 25 %.
 //
 // FROM: with kFromRows and kFromBags the gradient of every id's first occurrence is read from the caller's gradients

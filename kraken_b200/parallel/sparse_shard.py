@@ -38,7 +38,7 @@ def record_pitch(dim: int, used: int, counts: bool) -> int:
     """Floats from one slot of a table to the next.  A slot's value, its optimizer state (``used`` floats together) and,
     where the padding has room, its step counter (``counts``) lie side by side: an update, which reads and writes all of
     them at a random place, touches one run of sectors instead of one per slab: 0.55 M rows of 20 floats with Adam 203 us
-    in slabs, 115 us so; 3.2 M of one float with Adagrad 136 and 85; rows of 64 floats, whole sectors either way, 499 both
+    in slabs, 99 us so; 3.2 M of one float with Adagrad 136 and 85; rows of 64 floats, whole sectors either way, 499 both
     times.  Records end on a 32-byte sector where that costs at most a quarter of their size (small ones on a power of two);
     rows without state stay back to back."""
     if used == dim and not counts:
